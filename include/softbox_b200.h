@@ -891,8 +891,8 @@ sbx_status sbx_obs_stress(sbx_ctx* ctx, int32_t nNet, int32_t nSeg, const float*
                           const float* bondData, double headLen, const float* volume, double* out);
 /* Largest cluster: components over ACTIVE segments and backbones joined by chain links,
  * ACTIVE crosslinks and bound heads (segment -- its head's backbone, motorBackbone[m]).
- * `rounds` hook-and-compress rounds (each skipped once the previous one changed nothing);
- * flags[rounds] scratch, flags[rounds-1] != 0 afterwards means not converged. label
+ * One pass joins the edges' components completely; `rounds` is the length of flags less one
+ * (rounds + 1 words), and flags[rounds-1] != 0 afterwards means not converged. label
  * receives each node's component id (its smallest node id; -1 for FREE segments), size the
  * component sizes in segments; out[2k] = largest component (segments), out[2k+1] = ACTIVE
  * segments of network k. */
