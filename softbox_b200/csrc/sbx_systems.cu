@@ -879,44 +879,90 @@ extern "C" sbx_status sbx_grid_build(sbx_ctx* ctx, int32_t cap, const int32_t* b
     return counting_sort(ctx, cs, "sbx_grid_build");
 }
 
-__global__ void k_broad_phase(int cap, const float* center, const float* R, const int* bodyCell, const int* offsets,
-                              const int* contents, const int* gd, const float* gp, const int* counts, int* candPartner,
-                              int* candCount) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cap) return;
-    candCount[i] = 0;
-    int S = counts[1];
-    if (i >= S) return;
-    int c = bodyCell[i];
-    if (c < 0) return;
-    int nX = gd[0], nY = gd[1], nZ = gd[2], nXY = nX * nY;
-    float cutoff = gp[5];
-    int cz = c / nXY, rem = c - cz * nXY, cy = rem / nX, cx = rem - cy * nX;
-    float icx = center[i], icy = center[cap + i], icz = center[2 * cap + i], ri = R[i];
-    int x0 = max(cx - 1, 0), x1 = min(cx + 1, nX - 1);
-    int y0 = max(cy - 1, 0), y1 = min(cy + 1, nY - 1);
-    int z0 = max(cz - 1, 0), z1 = min(cz + 1, nZ - 1);
+// SpatialGrid.broadPhase (SpatialGrid.java:340-445). A body has BROAD_W lanes, which take the
+// entries of its nine stencil rows (three consecutive x-cells each: one contiguous range of
+// entries) BROAD_W at a time and append the passing ones in entry order, by ballot and the
+// popcount of the lower lanes' passes: the serial walk's list.
+// What bounds it is the latency of entry -> centre over some 35 entries a body, half of which
+// fail j > i. One thread a body, one entry at a time, took 75 us for 132,000 bodies at the
+// benchmark's density; this takes 35 us.
+constexpr int BROAD_W = 8;
+
+__global__ void __launch_bounds__(256) k_broad_phase(int cap, const float* center, const float* R, const int* bodyCell,
+                                                     const int* offsets, const int* contents, const int* gd,
+                                                     const float* gp, const int* counts, int* candPartner,
+                                                     int* candCount) {
+    constexpr int W = BROAD_W;
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(g / W), hl = (int)(threadIdx.x & (W - 1)), grp = (threadIdx.x & 31) / W;
+    const int c = (i < cap && i < counts[1]) ? bodyCell[i] : -1;
+    const bool valid = c >= 0;
+    const int nX = gd[0], nY = gd[1], nZ = gd[2], nXY = nX * nY;
+    float icx = 0.f, icy = 0.f, icz = 0.f, ri = 0.f;
+    if (valid) { icx = center[i]; icy = center[cap + i]; icz = center[2 * cap + i]; ri = R[i]; }
+    const float cutoff = gp[5];
+    // lane r reads stencil row r, lane 0 also row 8
+    int rs = 0, len = 0, rs8 = 0, len8 = 0;
+    const int cz = c / nXY, rem = c - cz * nXY, cy = rem / nX, cx = rem - cy * nX;
+    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, nX - 1);
+    auto row = [&](int r, int& s, int& l) {
+        const int zz = cz - 1 + r / 3, yy = cy - 1 + r % 3;
+        if (zz >= 0 && zz < nZ && yy >= 0 && yy < nY) {
+            const int c0 = x0 + yy * nX + zz * nXY;
+            s = offsets[c0];
+            l = offsets[c0 + (x1 - x0) + 1] - s;
+        }
+    };
+    if (valid) {
+        row(hl, rs, len);
+        if (hl == 0) row(8, rs8, len8);
+    }
+    int inc = len;
+#pragma unroll
+    for (int o = 1; o < W; o <<= 1) {
+        int y = __shfl_up_sync(0xffffffffu, inc, o, W);
+        if (hl >= o) inc += y;
+    }
+    const int rows8 = __shfl_sync(0xffffffffu, inc, W - 1, W);
+    const int total = rows8 + __shfl_sync(0xffffffffu, len8, 0, W);
+    int totalMax = total;
+#pragma unroll
+    for (int o = W; o < 32; o <<= 1) totalMax = max(totalMax, __shfl_xor_sync(0xffffffffu, totalMax, o));
+    int pre[9], at[9];
+#pragma unroll
+    for (int r = 0; r < 8; r++) {
+        pre[r] = __shfl_sync(0xffffffffu, inc - len, r, W);
+        at[r] = __shfl_sync(0xffffffffu, rs, r, W);
+    }
+    pre[8] = rows8;
+    at[8] = __shfl_sync(0xffffffffu, rs8, 0, W);
+    const unsigned lower = (1u << hl) - 1u;
     int cnt = 0;
-    for (int zz = z0; zz <= z1; zz++)
-        for (int yy = y0; yy <= y1; yy++)
-            for (int xx = x0; xx <= x1; xx++) {
-                int cc = xx + yy * nX + zz * nXY;
-                int start = offsets[cc], end = offsets[cc + 1];
-                for (int idx = start; idx < end; idx++) {
-                    int j = contents[idx];
-                    if (j <= i) continue;
-                    float dx = icx - center[j];
-                    float dy = icy - center[cap + j];
-                    float dz = icz - center[2 * cap + j];
-                    float distSq = dx * dx + dy * dy + dz * dz;
-                    float reach = ri + R[j] + cutoff;
-                    if (distSq <= reach * reach) {
-                        if (cnt < MAX_CAND) candPartner[(int64_t)i * MAX_CAND + cnt] = j;
-                        cnt++;
-                    }
-                }
+    for (int k0 = 0; k0 < totalMax; k0 += W) {
+        const int k = k0 + hl;
+        bool pass = false;
+        int j = 0;
+        if (k < total) {
+            int idx = at[0] + k;
+#pragma unroll
+            for (int r = 1; r < 9; r++)
+                if (k >= pre[r]) idx = at[r] + (k - pre[r]);
+            j = contents[idx];
+            if (j > i) {
+                float dx = icx - center[j];
+                float dy = icy - center[cap + j];
+                float dz = icz - center[2 * cap + j];
+                float distSq = dx * dx + dy * dy + dz * dz;
+                float reach = ri + R[j] + cutoff;
+                pass = distSq <= reach * reach;
             }
-    candCount[i] = cnt;
+        }
+        const unsigned mask = (__ballot_sync(0xffffffffu, pass) >> (W * grp)) & ((1u << W) - 1u);
+        const int pos = cnt + __popc(mask & lower);
+        if (pass && pos < MAX_CAND) candPartner[(int64_t)i * MAX_CAND + pos] = j;
+        cnt += __popc(mask);
+    }
+    if (hl == 0 && i < cap) candCount[i] = cnt;
 }
 
 extern "C" sbx_status sbx_grid_broad_phase(sbx_ctx* ctx, int32_t cap, const float* center, const float* R,
@@ -926,8 +972,8 @@ extern "C" sbx_status sbx_grid_broad_phase(sbx_ctx* ctx, int32_t cap, const floa
     SBX_REQUIRE(ctx && cap >= 0 && (cap == 0 || (center && R && bodyCell && offsets && contents && gd && gp && counts &&
                                                  candPartner && candCount)));
     if (cap == 0) return SBX_OK;
-    SBX_LAUNCH(ctx, k_broad_phase, blocks(cap, 128), 128, cap, center, R, bodyCell, offsets, contents, gd, gp, counts,
-               candPartner, candCount);
+    SBX_LAUNCH(ctx, k_broad_phase, blocks((int64_t)cap * BROAD_W), 256, cap, center, R, bodyCell, offsets, contents, gd,
+               gp, counts, candPartner, candCount);
     return check_launch(ctx, "sbx_grid_broad_phase");
 }
 
