@@ -12,7 +12,7 @@ torch = pytest.importorskip("torch")
 
 
 @pytest.mark.parametrize("cap,S,box,dims", [(1, 1, 1.0, (3, 3, 3)), (37, 33, 1.0, (4, 3, 2)), (1003, 1003, 2.0, (9, 8, 1)),
-                                            (1500, 1400, 0.6, (2, 2, 2)), (700, 700, 0.4, (1, 1, 1)),
+                                            (1500, 1400, 0.6, (2, 2, 2)), (700, 700, 0.3, (1, 1, 1)),
                                             (2051, 2049, 3.0, (1, 13, 12))])
 def test_broad_phase_bitwise(orc_dm, cap, S, box, dims):
     from softbox_b200.systems import SpatialGrid
