@@ -16,49 +16,198 @@ using namespace sbx;
 
 namespace {
 
+// One rod's per-step inputs that do not depend on its pose: the six Gaussians of step t0 + s.
 template <int MODE>   // 0 wang, 1 philox, 2 supplied
-__global__ void __launch_bounds__(128) k_free_rods(int n, float* coord, double* coord64, float* uVec, float* yVec,
-                                                   float* zVec, float* end1, float* end2, const float* segLength,
-                                                   const float* F, const float* T, float* rF, float* rT,
-                                                   const float* bTG, const float* bRG, const float* tSc,
-                                                   const float* rSc, const float* params, int* counts, int t0,
-                                                   int nsteps, uint64_t seed64, const float* noise) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+__device__ __forceinline__ void rod_gaussians(int n, int i, int t0, int s, int seed, uint64_t seed64,
+                                              const float* noise, float g[6]) {
+    if (MODE == 0) gauss6_wang(i, t0 + s, seed, g);
+    else if (MODE == 1) gauss6_philox(i, t0 + s, seed64, g);
+    else for (int k = 0; k < 6; k++) g[k] = noise[((int64_t)s * 6 + k) * n + i];
+}
+
+// A rod in registers: loaded once, stepped, stored once.
+struct RodState {
     Pose p;
-    float f[3], t[3], gT[3], gR[3], rf[3] = {0, 0, 0}, rt[3] = {0, 0, 0};
+    float f[3], t[3], gT[3], gR[3], rf[3], rt[3], z[3];
     double c64[3];
+    float tS, rS, mag, dt, L;
+};
+
+struct FreeArgs {
+    int n;
+    float* coord; double* coord64; float *uVec, *yVec, *zVec, *end1, *end2;
+    const float *segLength, *F, *T;
+    float *rF, *rT;
+    const float *bTG, *bRG, *tSc, *rSc, *params;
+    int* counts;
+    int t0, nsteps;
+    uint64_t seed64;
+    const float* noise;
+};
+
+__device__ __forceinline__ void rod_load(const FreeArgs& a, int i, RodState& r) {
+    const int n = a.n;
     for (int k = 0; k < 3; k++) {
-        p.c[k] = coord[k * n + i]; p.u[k] = uVec[k * n + i]; p.y[k] = yVec[k * n + i];
-        f[k] = F[k * n + i]; t[k] = T[k * n + i];
-        gT[k] = bTG[k * n + i]; gR[k] = bRG[k * n + i];
-        if (coord64) c64[k] = coord64[k * n + i];
+        r.p.c[k] = a.coord[k * n + i]; r.p.u[k] = a.uVec[k * n + i]; r.p.y[k] = a.yVec[k * n + i];
+        r.f[k] = a.F[k * n + i]; r.t[k] = a.T[k * n + i];
+        r.gT[k] = a.bTG[k * n + i]; r.gR[k] = a.bRG[k * n + i];
+        if (a.coord64) r.c64[k] = a.coord64[k * n + i];
+        r.rf[k] = r.rt[k] = r.z[k] = 0.f;
     }
-    float tS = tSc[i], rS = rSc[i], mag = params[1], dt = params[0], L = segLength[i];
-    int seed = counts[2];
-    float z[3] = {0, 0, 0}, e1[3] = {0, 0, 0}, e2[3] = {0, 0, 0};
-    for (int s = 0; s < nsteps; s++) {
-        int step = t0 + s;
+    r.tS = a.tSc[i]; r.rS = a.rSc[i]; r.mag = a.params[1]; r.dt = a.params[0]; r.L = a.segLength[i];
+}
+
+// the Langevin update and derived geometry of one step with the step's forces in rf / rt
+__device__ __forceinline__ void rod_step(RodState& r, bool fp64) {
+    Pose q;
+    float dc[3];
+    integrate_pose(r.p, r.f, r.t, r.rf, r.rt, r.gT, r.gR, r.dt, q, dc);
+    if (fp64)
+        for (int k = 0; k < 3; k++) { r.c64[k] = r.c64[k] + (double)dc[k]; q.c[k] = (float)r.c64[k]; }
+    float e1[3], e2[3];                   // (the stored ones follow from the last pose: rod_store)
+    derive_pose(q.c, q.u, q.y, r.z, e1, e2, r.L);
+    r.p = q;
+}
+
+// rod_step with the step's body velocities in rf / rt
+__device__ __forceinline__ void rod_step_vel(RodState& r, bool fp64) {
+    Pose q;
+    float dc[3], z[3];
+    pose_normal(r.p, z);
+    advance_pose(r.p, z, r.rf, r.rt, r.dt, q, dc);
+    if (fp64)
+        for (int k = 0; k < 3; k++) { r.c64[k] = r.c64[k] + (double)dc[k]; q.c[k] = (float)r.c64[k]; }
+    float e1[3], e2[3];
+    derive_pose(q.c, q.u, q.y, r.z, e1, e2, r.L);
+    r.p = q;
+}
+
+__device__ __forceinline__ void rod_store(const FreeArgs& a, int i, const RodState& r) {
+    const int n = a.n;
+    const float half = r.L * 0.5f;        // derive_pose's ends: c -/+ (L/2) u
+    for (int k = 0; k < 3; k++) {
+        a.coord[k * n + i] = r.p.c[k]; a.uVec[k * n + i] = r.p.u[k]; a.yVec[k * n + i] = r.p.y[k];
+        a.zVec[k * n + i] = r.z[k];
+        a.end1[k * n + i] = r.p.c[k] - half * r.p.u[k]; a.end2[k * n + i] = r.p.c[k] + half * r.p.u[k];
+        if (a.coord64) a.coord64[k * n + i] = r.c64[k];
+    }
+    if (i == 0) a.counts[1] = a.t0 + a.nsteps - 1;
+}
+
+// one thread a rod: each step's draw, then its update
+template <int MODE>
+__global__ void __launch_bounds__(128) k_free_rods(const FreeArgs a) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= a.n) return;
+    RodState r;
+    rod_load(a, i, r);
+    const int seed = a.counts[2];
+    for (int s = 0; s < a.nsteps; s++) {
         float g[6];
-        if (MODE == 0) gauss6_wang(i, step, seed, g);
-        else if (MODE == 1) gauss6_philox(i, step, seed64, g);
-        else for (int k = 0; k < 6; k++) g[k] = noise[((int64_t)s * 6 + k) * n + i];
-        brownian_amplitudes(g, tS, rS, mag, gT, gR, rf, rt);
-        Pose q;
-        float dc[3];
-        integrate_pose(p, f, t, rf, rt, gT, gR, dt, q, dc);
-        if (coord64)
-            for (int k = 0; k < 3; k++) { c64[k] = c64[k] + (double)dc[k]; q.c[k] = (float)c64[k]; }
-        derive_pose(q.c, q.u, q.y, z, e1, e2, L);
-        p = q;
+        rod_gaussians<MODE>(a.n, i, a.t0, s, seed, a.seed64, a.noise, g);
+        brownian_amplitudes(g, r.tS, r.rS, r.mag, r.gT, r.gR, r.rf, r.rt);
+        rod_step(r, a.coord64 != nullptr);
     }
-    for (int k = 0; k < 3; k++) {
-        coord[k * n + i] = p.c[k]; uVec[k * n + i] = p.u[k]; yVec[k * n + i] = p.y[k];
-        zVec[k * n + i] = z[k]; end1[k * n + i] = e1[k]; end2[k * n + i] = e2[k];
-        rF[k * n + i] = rf[k]; rT[k * n + i] = rt[k];
-        if (coord64) coord64[k * n + i] = c64[k];
+    rod_store(a, i, r);
+    for (int k = 0; k < 3; k++) { a.rF[k * a.n + i] = r.rf[k]; a.rT[k * a.n + i] = r.rt[k]; }
+}
+
+// A block of RODS rods: warp 0 steps them, one rod a lane, while the other warps draw the forces
+// of the next chunk of steps into shared memory. The draws are keyed by (rod, step) and do not
+// depend on the pose, so only the update (three square roots and divisions in a row) is left
+// on a rod's serial chain; the draw (three Box-Muller pairs in FP64, most of a step's work)
+// spreads over the block. For a rod without external force and torque the drawing threads
+// also make its body velocities (six more divisions off the chain): with F = T = 0 the body
+// forces are sums of zeros and the draw, so they equal the draw wherever it is not zero.
+// 1,024 rods take 0.43 us a step, one thread a rod 1.67 us.
+template <int RODS>
+struct PipeShape {
+    static constexpr int STEPS = 256 / RODS;                 // steps of a chunk: 256 draws
+    static constexpr int THREADS = 32 + 256;                 // the stepping warp, one thread a draw
+};
+
+__device__ __forceinline__ bool all_zero(const float f[3], const float t[3]) {
+    return f[0] == 0.f && f[1] == 0.f && f[2] == 0.f && t[0] == 0.f && t[1] == 0.f && t[2] == 0.f;
+}
+
+template <int MODE, int RODS>
+__global__ void __launch_bounds__(PipeShape<RODS>::THREADS) k_free_pipe(const FreeArgs a) {
+    constexpr int STEPS = PipeShape<RODS>::STEPS;
+    __shared__ float buf[2][STEPS][6][RODS];
+    __shared__ unsigned char vel[2][STEPS][RODS];            // buf holds body velocities, not forces
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = blockIdx.x * RODS;
+    const int seed = a.counts[2];
+    const int chunks = (a.nsteps + STEPS - 1) / STEPS;
+    const bool steps = warp == 0 && lane < RODS && first + lane < a.n;
+    RodState r;
+    if (steps) rod_load(a, first + lane, r);
+    // the drawing threads: rod (threadIdx - 32) % RODS, step (threadIdx - 32) / RODS of a chunk
+    const int d = (int)threadIdx.x - 32, dr = d & (RODS - 1), ds = d / RODS;
+    const int di = first + dr;
+    const bool draws = warp > 0 && di < a.n;
+    float gT[3], gR[3], tS = 0.f, rS = 0.f, mag = 0.f;
+    bool loose = false;                                      // the rod has no external force or torque
+    if (draws) {
+        float f[3], t[3];
+        for (int k = 0; k < 3; k++) {
+            gT[k] = a.bTG[k * a.n + di]; gR[k] = a.bRG[k * a.n + di];
+            f[k] = a.F[k * a.n + di]; t[k] = a.T[k * a.n + di];
+        }
+        tS = a.tSc[di]; rS = a.rSc[di]; mag = a.params[1];
+        loose = all_zero(f, t);
     }
-    if (i == 0) counts[1] = t0 + nsteps - 1;
+    for (int c = 0; c <= chunks; c++) {
+        if (draws && c < chunks) {
+            const int s = c * STEPS + ds;
+            if (s < a.nsteps) {
+                float g[6], rf[3], rt[3];
+                rod_gaussians<MODE>(a.n, di, a.t0, s, seed, a.seed64, a.noise, g);
+                brownian_amplitudes(g, tS, rS, mag, gT, gR, rf, rt);
+                if (s == a.nsteps - 1)
+                    for (int k = 0; k < 3; k++) { a.rF[k * a.n + di] = rf[k]; a.rT[k * a.n + di] = rt[k]; }
+                const bool v = loose && rf[0] != 0.f && rf[1] != 0.f && rf[2] != 0.f && rt[0] != 0.f &&
+                               rt[1] != 0.f && rt[2] != 0.f;
+                vel[c & 1][ds][dr] = v;
+                for (int k = 0; k < 3; k++) {
+                    buf[c & 1][ds][k][dr] = v ? 1.0e6f * rf[k] / gT[k] : rf[k];
+                    buf[c & 1][ds][3 + k][dr] = v ? rt[k] / gR[k] : rt[k];
+                }
+            }
+        }
+        if (steps && c > 0) {
+            const int left = a.nsteps - (c - 1) * STEPS, m = left < STEPS ? left : STEPS;
+            for (int s = 0; s < m; s++) {
+                for (int k = 0; k < 3; k++) { r.rf[k] = buf[(c - 1) & 1][s][k][lane]; r.rt[k] = buf[(c - 1) & 1][s][3 + k][lane]; }
+                if (vel[(c - 1) & 1][s][lane]) rod_step_vel(r, a.coord64 != nullptr);
+                else rod_step(r, a.coord64 != nullptr);
+            }
+        }
+        __syncthreads();
+    }
+    if (steps) rod_store(a, first + lane, r);                // (the last step's forces: stored by its draw)
+}
+
+// The pipeline while the rods leave the GPU idle: as few rods a block as give at most two
+// blocks an SM, 32 up to four blocks an SM. More rods fill the GPU one thread a rod, where the
+// pipeline's stepping warps are in the way. Measured before the velocities moved to the drawing
+// warps, us a step, pipeline / one thread a rod: 4,096 rods 0.67 (16 a block; 1.25 with 8)
+// / 1.71, 8,192 0.72 (32) / 1.71, 16,384 1.44 (32) / 1.73, 32,768 2.84 (32) / 2.02. A few
+// steps are not worth filling the pipeline.
+constexpr int PIPE_MIN_STEPS = 4;
+template <int MODE>
+void free_launch(sbx_ctx* ctx, const FreeArgs& a) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess) sms = 0;
+    const int64_t two = 2 * (int64_t)sms;
+    if (a.nsteps < PIPE_MIN_STEPS || a.n > 2 * 32 * two)
+        SBX_LAUNCH(ctx, k_free_rods<MODE>, blocks(a.n, 128), 128, a);
+    else if (a.n <= 8 * two)
+        SBX_LAUNCH(ctx, (k_free_pipe<MODE, 8>), blocks(a.n, 8), PipeShape<8>::THREADS, a);
+    else if (a.n <= 16 * two)
+        SBX_LAUNCH(ctx, (k_free_pipe<MODE, 16>), blocks(a.n, 16), PipeShape<16>::THREADS, a);
+    else
+        SBX_LAUNCH(ctx, (k_free_pipe<MODE, 32>), blocks(a.n, 32), PipeShape<32>::THREADS, a);
 }
 
 }  // namespace
@@ -81,12 +230,11 @@ extern "C" sbx_status sbx_free_rods_run(sbx_ctx* ctx, sbx_filament_store* fil, i
         if (st) return st;
         if (bad) return fail(ctx, SBX_ENONFINITE, "sbx_free_rods_run: noise holds NaN/Inf");
     }
-#define FREE_ARGS n, b.coord, b.coord64, b.uVec, b.yVec, b.zVec, b.end1, b.end2, b.segLength, b.forceSum, b.torqueSum, \
-                  b.randForce, b.randTorque, b.bTransGam, b.bRotGam, b.brownTransScale, b.brownRotScale, fil->params, \
-                  fil->counts, t0, nsteps, philox_seed, noise
-    if (noise_mode == 0) SBX_LAUNCH(ctx, k_free_rods<0>, blocks(n, 128), 128, FREE_ARGS);
-    else if (noise_mode == 1) SBX_LAUNCH(ctx, k_free_rods<1>, blocks(n, 128), 128, FREE_ARGS);
-    else SBX_LAUNCH(ctx, k_free_rods<2>, blocks(n, 128), 128, FREE_ARGS);
-#undef FREE_ARGS
+    FreeArgs a{n, b.coord, b.coord64, b.uVec, b.yVec, b.zVec, b.end1, b.end2, b.segLength, b.forceSum, b.torqueSum,
+               b.randForce, b.randTorque, b.bTransGam, b.bRotGam, b.brownTransScale, b.brownRotScale, fil->params,
+               fil->counts, t0, nsteps, philox_seed, noise};
+    if (noise_mode == 0) free_launch<0>(ctx, a);
+    else if (noise_mode == 1) free_launch<1>(ctx, a);
+    else free_launch<2>(ctx, a);
     return check_launch(ctx, "sbx_free_rods_run");
 }

@@ -112,51 +112,57 @@ struct Pose {
 
 // RigidRodLangevinIntegrationSystem.java:53-110 (and MechanicsFusion.java:134-176).
 // Returns the new pose; `dc` receives the FP32 increments dt*v for FP64 accumulation.
-SBX_DEV void integrate_pose(const Pose& p, const float F[3], const float T[3], const float rF[3],
-                            const float rT[3], const float gT[3], const float gR[3], float dt, Pose& q,
-                            float dc[3]) {
+SBX_DEV void pose_normal(const Pose& p, float z[3]) {          // z = unit(u x y)
+    float zx = p.u[1] * p.y[2] - p.u[2] * p.y[1];
+    float zy = p.u[2] * p.y[0] - p.u[0] * p.y[2];
+    float zz = p.u[0] * p.y[1] - p.u[1] * p.y[0];
+    float zlen = 1.0f / fsqrt(zx * zx + zy * zy + zz * zz);
+    z[0] = zx * zlen; z[1] = zy * zlen; z[2] = zz * zlen;
+}
+
+// the second half: from the body-frame velocities bv (um/s) and bw (rad/s)
+SBX_DEV void advance_pose(const Pose& p, const float z[3], const float bv[3], const float bw[3], float dt, Pose& q,
+                          float dc[3]) {
     float ux = p.u[0], uyc = p.u[1], uzc = p.u[2];
     float yx = p.y[0], yyc = p.y[1], yzc = p.y[2];
-    float zx = uyc * yzc - uzc * yyc;
-    float zy = uzc * yx - ux * yzc;
-    float zz = ux * yyc - uyc * yx;
-    float zlen = 1.0f / fsqrt(zx * zx + zy * zy + zz * zz);
-    zx *= zlen; zy *= zlen; zz *= zlen;
-    float fx = F[0], fy = F[1], fz = F[2];
-    float tx = T[0], ty = T[1], tz = T[2];
-    float bfx = ux * fx + uyc * fy + uzc * fz + rF[0];
-    float bfy = yx * fx + yyc * fy + yzc * fz + rF[1];
-    float bfz = zx * fx + zy * fy + zz * fz + rF[2];
-    float btx = ux * tx + uyc * ty + uzc * tz + rT[0];
-    float bty = yx * tx + yyc * ty + yzc * tz + rT[1];
-    float btz = zx * tx + zy * ty + zz * tz + rT[2];
-    float bvx = 1.0e6f * bfx / gT[0];
-    float bvy = 1.0e6f * bfy / gT[1];
-    float bvz = 1.0e6f * bfz / gT[2];
-    float bwx = btx / gR[0];
-    float bwy = bty / gR[1];
-    float bwz = btz / gR[2];
-    float vx = ux * bvx + yx * bvy + zx * bvz;
-    float vy = uyc * bvx + yyc * bvy + zy * bvz;
-    float vz = uzc * bvx + yzc * bvy + zz * bvz;
+    float zx = z[0], zy = z[1], zz = z[2];
+    float vx = ux * bv[0] + yx * bv[1] + zx * bv[2];
+    float vy = uyc * bv[0] + yyc * bv[1] + zy * bv[2];
+    float vz = uzc * bv[0] + yzc * bv[1] + zz * bv[2];
     dc[0] = dt * vx; dc[1] = dt * vy; dc[2] = dt * vz;
     q.c[0] = p.c[0] + dc[0];
     q.c[1] = p.c[1] + dc[1];
     q.c[2] = p.c[2] + dc[2];
-    float uTransInZ = -bwy * dt;
-    float uTransInY = bwz * dt;
+    float uTransInZ = -bw[1] * dt;
+    float uTransInY = bw[2] * dt;
     float nuX = ux + yx * uTransInY + zx * uTransInZ;
     float nuY = uyc + yyc * uTransInY + zy * uTransInZ;
     float nuZ = uzc + yzc * uTransInY + zz * uTransInZ;
     float nuInv = 1.0f / fsqrt(nuX * nuX + nuY * nuY + nuZ * nuZ);
     q.u[0] = nuX * nuInv; q.u[1] = nuY * nuInv; q.u[2] = nuZ * nuInv;
     float yTransInX = -uTransInY;
-    float yTransInZ = bwx * dt;
+    float yTransInZ = bw[0] * dt;
     float nyX = ux * yTransInX + yx + zx * yTransInZ;
     float nyY = uyc * yTransInX + yyc + zy * yTransInZ;
     float nyZ = uzc * yTransInX + yzc + zz * yTransInZ;
     float nyInv = 1.0f / fsqrt(nyX * nyX + nyY * nyY + nyZ * nyZ);
     q.y[0] = nyX * nyInv; q.y[1] = nyY * nyInv; q.y[2] = nyZ * nyInv;
+}
+
+SBX_DEV void integrate_pose(const Pose& p, const float F[3], const float T[3], const float rF[3],
+                            const float rT[3], const float gT[3], const float gR[3], float dt, Pose& q,
+                            float dc[3]) {
+    float z[3], bv[3], bw[3];
+    pose_normal(p, z);
+    const float* axis[3] = {p.u, p.y, z};
+    for (int k = 0; k < 3; k++) {
+        const float* e = axis[k];
+        float bf = e[0] * F[0] + e[1] * F[1] + e[2] * F[2] + rF[k];
+        float bt = e[0] * T[0] + e[1] * T[1] + e[2] * T[2] + rT[k];
+        bv[k] = 1.0e6f * bf / gT[k];
+        bw[k] = bt / gR[k];
+    }
+    advance_pose(p, z, bv, bw, dt, q, dc);
 }
 
 // DerivedGeometrySystem.java:43-71: z = unit(u x y), y' = z x u, ends = c -/+ (L/2) u
