@@ -929,6 +929,26 @@ sbx_status sbx_mlp_mse_grad(sbx_ctx* ctx, int32_t nz, int32_t M, int32_t Np, int
 sbx_status sbx_mlp_adam(sbx_ctx* ctx, int32_t nz, int32_t N, int32_t K, float* w, const float* gw, float* m, float* v,
                         int64_t stride, float lr, float beta1, float beta2, float eps, int32_t stepNumber,
                         void* wBf16, void* wBf16T, int64_t strideB, int64_t strideBT);
+/* The ensemble's networks for the whole-network entry points: layer l maps Kp[l] columns to
+ * Np[l] (Kp[0] = 16: the nin inputs padded; Np of the last layer = 16: the nout outputs
+ * padded), every array holding the nz networks one after another. Wb: BF16 weights
+ * [nz][Np][Kp], b: biases [nz][Np]. */
+#define SBX_MLP_MAX_LAYERS 8
+typedef struct sbx_mlp_net {
+    int32_t nz, nLayers, nin, nout;
+    int32_t Kp[SBX_MLP_MAX_LAYERS], Np[SBX_MLP_MAX_LAYERS];
+    void* Wb[SBX_MLP_MAX_LAYERS];
+    float* b[SBX_MLP_MAX_LAYERS];
+} sbx_mlp_net;
+/* 1 if the whole-network kernels take this ensemble: at most 16 inputs and outputs, hidden
+ * widths multiples of 32 up to 256, at most SBX_MLP_MAX_LAYERS layers (training: at least 2) */
+int32_t sbx_mlp_net_fits(const sbx_mlp_net* net, int32_t train);
+/* Predictions for P points X [P][nin] (FP64, not normalised): out [2 + nz][P][nout] FP64 holds
+ * the ensemble mean, its population standard deviation and each network's outputs.
+ * Inputs are normalised as bf16(float((x - xMean) / xStd)), outputs as y * yStd + yMean. */
+sbx_status sbx_mlp_predict(sbx_ctx* ctx, const sbx_mlp_net* net, const double* X, int32_t P, const double* xMean,
+                           const double* xStd, const double* yMean, const double* yStd, double* out,
+                           int32_t* errFlag);
 /* A plan over a packed scene (graph and per-system paths; the fused kernel is for one
  * network). `batch` is copied; its arrays must stay alive. */
 sbx_status sbx_dense_plan_create_batched(sbx_ctx* ctx, const sbx_dense_scene* scene, const sbx_batch* batch,

@@ -105,3 +105,12 @@ class TurnoverBatchDesc(C.Structure):   # packed-network turnover tables (sbx_tu
 
 class DenseNoiseDesc(C.Structure):      # supplied Gaussians of the dense step (sbx_dense_noise)
     _fields_ = [("fil", f32p), ("mot", f32p), ("bb", f32p), ("t0", C.c_int32), ("nsteps", C.c_int32)]
+
+
+MLP_MAX_LAYERS = 8
+
+
+class MlpNet(C.Structure):              # an ensemble's networks (sbx_mlp_net)
+    _fields_ = [(k, C.c_int32) for k in ("nz", "nLayers", "nin", "nout")] + [
+        (k, C.c_int32 * MLP_MAX_LAYERS) for k in ("Kp", "Np")] + [
+        (k, C.c_void_p * MLP_MAX_LAYERS) for k in ("Wb", "b")]

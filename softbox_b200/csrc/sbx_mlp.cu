@@ -261,6 +261,227 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_gemm(GemmArgs g) {
     }
 }
 
+// ---------------------------------------------------------------- whole networks
+// The ensemble's networks as the whole-network kernels take them: layer l is Np[l] x Kp[l]
+// (inputs and outputs padded to 16), arrays hold nz networks one after another.
+constexpr int NET_MAX_LAYERS = 8;
+struct Net {
+    int nz, L, nin, nout;
+    int Kp[NET_MAX_LAYERS], Np[NET_MAX_LAYERS];
+    const __nv_bfloat16* Wb[NET_MAX_LAYERS];
+    const float* b[NET_MAX_LAYERS];
+};
+
+// one 128 x N x Kp product from the staged operands into tensor memory, issued by one thread;
+// the commit arrives on mbar
+__device__ __forceinline__ void issue_mma(unsigned tmem, unsigned aBase, unsigned bBase, int N, int Kp,
+                                          unsigned long long* mbar) {
+    const unsigned idesc = idesc_bf16(MT, N);
+    const unsigned sbo = (unsigned)(Kp >> 3) * 128u;
+    for (int kk = 0; kk < Kp / 16; kk++) {
+        unsigned long long ad = kmajor_desc(aBase + kk * 256u, 128u, sbo);
+        unsigned long long bd = kmajor_desc(bBase + kk * 256u, 128u, sbo);
+        unsigned acc = kk > 0 ? 1u : 0u;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+            "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+    }
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+        smem_u32(mbar)));
+}
+
+// bounded wait for phase `parity` of mbar; one verdict for the block
+__device__ __forceinline__ bool wait_mma(unsigned long long* mbar, unsigned parity) {
+    bool done_ok = false;
+    long long t0 = gtimer();
+    for (;;) {
+        unsigned done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(smem_u32(mbar)), "r"(parity));
+        if (done) { done_ok = true; break; }
+        if (gtimer() - t0 > WAIT_NS) break;
+    }
+    return __syncthreads_and(done_ok ? 1 : 0) != 0;
+}
+
+// 16 accumulator columns of this warp's 32 rows (TMEM lanes 32 * quarter ..)
+__device__ __forceinline__ void load_acc16(unsigned tmem, int quarter, int c0, float v[16]) {
+    unsigned r[16];
+    unsigned taddr = tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)c0;
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
+        "[%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
+}
+
+__device__ __forceinline__ void pack16(const float a[16], uint4& lo, uint4& hi) {
+    unsigned w[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        __nv_bfloat162 h = __floats2bfloat162_rn(a[2 * j], a[2 * j + 1]);
+        w[j] = *reinterpret_cast<unsigned*>(&h);
+    }
+    lo = make_uint4(w[0], w[1], w[2], w[3]);
+    hi = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
+// byte offset of element (r, c) of a staged operand with contraction length Kp
+__device__ __forceinline__ int core_at(int r, int c, int Kp) {
+    return ((r >> 3) * (Kp >> 3) + (c >> 3)) * 128 + (r & 7) * 16 + (c & 7) * 2;
+}
+
+// rows [0, rows) x [0, Kp) of a row-major BF16 matrix (16-byte aligned rows) into the
+// core-matrix layout by 16-byte async copies; rows past rowsValid are zero
+__device__ __forceinline__ void stage_rows(char* dst, const __nv_bfloat16* src, int ld, int rows, int rowsValid,
+                                           int Kp) {
+    const int kg = Kp >> 3;
+    for (int u = threadIdx.x; u < rows * kg; u += blockDim.x) {
+        const int r = u / kg, c = u - r * kg;
+        char* d = dst + ((r >> 3) * kg + c) * 128 + (r & 7) * 16;
+        if (r < rowsValid) {
+            const __nv_bfloat16* p = src + (long long)r * ld + c * 8;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(d)), "l"(p));
+        } else {
+            *reinterpret_cast<uint4*>(d) = make_uint4(0, 0, 0, 0);
+        }
+    }
+}
+
+// ---------------------------------------------------------------- prediction
+// Every layer of every network for 128 points a tile, in one launch: the activations of the
+// tile stay in shared memory between layers (BF16, as the GEMM path stores them), a whole
+// layer's weights sit beside them, and the next layer's are fetched while the epilogue runs.
+// What bounds it is the epilogue: GELU on 1,024 hidden values a point and network, some 30
+// instructions each, an order of magnitude above the MMAs' time. So one block of 16 warps an
+// SM does the epilogues back to back; the separate GEMMs moved each layer's activations
+// through memory and left normalisation, de-normalisation and the ensemble statistics to the
+// host. 100,000 points on 5 networks: 1.13 ms, and 1.63 ms in ten GEMMs before (17 ms a call with
+// the host's part, 2.4 ms now).
+// The inputs are normalised here ((x - mean) / std in FP64, then FP32, then BF16) and the
+// outputs de-normalised in FP64 (y * std + mean), operation for operation as the host does.
+struct PredictArgs {
+    Net net;
+    const double *X, *xMean, *xStd, *yMean, *yStd;
+    int P;
+    double* out;      // [2 + nz][P][nout]: mean, standard deviation, each network's outputs
+    int* err;
+};
+
+__global__ void __launch_bounds__(GEMM_THREADS, 1) k_predict(const __grid_constant__ PredictArgs g) {
+    extern __shared__ __align__(1024) char smem[];
+    char* sA = smem;                               // 128 x 256
+    char* sB = smem + MT * KMAX * 2;               // 256 x 256
+    __shared__ __align__(8) unsigned long long mbar;
+    __shared__ unsigned tmemSlot;
+    __shared__ float sBias[2][NT];
+    const Net& net = g.net;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quarter = warp & 3, cgroup = warp >> 2;
+    const int tiles = (g.P + MT - 1) / MT, z = blockIdx.y, L = net.L;
+    if (threadIdx.x == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)));
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmemSlot)),
+                     "r"(256));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    auto weights = [&](int l, int slot) {
+        stage_rows(sB, net.Wb[l] + (long long)z * net.Np[l] * net.Kp[l], net.Kp[l], net.Np[l], net.Np[l], net.Kp[l]);
+        if ((int)threadIdx.x < net.Np[l]) sBias[slot][threadIdx.x] = net.b[l][z * net.Np[l] + threadIdx.x];
+    };
+    bool ok = true;
+    unsigned phase = 0;                            // the barrier's phase, and the bias slot in use
+    if ((int)blockIdx.x < tiles) weights(0, 0);
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        const int m0 = tile * MT;
+        // the tile's inputs: 16 padded columns, thread (row, half)
+        if (threadIdx.x < 2 * MT) {
+            const int r = threadIdx.x >> 1, c0 = (threadIdx.x & 1) * 8, row = m0 + r;
+            unsigned short h[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                float x = 0.f;
+                if (row < g.P && c0 + j < net.nin)
+                    x = (float)((g.X[(long long)row * net.nin + c0 + j] - g.xMean[c0 + j]) / g.xStd[c0 + j]);
+                h[j] = __bfloat16_as_ushort(__float2bfloat16_rn(x));
+            }
+            *reinterpret_cast<uint4*>(sA + core_at(r, c0, 16)) =
+                make_uint4(h[0] | (unsigned)h[1] << 16, h[2] | (unsigned)h[3] << 16, h[4] | (unsigned)h[5] << 16,
+                           h[6] | (unsigned)h[7] << 16);
+        }
+        for (int l = 0; l < L && ok; l++) {
+            const int Np = net.Np[l], Kp = net.Kp[l];
+            const bool last = l == L - 1;
+            cp_async_wait_all();                           // this layer's weights
+            asm volatile("fence.proxy.async.shared::cta;");
+            asm volatile("tcgen05.fence::before_thread_sync;");
+            __syncthreads();
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const unsigned tmem = tmemSlot;
+            if (threadIdx.x == 0) issue_mma(tmem, smem_u32(sA), smem_u32(sB), Np, Kp, &mbar);
+            ok = wait_mma(&mbar, phase);
+            const float* bias = sBias[phase];
+            phase ^= 1u;
+            if (!ok && threadIdx.x == 0 && g.err) atomicOr(g.err, 1);
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            if (!ok) break;
+            // the product has read both operands: fetch the next weights, then the epilogue
+            if (!last) weights(l + 1, phase);
+            else if (tile + (int)gridDim.x < tiles) weights(0, phase);
+            const int r = quarter * 32 + lane, row = m0 + r;
+            for (int c0 = cgroup * 16; c0 < Np; c0 += COL_GROUPS * 16) {
+                float v[16];
+                load_acc16(tmem, quarter, c0, v);
+#pragma unroll
+                for (int j = 0; j < 16; j++) v[j] += bias[c0 + j];
+                if (!last) {
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] = gelu(v[j]);
+                    uint4 lo, hi;
+                    pack16(v, lo, hi);
+                    *reinterpret_cast<uint4*>(sA + core_at(r, c0, Np)) = lo;
+                    *reinterpret_cast<uint4*>(sA + core_at(r, c0 + 8, Np)) = hi;
+                } else if (row < g.P) {
+                    double* o = g.out + ((long long)(2 + z) * g.P + row) * net.nout;
+                    for (int j = 0; j < 16; j++)
+                        if (c0 + j < net.nout) o[c0 + j] = (double)v[j] * g.yStd[c0 + j] + g.yMean[c0 + j];
+                }
+            }
+        }
+    }
+    cp_async_wait_all();
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmemSlot), "r"(256));
+    }
+}
+
+// the ensemble's mean and (population) standard deviation of every output, networks in order
+__global__ void k_predict_stats(int nz, long long n, double* out) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double* y = out + 2 * n;
+    double s = y[i];
+    for (int z = 1; z < nz; z++) s += y[z * n + i];
+    const double mean = s / (double)nz;
+    double q = 0.0;
+    for (int z = 0; z < nz; z++) {
+        const double d = y[z * n + i] - mean;
+        q = z == 0 ? d * d : q + d * d;
+    }
+    out[i] = mean;
+    out[n + i] = sqrt(q / (double)nz);
+}
+
 // dZ = dA * GELU'(Z) (or dA when Z is NULL) -> BF16 row-major and transposed; M x N, per z
 __global__ void k_gelu_back(int M, int N, const float* dA, const float* Z, long long sMN, __nv_bfloat16* g,
                             __nv_bfloat16* gT, long long sG, long long sGT) {
@@ -409,4 +630,58 @@ extern "C" sbx_status sbx_mlp_adam(sbx_ctx* ctx, int32_t nz, int32_t N, int32_t 
     SBX_LAUNCH_SMEM(ctx, k_adam, grid, 256, 0, N, K, w, gw, m, v, stride, lr, beta1, beta2, eps, c1, c2,
                (__nv_bfloat16*)wBf16, (__nv_bfloat16*)wBf16T, strideB, strideBT);
     return check_launch(ctx, "sbx_mlp_adam");
+}
+
+// ---------------------------------------------------------------- whole networks
+// Which ensembles the whole-network kernels take: inputs and outputs within their 16 padded
+// columns, hidden widths whole tiles. Others keep the GEMM path.
+static bool net_fits(const sbx_mlp_net* n, bool train) {
+    if (!n || n->nz < 1 || n->nz > 65535 || n->nLayers < (train ? 2 : 1) || n->nLayers > NET_MAX_LAYERS || n->nin < 1 ||
+        n->nin > 16 || n->nout < 1 || n->nout > 16)
+        return false;
+    for (int l = 0; l < n->nLayers; l++) {
+        const int N = n->Np[l], K = n->Kp[l];
+        if (K != (l == 0 ? 16 : n->Np[l - 1])) return false;
+        if (l == n->nLayers - 1 ? N != 16 : (N < 32 || N > KMAX || N % 32)) return false;
+        if (!n->Wb[l] || !n->b[l] || ((uintptr_t)n->Wb[l] & 15)) return false;
+    }
+    return true;
+}
+
+static Net net_of(const sbx_mlp_net* n) {
+    Net o{};
+    o.nz = n->nz; o.L = n->nLayers; o.nin = n->nin; o.nout = n->nout;
+    for (int l = 0; l < o.L; l++) {
+        o.Kp[l] = n->Kp[l];
+        o.Np[l] = n->Np[l];
+        o.Wb[l] = (const __nv_bfloat16*)n->Wb[l];
+        o.b[l] = n->b[l];
+    }
+    return o;
+}
+
+static int sm_count(sbx_ctx* ctx) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess) sms = 0;
+    return sms;
+}
+
+extern "C" int32_t sbx_mlp_net_fits(const sbx_mlp_net* net, int32_t train) { return net_fits(net, train != 0) ? 1 : 0; }
+
+extern "C" sbx_status sbx_mlp_predict(sbx_ctx* ctx, const sbx_mlp_net* net, const double* X, int32_t P,
+                                      const double* xMean, const double* xStd, const double* yMean,
+                                      const double* yStd, double* out, int32_t* errFlag) {
+    SBX_REQUIRE(ctx && net_fits(net, false) && P >= 0 && (P == 0 || (X && xMean && xStd && yMean && yStd && out)));
+    if (P == 0) return SBX_OK;
+    const size_t smem = (size_t)(MT + NT) * KMAX * 2;
+    if (cudaFuncSetAttribute(k_predict, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return fail(ctx, SBX_ECUDA, "sbx_mlp_predict: shared memory attribute");
+    PredictArgs g{net_of(net), X, xMean, xStd, yMean, yStd, P, out, errFlag};
+    const int sms = sm_count(ctx), tiles = (P + MT - 1) / MT;
+    int gx = sms / net->nz;                        // one wave: a block's shared memory fills an SM
+    gx = gx < 1 ? 1 : (gx > tiles ? tiles : gx);
+    SBX_LAUNCH_SMEM(ctx, k_predict, dim3(gx, net->nz), GEMM_THREADS, smem, g);
+    const long long n = (long long)P * net->nout;
+    SBX_LAUNCH(ctx, k_predict_stats, blocks(n), 256, net->nz, n, out);
+    return check_launch(ctx, "sbx_mlp_predict");
 }

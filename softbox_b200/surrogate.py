@@ -7,19 +7,25 @@ fallback wherever the ensemble disagrees.
     mean, std = ens.predict(X_new)                   # per output, de-normalised
     rerun = fallback_mask(mean, std, 0.10)           # points for the plain simulator
 
-Every GEMM of the forward and backward passes (C = A B^T with BF16 operands and FP32
-accumulation in tensor memory) is sbx_mlp_gemm_bf16 with all ensemble members in one
-launch (blockIdx.z); the epilogues write the BF16 activations, their transposes (the
-operands of the weight-gradient GEMMs) and the FP32 pre-activations. The GELU backward,
-bias gradients, loss gradient and Adam (FP32 master weights, BF16 copies and transposes)
-are the library's elementwise kernels. Torch provides the device buffers and the batch
-gathers only.
+Ensembles that sbx_mlp_net_fits accepts (the default one does) run whole: sbx_mlp_predict
+takes all layers of all members for a tile of points in one launch. For other widths, and for
+training, every GEMM of a pass (C = A B^T with BF16 operands and FP32 accumulation in tensor memory)
+is sbx_mlp_gemm_bf16 with all members in one launch (blockIdx.z); the epilogues write the
+BF16 activations, their transposes (the operands of the weight-gradient GEMMs) and the FP32
+pre-activations. The GELU backward, bias gradients, loss gradient and Adam (FP32 master
+weights, BF16 copies and transposes) are then the library's elementwise kernels. Both ways
+do the same operations on every element. Torch provides the device buffers and, on the
+second way, the batch gathers.
 
 Shapes are padded for the tensor cores: the 6 inputs to 16 columns and the 3 outputs to
 16 rows of the last weight matrix; the padding stays exactly zero (zero inputs and zero
 output gradients give it zero gradients).
 """
+import ctypes as C
+
 import numpy as np
+
+from . import abi_types as T
 
 KPAD_IN = 16
 NPAD_OUT = 16
@@ -90,6 +96,18 @@ class MLPEnsemble:
             wb = self.W[l].to(t.bfloat16)
             self.Wb[l].copy_(wb.view(t.int16))
             self.WbT[l].copy_(wb.transpose(1, 2).contiguous().view(t.int16))
+
+    # ---------------------------------------------------------------- whole networks
+    def _net(self, train):
+        """The ensemble as the whole-network entry points take it, or None if they do not."""
+        from .runtime import LIB
+        if self.L > T.MLP_MAX_LAYERS:
+            return None
+        d = T.MlpNet(self.nz, self.L, self.nin, self.nout)
+        for l in range(self.L):
+            d.Kp[l], d.Np[l] = self.Kp[l], self.Np[l]
+            d.Wb[l], d.b[l] = self.Wb[l].data_ptr(), self.b[l].data_ptr()
+        return d if LIB.sbx_mlp_net_fits(C.byref(d), 1 if train else 0) else None
 
     # ---------------------------------------------------------------- passes
     def _gemm(self, M, N, K, A, lda, sA, B, ldb, sB, bias=None, act=0, out=None, outT=None, outF=None, ldt=None):
@@ -220,10 +238,17 @@ class MLPEnsemble:
 
     def predict(self, X, chunk=65536):
         """Ensemble mean and standard deviation of the de-normalised outputs for X [P, nin].
-        Runs on inference buffers of its own (allocated on first use of a chunk size, then
-        reused), so a prediction allocates nothing once they exist."""
+        An ensemble that does not run whole uses inference buffers for `chunk` points
+        (allocated on first use of a chunk size, then reused)."""
         t = self.torch
-        Xn = t.tensor((np.asarray(X) - self.x_mean) / self.x_std, dtype=t.float32, device=self.dev)
+        X = np.asarray(X)
+        net = self._net(False)
+        norm = ((self.x_mean, self.nin), (self.x_std, self.nin), (self.y_mean, self.nout), (self.y_std, self.nout))
+        if (net is not None and X.ndim == 2 and 0 < X.shape[0] < 2**31 and X.shape[1] == self.nin
+                and all(np.shape(v) == (n,) for v, n in norm)
+                and np.result_type(X, self.x_mean, self.x_std) == np.float64):
+            return self._predict_whole(net, X)
+        Xn = t.tensor((X - self.x_mean) / self.x_std, dtype=t.float32, device=self.dev)
         P = Xn.shape[0]
         need = min(max(P, 1), chunk)
         if getattr(self, "_inf_M", 0) < need:
@@ -238,6 +263,21 @@ class MLPEnsemble:
             outs.append(self._forward_infer(m)[:, :m, :self.nout].clone())
         y = t.cat(outs, dim=1).cpu().numpy().astype(np.float64) * self.y_std + self.y_mean
         return y.mean(axis=0), y.std(axis=0), y
+
+    def _predict_whole(self, net, X):
+        """predict() in one launch over all points, with one upload of X and one read of the
+        results: normalisation and the ensemble statistics run on the device, operation for
+        operation as the host's."""
+        t = self.torch
+        P = X.shape[0]
+        norm = t.from_numpy(np.concatenate([np.asarray(v, np.float64) for v in (
+            self.x_mean, self.x_std, self.y_mean, self.y_std)])).to(self.dev)
+        xm, xs, ym, ys = t.split(norm, [self.nin, self.nin, self.nout, self.nout])
+        Xd = t.from_numpy(np.ascontiguousarray(X, dtype=np.float64)).to(self.dev)
+        out = t.empty((2 + self.nz, P, self.nout), dtype=t.float64, device=self.dev)
+        self._ctx()("sbx_mlp_predict", net, Xd, P, xm, xs, ym, ys, out, self.err)
+        out = out.cpu().numpy()
+        return out[0], out[1], out[2:]
 
 
 def fallback_mask(mean, std, threshold=0.10, outputs=None, scale=None):
