@@ -940,6 +940,22 @@ typedef struct sbx_mlp_net {
     void* Wb[SBX_MLP_MAX_LAYERS];
     float* b[SBX_MLP_MAX_LAYERS];
 } sbx_mlp_net;
+/* The training state beside it: FP32 master weights, Adam moments and last gradients, the
+ * transposed BF16 weights [nz][Kp][Np], and buffers of a pass of B rows: activations A and
+ * their transposes AT (not for the last layer), pre-activations Z, gradients G and GT, the
+ * transposed inputs X0T [nz][16][B]. loss: nz floats (the last step's). bar: nz uint64 words
+ * of scratch. err gets bit 0 when a wait ran out. */
+typedef struct sbx_mlp_train_state {
+    float *W[SBX_MLP_MAX_LAYERS], *mW[SBX_MLP_MAX_LAYERS], *vW[SBX_MLP_MAX_LAYERS], *mb[SBX_MLP_MAX_LAYERS],
+        *vb[SBX_MLP_MAX_LAYERS], *dW[SBX_MLP_MAX_LAYERS], *db[SBX_MLP_MAX_LAYERS];
+    void* WbT[SBX_MLP_MAX_LAYERS];
+    void *A[SBX_MLP_MAX_LAYERS], *AT[SBX_MLP_MAX_LAYERS], *G[SBX_MLP_MAX_LAYERS], *GT[SBX_MLP_MAX_LAYERS];
+    float* Z[SBX_MLP_MAX_LAYERS];
+    void* X0T;
+    float* loss;
+    void* bar;
+    int32_t* err;
+} sbx_mlp_train_state;
 /* 1 if the whole-network kernels take this ensemble: at most 16 inputs and outputs, hidden
  * widths multiples of 32 up to 256, at most SBX_MLP_MAX_LAYERS layers (training: at least 2) */
 int32_t sbx_mlp_net_fits(const sbx_mlp_net* net, int32_t train);
@@ -949,6 +965,14 @@ int32_t sbx_mlp_net_fits(const sbx_mlp_net* net, int32_t train);
 sbx_status sbx_mlp_predict(sbx_ctx* ctx, const sbx_mlp_net* net, const double* X, int32_t P, const double* xMean,
                            const double* xStd, const double* yMean, const double* yStd, double* out,
                            int32_t* errFlag);
+/* nsteps Adam steps of every network on batches of B rows (a multiple of 16, 16..256) of the
+ * normalised points X [n][nin], Y [n][nout]: step s, row r of network z is point
+ * idx[z * idxStride + s * B + r] (idx NULL: point z * B + r, one step). stepNumber: the first
+ * step's number (from 1). The same operations as forward, sbx_mlp_mse_grad, backward and
+ * sbx_mlp_adam in turn. */
+sbx_status sbx_mlp_train(sbx_ctx* ctx, const sbx_mlp_net* net, const sbx_mlp_train_state* state, int32_t B,
+                         const float* X, const float* Y, const int64_t* idx, int64_t idxStride, int32_t nsteps,
+                         int32_t stepNumber, float lr, float beta1, float beta2, float eps);
 /* A plan over a packed scene (graph and per-system paths; the fused kernel is for one
  * network). `batch` is copied; its arrays must stay alive. */
 sbx_status sbx_dense_plan_create_batched(sbx_ctx* ctx, const sbx_dense_scene* scene, const sbx_batch* batch,

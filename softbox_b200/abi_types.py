@@ -114,3 +114,9 @@ class MlpNet(C.Structure):              # an ensemble's networks (sbx_mlp_net)
     _fields_ = [(k, C.c_int32) for k in ("nz", "nLayers", "nin", "nout")] + [
         (k, C.c_int32 * MLP_MAX_LAYERS) for k in ("Kp", "Np")] + [
         (k, C.c_void_p * MLP_MAX_LAYERS) for k in ("Wb", "b")]
+
+
+class MlpTrainState(C.Structure):       # its training state (sbx_mlp_train_state)
+    _fields_ = [(k, C.c_void_p * MLP_MAX_LAYERS) for k in (
+        "W", "mW", "vW", "mb", "vb", "dW", "db", "WbT", "A", "AT", "G", "GT", "Z")] + [
+        (k, C.c_void_p) for k in ("X0T", "loss", "bar", "err")]

@@ -482,6 +482,319 @@ __global__ void k_predict_stats(int nz, long long n, double* out) {
     out[n + i] = sqrt(q / (double)nz);
 }
 
+// ---------------------------------------------------------------- training
+// Whole Adam steps of the ensemble in one cooperative launch. A network's blocks (gridDim.x of
+// them, at most one an SM) work on its passes together and meet at a barrier of their own
+// after each: L forward products, then for each layer from the last the input gradient
+// together with the weight gradient and Adam update of the layer above it (whose weights
+// nothing reads any more). Every product is split into 128 x 32 tiles; the epilogues take in
+// what the separate kernels passed through memory: bias and GELU, the loss gradient, the GELU
+// gradient, Adam with the BF16 copies; the bias gradients are summed from the staged operand
+// in row order. The arithmetic, element by element, is that of the separate kernels.
+// What bounds it is latency: per pass an operand fetch from L2, a short MMA chain, an
+// epilogue and a barrier. As 42 launches a step the host's calls bounded it: 551 us a step of 5 networks at a batch of 256,
+// 127 us now.
+constexpr int TRAIN_THREADS = 256;
+constexpr int TRAIN_N = 32;                        // columns of a tile
+constexpr int TRAIN_STEPS = 64;                    // steps a launch takes (the bias corrections are arguments)
+struct TrainArgs {
+    Net net;
+    int B, nsteps;
+    const float *X, *Y;                            // [points][nin], [points][nout], normalised
+    const long long* idx;                          // [nz][idxStride] points of each network's steps, or null:
+    long long idxStride;                           //   network z's row r is point z * B + r
+    float *W[NET_MAX_LAYERS], *bias[NET_MAX_LAYERS], *mW[NET_MAX_LAYERS], *vW[NET_MAX_LAYERS], *mb[NET_MAX_LAYERS],
+        *vb[NET_MAX_LAYERS], *dW[NET_MAX_LAYERS], *db[NET_MAX_LAYERS];
+    __nv_bfloat16 *Wb[NET_MAX_LAYERS], *WbT[NET_MAX_LAYERS];
+    // the pass's activations and gradients, [nz][B][Np] (and transposed)
+    __nv_bfloat16 *A[NET_MAX_LAYERS], *AT[NET_MAX_LAYERS], *G[NET_MAX_LAYERS], *GT[NET_MAX_LAYERS], *X0T;
+    float* Z[NET_MAX_LAYERS];
+    float* loss;
+    float lr, b1, b2, eps, c1[TRAIN_STEPS], c2[TRAIN_STEPS];
+    unsigned long long* bar;                       // [nz] arrival counters, zero at launch
+    int* err;                                      // bit 0: an MMA or barrier wait ran out
+};
+
+__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// barrier of a network's blocks; false (for the whole block) once a wait has run out anywhere
+__device__ bool net_sync(unsigned long long* ctr, unsigned long long& target, int* err) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        target += gridDim.x;
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(ctr), "l"(1ULL) : "memory");
+        bool ok = true;
+        long long t0 = 0;
+        unsigned it = 0;
+        while (ld_acquire_u64(ctr) < target) {
+            if ((++it & 63u) == 0) {
+                if (*(volatile int*)err & 1) { ok = false; break; }
+                long long now = gtimer();
+                if (t0 == 0) t0 = now;
+                else if (now - t0 > WAIT_NS) { atomicOr(err, 1); ok = false; break; }
+            }
+        }
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// Adam of one weight with the step's corrections (the arithmetic of k_adam)
+__device__ __forceinline__ float adam_one(const TrainArgs& g, int s, float gg, float& m, float& v, float w) {
+    m = g.b1 * m + (1.0f - g.b1) * gg;
+    v = g.b2 * v + (1.0f - g.b2) * gg * gg;
+    return w - g.lr * (m / g.c1[s]) / (sqrtf(v / g.c2[s]) + g.eps);
+}
+
+__global__ void __launch_bounds__(TRAIN_THREADS, 1) k_train(const __grid_constant__ TrainArgs g) {
+    extern __shared__ __align__(1024) char smem[];
+    char* sA = smem;                               // 128 x 256
+    char* sB = smem + MT * KMAX * 2;               // 32 x 256
+    __shared__ __align__(8) unsigned long long mbar;
+    __shared__ unsigned tmemSlot;
+    const Net& net = g.net;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quarter = warp & 3, half = warp >> 2;
+    const int z = blockIdx.y, L = net.L, B = g.B;
+    const int mTiles = (B + MT - 1) / MT;
+    if (threadIdx.x == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)));
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmemSlot)),
+                     "r"(TRAIN_N));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const unsigned tmem = tmemSlot;
+    unsigned phase = 0;
+    unsigned long long target = 0;
+    bool ok = true;
+
+    // the product of the staged operands (128 x N x Kp): true when it is in tensor memory
+    auto product = [&](int N, int Kp) {
+        cp_async_wait_all();
+        asm volatile("fence.proxy.async.shared::cta;");
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        if (threadIdx.x == 0) issue_mma(tmem, smem_u32(sA), smem_u32(sB), N, Kp, &mbar);
+        const bool done = wait_mma(&mbar, phase);
+        phase ^= 1u;
+        if (!done && threadIdx.x == 0) atomicOr(g.err, 1);
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        return done;
+    };
+    // every warp is done with the operands and the accumulators
+    auto release = [&]() {
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncthreads();
+    };
+    // row-major [rows][N] BF16 and its transpose [N][rows] from 16 columns of a row
+    auto put = [&](__nv_bfloat16* rowMajor, __nv_bfloat16* transposed, int rows, int N, int row, int c0,
+                   const float a[16]) {
+        if (row >= rows) return;
+        uint4 lo, hi;
+        pack16(a, lo, hi);
+        uint4* o = reinterpret_cast<uint4*>(rowMajor + (long long)row * N + c0);
+        o[0] = lo;
+        o[1] = hi;
+#pragma unroll
+        for (int j = 0; j < 16; j++) transposed[(long long)(c0 + j) * rows + row] = __float2bfloat16_rn(a[j]);
+    };
+
+    // dW of layer l for rows [128 mt, ..) and columns [32 kt, ..), its Adam update and, with the
+    // first columns, the rows' bias gradient and update
+    auto weight_tile = [&](int l, int tile, int s) {
+        const int N = net.Np[l], K = net.Kp[l], kTiles = (K + TRAIN_N - 1) / TRAIN_N;
+        const int mt = tile / kTiles, kt = tile - mt * kTiles, n0 = mt * MT, k0 = kt * TRAIN_N;
+        const int kc = min(TRAIN_N, K - k0);
+        const long long wz = (long long)z * N * K;
+        const __nv_bfloat16* prevT = l == 0 ? g.X0T : g.AT[l - 1];
+        stage_rows(sA, g.GT[l] + ((long long)z * N + n0) * B, B, MT, min(MT, N - n0), B);
+        stage_rows(sB, prevT + ((long long)z * K + k0) * B, B, kc, kc, B);
+        const int n = n0 + quarter * 32 + lane, c0 = 16 * half;
+        const bool mine = n < N && c0 < kc;
+        float w[16], m[16], v[16];
+        const long long o = wz + (long long)n * K + k0 + c0;
+        if (mine) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                *reinterpret_cast<float4*>(w + 4 * j) = reinterpret_cast<const float4*>(g.W[l] + o)[j];
+                *reinterpret_cast<float4*>(m + 4 * j) = reinterpret_cast<const float4*>(g.mW[l] + o)[j];
+                *reinterpret_cast<float4*>(v + 4 * j) = reinterpret_cast<const float4*>(g.vW[l] + o)[j];
+            }
+        }
+        if (!product(kc, B)) return false;
+        if (kt == 0 && threadIdx.x < MT && n0 + (int)threadIdx.x < N) {
+            // the bias gradient: the row's B values in row order, from the staged operand
+            const int r = threadIdx.x;
+            float sum = 0.f;
+            for (int c = 0; c < B; c += 8) {
+                const uint4 q = *reinterpret_cast<const uint4*>(sA + core_at(r, c, B));
+                const unsigned h[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    sum += __bfloat162float(__ushort_as_bfloat16((unsigned short)(h[j] & 0xffffu)));
+                    sum += __bfloat162float(__ushort_as_bfloat16((unsigned short)(h[j] >> 16)));
+                }
+            }
+            const int bo = z * N + n0 + r;
+            g.db[l][bo] = sum;
+            float mm = g.mb[l][bo], vv = g.vb[l][bo];
+            g.bias[l][bo] = adam_one(g, s, sum, mm, vv, g.bias[l][bo]);
+            g.mb[l][bo] = mm;
+            g.vb[l][bo] = vv;
+        }
+        float d[16];
+        if (c0 < kc) load_acc16(tmem, quarter, c0, d);
+        if (mine) {
+#pragma unroll
+            for (int j = 0; j < 16; j++) w[j] = adam_one(g, s, d[j], m[j], v[j], w[j]);
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                reinterpret_cast<float4*>(g.dW[l] + o)[j] = *reinterpret_cast<float4*>(d + 4 * j);
+                reinterpret_cast<float4*>(g.W[l] + o)[j] = *reinterpret_cast<float4*>(w + 4 * j);
+                reinterpret_cast<float4*>(g.mW[l] + o)[j] = *reinterpret_cast<float4*>(m + 4 * j);
+                reinterpret_cast<float4*>(g.vW[l] + o)[j] = *reinterpret_cast<float4*>(v + 4 * j);
+            }
+            uint4 lo, hi;
+            pack16(w, lo, hi);
+            uint4* wb = reinterpret_cast<uint4*>(g.Wb[l] + o);
+            wb[0] = lo;
+            wb[1] = hi;
+#pragma unroll
+            for (int j = 0; j < 16; j++) g.WbT[l][wz + (long long)(k0 + c0 + j) * N + n] = __float2bfloat16_rn(w[j]);
+        }
+        release();
+        return true;
+    };
+    auto weight_tiles = [&](int l) { return ((net.Np[l] + MT - 1) / MT) * ((net.Kp[l] + TRAIN_N - 1) / TRAIN_N); };
+
+    for (int s = 0; s < g.nsteps && ok; s++) {
+        auto point = [&](int row) {
+            return g.idx ? g.idx[z * g.idxStride + (long long)s * B + row] : (long long)z * B + row;
+        };
+        // ---- forward
+        for (int l = 0; l < L && ok; l++) {
+            const int N = net.Np[l], K = net.Kp[l], nTiles = (N + TRAIN_N - 1) / TRAIN_N;
+            const bool last = l == L - 1;
+            if (l == 0 && blockIdx.x == 0 && threadIdx.x == 0) g.loss[z] = 0.f;
+            for (int tile = blockIdx.x; tile < mTiles * nTiles && ok; tile += gridDim.x) {
+                const int mt = tile / nTiles, nt = tile - mt * nTiles, m0 = mt * MT, n0 = nt * TRAIN_N;
+                const int nc = min(TRAIN_N, N - n0);
+                if (l == 0) {
+                    // the batch's inputs (16 padded columns), with their transpose for dW of layer 0
+                    const int r = threadIdx.x >> 1, q0 = (threadIdx.x & 1) * 8, row = m0 + r;
+                    unsigned short h[8];
+                    const long long pt = row < B ? point(row) : 0;
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const float x = (row < B && q0 + j < net.nin) ? g.X[pt * net.nin + q0 + j] : 0.f;
+                        h[j] = __bfloat16_as_ushort(__float2bfloat16_rn(x));
+                        if (nt == 0 && row < B)
+                            g.X0T[((long long)z * K + q0 + j) * B + row] = __ushort_as_bfloat16(h[j]);
+                    }
+                    *reinterpret_cast<uint4*>(sA + core_at(r, q0, 16)) =
+                        make_uint4(h[0] | (unsigned)h[1] << 16, h[2] | (unsigned)h[3] << 16,
+                                   h[4] | (unsigned)h[5] << 16, h[6] | (unsigned)h[7] << 16);
+                } else {
+                    stage_rows(sA, g.A[l - 1] + ((long long)z * B + m0) * K, K, MT, min(MT, B - m0), K);
+                }
+                stage_rows(sB, g.Wb[l] + ((long long)z * N + n0) * K, K, nc, nc, K);
+                const int r = quarter * 32 + lane, row = m0 + r, c0 = 16 * half;
+                ok = product(nc, K);
+                if (ok && c0 < nc) {
+                    float v[16];
+                    load_acc16(tmem, quarter, c0, v);
+#pragma unroll
+                    for (int j = 0; j < 16; j++) v[j] += __ldcg(g.bias[l] + z * N + n0 + c0 + j);
+                    if (row < B) {
+                        float4* zo = reinterpret_cast<float4*>(g.Z[l] + ((long long)z * B + row) * N + n0 + c0);
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            zo[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    }
+                    if (!last) {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) v[j] = gelu(v[j]);
+                        put(g.A[l] + (long long)z * B * N, g.AT[l] + (long long)z * B * N, B, N, row, n0 + c0, v);
+                    } else {
+                        // the loss gradient of the outputs (0 on the padding), and the loss
+                        float e = 0.f;
+                        const long long pt = row < B ? point(row) : 0;
+#pragma unroll
+                        for (int j = 0; j < 16; j++) {
+                            float gr = 0.f;
+                            if (row < B && c0 + j < net.nout) {
+                                const float d = v[j] - g.Y[pt * net.nout + c0 + j];
+                                gr = 2.0f * d / (float)(B * net.nout);
+                                e += d * d / (float)(B * net.nout);
+                            }
+                            v[j] = gr;
+                        }
+                        put(g.G[l] + (long long)z * B * N, g.GT[l] + (long long)z * B * N, B, N, row, c0, v);
+                        for (int q = 16; q > 0; q >>= 1) e += __shfl_xor_sync(0xffffffffu, e, q);
+                        if (lane == 0) atomicAdd(&g.loss[z], e);
+                    }
+                }
+                if (ok) release();
+            }
+            ok = ok && net_sync(g.bar + z, target, g.err);
+        }
+        // ---- backward: the gradient of layer l's input, with the update of layer l + 1
+        for (int l = L - 1; l >= 1 && ok; l--) {
+            const int N = net.Np[l], K = net.Kp[l], kTiles = (K + TRAIN_N - 1) / TRAIN_N;
+            const int nGrad = mTiles * kTiles, nAll = nGrad + (l + 1 < L ? weight_tiles(l + 1) : 0);
+            for (int tile = blockIdx.x; tile < nAll && ok; tile += gridDim.x) {
+                if (tile >= nGrad) {
+                    ok = weight_tile(l + 1, tile - nGrad, s);
+                    continue;
+                }
+                const int mt = tile / kTiles, kt = tile - mt * kTiles, m0 = mt * MT, k0 = kt * TRAIN_N;
+                const int kc = min(TRAIN_N, K - k0);
+                stage_rows(sA, g.G[l] + ((long long)z * B + m0) * N, N, MT, min(MT, B - m0), N);
+                stage_rows(sB, g.WbT[l] + ((long long)z * K + k0) * N, N, kc, kc, N);
+                const int row = m0 + quarter * 32 + lane, c0 = 16 * half;
+                float zv[16];
+                if (row < B && c0 < kc) {
+                    const float4* zp = reinterpret_cast<const float4*>(g.Z[l - 1] + ((long long)z * B + row) * K + k0 + c0);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) *reinterpret_cast<float4*>(zv + 4 * j) = __ldcg(zp + j);
+                }
+                ok = product(kc, N);
+                if (ok && c0 < kc) {
+                    float v[16];
+                    load_acc16(tmem, quarter, c0, v);
+                    if (row < B) {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) v[j] *= gelu_grad(zv[j]);
+                        put(g.G[l - 1] + (long long)z * B * K, g.GT[l - 1] + (long long)z * B * K, B, K, row, k0 + c0, v);
+                    }
+                }
+                if (ok) release();
+            }
+            ok = ok && net_sync(g.bar + z, target, g.err);
+        }
+        // ---- the updates that are left: layer 0, and layer 1 of a network with more than one
+        const int w1 = L > 1 ? weight_tiles(1) : 0, w0 = weight_tiles(0);
+        for (int tile = blockIdx.x; tile < w1 + w0 && ok; tile += gridDim.x)
+            ok = tile < w1 ? weight_tile(1, tile, s) : weight_tile(0, tile - w1, s);
+        ok = ok && net_sync(g.bar + z, target, g.err);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    if (warp == 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TRAIN_N));
+    }
+}
+
 // dZ = dA * GELU'(Z) (or dA when Z is NULL) -> BF16 row-major and transposed; M x N, per z
 __global__ void k_gelu_back(int M, int N, const float* dA, const float* Z, long long sMN, __nv_bfloat16* g,
                             __nv_bfloat16* gT, long long sG, long long sGT) {
@@ -684,4 +997,63 @@ extern "C" sbx_status sbx_mlp_predict(sbx_ctx* ctx, const sbx_mlp_net* net, cons
     const long long n = (long long)P * net->nout;
     SBX_LAUNCH(ctx, k_predict_stats, blocks(n), 256, net->nz, n, out);
     return check_launch(ctx, "sbx_mlp_predict");
+}
+
+extern "C" sbx_status sbx_mlp_train(sbx_ctx* ctx, const sbx_mlp_net* net, const sbx_mlp_train_state* st, int32_t B,
+                                    const float* X, const float* Y, const int64_t* idx, int64_t idxStride,
+                                    int32_t nsteps, int32_t stepNumber, float lr, float beta1, float beta2, float eps) {
+    SBX_REQUIRE(ctx && net_fits(net, true) && st && B >= 16 && B <= KMAX && B % 16 == 0 && X && Y && nsteps >= 0 &&
+                stepNumber >= 1 && st->X0T && st->loss && st->bar && st->err);
+    for (int l = 0; l < net->nLayers; l++)
+        SBX_REQUIRE(st->W[l] && st->mW[l] && st->vW[l] && st->mb[l] && st->vb[l] && st->dW[l] && st->db[l] &&
+                    st->WbT[l] && st->Z[l] && st->G[l] && st->GT[l] &&
+                    (l == net->nLayers - 1 || (st->A[l] && st->AT[l])));
+    const size_t smem = (size_t)(MT + TRAIN_N) * KMAX * 2;
+    if (cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return fail(ctx, SBX_ECUDA, "sbx_mlp_train: shared memory attribute");
+    int per = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_train, TRAIN_THREADS, smem) != cudaSuccess || per < 1)
+        return fail(ctx, SBX_ECUDA, "sbx_mlp_train: occupancy");
+    // a network's blocks: one an SM, no more than a backward pass has tiles (two products of 16)
+    int gx = sm_count(ctx) / net->nz;
+    if (gx < 1) return fail(ctx, SBX_EINVAL, "sbx_mlp_train: more networks than SMs");
+    if (gx > 32) gx = 32;
+    TrainArgs g{};
+    g.net = net_of(net);
+    g.B = B;
+    g.X = X; g.Y = Y;
+    g.idx = (const long long*)idx;
+    g.idxStride = idxStride;
+    for (int l = 0; l < net->nLayers; l++) {
+        g.W[l] = st->W[l]; g.bias[l] = net->b[l]; g.mW[l] = st->mW[l]; g.vW[l] = st->vW[l];
+        g.mb[l] = st->mb[l]; g.vb[l] = st->vb[l]; g.dW[l] = st->dW[l]; g.db[l] = st->db[l];
+        g.Wb[l] = (__nv_bfloat16*)net->Wb[l]; g.WbT[l] = (__nv_bfloat16*)st->WbT[l];
+        g.A[l] = (__nv_bfloat16*)st->A[l]; g.AT[l] = (__nv_bfloat16*)st->AT[l];
+        g.G[l] = (__nv_bfloat16*)st->G[l]; g.GT[l] = (__nv_bfloat16*)st->GT[l];
+        g.Z[l] = st->Z[l];
+    }
+    g.X0T = (__nv_bfloat16*)st->X0T;
+    g.loss = st->loss;
+    g.bar = (unsigned long long*)st->bar;
+    g.err = st->err;
+    g.lr = lr; g.b1 = beta1; g.b2 = beta2; g.eps = eps;
+    for (int s0 = 0; s0 < nsteps; s0 += TRAIN_STEPS) {
+        g.nsteps = nsteps - s0 < TRAIN_STEPS ? nsteps - s0 : TRAIN_STEPS;
+        g.idx = idx ? (const long long*)idx + (int64_t)s0 * B : nullptr;
+        for (int s = 0; s < g.nsteps; s++) {
+            g.c1[s] = 1.0f - powf(beta1, (float)(stepNumber + s0 + s));
+            g.c2[s] = 1.0f - powf(beta2, (float)(stepNumber + s0 + s));
+        }
+        if (cudaMemsetAsync(g.bar, 0, sizeof(unsigned long long) * net->nz, ctx->stream) != cudaSuccess)
+            return fail(ctx, SBX_ECUDA, "sbx_mlp_train: memset");
+        void* args[] = {&g};
+        cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_train, dim3(gx, net->nz), dim3(TRAIN_THREADS), args,
+                                                    smem, ctx->stream);
+        ctx->launches++;
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return fail(ctx, SBX_ECUDA, std::string("sbx_mlp_train: ") + cudaGetErrorString(e));
+        }
+    }
+    return check_launch(ctx, "sbx_mlp_train");
 }

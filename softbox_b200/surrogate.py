@@ -8,8 +8,9 @@ fallback wherever the ensemble disagrees.
     rerun = fallback_mask(mean, std, 0.10)           # points for the plain simulator
 
 Ensembles that sbx_mlp_net_fits accepts (the default one does) run whole: sbx_mlp_predict
-takes all layers of all members for a tile of points in one launch. For other widths, and for
-training, every GEMM of a pass (C = A B^T with BF16 operands and FP32 accumulation in tensor memory)
+takes all layers of all members for a tile of points in one launch, sbx_mlp_train an epoch's
+Adam steps in one launch. For other widths, and for forward() and backward() by themselves,
+every GEMM of a pass (C = A B^T with BF16 operands and FP32 accumulation in tensor memory)
 is sbx_mlp_gemm_bf16 with all members in one launch (blockIdx.z); the epilogues write the
 BF16 activations, their transposes (the operands of the weight-gradient GEMMs) and the FP32
 pre-activations. The GELU backward, bias gradients, loss gradient and Adam (FP32 master
@@ -84,6 +85,7 @@ class MLPEnsemble:
         self.dA = [t.zeros((nz, M, self.Kp[l]), **f32) for l in range(self.L)]     # dL / d(input of layer l)
         self.gout = t.zeros((nz, M, NPAD_OUT), **f32)
         self.loss = t.zeros(nz, **f32)
+        self.bar = t.zeros(nz, dtype=t.int64, device=self.dev)
 
     def _ctx(self):
         from .runtime import default_context
@@ -108,6 +110,21 @@ class MLPEnsemble:
             d.Kp[l], d.Np[l] = self.Kp[l], self.Np[l]
             d.Wb[l], d.b[l] = self.Wb[l].data_ptr(), self.b[l].data_ptr()
         return d if LIB.sbx_mlp_net_fits(C.byref(d), 1 if train else 0) else None
+
+    def _train_whole(self, net, X, Y, idx, nsteps):
+        """nsteps Adam steps in one call: X [n, nin], Y [n, nout] float32, idx [nz, ...] int64
+        (None: member z's row r is point z * B + r)."""
+        s = T.MlpTrainState()
+        for l in range(self.L):
+            for k in ("W", "mW", "vW", "mb", "vb", "dW", "db", "WbT", "A", "AT", "G", "GT", "Z"):
+                getattr(s, k)[l] = getattr(self, k)[l].data_ptr()
+        s.X0T, s.loss, s.bar, s.err = (x.data_ptr() for x in (self.X0T, self.loss, self.bar, self.err))
+        self._ctx()("sbx_mlp_train", net, s, self.B, X, Y, idx, 0 if idx is None else idx.stride(0), nsteps,
+                    self.step_no + 1, self.lr, 0.9, 0.999, 1e-8)
+        self.step_no += nsteps
+
+    def _trains_whole(self):
+        return self._net(True) if self.B % 16 == 0 and 16 <= self.B <= 256 and self.M == self.B else None
 
     # ---------------------------------------------------------------- passes
     def _gemm(self, M, N, K, A, lda, sA, B, ldb, sB, bias=None, act=0, out=None, outT=None, outF=None, ldt=None):
@@ -181,6 +198,13 @@ class MLPEnsemble:
     def train_step(self, xb, tb):
         """One Adam step per member on its own batch: xb [nz, B, nin], tb [nz, B, nout]
         (normalised, device). Returns nothing; the losses stay in self.loss."""
+        t = self.torch
+        shapes = ((xb, (self.nz, self.B, self.nin)), (tb, (self.nz, self.B, self.nout)))
+        net = self._trains_whole()
+        if net is not None and all(tuple(x.shape) == sh and x.dtype == t.float32 and x.is_contiguous()
+                                   and x.device == self.loss.device for x, sh in shapes):
+            self._train_whole(net, xb, tb, None, 1)
+            return
         self._stage_inputs(xb)
         self.T.copy_(tb)
         self.forward()
@@ -203,7 +227,11 @@ class MLPEnsemble:
         steps = max(1, n // self.B)
         for ep in range(epochs):
             perms = t.stack([smp[t.randperm(n, generator=g)] for smp in samples]).to(self.dev)
-            for s in range(steps):
+            net = self._trains_whole() if n >= self.B and Xn.shape[1:] == (self.nin,) and Yn.shape == (
+                n, self.nout) else None
+            if net is not None:
+                self._train_whole(net, Xn, Yn, perms, steps)
+            for s in range(steps if net is None else 0):
                 idx = perms[:, s * self.B:(s + 1) * self.B]
                 if idx.shape[1] < self.B:
                     break

@@ -1,7 +1,9 @@
-"""The whole-network prediction kernel (sbx_mlp_predict) against the GEMM path, which the
+"""The whole-network kernels (sbx_mlp_predict, sbx_mlp_train) against the GEMM path, which the
 oracle checks (tests/test_gpu_surrogate.py): ragged point counts around the 128-row tiles, one
-and several networks, narrow and wide layers. Both paths do the same operations on every
-element, so predictions agree to FP64 rounding of the statistics."""
+and several networks, narrow and wide layers, batches of part of a tile to two tiles. Both
+paths do the same operations on every element, so predictions agree to FP64 rounding of the
+statistics. Training may differ by a BF16 rounding where two FP32 values straddle one: one
+such flip among a layer's 256 inputs moves a sum by 2^-8 / 256 of itself, 1.5e-5."""
 import numpy as np
 import pytest
 
@@ -34,3 +36,39 @@ def test_predict_equals_the_gemm_path(dims, nz, P, monkeypatch):
     for a, b, name in zip(whole, ref, ("mean", "std", "y")):
         assert a.shape == b.shape and a.dtype == b.dtype
         assert np.allclose(a, b, rtol=1e-12, atol=1e-12), name
+
+
+@pytest.mark.parametrize("dims,nz,B", [((6, 256, 256, 256, 256, 3), 5, 256), ((6, 64, 32, 3), 2, 16),
+                                       ((16, 96, 16), 1, 144), ((3, 32, 256, 1), 3, 128)])
+def test_train_equals_the_separate_kernels(dims, nz, B, monkeypatch):
+    steps = 3
+    a, x, y = _ensemble(dims, nz, B)
+    b, _, _ = _ensemble(dims, nz, B)
+    n = steps * B
+    ha = a.fit(x[:n], y[:n], epochs=1, seed=5)
+    monkeypatch.setattr(type(b), "_net", lambda self, train: None)
+    hb = b.fit(x[:n], y[:n], epochs=1, seed=5)
+    torch.cuda.synchronize()
+    assert a.err.item() == 0 and a.step_no == b.step_no == steps
+    assert abs(ha[0] - hb[0]) <= 1e-5 * abs(hb[0])
+    for l in range(a.L):
+        for k in ("W", "b", "mW", "mb", "vW", "vb", "dW", "db"):
+            p, q = getattr(a, k)[l].double(), getattr(b, k)[l].double()
+            assert (p - q).norm() <= 2e-5 * q.norm(), f"{k}[{l}]"
+        assert torch.equal(a.Wb[l].view(torch.bfloat16), a.W[l].to(torch.bfloat16))
+        assert torch.equal(a.WbT[l], a.Wb[l].transpose(1, 2))
+        assert a.W[l][:, dims[l + 1]:].abs().sum().item() == 0        # the padding stays zero
+    assert a.W[0][:, :, dims[0]:].abs().sum().item() == 0
+
+
+def test_one_step_on_given_batches_equals_fit():
+    a, x, y = _ensemble((6, 64, 64, 3), 2, 64)
+    b, _, _ = _ensemble((6, 64, 64, 3), 2, 64)
+    t = lambda v, m, s: torch.tensor((v - m) / s, dtype=torch.float32, device="cuda")  # noqa: E731
+    X, Y = t(x[:64], a.x_mean, a.x_std), t(y[:64], a.y_mean, a.y_std)
+    a.train_step(X.expand(2, 64, 6).contiguous(), Y.expand(2, 64, 3).contiguous())
+    idx = torch.arange(64, device="cuda").repeat(2, 1)
+    b._train_whole(b._net(True), X, Y, idx, 1)
+    torch.cuda.synchronize()
+    for l in range(a.L):
+        assert torch.equal(a.W[l], b.W[l]) and torch.equal(a.b[l], b.b[l])
