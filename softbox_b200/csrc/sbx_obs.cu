@@ -212,11 +212,13 @@ __global__ void k_cl_init(int nSeg, int nNode, const int* filState, int* label, 
 // one as its parent if it still is a root; otherwise another edge got there first and this
 // one goes on from the two nodes' roots as they are now. A failed exchange means that a root
 // has gone, so the tries of all edges together are bounded by the nodes; a thread that runs
-// out of its own limit marks the labelling as not converged.
-__global__ void k_cl_join(int nSeg, const int* e2, int nLinks, const int* linkA, const int* linkB,
+// out of its own limit marks the labelling as not converged. The chain links go first (edges
+// [0, nSeg)), then every path is flattened, then the other edges ([nSeg, ..)): a walk from a
+// crosslink or a head then starts one step from its filament's root, not at the end of a chain.
+__global__ void k_cl_join(int first, int nSeg, const int* e2, int nLinks, const int* linkA, const int* linkB,
                           const int* linkState, int nM, const int* boundSeg, const int* motorBackbone, int* label,
                           int* notDone) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int i = first + blockIdx.x * blockDim.x + threadIdx.x;
     int u = -1, v = -1;
     if (i < nSeg) {
         u = i;
@@ -238,6 +240,11 @@ __global__ void k_cl_join(int nSeg, const int* e2, int nLinks, const int* linkA,
         if (atomicCAS(&label[hi], hi, lo) == hi) return;
     }
     *notDone = 1;
+}
+
+__global__ void k_cl_flatten(int nNode, int* label) {
+    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nNode && __ldcg(label + i) >= 0) __stcg(label + i, find_root<false>(label, i));
 }
 
 // every node's label: its component's root; the component sizes in segments
@@ -328,9 +335,13 @@ extern "C" sbx_status sbx_obs_clusters(sbx_ctx* ctx, int32_t nNet, const int32_t
     int nInit = nNode > rounds + 1 ? nNode : rounds + 1;
     if (nInit < 2 * nNet) nInit = 2 * nNet;
     SBX_LAUNCH(ctx, k_cl_init, blocks(nInit), 256, nSeg, nNode, filState, label, size, flags, rounds, nNet, out);
-    int nEdge = nSeg + nLinks + nMotors;
-    SBX_LAUNCH(ctx, k_cl_join, blocks(nEdge), 256, nSeg, end2NbrSlot, nLinks, linkFilA, linkFilB, linkState, nMotors,
-               boundSeg, motorBackbone, label, flags + (rounds - 1));
+    SBX_LAUNCH(ctx, k_cl_join, blocks(nSeg), 256, 0, nSeg, end2NbrSlot, 0, linkFilA, linkFilB, linkState, 0, boundSeg,
+               motorBackbone, label, flags + (rounds - 1));
+    if (nLinks + nMotors > 0) {
+        SBX_LAUNCH(ctx, k_cl_flatten, blocks(nNode), 256, nNode, label);
+        SBX_LAUNCH(ctx, k_cl_join, blocks((int64_t)nLinks + nMotors), 256, nSeg, nSeg, end2NbrSlot, nLinks, linkFilA,
+                   linkFilB, linkState, nMotors, boundSeg, motorBackbone, label, flags + (rounds - 1));
+    }
     SBX_LAUNCH(ctx, k_cl_label, blocks(nNode), 256, nSeg, nNode, label, size);
     SBX_LAUNCH(ctx, k_cl_largest, nNet * CL_PARTS, OBS_THREADS, segBase, label, size, out);
     return check_launch(ctx, "sbx_obs_clusters");
