@@ -15,6 +15,7 @@
 #include "sbx_internal.cuh"
 #include "sbx_physics.cuh"
 #include "sbx_trace.h"
+#include "sbx_wide.cuh"
 
 #include <vector>
 
@@ -400,6 +401,10 @@ struct sbx_dense_plan {
     FusedArgs fa{};
     int fused_grid = 0;
     std::vector<void*> allocs;
+    // the graph path's wide kernels (harness layouts); other scenes capture the per-system sequence
+    bool wide_ok = false;
+    WideArgs wide{};
+    WideStreams wideStreams{};
     // packed networks (graph and per-system paths only)
     bool batched = false;
     sbx_batch batch{};
@@ -528,75 +533,37 @@ bool fused_topology(sbx_dense_plan* p) {
     return true;
 }
 
-bool fused_prepare(sbx_dense_plan* p) {
+// Sizes and the harness layout that the fused kernel and the wide kernels rely on: motors 2d and
+// 2d + 1 of dimer d, the same number of dimers on every backbone in backbone order, the body
+// view = segments then heads. Returns why a scene has another layout, or null.
+const char* step_layout(sbx_dense_plan* p, FusedArgs& a) {
     const sbx_dense_scene& sc = p->scene;
     cudaStream_t st = p->ctx->stream;
-    FusedArgs& a = p->fa;
     a.sc = sc;
     a.nSeg = sc.fil.body.n; a.nM = sc.mot.nMotors; a.nB = sc.mot.body.n; a.nBb = sc.mini.backbone.n;
     a.nD = sc.dim.nDimers; a.nL = sc.xl.nLinks; a.cap = sc.grid.cap; a.C = sc.grid.totalCells;
     a.xlOn = (sc.xlinkOn && sc.xl.nLinks > 0) ? 1 : 0;
     a.xlUnbind = sc.xlUnbind ? 1 : 0;
-    auto why = [&](const char* w) { p->fused_why = w; return false; };
-    if (a.nSeg <= 0 || a.nM <= 0 || a.nBb <= 0) return why("empty stores");
-    if (a.nB != 3 * a.nM || a.nM != 2 * a.nD || sc.mini.nDimers != a.nD) return why("motor/dimer counts");
-    if (a.nD % a.nBb) return why("dimers per backbone not uniform");
+    if (a.nSeg <= 0 || a.nM <= 0 || a.nBb <= 0) return "empty stores";
+    if (a.nB != 3 * a.nM || a.nM != 2 * a.nD || sc.mini.nDimers != a.nD) return "motor/dimer counts";
+    if (a.nD % a.nBb) return "dimers per backbone not uniform";
     a.dpm = a.nD / a.nBb;
-    if (6 * a.dpm > FUSED_MAX_SUB || 2 * a.dpm > 32) return why("too many dimers per backbone");
+    if (6 * a.dpm > FUSED_MAX_SUB || 2 * a.dpm > 32) return "too many dimers per backbone";
     auto mA = d2h(sc.dim.motorA, a.nD, st), mB = d2h(sc.dim.motorB, a.nD, st);
     auto hbs = d2h(sc.mini.headBackboneSlot, a.nD, st), mmA = d2h(sc.mini.motorA, a.nD, st);
     for (int d = 0; d < a.nD; d++)
         if (mA[d] != 2 * d || mB[d] != 2 * d + 1 || hbs[d] != d / a.dpm || mmA[d] != 2 * d)
-            return why("dimer/minifilament topology is not the harness layout");
+            return "dimer/minifilament topology is not the harness layout";
     auto pub = d2h(sc.mot.publishParams, 1, st);
-    if (pub[0] != a.nSeg || a.cap < a.nSeg + a.nM) return why("body-view layout");
+    if (pub[0] != a.nSeg || a.cap < a.nSeg + a.nM) return "body-view layout";
     auto gc = d2h(sc.grid.gridCounts, 4, st);
     a.S = gc[1];
-    if (a.S < 0 || a.S > a.cap) return why("grid counts");
+    if (a.S < 0 || a.S > a.cap) return "grid counts";
     auto gd = d2h(sc.grid.gridDims, 4, st);
     a.nX = gd[0]; a.nY = gd[1]; a.nZ = gd[2];
-    if (gd[3] != a.C || (long long)a.nX * a.nY * a.nZ != a.C) return why("grid dims");
-    int dev = 0, sms = 0, coop = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    int per = fused_max_blocks_per_sm();
-    if (!coop || per <= 0) return why("cooperative launch unavailable");
-    p->fused_grid = sms * per;
-    if (!fused_topology(p)) return false;
+    if (gd[3] != a.C || (!p->batched && (long long)a.nX * a.nY * a.nZ != a.C)) return "grid dims";
     a.tilesC = (a.C + SCAN_CHUNK - 1) / SCAN_CHUNK;
     a.tilesS = (a.nSeg + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    auto fc = d2h(sc.fil.counts, 4, st);
-    a.filSeed = fc[2];
-    // plan-owned scratch
-    auto alloc = [&](size_t bytes) -> void* {
-        void* q = nullptr;
-        if (cudaMalloc(&q, bytes ? bytes : 4) != cudaSuccess) return nullptr;
-        p->allocs.push_back(q);
-        return q;
-    };
-    size_t nS = a.nSeg;
-    a.cntCell = (int*)alloc(4 * (size_t)a.C);
-    a.cntSeg = (int*)alloc(4 * (size_t)a.C);
-    a.segCellOff = (int*)alloc(4 * ((size_t)a.C + 1));
-    a.cntAct = (int*)alloc(4 * nS); a.cntA = (int*)alloc(4 * nS); a.cntB = (int*)alloc(4 * nS);
-    a.cntM = (int*)alloc(4 * nS);
-    a.tileSum = (int*)alloc(4 * (size_t)(2 * a.tilesC + 2 * a.tilesS + 1));
-    a.mTileSum = (int*)alloc(4 * (size_t)(a.tilesS + 1));
-    a.cellSlot = (int*)alloc(4 * (size_t)a.C * FUSED_CELL_SLOTS);
-    a.slotA = (int*)alloc(4 * nS * FUSED_ROW_SLOTS); a.slotB = (int*)alloc(4 * nS * FUSED_ROW_SLOTS);
-    a.slotM = (int*)alloc(4 * nS * FUSED_MOTOR_SLOTS);
-    a.cellHead = (int*)alloc(4 * (size_t)a.C); a.cellNext = (int*)alloc(4 * (size_t)a.cap);
-    size_t nLk = (size_t)std::max(a.nL, 1);
-    a.headA = (int*)alloc(4 * nS); a.nextA = (int*)alloc(4 * nLk);
-    a.headB = (int*)alloc(4 * nS); a.nextB = (int*)alloc(4 * nLk);
-    a.headM = (int*)alloc(4 * nS); a.nextM = (int*)alloc(4 * (size_t)a.nM);
-    a.segE1 = (float4*)alloc(16 * nS); a.segE2 = (float4*)alloc(16 * nS);
-    a.joints = alloc(2 * nS * FUSED_JOINT_BYTES);
-    a.terms = alloc((2 * (size_t)a.nM + 4 * (size_t)a.nD) * FUSED_TERM_BYTES);
-    a.uSnap = (float*)alloc(12 * nS);
-    a.bar = (unsigned long long*)alloc(32);
-    a.err = (int*)alloc(16);
     a.d_step = p->d_step;
     a.stats = p->stats;
     a.entCap = FUSED_ENT_CAP;
@@ -605,12 +572,129 @@ bool fused_prepare(sbx_dense_plan* p) {
     a.cellUse = FUSED_CELL_SLOTS;
     a.rowUse = FUSED_ROW_SLOTS;
     a.mRowUse = FUSED_MOTOR_SLOTS;
-    for (void* q : p->allocs)
-        if (!q) return why("scratch allocation failed");
+    return nullptr;
+}
+
+// A path's scratch is one allocation, carved twice by the same code: once for its size, once for
+// the pointers.
+struct Arena {
+    char* base = nullptr;
+    size_t used = 0;
+    template <class T>
+    void take(T*& p, size_t bytes) {
+        p = base ? reinterpret_cast<T*>(base + used) : nullptr;
+        used += (std::max(bytes, (size_t)4) + 255) & ~(size_t)255;
+    }
+    template <class Carve>
+    bool build(sbx_dense_plan* p, const Carve& carve) {
+        carve();
+        void* q = nullptr;
+        if (cudaMalloc(&q, used) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        p->allocs.push_back(q);
+        base = static_cast<char*>(q);
+        used = 0;
+        carve();
+        return true;
+    }
+};
+
+// the row slots, lists, snapshots and terms both shapes of the step use (each its own set)
+void step_carve(Arena& m, FusedArgs& a, int cellSlots) {
+    const size_t nS = a.nSeg, nLk = (size_t)std::max(a.nL, 1), C = a.C;
+    m.take(a.cntCell, 4 * C); m.take(a.cntSeg, 4 * C);
+    m.take(a.segCellOff, 4 * (C + 1));
+    for (int** q : {&a.cntAct, &a.cntA, &a.cntB, &a.cntM, &a.headA, &a.headB, &a.headM}) m.take(*q, 4 * nS);
+    m.take(a.cellSlot, 4 * C * cellSlots);
+    m.take(a.slotA, 4 * nS * FUSED_ROW_SLOTS); m.take(a.slotB, 4 * nS * FUSED_ROW_SLOTS);
+    m.take(a.slotM, 4 * nS * FUSED_MOTOR_SLOTS);
+    m.take(a.cellHead, 4 * C); m.take(a.cellNext, 4 * (size_t)a.cap);
+    m.take(a.nextA, 4 * nLk); m.take(a.nextB, 4 * nLk); m.take(a.nextM, 4 * (size_t)a.nM);
+    m.take(a.segE1, 16 * nS); m.take(a.segE2, 16 * nS);
+    m.take(a.joints, 2 * nS * FUSED_JOINT_BYTES);
+    m.take(a.terms, (2 * (size_t)a.nM + 4 * (size_t)a.nD) * FUSED_TERM_BYTES);
+    m.take(a.uSnap, 12 * nS);
+    m.take(a.reachMax, 4);
+    m.take(a.err, 16);
+}
+
+// empty histograms and lists, as every completed step leaves them
+void step_reset(sbx_ctx* ctx, FusedArgs& a) {
+    cudaMemsetAsync(a.cntCell, 0, 4 * (size_t)a.C, ctx->stream);
+    cudaMemsetAsync(a.cntSeg, 0, 4 * (size_t)a.C, ctx->stream);
+    for (int* q : {a.cntAct, a.cntA, a.cntB, a.cntM}) cudaMemsetAsync(q, 0, 4 * (size_t)a.nSeg, ctx->stream);
+    cudaMemsetAsync(a.cellHead, 0xff, 4 * (size_t)a.C, ctx->stream);
+    for (int* q : {a.headA, a.headB, a.headM}) cudaMemsetAsync(q, 0xff, 4 * (size_t)a.nSeg, ctx->stream);
+    cudaMemsetAsync(a.reachMax, 0, 4, ctx->stream);
+    cudaMemsetAsync(a.err, 0, 16, ctx->stream);
+}
+
+bool fused_prepare(sbx_dense_plan* p) {
+    const sbx_dense_scene& sc = p->scene;
+    cudaStream_t st = p->ctx->stream;
+    FusedArgs& a = p->fa;
+    auto why = [&](const char* w) { p->fused_why = w; return false; };
+    if (const char* w = step_layout(p, a)) return why(w);
+    int dev = 0, sms = 0, coop = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    int per = fused_max_blocks_per_sm();
+    if (!coop || per <= 0) return why("cooperative launch unavailable");
+    p->fused_grid = sms * per;
+    if (!fused_topology(p)) return false;
+    auto fc = d2h(sc.fil.counts, 4, st);
+    a.filSeed = fc[2];
+    Arena m;
+    if (!m.build(p, [&] {
+            step_carve(m, a, FUSED_CELL_SLOTS);
+            m.take(a.tileSum, 4 * (size_t)(2 * a.tilesC + 2 * a.tilesS + 1));
+            m.take(a.mTileSum, 4 * (size_t)(a.tilesS + 1));
+            m.take(a.bar, 32);
+        }))
+        return why("scratch allocation failed");
     // the error word and barrier counters are read by the plan status before any fused run
     cudaMemsetAsync(a.err, 0, 16, st);
     cudaMemsetAsync(a.bar, 0, 32, st);
     p->fused_prepared = true;
+    return true;
+}
+
+void wide_reset(sbx_dense_plan* p) {
+    const WideArgs& w = p->wide;
+    step_reset(p->ctx, p->wide.a);
+    cudaMemsetAsync(w.sumCell, 0, 4 * (size_t)WIDE_SUM_STRIDE * (2 * (size_t)w.tilesC + 3 * (size_t)w.tilesS),
+                    p->ctx->stream);
+}
+
+// The wide kernels of the graph path: any network of the harness layout, single or packed.
+bool wide_prepare(sbx_dense_plan* p) {
+    WideArgs& w = p->wide;
+    FusedArgs& a = w.a;
+    if (step_layout(p, a)) return false;
+    if (p->batched) w.bt = p->batch;
+    w.errDev = p->ctx->err_dev;
+    a.cellUse = WIDE_CELL_SLOTS;
+    w.tilesC = (a.C + WIDE_TILE - 1) / WIDE_TILE;
+    w.tilesS = (a.nSeg + WIDE_TILE - 1) / WIDE_TILE;
+    const size_t nLk = (size_t)std::max(a.nL, 1), words = WIDE_SUM_STRIDE * (2 * (size_t)w.tilesC + 3 * (size_t)w.tilesS);
+    int* sums = nullptr;
+    Arena m;
+    if (!m.build(p, [&] {
+            step_carve(m, a, WIDE_CELL_SLOTS);
+            m.take(w.payA, 24 * nLk);
+            m.take(w.payB, 24 * nLk);
+            m.take(sums, 4 * words);
+        }) || !wide_streams_create(p->wideStreams))
+        return false;
+    w.sumCell = sums;
+    w.sumSeg = w.sumCell + WIDE_SUM_STRIDE * w.tilesC;
+    w.sumA = w.sumSeg + WIDE_SUM_STRIDE * w.tilesC;
+    w.sumB = w.sumA + WIDE_SUM_STRIDE * w.tilesS;
+    w.sumM = w.sumB + WIDE_SUM_STRIDE * w.tilesS;
+    wide_reset(p);
     return true;
 }
 
@@ -633,12 +717,21 @@ static sbx_status capture_step(sbx_dense_plan* p) {
         return fail(ctx, SBX_ECUDA, "dense plan: begin capture");
     sbx_status st;
     StepNoise sn{p->noise, p->noiseErr};
-    {
+    if (p->wide_ok) {
+        FusedArgs& a = p->wide.a;
+        a.nzFil = p->noiseOn ? p->noise.fil : nullptr;
+        a.nzMot = p->noiseOn ? p->noise.mot : nullptr;
+        a.nzBb = p->noiseOn ? p->noise.bb : nullptr;
+        a.nzT0 = p->noise.t0;
+        a.nzN = p->noise.nsteps;
+        p->wide.noiseErr = p->noiseErr;
+        st = wide_step(ctx, p->wide, p->batched, p->wideStreams);
+    } else {
         PlanScratch use(p);
         st = dense_sequence(ctx, &p->scene, p->d_step, 0, p->batched ? &p->batch : nullptr, &p->side,
                             p->noiseOn ? &sn : nullptr);
     }
-    if (st == SBX_OK) SBX_LAUNCH(ctx, k_step_advance, 1, 1, p->d_step);
+    if (st == SBX_OK && !p->wide_ok) SBX_LAUNCH(ctx, k_step_advance, 1, 1, p->d_step);
     cudaGraph_t g = nullptr;
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
     if (st != SBX_OK || ce != cudaSuccess) {
@@ -708,9 +801,12 @@ static sbx_status plan_create(sbx_ctx* ctx, const sbx_dense_scene* sc, const sbx
         cudaGetLastError();
         return fail(ctx, SBX_ENOMEM, "sbx_dense_plan_create: counters");
     }
+    p->wide_ok = wide_prepare(p);
     // capture one step into a graph
     sbx_status st = capture_step(p);
     if (st != SBX_OK) {
+        wide_streams_destroy(p->wideStreams);
+        for (void* q : p->allocs) cudaFree(q);
         cudaFree(p->stats);
         cudaFree(p->d_step);
         cudaFree(p->scratch);
@@ -753,14 +849,8 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
         // the kernel leaves its histograms zeroed and its barrier words consistent at the
         // end of every completed run; they are reset here only after a failed run
         if (p->fused_dirty) {
-            FusedArgs& a = p->fa;
-            cudaMemsetAsync(a.cntCell, 0, 4 * (size_t)a.C, ctx->stream);
-            cudaMemsetAsync(a.cntSeg, 0, 4 * (size_t)a.C, ctx->stream);
-            for (int* q : {a.cntAct, a.cntA, a.cntB, a.cntM}) cudaMemsetAsync(q, 0, 4 * (size_t)a.nSeg, ctx->stream);
-            cudaMemsetAsync(a.cellHead, 0xff, 4 * (size_t)a.C, ctx->stream);
-            for (int* q : {a.headA, a.headB, a.headM}) cudaMemsetAsync(q, 0xff, 4 * (size_t)a.nSeg, ctx->stream);
-            cudaMemsetAsync(a.bar, 0, 32, ctx->stream);
-            cudaMemsetAsync(a.err, 0, 16, ctx->stream);
+            step_reset(ctx, p->fa);
+            cudaMemsetAsync(p->fa.bar, 0, 32, ctx->stream);
             p->fused_dirty = false;
         }
         SBX_TRACE("sbx.dense.fused_launch");
@@ -797,6 +887,17 @@ extern "C" sbx_status sbx_dense_plan_status(sbx_dense_plan* p, int32_t* flags) {
         if (ne) {
             cudaMemsetAsync(p->noiseErr, 0, sizeof(int), p->ctx->stream);
             return fail(p->ctx, SBX_EINVAL, "dense step: a step ran outside the supplied-noise range");
+        }
+    }
+    if (p->wide_ok) {
+        int we = 0;
+        cudaMemcpyAsync(&we, p->wide.a.err, sizeof(int), cudaMemcpyDeviceToHost, p->ctx->stream);
+        CHK(sbx_ctx_sync(p->ctx));
+        if (we) cudaMemsetAsync(p->wide.a.err, 0, 16, p->ctx->stream);
+        if (we & 8) {
+            wide_reset(p);
+            *flags = 8;
+            return fail(p->ctx, SBX_ESTATE, "graph step: a linked-list walk ran past its bound");
         }
     }
     if (!p->fused_ok) return SBX_OK;
@@ -892,13 +993,15 @@ extern "C" sbx_status sbx_dense_plan_test_caps(sbx_dense_plan* p, int32_t entCap
                                                int32_t rowSlots, int32_t cellSlots) {
     if (!p) return SBX_EINVAL;
     auto clampCap = [](int v, int cap) { return v < 0 ? cap : (v > cap ? cap : v); };
-    p->fa.entCap = clampCap(entCap, FUSED_ENT_CAP);
-    p->fa.mCap = clampCap(motorCap, FUSED_MCAP);
-    p->fa.mIds = clampCap(motorIds, FUSED_MIDS);
-    p->fa.rowUse = clampCap(rowSlots, FUSED_ROW_SLOTS);
-    p->fa.mRowUse = clampCap(rowSlots, FUSED_MOTOR_SLOTS);
-    p->fa.cellUse = clampCap(cellSlots, FUSED_CELL_SLOTS);
-    return SBX_OK;
+    for (FusedArgs* a : {&p->fa, &p->wide.a}) {
+        a->entCap = clampCap(entCap, FUSED_ENT_CAP);
+        a->mCap = clampCap(motorCap, FUSED_MCAP);
+        a->mIds = clampCap(motorIds, FUSED_MIDS);
+        a->rowUse = clampCap(rowSlots, FUSED_ROW_SLOTS);
+        a->mRowUse = clampCap(rowSlots, FUSED_MOTOR_SLOTS);
+        a->cellUse = clampCap(cellSlots, a == &p->fa ? FUSED_CELL_SLOTS : WIDE_CELL_SLOTS);
+    }
+    return p->wide_ok ? capture_step(p) : SBX_OK;      // the captured step holds its arguments
 }
 
 extern "C" sbx_status sbx_dense_plan_destroy(sbx_dense_plan* p) {
@@ -913,6 +1016,7 @@ extern "C" sbx_status sbx_dense_plan_destroy(sbx_dense_plan* p) {
     if (p->noiseErr) cudaFree(p->noiseErr);
     if (p->stats) cudaFree(p->stats);
     release_side(p);
+    wide_streams_destroy(p->wideStreams);
     for (void* q : p->allocs) cudaFree(q);
     delete p;
     return SBX_OK;

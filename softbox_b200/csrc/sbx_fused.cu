@@ -37,13 +37,15 @@
 #include "sbx_fused.cuh"
 #include "sbx_internal.cuh"
 #include "sbx_physics.cuh"
+#include "sbx_step.cuh"
 
 using namespace sbx;
 
 namespace {
 
 constexpr unsigned long long WAIT_NS = 1000000000ULL;   // barrier and bulk-copy waits give up after one second
-constexpr int ERR_BARRIER = 1, ERR_REACH_OVERFLOW = 2, ERR_TMA = 4, ERR_LIST = 8;
+
+constexpr int ERR_BARRIER = 1, ERR_TMA = 4;
 
 // shared memory of one CTA, reused by the phases
 struct RodSmem {
@@ -57,34 +59,10 @@ struct RodSmem {
     int mIds[FUSED_MAX_ROD][FUSED_MIDS];          // their slots, ascending (the first FUSED_MIDS)
     float mPay[FUSED_MAX_ROD][FUSED_MCAP][6];     // the first FUSED_MCAP bond reactions
 };
-struct MiniSmem {
-    float sF[3 * FUSED_MAX_SUB], sT[3 * FUSED_MAX_SUB];
-};
-static_assert(sizeof(ChainJoint) <= FUSED_JOINT_BYTES, "joint slot size");
-static_assert(sizeof(MotorJoint) <= FUSED_TERM_BYTES && sizeof(CoupleTerm) <= FUSED_TERM_BYTES &&
-                  sizeof(LeverTerm) <= FUSED_TERM_BYTES && sizeof(TetherTerm) <= FUSED_TERM_BYTES,
-              "myosin term slot size");
-
-// slots of the step's myosin terms (FusedArgs::terms)
-__device__ __forceinline__ MotorJoint& term_joint(const FusedArgs& a, int m, int which) {
-    return *reinterpret_cast<MotorJoint*>((char*)a.terms + ((size_t)which * a.nM + m) * FUSED_TERM_BYTES);
-}
-__device__ __forceinline__ CoupleTerm& term_couple(const FusedArgs& a, int d, int variant) {
-    return *reinterpret_cast<CoupleTerm*>((char*)a.terms + (2 * (size_t)a.nM + 2 * d + variant) * FUSED_TERM_BYTES);
-}
-__device__ __forceinline__ LeverTerm& term_lever(const FusedArgs& a, int d) {
-    return *reinterpret_cast<LeverTerm*>((char*)a.terms + (2 * (size_t)a.nM + 2 * (size_t)a.nD + d) * FUSED_TERM_BYTES);
-}
-__device__ __forceinline__ TetherTerm& term_tether(const FusedArgs& a, int d) {
-    return *reinterpret_cast<TetherTerm*>((char*)a.terms + (2 * (size_t)a.nM + 3 * (size_t)a.nD + d) * FUSED_TERM_BYTES);
-}
-
 union FusedSmem {
     RodSmem rod;
     MiniSmem mini;
 };
-
-__device__ __forceinline__ int vload(const int* p) { return *(const volatile int*)p; }
 
 __device__ __forceinline__ unsigned long long gtimer() {
     unsigned long long ns;
@@ -136,78 +114,6 @@ __device__ __forceinline__ unsigned long long counter_base(const unsigned long l
 
 __device__ __forceinline__ int gtid() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int gthreads() { return gridDim.x * blockDim.x; }
-
-// BrownianForceSystem.brownianForce (BrownianForceSystem.java:44-106), component j (0..2) of
-// one slot: the slot's j-th Box-Muller pair gives its random force and torque components j
-// (randF = ((tS * mag) * sqrt(gamma)) * g, :94-104). In supplied-noise mode the Gaussians come
-// from noise[t - t0][6][n] (a step outside the supplied range, which the host rejects before
-// the launch, draws zeros).
-__device__ __forceinline__ void brownian_component(const FusedArgs& a, const sbx_rigid_body& b, int s, int j, int t,
-                                                   int seed, float mag, const float* noise) {
-    const int n = b.n;
-    float gf, gt;
-    if (noise) {
-        int k = t - a.nzT0;
-        bool in = k >= 0 && k < a.nzN;
-        const float* q = noise + (int64_t)(in ? k : 0) * 6 * n + s;
-        gf = in ? q[(int64_t)j * n] : 0.f;
-        gt = in ? q[(int64_t)(3 + j) * n] : 0.f;
-    } else {
-        gauss_pair_wang(s, t, seed, j, &gf, &gt);
-    }
-    const float tS = b.brownTransScale[s], rS = b.brownRotScale[s];
-    b.randForce[j * n + s] = tS * mag * fsqrt(b.bTransGam[j * n + s]) * gf;
-    b.randTorque[j * n + s] = rS * mag * fsqrt(b.bRotGam[j * n + s]) * gt;
-}
-
-// ---------------------------------------------------------------- rows: slots + overflow lists
-// Rank of `self` in a row = the number of the row's items with a smaller index, counted
-// along the row's list: the position the reference's serial scatter gives it (items are
-// scattered in ascending index). A walk longer than `bound` marks the list corrupt.
-__device__ __forceinline__ int list_rank(const FusedArgs& a, int head, const int* next, int self, int bound) {
-    int r = 0, it = 0;
-    for (int j = head; j >= 0; j = next[j]) {
-        if (!SBX_IDX_OK(j, bound, CK_LIST_ENTRY)) break;
-        r += j < self;
-        if (++it > bound) {
-            atomicOr(a.err, ERR_LIST);
-            break;
-        }
-    }
-    return r;
-}
-
-// Appends `item` to row r: the histogram's old count is its arrival index; the first `use`
-// (<= S, the slot stride) arrivals take the row's fixed slots, later ones join the row's
-// overflow list (returns 1).
-__device__ __forceinline__ int row_insert(int* cnt, int* slot, int S, int use, int* head, int* next, int r,
-                                          int item) {
-    int j = atomicAdd(&cnt[r], 1);
-    if (j < use) {
-        slot[(size_t)r * S + j] = item;
-        return 0;
-    }
-    next[item] = atomicExch(&head[r], item);
-    return 1;
-}
-
-// adds a thread's count of a capacity fallback to the plan's counters
-__device__ __forceinline__ void stat_add(const FusedArgs& a, int which, int v) {
-    if (v) atomicAdd(&a.stats[which], (unsigned long long)v);
-}
-
-// rank of `item` in row r: the row's members with a smaller index (slots, then the list)
-template <int S>
-__device__ __forceinline__ int row_rank(const FusedArgs& a, const int* cnt, const int* slot, int use,
-                                        const int* head, const int* next, int r, int item, int bound) {
-    int n = cnt[r];
-    int rank = 0;
-#pragma unroll
-    for (int j = 0; j < S; j++)
-        if (j < n && j < use) rank += slot[(size_t)r * S + j] < item;
-    if (n > use) rank += list_rank(a, head[r], next, item, bound);
-    return rank;
-}
 
 // ---------------------------------------------------------------- phase A
 __device__ void phase_publish_bin(const FusedArgs& a, int t) {
@@ -323,137 +229,19 @@ __device__ void motor_brownian(const FusedArgs& a, int t, int firstWarp) {
     const int nB = a.nB, n = nB + a.nBb;
     for (int q = (w - firstWarp) * 32 + (threadIdx.x & 31); q < 3 * n; q += (nw - firstWarp) * 32) {
         const int c = q / n, j = q - c * n;
-        if (j < nB) brownian_component(a, sc.mot.body, j, c, t, sc.seed, sc.mot.bodyParams[1], a.nzMot);
-        else brownian_component(a, sc.mini.backbone, j - nB, c, t, sc.seedBb, sc.mini.bbBodyParams[1], a.nzBb);
+        if (j < nB) brownian_component(a, sc.mot.body, j, j, c, t, sc.seed, sc.mot.bodyParams[1], a.nzMot);
+        else brownian_component(a, sc.mini.backbone, j - nB, j - nB, c, t, sc.seedBb, sc.mini.bbBodyParams[1], a.nzBb);
     }
 }
 
-// The position-only terms of the myosin mechanics, none of which depends on this step's
-// binding or forces (MotorJointSystem.java:72-123 joint geometry, DimerCouplingSystem.java:
-// 99-182 end variants and lever torsion, MiniFilamentSystem tethers with their backbone
-// reaction rows), one item per term on the warps from `firstWarp` on (all warps when
-// there are none); the minifilament phase accumulates them in the reference's order.
+// The myosin terms, one item per thread on the warps from `firstWarp` on (all warps when there
+// are none); the minifilament phase accumulates them in the reference's order.
 __device__ void myosin_terms(const FusedArgs& a, int firstWarp) {
-    const sbx_dense_scene& sc = a.sc;
-    const sbx_motor_store& mot = sc.mot;
-    const sbx_rigid_body& mb = mot.body;
-    const sbx_minifilament_store& mini = sc.mini;
-    const sbx_rigid_body& bb = mini.backbone;
     int w = gtid() >> 5, nw = gthreads() >> 5;
     if (firstWarp >= nw) firstWarp = 0;
     if (w < firstWarp) return;
-    const int nM = a.nM, nD = a.nD, nB = a.nB;
-    const int total = 2 * nM + 4 * nD;
-    for (int k = (w - firstWarp) * 32 + (threadIdx.x & 31); k < total; k += (nw - firstWarp) * 32) {
-        if (k < 2 * nM) {
-            const int which = k >= nM, m = k - which * nM;
-            term_joint(a, m, which) = motor_joint(m, which, nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam,
-                                                  mb.bRotGam, mot.jointParams);
-        } else if (k < 2 * nM + 2 * nD) {
-            const int q = k - 2 * nM, d = q >> 1;
-            term_couple(a, d, q & 1) = couple_variant(nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam, mb.bRotGam,
-                                                      2 * d, 2 * d + 1, sc.dim.parallel[d] != 0, sc.dim.dimerParams,
-                                                      q & 1);
-        } else if (k < 2 * nM + 3 * nD) {
-            const int d = k - 2 * nM - 2 * nD;
-            term_lever(a, d) = couple_lever(nB, mb.uVec, mb.bRotGam, 2 * d, 2 * d + 1, sc.dim.dimerParams);
-        } else {
-            const int d = k - 2 * nM - 3 * nD, u = d / a.dpm;
-            TetherTerm T = tether_terms(nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam, mb.bRotGam, a.nBb, bb.coord,
-                                        bb.uVec, mini.bbInvDragY, u, 2 * d, mini.attachAxial[d], mini.miniParams);
-            term_tether(a, d) = T;
-            float* o = mini.miniData + (int64_t)MINI_STRIDE * d;
-            for (int j = 0; j < 6; j++) o[j] = T.row[j];
-            // backbone CSR of the reference (rows = backbones, items = dimers in index order)
-            mini.bbDimerList[d] = d;
-        }
-    }
-}
-
-// ---------------------------------------------------------------- scans (B, C, G, H)
-struct ScanArr {
-    const int* cnt;   // histogram
-    int n;            // rows
-    int tile0;        // first tile index in the shared tile-sum array
-};
-
-__device__ __forceinline__ int warp_sum(int v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__device__ void tile_sums(const ScanArr* arrs, int narr, int* tileSum, int warp, int nwarps) {
-    int lane = threadIdx.x & 31;
-    int total = arrs[narr - 1].tile0 + (arrs[narr - 1].n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    for (int tl = warp; tl < total; tl += nwarps) {
-        int ai = 0;
-        while (ai + 1 < narr && tl >= arrs[ai + 1].tile0) ai++;
-        const ScanArr& s = arrs[ai];
-        int base = (tl - s.tile0) * SCAN_CHUNK;
-        int v = 0;
-        for (int j = lane; j < SCAN_CHUNK; j += 32) v += (base + j < s.n) ? s.cnt[base + j] : 0;
-        v = warp_sum(v);
-        if (lane == 0) tileSum[tl] = v;
-    }
-}
-
-// exclusive scan of each array into out[ai][0..n] (terminator = min(total, clamp[ai]));
-// copy[ai] (optional) receives the counts — the row lengths the reference's serial
-// scatter leaves in its write cursors; chunkOut (optional, array 0) gets the tile-prefix
-// layout of SpatialGrid.gridScanChunks.
-__device__ void tile_scan(const ScanArr* arrs, int narr, const int* tileSum, int* const* out, int* const* copy,
-                          const int* clampTotal, int* chunkOut, int warp, int nwarps) {
-    int lane = threadIdx.x & 31;
-    int total = arrs[narr - 1].tile0 + (arrs[narr - 1].n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    for (int tl = warp; tl < total; tl += nwarps) {
-        int ai = 0;
-        while (ai + 1 < narr && tl >= arrs[ai + 1].tile0) ai++;
-        const ScanArr& s = arrs[ai];
-        int ntiles = (s.n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-        int local = tl - s.tile0;
-        // the preceding tiles' sums: 16 predicated loads per lane in flight together
-        int b = 0;
-#pragma unroll
-        for (int q = 0; q < 16; q++) {
-            int j = lane + 32 * q;
-            b += (j < local) ? tileSum[s.tile0 + j] : 0;
-        }
-        for (int j = lane + 512; j < local; j += 32) b += tileSum[s.tile0 + j];
-        b = warp_sum(b);
-        int base = local * SCAN_CHUNK;
-        constexpr int PER = SCAN_CHUNK / 32;
-        // coalesced: row j of the tile is elements base + 32 j + lane
-        int vals[PER];
-#pragma unroll
-        for (int j = 0; j < PER; j++) {
-            int r = base + 32 * j + lane;
-            vals[j] = r < s.n ? s.cnt[r] : 0;
-        }
-        int run = b;
-#pragma unroll
-        for (int j = 0; j < PER; j++) {
-            int v = vals[j], x = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            int r = base + 32 * j + lane;
-            if (r < s.n) {
-                out[ai][r] = run + x - v;
-                if (copy[ai]) copy[ai][r] = v;
-            }
-            run += __shfl_sync(0xffffffffu, x, 31);
-        }
-        if (lane == 0 && ai == 0 && chunkOut) chunkOut[local] = b;
-        if (local == ntiles - 1) {
-            int tot = run;
-            if (lane == 0) {
-                out[ai][s.n] = tot < clampTotal[ai] ? tot : clampTotal[ai];
-                if (ai == 0 && chunkOut) chunkOut[ntiles] = tot;
-            }
-        }
-    }
+    const int total = 2 * a.nM + 4 * a.nD;
+    for (int k = (w - firstWarp) * 32 + (threadIdx.x & 31); k < total; k += (nw - firstWarp) * 32) myosin_term(a, k);
 }
 
 // ---------------------------------------------------------------- E: stable placement
@@ -464,6 +252,7 @@ __device__ void phase_place(const FusedArgs& a) {
     const sbx_rigid_body& fb = sc.fil.body;
     const int nSeg = a.nSeg;
     int total = a.cap + (a.xlOn ? a.nL : 0);
+    float span = 0.f;
     for (int i = gtid(); i < total; i += gthreads()) {
         if (i < a.cap) {
             int c = g.bodyCell[i];
@@ -477,8 +266,15 @@ __device__ void phase_place(const FusedArgs& a) {
             if (i < nSeg && SBX_IDX_OK(a.segCellOff[c] + rank, nSeg, CK_CSR_POS)) {
                 int q = a.segCellOff[c] + rank;
                 if (g.ownerStore[i] == STORE_FILAMENT) {
-                    a.segE1[q] = make_float4(fb.end1[i], fb.end1[nSeg + i], fb.end1[2 * nSeg + i], __int_as_float(i));
-                    a.segE2[q] = make_float4(fb.end2[i], fb.end2[nSeg + i], fb.end2[2 * nSeg + i], 0.f);
+                    float c3[3], e1[3], e2[3];
+                    for (int k = 0; k < 3; k++) {
+                        c3[k] = g.center[k * a.cap + i];
+                        e1[k] = fb.end1[k * nSeg + i];
+                        e2[k] = fb.end2[k * nSeg + i];
+                    }
+                    span = fmaxf(span, segment_span(c3, e1, e2));
+                    a.segE1[q] = make_float4(e1[0], e1[1], e1[2], __int_as_float(i));
+                    a.segE2[q] = make_float4(e2[0], e2[1], e2[2], 0.f);
                 } else {
                     a.segE1[q] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
                     a.segE2[q] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -496,121 +292,11 @@ __device__ void phase_place(const FusedArgs& a) {
                            row_rank<FUSED_ROW_SLOTS>(a, a.cntB, a.slotB, a.rowUse, a.headB, a.nextB, lb, k, a.nL)] = k;
         }
     }
+    __syncwarp();
+    span_max(a.reachMax, span);
 }
 
 // ---------------------------------------------------------------- F: minifilaments + links
-// BindingDetectionSystem.gridReachable (BindingDetectionSystem.java:161-227) over the
-// segment-only cell-ordered endpoints, fused with bindNearest's selection
-// (BindingDetectionSystem.java:366-388): the same 27 cells in the same order (nine rows of
-// three consecutive x-cells), the same predicate, and the first nearest among the first
-// MAX_CAND candidates. A group of W lanes (8 or 16) walks one head (the 32 / W groups of a
-// warp walk as many heads side by side; every lane of a group calls it with its group's
-// head, `valid` false for a group without one): lane r of the group reads stencil row r's
-// range (with 8 lanes, lane 0 also row 8), then the entries are tested W at a time, lane k
-// of the group taking entry k0 + k. Passing entries are appended in entry order (ballot,
-// and the popcount of the group's lower lanes' passes), so the list is the serial walk's
-// list; the nearest of the first MAX_CAND (strict <, the first in list order wins) is the
-// serial choice: a chunk's minimum with ties to its lowest lane replaces the running best
-// only when strictly smaller. Every group runs the same number of chunks (the longest
-// walk's), so every shuffle has the whole warp. Returns the reach count; best and arc are
-// the same on every lane of the group.
-template <int W>
-__device__ int group_reach_bind(const FusedArgs& a, int lane, bool valid, float mx, float my, float mz, float mux,
-                                float muy, float muz, float rux, float ruy, float ruz, int* out, float tol,
-                                float align, int* bestSeg, float* bestArc) {
-    static_assert(W == 8 || W == 16, "a group of 8 or 16 lanes walks one head");
-    const float* gp = a.sc.grid.gridParams;
-    const int* off = a.segCellOff;
-    const int hl = lane & (W - 1), grp = lane / W;
-    const int nX = a.nX, nY = a.nY, nZ = a.nZ, nXY = nX * nY;
-    const int cx = cell_coord(mx, gp[0], gp[4], nX), cy = cell_coord(my, gp[1], gp[4], nY),
-              cz = cell_coord(mz, gp[2], gp[4], nZ);
-    const int x0 = max(cx - 1, 0), x1 = min(cx + 1, nX - 1);
-    // lane hl reads stencil row hl; with 8 lanes, lane 0 also reads row 8
-    int rs = 0, len = 0, rs8 = 0, len8 = 0;
-    auto row = [&](int r, int& s, int& l) {
-        int zz = cz - 1 + r / 3, yy = cy - 1 + r % 3;
-        if (zz >= 0 && zz < nZ && yy >= 0 && yy < nY) {
-            int c0 = x0 + yy * nX + zz * nXY;
-            s = off[c0];
-            l = off[c0 + (x1 - x0) + 1] - s;
-        }
-    };
-    if (valid && hl < 9) row(hl, rs, len);
-    if (W == 8 && valid && hl == 0) row(8, rs8, len8);
-    int inc = len;
-#pragma unroll
-    for (int o = 1; o < W; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, inc, o, W);
-        if (hl >= o) inc += y;
-    }
-    const int lanesTotal = __shfl_sync(0xffffffffu, inc, W - 1, W);     // rows 0 .. min(8, W - 1)
-    const int total = lanesTotal + (W == 8 ? __shfl_sync(0xffffffffu, len8, 0, W) : 0);
-    int totalMax = total;
-#pragma unroll
-    for (int o = W; o < 32; o <<= 1) totalMax = max(totalMax, __shfl_xor_sync(0xffffffffu, totalMax, o));
-    // every lane holds its group's nine (start of row in the sequence, start of row in memory) pairs
-    int preR[9], rsR[9];
-#pragma unroll
-    for (int r = 0; r < 9; r++) {
-        if (r < W) {
-            preR[r] = __shfl_sync(0xffffffffu, inc - len, r, W);
-            rsR[r] = __shfl_sync(0xffffffffu, rs, r, W);
-        } else {
-            preR[r] = lanesTotal;
-            rsR[r] = __shfl_sync(0xffffffffu, rs8, 0, W);
-        }
-    }
-    const unsigned lower = (1u << hl) - 1u;
-    int cnt = 0, best = -1;
-    float bestD = 1.0e30f, arc = 0.f;
-    for (int k0 = 0; k0 < totalMax; k0 += W) {
-        const int k = k0 + hl;
-        bool pass = false;
-        float d = 0.f;
-        float4 e1 = make_float4(0.f, 0.f, 0.f, 0.f), e2 = e1;
-        if (k < total) {
-            int idx = rsR[0] + k;
-#pragma unroll
-            for (int r = 1; r < 9; r++)
-                if (k >= preR[r]) idx = rsR[r] + (k - preR[r]);
-            if (SBX_IDX_OK(idx, a.nSeg, CK_REACH_ENTRY)) {
-                e1 = a.segE1[idx];
-                e2 = a.segE2[idx];
-                d = reach_test_dist_sq(mx, my, mz, mux, muy, muz, rux, ruy, ruz, e1.x, e1.y, e1.z, e2.x, e2.y, e2.z,
-                                       tol, align);
-                pass = d >= 0.f && __float_as_int(e1.w) >= 0;
-            }
-        }
-        const unsigned mask = (__ballot_sync(0xffffffffu, pass) >> (W * grp)) & ((1u << W) - 1u);
-        const int pos = cnt + __popc(mask & lower);
-        const int sg = __float_as_int(e1.w);
-        const bool elig = pass && pos < MAX_CAND;
-        if (elig) out[pos] = sg;
-        float v = elig ? d : 3.0e38f;
-        int who = hl;
-#pragma unroll
-        for (int o = W / 2; o > 0; o >>= 1) {
-            float ov = __shfl_xor_sync(0xffffffffu, v, o);
-            int ow = __shfl_xor_sync(0xffffffffu, who, o);
-            if (ov < v || (ov == v && ow < who)) { v = ov; who = ow; }
-        }
-        float myArc = 0.f;
-        if (v < bestD && hl == who) myArc = bind_arc(mx, my, mz, e1.x, e1.y, e1.z, e2.x, e2.y, e2.z);
-        const int bw = __shfl_sync(0xffffffffu, sg, who, W);
-        const float ba = __shfl_sync(0xffffffffu, myArc, who, W);
-        if (v < bestD) {
-            bestD = v;
-            best = bw;
-            arc = ba;
-        }
-        cnt += __popc(mask);
-    }
-    *bestSeg = best;
-    *bestArc = arc;
-    return cnt;
-}
-
 // BindingDetectionSystem / NucleotideCycleSystem for every head: the
 // catch-slip release (NucleotideCycleSystem.java:77-134), the reach walk fused with
 // bindNearest's choice (BindingDetectionSystem.java:161-227, :366-388), the nucleotide cycle
@@ -626,6 +312,7 @@ __device__ void phase_bind(const FusedArgs& a, int t) {
     const float* kp = mot.kinParams;
     const int lane = threadIdx.x & 31, gw = gtid() >> 5, nw = gthreads() >> 5;
     const int nM = a.nM;
+    const GridView gv{sc.grid.gridParams, a.nX, a.nY, a.nZ, a.segCellOff};
     int listed = 0;
     for (int base = gw; base < nM; base += 32 * nw) {
         const int myM = base + lane * nw;
@@ -647,7 +334,7 @@ __device__ void phase_bind(const FusedArgs& a, int t) {
             float rux = mot.rodUVec[mm], ruy = mot.rodUVec[nM + mm], ruz = mot.rodUVec[2 * nM + mm];
             int best;
             float arc;
-            int rc = group_reach_bind<BIND_W>(a, lane, valid, mx, my, mz, mux, muy, muz, rux, ruy, ruz,
+            int rc = group_reach_bind<BIND_W>(a, gv, lane, valid, mx, my, mz, mux, muy, muz, rux, ruy, ruz,
                                      sc.grid.reachSeg + (int64_t)mm * MAX_CAND, kp[7], kp[8], &best, &arc);
             if ((lane & (BIND_W - 1)) == 0 && valid) {
                 sc.grid.reachCount[m] = rc;
@@ -678,114 +365,6 @@ __device__ void phase_bind(const FusedArgs& a, int t) {
     stat_add(a, ST_MOTOR_LIST, listed);
 }
 
-// One minifilament per CTA (its heads' binding and its position-only terms ran in earlier
-// phases). Stage 2: each sub-body accumulates its terms in the order of the reference's
-// System sequence (joints, coupling, tether; the head's bond after its joint). Stage 3:
-// integrate.
-__device__ void mini_unit(const FusedArgs& a, MiniSmem& ms, int u, int t) {
-    const sbx_dense_scene& sc = a.sc;
-    const sbx_motor_store& mot = sc.mot;
-    const sbx_rigid_body& mb = mot.body;
-    const sbx_minifilament_store& mini = sc.mini;
-    const sbx_rigid_body& bb = mini.backbone;
-    const sbx_rigid_body& fb = sc.fil.body;
-    const int nB = a.nB, nSeg = a.nSeg, nBb = a.nBb;
-    const int dpm = a.dpm, mpm = 2 * dpm, spm = 6 * dpm;
-    const int m0 = u * mpm, s0 = u * spm, d0 = u * dpm;
-    const int tid = threadIdx.x;
-    float* sF = ms.sF;
-    float* sT = ms.sT;
-    LocalAcc acc{sF, sT, s0, spm};
-
-    // ---- stage 2
-    if (tid < 32) {
-        if (tid < mpm) {
-            // CrossBridgeSystem.bondForces, then the head's sums: joint 1, then the bond
-            int m = m0 + tid;
-            float out[XB_STRIDE];
-            int bs = mot.boundSeg[m];
-            if (!SBX_IDX_OK_OR_NONE(bs, nSeg, CK_BOUND_SEG)) bs = -1;
-            bond_one(m, nB, mb.coord, mb.uVec, mb.yVec, mb.bRotGam, nSeg, fb.coord, fb.uVec, fb.yVec, fb.bRotGam,
-                     fb.segLength, bs, mot.bindArc[m], mot.nucleotideState[m], sc.xbParams, out);
-            for (int k = 0; k < XB_STRIDE; k++) sc.bondData[m * XB_STRIDE + k] = out[k];
-            int hl = 3 * tid + 2;
-            double f[3] = {0.0, 0.0, 0.0}, tq[3] = {0.0, 0.0, 0.0};
-            motor_joint_apply(term_joint(a, m, 1), 1, true, mot.nucleotideState[m], s0 + hl, nB, mb.uVec,
-                              mb.segLength, mot.jointParams, f, tq);
-            for (int k = 0; k < 3; k++) {
-                float F = (float)(0.0 + f[k]), T = (float)(0.0 + tq[k]);
-                sF[k * spm + hl] = F + out[k];
-                sT[k * spm + hl] = T + out[3 + k];
-            }
-        }
-    } else {
-        int w = tid - 32;
-        if (w < 2 * mpm) {
-            // rods (role 0) and levers (role 1): joints, then dimer coupling, then the tether
-            int ml = w >> 1, role = w & 1;
-            int m = m0 + ml, sl = 3 * ml + role, s = s0 + sl;
-            int nuc = mot.nucleotideState[m];
-            double f[3] = {0.0, 0.0, 0.0}, tq[3] = {0.0, 0.0, 0.0};
-            if (role == 0) {
-                motor_joint_apply(term_joint(a, m, 0), 0, false, nuc, s, nB, mb.uVec, mb.segLength, mot.jointParams, f,
-                                  tq);
-            } else {
-                motor_joint_apply(term_joint(a, m, 0), 0, true, nuc, s, nB, mb.uVec, mb.segLength, mot.jointParams, f,
-                                  tq);
-                motor_joint_apply(term_joint(a, m, 1), 1, false, nuc, s, nB, mb.uVec, mb.segLength, mot.jointParams, f,
-                                  tq);
-            }
-            for (int k = 0; k < 3; k++) {
-                sF[k * spm + sl] = (float)(0.0 + f[k]);
-                sT[k * spm + sl] = (float)(0.0 + tq[k]);
-            }
-            int dl = ml >> 1, d = d0 + dl;
-            bool isA = (ml & 1) == 0;            // motorA = 2d, motorB = 2d + 1
-            if (role == 0) {
-                couple_apply_rod(acc, s, isA, term_couple(a, d, 0));
-                couple_apply_rod(acc, s, isA, term_couple(a, d, 1));
-                if (isA) tether_apply(acc, s, term_tether(a, d));
-            } else {
-                bool bothBound = mot.boundSeg[2 * d] >= 0 && mot.boundSeg[2 * d + 1] >= 0;
-                if (sc.dim.parallel[d] != 0 && !bothBound) couple_apply_lever(acc, s, isA, term_lever(a, d));
-            }
-        } else if (w == 2 * mpm) {
-            // the backbone: gather its dimers' reactions, confine, integrate, derive
-            mini.bbDimerCount[u] = dpm;
-            mini.bbDimerOffsets[u] = d0;
-            if (u == nBb - 1) mini.bbDimerOffsets[nBb] = d0 + dpm;
-            // MiniFilamentSystem.backboneGather over this backbone's CSR row (its dimers, ascending)
-            double f[3] = {0, 0, 0}, tq[3] = {0, 0, 0};
-            for (int d = d0; d < d0 + dpm; d++) {
-                const float* p = mini.miniData + (int64_t)d * MINI_STRIDE;
-                f[0] += p[0]; f[1] += p[1]; f[2] += p[2];
-                tq[0] += p[3]; tq[1] += p[4]; tq[2] += p[5];
-            }
-            float F[3], T[3];
-            for (int k = 0; k < 3; k++) { F[k] = (float)(0.0f + f[k]); T[k] = (float)(0.0f + tq[k]); }
-            BoxParams bx = box_params(sc.boxParams, t);
-            float c[3] = {bb.coord[u], bb.coord[nBb + u], bb.coord[2 * nBb + u]};
-            float uu[3] = {bb.uVec[u], bb.uVec[nBb + u], bb.uVec[2 * nBb + u]};
-            if (bx.active) confine_one(bx, c, uu, bb.segLength[u], bb.bTransGam[u], F, T);
-            integrate_derive_store(bb, u, F, T, mini.bbBodyParams[0]);
-        }
-    }
-    __syncthreads();
-    // ---- stage 3: integrate + derive the sub-bodies; force-dot registry
-    if (tid < spm) {
-        int s = s0 + tid;
-        float F[3] = {sF[tid], sF[spm + tid], sF[2 * spm + tid]};
-        float T[3] = {sT[tid], sT[spm + tid], sT[2 * spm + tid]};
-        integrate_derive_store(mb, s, F, T, mot.bodyParams[0]);
-    }
-    if (tid < mpm) {
-        int m = m0 + tid;
-        register_force_dot_one(m, sc.bondData, mot.boundSeg[m] >= 0, mot.forceDotFil, mot.forceMag,
-                               mot.forceDotHist, mot.forceDotPlace);
-    }
-    __syncthreads();
-}
-
 __device__ void link_item(const FusedArgs& a, int k) {
     const sbx_dense_scene& sc = a.sc;
     const sbx_crosslinker_store& xl = sc.xl;
@@ -806,7 +385,11 @@ __device__ void phase_motors_links(const FusedArgs& a, FusedSmem& sm, int t) {
     int units = a.nBb + linkChunks;
     for (int w = blockIdx.x; w < units; w += gridDim.x) {
         if (w < a.nBb) {
-            mini_unit(a, sm.mini, w, t);
+            // the sub-bodies on three warps, the backbone on the fourth
+            if (threadIdx.x < 96) mini_bodies(a, sm.mini, w, GlobalTerms{a});
+            else if (threadIdx.x == 96)
+                mini_backbone(a, w, t, GlobalTerms{a}, a.sc.boxParams, a.sc.mini.bbBodyParams[0]);
+            __syncthreads();
         } else {
             int k = (w - a.nBb) * blockDim.x + threadIdx.x;
             if (k < a.nL) link_item(a, k);
@@ -853,7 +436,7 @@ __device__ void phase_motors_links(const FusedArgs& a, FusedSmem& sm, int t) {
                 }
             } else {
                 const int r = q - nJ, c = r / n, i = r - c * n;
-                brownian_component(a, fb, i, c, t, a.filSeed, fs.params[1], a.nzFil);
+                brownian_component(a, fb, i, i, c, t, a.filSeed, fs.params[1], a.nzFil);
             }
         }
     }
@@ -1218,6 +801,7 @@ __device__ bool phase_rods(const FusedArgs& a, FusedSmem& sm, int t, uint64_t* m
         if (!rod_unit(a, sm.rod, u, t, mbar, phase)) return false;
     if ((int)blockIdx.x >= a.kHelp0) motor_csr(a, blockIdx.x - a.kHelp0, gridDim.x - a.kHelp0, hTarget);
     // reset the histograms and lists of this step's grid and link CSRs for the next step
+    if (gtid() == 0) *a.reachMax = 0;
     for (int i = gtid(); i < a.C; i += gthreads()) { a.cntCell[i] = 0; a.cntSeg[i] = 0; a.cellHead[i] = -1; }
     for (int i = gtid(); i < a.nSeg; i += gthreads()) {
         a.cntAct[i] = 0; a.cntA[i] = 0; a.cntB[i] = 0; a.headA[i] = -1; a.headB[i] = -1;

@@ -875,9 +875,10 @@ SBX_DEV void link_forces_one(int k, int nSeg, const float* fC, const float* fU, 
     out[9] = (float)TBx; out[10] = (float)TBy; out[11] = (float)TBz;
 }
 
-// CrosslinkerSystem.linkTorsion per link (CrosslinkerSystem.java:777-806); adds into xd row k
-SBX_DEV void link_torsion_one(int k, int nSeg, const float* fU, int a, int b, int state, int orient, float* hist,
-                              int* place, float* xd, double spring) {
+// CrosslinkerSystem.linkTorsion per link (CrosslinkerSystem.java:777-806); adds into the link's
+// payload row r
+SBX_DEV void link_torsion_row(int k, int nSeg, const float* fU, int a, int b, int state, int orient, float* hist,
+                              int* place, float* r, double spring) {
     if (state < 0) return;
     if (a < 0 || b < 0) return;
     double uax = fU[a], uay = fU[nSeg + a], uaz = fU[2 * nSeg + a];
@@ -902,13 +903,17 @@ SBX_DEV void link_torsion_one(int k, int nSeg, const float* fU, int a, int b, in
     for (int j = 0; j < TORQUE_WIN; j++) avg += hist[base + j];
     avg /= TORQUE_WIN;
     double Tx = avg * tx, Ty = avg * ty, Tz = avg * tz;
-    float* r = xd + (int64_t)k * XL_STRIDE;
     r[3] = (float)(r[3] + Tx);
     r[4] = (float)(r[4] + Ty);
     r[5] = (float)(r[5] + Tz);
     r[9] = (float)(r[9] - Tx);
     r[10] = (float)(r[10] - Ty);
     r[11] = (float)(r[11] - Tz);
+}
+
+SBX_DEV void link_torsion_one(int k, int nSeg, const float* fU, int a, int b, int state, int orient, float* hist,
+                              int* place, float* xd, double spring) {
+    link_torsion_row(k, nSeg, fU, a, b, state, orient, hist, place, xd + (int64_t)k * XL_STRIDE, spring);
 }
 
 // CrosslinkerSystem.unbind per ACTIVE link (CrosslinkerSystem.java:245-280); true = break
@@ -1265,37 +1270,52 @@ SBX_DEV void tether_one(int d, int nMB, const float* mC, const float* mU, const 
     for (int k = 0; k < 6; k++) o[k] = T.row[k];
 }
 
-// integrate + derive one body slot from accumulated F/T (registers), the slot's stored
-// Brownian draws and drag, then store pose, derived geometry and the final F/T sums
-// (MechanicsFusion.integDerive, MechanicsFusion.java:129-200)
-SBX_DEV void integrate_derive_store(const sbx_rigid_body& b, int s, const float F[3], const float T[3], float dt) {
+// What the integration of one body slot reads: pose, the slot's stored Brownian draws and drag.
+struct BodyIn {
+    Pose p;
+    float rf[3], rt[3], gT[3], gR[3], len;
+    double c64[3];
+};
+
+// every input read up front, so that the loads are in flight together
+SBX_DEV BodyIn body_load(const sbx_rigid_body& b, int s) {
     const int n = b.n;
-    Pose p, q;
-    float rf[3], rt[3], gT[3], gR[3], dc[3];
-    // every input read up front, so that the loads are in flight together
-    double c64[3] = {0.0, 0.0, 0.0};
+    BodyIn i;
     for (int k = 0; k < 3; k++) {
-        p.c[k] = b.coord[k * n + s]; p.u[k] = b.uVec[k * n + s]; p.y[k] = b.yVec[k * n + s];
-        rf[k] = b.randForce[k * n + s]; rt[k] = b.randTorque[k * n + s];
-        gT[k] = b.bTransGam[k * n + s]; gR[k] = b.bRotGam[k * n + s];
-        if (b.coord64) c64[k] = b.coord64[k * n + s];
+        i.p.c[k] = b.coord[k * n + s]; i.p.u[k] = b.uVec[k * n + s]; i.p.y[k] = b.yVec[k * n + s];
+        i.rf[k] = b.randForce[k * n + s]; i.rt[k] = b.randTorque[k * n + s];
+        i.gT[k] = b.bTransGam[k * n + s]; i.gR[k] = b.bRotGam[k * n + s];
+        i.c64[k] = b.coord64 ? b.coord64[k * n + s] : 0.0;
     }
-    const float len = b.segLength[s];
-    integrate_pose(p, F, T, rf, rt, gT, gR, dt, q, dc);
+    i.len = b.segLength[s];
+    return i;
+}
+
+// integrate + derive one body slot from accumulated F/T (registers), then store pose, derived
+// geometry and the final F/T sums (MechanicsFusion.integDerive, MechanicsFusion.java:129-200)
+SBX_DEV void body_step(const sbx_rigid_body& b, int s, const BodyIn& i, const float F[3], const float T[3], float dt) {
+    const int n = b.n;
+    Pose q;
+    float dc[3];
+    integrate_pose(i.p, F, T, i.rf, i.rt, i.gT, i.gR, dt, q, dc);
     if (b.coord64) {
         for (int k = 0; k < 3; k++) {
-            double c = c64[k] + (double)dc[k];
+            double c = i.c64[k] + (double)dc[k];
             b.coord64[k * n + s] = c;
             q.c[k] = (float)c;
         }
     }
     float z[3], e1[3], e2[3];
-    derive_pose(q.c, q.u, q.y, z, e1, e2, len);
+    derive_pose(q.c, q.u, q.y, z, e1, e2, i.len);
     for (int k = 0; k < 3; k++) {
         b.coord[k * n + s] = q.c[k]; b.uVec[k * n + s] = q.u[k]; b.yVec[k * n + s] = q.y[k];
         b.zVec[k * n + s] = z[k]; b.end1[k * n + s] = e1[k]; b.end2[k * n + s] = e2[k];
         b.forceSum[k * n + s] = F[k]; b.torqueSum[k * n + s] = T[k];
     }
+}
+
+SBX_DEV void integrate_derive_store(const sbx_rigid_body& b, int s, const float F[3], const float T[3], float dt) {
+    body_step(b, s, body_load(b, s), F, T, dt);
 }
 
 }  // namespace sbx

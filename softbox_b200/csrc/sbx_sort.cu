@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include "sbx_internal.cuh"
+#include "sbx_scan.cuh"
 
 namespace {
 
@@ -39,35 +40,6 @@ __global__ void k_cs_hist(const int* keys, const int* nDev, int useDevN, int nBo
         int c = keys[i];
         if (key_ok(c, nRows, errFlag)) atomicAdd(&rowCount[c], 1);
     }
-}
-
-// block-wide exclusive scan of one int per thread; returns the exclusive prefix, *total = sum
-template <int NT>
-__device__ __forceinline__ int block_exclusive_scan(int v, int* total) {
-    __shared__ int warp_sums[NT / 32];
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        int w = (lane < NT / 32) ? warp_sums[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        if (lane < NT / 32) warp_sums[lane] = w;
-    }
-    __syncthreads();
-    int warp_prefix = warp > 0 ? warp_sums[warp - 1] : 0;
-    *total = warp_sums[NT / 32 - 1];
-    __syncthreads();
-    return warp_prefix + x - v;
 }
 
 // SpatialGrid.gridScanLocal (SpatialGrid.java:99-117), one block per 512-row tile
@@ -117,11 +89,6 @@ __global__ void __launch_bounds__(1024) k_scan_chunks(int* chunkSum, int numChun
 // inter-block wait), scans its tile through shared memory and writes offsets, the chunk
 // prefixes chunkSum[c] (chunkSum[numChunks] = the total), offsets[nRows] = min(total, listCap),
 // and resets the counts to zero (the scatter cursor).
-constexpr int SCAN_TILE_ROWS = 8 * SCAN_CHUNK;
-constexpr int TILE_PER_THREAD = SCAN_TILE_ROWS / 256;
-
-__device__ __forceinline__ int tile_slot(int r) { return r + (r >> 5); }     // padded: no bank conflicts
-
 __global__ void __launch_bounds__(256) k_tile_reduce(const int* rowCount, int nRows, int* tileSum) {
     const int base = blockIdx.x * SCAN_TILE_ROWS;
     int s = 0;

@@ -106,6 +106,7 @@ extern "C" int64_t sbx_ctx_scratch_bytes(sbx_ctx* ctx) { return ctx ? (int64_t)c
 #ifdef SBX_CHECK
 extern "C" int sbx_check_collect_systems(unsigned long long*, unsigned long long*, int);
 extern "C" int sbx_check_collect_fused(unsigned long long*, unsigned long long*, int);
+extern "C" int sbx_check_collect_wide(unsigned long long*, unsigned long long*, int);
 #endif
 
 extern "C" int32_t sbx_check_build(void) {
@@ -124,7 +125,8 @@ extern "C" sbx_status sbx_check_report(int64_t* count, int32_t* site, int64_t* i
 #ifdef SBX_CHECK
     // the translation units with checked kernels, each with its own counters
     int (*collect[])(unsigned long long*, unsigned long long*, int) = {sbx_check_collect_systems,
-                                                                      sbx_check_collect_fused};
+                                                                      sbx_check_collect_fused,
+                                                                      sbx_check_collect_wide};
     for (auto fn : collect) {
         unsigned long long c = 0, f = 0;
         if (fn(&c, &f, reset) != 0) return SBX_ECUDA;

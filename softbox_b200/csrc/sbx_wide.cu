@@ -1,0 +1,756 @@
+// sbx_wide.cu — the dense contractile step (DenseContractileHarness.cpuStep,
+// DenseContractileHarness.java:350-429) as fourteen wide kernels, single or packed networks.
+//
+//   main stream                                    ahead         link               csr
+//   publish: body view, cells, row slots           draws         rows, unbinding
+//   scan: cell offsets                             myosin terms  scan
+//   place: contents, endpoints in cell order       joints        forces, lists
+//   bind: release, reach, nearest, cycle
+//   mini: one block a minifilament  <- draws, terms                                 scan
+//   rods: gathers, walls, integrate <- joints, link                                 lists
+//
+// The per-system sequence (sbx_dense.cu: dense_sequence) takes 53 launches: five counting sorts
+// of five kernels and many kernels of 3-5 us each, in a row. Here the inverse maps are made as
+// the fused kernel makes them (fixed slots per row filled by atomics, placed by rank), what
+// needs only the step's start view runs beside the grid, a minifilament is one block's work, and
+// what a later kernel reads again is written once.
+// Every slot is computed by the same device functions as the per-system kernels, in the
+// reference's accumulation order: the same bits.
+// A step takes 105 us at 100,000 rods and 375 us at 500,000 (200 and 434 as the per-system
+// sequence), a packed step of 12 networks (0.17e6 rods, 0.18e6 heads) 280 us (366).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "../../include/softbox_b200.h"
+#include "sbx_scan.cuh"
+#include "sbx_step.cuh"
+#include "sbx_trace.h"
+#include "sbx_wide.cuh"
+
+namespace {
+
+// network and local index of an item in packed networks (a single network: 0 and the index)
+template <bool B>
+__device__ __forceinline__ int2 key_of(const int* key, int i) {
+    return B ? make_int2(key[2 * i], key[2 * i + 1]) : make_int2(0, i);
+}
+
+template <bool B>
+__device__ __forceinline__ GridView grid_view(const WideArgs& w, int net) {
+    const sbx_grid_state& g = w.a.sc.grid;
+    if (B) {
+        const int* gd = w.bt.gridDims + 4 * net;
+        return GridView{w.bt.gridParams + 6 * net, gd[0], gd[1], gd[2], w.a.segCellOff + gd[3]};
+    }
+    return GridView{g.gridParams, g.gridDims[0], g.gridDims[1], g.gridDims[2], w.a.segCellOff};
+}
+
+// a link end names a rod; one at or past the rod count is left out and reported
+__device__ __forceinline__ bool end_ok(const WideArgs& w, int s) {
+    if (s < 0) return false;
+    if (SBX_IDX_OK(s, w.a.nSeg, CK_LINK_END) && s < w.a.nSeg) return true;
+    if (w.errDev) *(volatile int*)w.errDev = 1;
+    return false;
+}
+
+// one addition per distinct tile of a warp: tile sums[tile] += the warp's items of that tile
+__device__ __forceinline__ void tile_add(int* sums, int tile) {
+    const unsigned same = __match_any_sync(0xffffffffu, tile);
+    if (tile >= 0 && (int)(threadIdx.x & 31) == __ffs(same) - 1)
+        atomicAdd(&sums[tile * WIDE_SUM_STRIDE], __popc(same));
+}
+
+// ---------------------------------------------------------------- ahead: draws and joints
+// What depends only on the step's start poses and the step index. The Brownian forces of every
+// body (BrownianForceSystem.java:44-106), one body a thread: its three Box-Muller pairs are
+// independent chains of FP64 operations.
+template <bool B>
+__global__ void __launch_bounds__(256) k_wide_draws(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_dense_scene& sc = a.sc;
+    const int nB = a.nB, nBb = a.nBb;
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= nB + nBb + a.nSeg) return;
+    const int t = *a.d_step;
+    if (j == 0 && a.nzFil && w.noiseErr && (t < a.nzT0 || t >= a.nzT0 + a.nzN)) atomicOr(w.noiseErr, 1);
+    const sbx_rigid_body* b;
+    const float* noise;
+    int i, key, seed;
+    float mag;
+    if (j < nB) {
+        b = &sc.mot.body;
+        i = j;
+        const int m = j / 3;
+        const int2 k = key_of<B>(w.bt.motKey, m);
+        key = 3 * k.y + (j - 3 * m);
+        seed = B ? w.bt.seeds[3 * k.x] : sc.seed;
+        mag = sc.mot.bodyParams[1];
+        noise = a.nzMot;
+    } else if (j < nB + nBb) {
+        b = &sc.mini.backbone;
+        i = j - nB;
+        const int2 k = key_of<B>(w.bt.bbKey, i);
+        key = k.y;
+        seed = B ? w.bt.seeds[3 * k.x + 1] : sc.seedBb;
+        mag = sc.mini.bbBodyParams[1];
+        noise = a.nzBb;
+    } else {
+        b = &sc.fil.body;
+        i = j - nB - nBb;
+        const int2 k = key_of<B>(w.bt.segKey, i);
+        key = k.y;
+        seed = B ? w.bt.seeds[3 * k.x + 2] : sc.fil.counts[2];
+        mag = sc.fil.params[1];
+        noise = a.nzFil;
+    }
+    const int n = b->n;
+    float g[6];
+    if (noise) {
+        const int s = t - a.nzT0;
+        const bool in = s >= 0 && s < a.nzN;
+        const float* q = noise + (int64_t)(in ? s : 0) * 6 * n + i;
+        for (int k = 0; k < 6; k++) g[k] = in ? q[(int64_t)k * n] : 0.f;
+    } else {
+        gauss6_wang(key, t, seed, g);
+    }
+    float gT[3], gR[3], rf[3], rt[3];
+    for (int k = 0; k < 3; k++) { gT[k] = b->bTransGam[k * n + i]; gR[k] = b->bRotGam[k * n + i]; }
+    brownian_amplitudes(g, b->brownTransScale[i], b->brownRotScale[i], mag, gT, gR, rf, rt);
+    for (int k = 0; k < 3; k++) { b->randForce[k * n + i] = rf[k]; b->randTorque[k * n + i] = rt[k]; }
+}
+
+// the chain joints, each by its lower-slot rod (as k_chain)
+__global__ void __launch_bounds__(128, 5) k_wide_joints(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_filament_store& fs = a.sc.fil;
+    const sbx_rigid_body& fb = fs.body;
+    const int n = a.nSeg, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    int s2 = fs.end2NbrSlot[i], s1 = fs.end1NbrSlot[i];
+    if (!SBX_IDX_OK_OR_NONE(s2, n, CK_NEIGHBOUR)) s2 = -1;
+    if (!SBX_IDX_OK_OR_NONE(s1, n, CK_NEIGHBOUR)) s1 = -1;
+    ChainJoint* J = reinterpret_cast<ChainJoint*>(a.joints);
+    const ChainParams cp = chain_params(fs.chainParams);
+    for (int side = 0; side < 2; side++) {
+        const int nb = side == 0 ? s2 : s1;
+        if (nb <= i) continue;
+        J[2 * (int64_t)i + side] =
+            chain_joint(cp, i, side, nb, side == 0 ? fs.end2NbrSide[i] : fs.end1NbrSide[i],
+                        load_rod(n, i, fb.coord, fb.uVec, fb.segLength, fb.bTransGam, fb.bRotGam),
+                        load_rod(n, nb, fb.coord, fb.uVec, fb.segLength, fb.bTransGam, fb.bRotGam));
+    }
+}
+
+// ---------------------------------------------------------------- publish
+// The body view, the cells with their row slots and tile sums, the start view's orientations
+// (the rods kernel reads a neighbour from the start view: its own block may have stepped it
+// already) and the step's counts.
+template <bool B>
+__global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_dense_scene& sc = a.sc;
+    const sbx_grid_state& g = sc.grid;
+    const int nSeg = a.nSeg, nM = a.nM, nB = a.nB, cap = a.cap;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        const int t = *a.d_step;
+        int* mc = sc.mot.counts; mc[0] = nM; mc[1] = t; mc[2] = sc.seed; mc[3] = nSeg;
+        int* bc = sc.mini.bbCounts; bc[0] = a.nBb; bc[1] = t; bc[2] = sc.seedBb; bc[3] = a.nBb;
+        sc.fil.counts[1] = t;
+        if (a.xlOn) { sc.xl.counts[1] = t; sc.xl.counts[2] = sc.seed; }
+    }
+    int cell = -1;
+    if (i < nSeg + nM) {
+        float c[3];
+        int net;
+        if (i < nSeg) {
+            const sbx_rigid_body& fb = sc.fil.body;
+            const int* state = sc.fil.filState;              // FREE (< 0) slots of turnover, or none
+            // (all loads before the first store: nothing tells the compiler that they differ)
+            float u[3];
+            for (int k = 0; k < 3; k++) { c[k] = fb.coord[k * nSeg + i]; u[k] = fb.uVec[k * nSeg + i]; }
+            const float r = 0.5f * fb.segLength[i] + g.viewParams[0];
+            const int owner = (state && state[i] < 0) ? STORE_NONE : STORE_FILAMENT;
+            net = key_of<B>(w.bt.segKey, i).x;
+            for (int k = 0; k < 3; k++) a.uSnap[k * nSeg + i] = u[k];
+            g.boundingRadius[i] = r;
+            g.ownerStore[i] = owner;
+            g.ownerSlot[i] = i;
+            // the motor rows of the previous step were last read by its rods and motor CSR kernels
+            a.headM[i] = -1;
+            a.cntM[i] = 0;
+        } else {
+            const sbx_rigid_body& mb = sc.mot.body;
+            const int m = i - nSeg, h = 3 * m + 2, r = 3 * m;
+            const float hl = mb.segLength[h], reach = sc.mot.reach[m];
+            float u[3], ru[3];
+            for (int k = 0; k < 3; k++) {
+                u[k] = mb.uVec[k * nB + h];
+                ru[k] = mb.uVec[k * nB + r];
+                c[k] = mb.coord[k * nB + h] + 0.5f * hl * u[k];
+            }
+            net = key_of<B>(w.bt.motKey, m).x;
+            for (int k = 0; k < 3; k++) {
+                sc.mot.head[k * nM + m] = c[k];
+                sc.mot.uVec[k * nM + m] = u[k];
+                sc.mot.rodUVec[k * nM + m] = ru[k];
+            }
+            g.boundingRadius[i] = reach;
+            g.ownerStore[i] = STORE_MOTOR;
+            g.ownerSlot[i] = m;
+        }
+        for (int k = 0; k < 3; k++) g.center[k * cap + i] = c[k];
+        if (i < g.gridCounts[1]) {
+            const GridView v = grid_view<B>(w, net);
+            cell = (int)(v.off - a.segCellOff) + cell_coord(c[0], v.gp[0], v.gp[4], v.nX) +
+                   cell_coord(c[1], v.gp[1], v.gp[4], v.nY) * v.nX + cell_coord(c[2], v.gp[2], v.gp[4], v.nZ) * (v.nX * v.nY);
+        }
+    }
+    if (i < cap) g.bodyCell[i] = cell;
+    int over = 0;
+    if (cell >= 0) {
+        if (i < nSeg) atomicAdd(&a.cntSeg[cell], 1);
+        over = row_insert(a.cntCell, a.cellSlot, WIDE_CELL_SLOTS, a.cellUse, a.cellHead, a.cellNext, cell, i);
+    }
+    __syncwarp();
+    const int tile = cell >= 0 ? cell / WIDE_TILE : -1;
+    tile_add(w.sumCell, tile);
+    tile_add(w.sumSeg, i < nSeg ? tile : -1);
+    stat_add(a, ST_CELL_LIST, over);
+}
+
+// ---------------------------------------------------------------- link rows
+// One link a thread: its entries in the rows of its two rods, the Bell unbinding
+// (CrosslinkerSystem.java:727-756) and the active counts (:694-708)
+template <bool B>
+__global__ void __launch_bounds__(128) k_wide_link_rows(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_dense_scene& sc = a.sc;
+    const sbx_crosslinker_store& xl = sc.xl;
+    const sbx_rigid_body& fb = sc.fil.body;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    int la = -1, lb = -1, over = 0;
+    if (k < a.nL) {
+        la = xl.linkFilA[k];
+        lb = xl.linkFilB[k];
+        if (!end_ok(w, la)) la = -1;
+        if (!end_ok(w, lb)) lb = -1;
+        if (la >= 0) over += row_insert(a.cntA, a.slotA, FUSED_ROW_SLOTS, a.rowUse, a.headA, a.nextA, la, k);
+        if (lb >= 0) over += row_insert(a.cntB, a.slotB, FUSED_ROW_SLOTS, a.rowUse, a.headB, a.nextB, lb, k);
+    }
+    __syncwarp();
+    tile_add(w.sumA, la >= 0 ? la / WIDE_TILE : -1);
+    tile_add(w.sumB, lb >= 0 ? lb / WIDE_TILE : -1);
+    stat_add(a, ST_LINK_LIST, over);
+    if (la < 0 || lb < 0 || xl.linkState[k] < 0) return;
+    if (a.xlUnbind) {
+        const int2 key = key_of<B>(w.bt.linkKey, k);
+        // the draw is keyed by the local index, which also indexes the strain ring: shift the
+        // ring pointers so that it addresses this link's own ring
+        const int off = k - key.y;
+        if (unbind_one(key.y, a.nSeg, fb.uVec, fb.end1, la, lb, xl.loc1[k], xl.loc2[k],
+                       xl.strainHist + (int64_t)off * STRAIN_WIN, xl.strainPlace + off, xl.offParams, *a.d_step,
+                       B ? w.bt.seeds[3 * key.x] : sc.seed)) {
+            xl.linkState[k] = LINK_FREE;
+            return;
+        }
+    }
+    atomicAdd(&a.cntAct[la], 1);
+    atomicAdd(&a.cntAct[lb], 1);
+}
+
+// ---------------------------------------------------------------- scans
+// Exclusive scan of one tile of a histogram into out, with the tile sums made by the kernel that
+// filled it: a block adds the sums before its tile and scans the tile through shared memory.
+// copy (optional) gets the row lengths, chunkOut (optional) the prefix of every SCAN_CHUNK rows;
+// the histogram is left at zero for the next step.
+__device__ void scan_one_tile(int tile, int tiles, int* cnt, int n, const int* sums, int* out, int* copy, int clampTotal,
+                              int* chunkOut, bool keep) {
+    __shared__ int sv[WIDE_TILE + WIDE_TILE / 32];
+    static_assert(WIDE_TILE == SCAN_TILE_ROWS, "the scan's tile");
+    const int base = tile * WIDE_TILE;
+    int v[TILE_PER_THREAD], s = 0;
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; k++) {
+        const int g = base + threadIdx.x + 256 * k;
+        v[k] = g < n ? cnt[g] : 0;
+    }
+    int p = 0;
+    for (int k = threadIdx.x; k < tile; k += 256) p += sums[k * WIDE_SUM_STRIDE];
+    int prefix;
+    block_exclusive_scan<256>(p, &prefix);
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; k++) {
+        const int r = threadIdx.x + 256 * k, g = base + r;
+        sv[tile_slot(r)] = v[k];
+        if (g < n) {
+            if (copy) copy[g] = v[k];
+            if (!keep) cnt[g] = 0;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; k++) {
+        v[k] = sv[tile_slot(TILE_PER_THREAD * threadIdx.x + k)];
+        s += v[k];
+    }
+    int tot;
+    int run = block_exclusive_scan<256>(s, &tot);
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; k++) {
+        sv[tile_slot(TILE_PER_THREAD * threadIdx.x + k)] = run;
+        run += v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < TILE_PER_THREAD; k++) {
+        const int r = threadIdx.x + 256 * k, g = base + r;
+        if (g < n) out[g] = prefix + sv[tile_slot(r)];
+    }
+    if (chunkOut && threadIdx.x < WIDE_TILE / SCAN_CHUNK) {
+        const int c = tile * (WIDE_TILE / SCAN_CHUNK) + threadIdx.x;
+        if (c < (n + SCAN_CHUNK - 1) / SCAN_CHUNK) chunkOut[c] = prefix + sv[tile_slot(threadIdx.x * SCAN_CHUNK)];
+    }
+    if (tile == tiles - 1 && threadIdx.x == 0) {
+        const int total = prefix + tot;
+        out[n] = total < clampTotal ? total : clampTotal;
+        if (chunkOut) chunkOut[(n + SCAN_CHUNK - 1) / SCAN_CHUNK] = total;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_wide_cell_scan(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_grid_state& g = a.sc.grid;
+    const int b = blockIdx.x;
+    if (b < w.tilesC)
+        scan_one_tile(b, w.tilesC, a.cntCell, a.C, w.sumCell, g.gridCellOffsets, g.cellCount, a.cap, g.chunkSum, false);
+    else
+        scan_one_tile(b - w.tilesC, w.tilesC, a.cntSeg, a.C, w.sumSeg, a.segCellOff, nullptr, a.nSeg, nullptr, false);
+}
+
+__global__ void __launch_bounds__(256) k_wide_link_scan(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_crosslinker_store& xl = a.sc.xl;
+    const int b = blockIdx.x;
+    if (b < w.tilesS)
+        scan_one_tile(b, w.tilesS, a.cntA, a.nSeg, w.sumA, xl.segOffsetsA, xl.segCountA, a.nL, nullptr, false);
+    else
+        scan_one_tile(b - w.tilesS, w.tilesS, a.cntB, a.nSeg, w.sumB, xl.segOffsetsB, xl.segCountB, a.nL, nullptr, false);
+}
+
+// ---------------------------------------------------------------- place
+// Each body at its rank in its cell: the serial scatter's position. The segments' endpoints go
+// into cell order for the reach walk (segments precede heads within a cell, so a segment's
+// rank in its cell is its rank among the cell's segments), and the largest reach of a segment
+// from its centre is kept for it.
+__global__ void __launch_bounds__(256) k_wide_place(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_dense_scene& sc = a.sc;
+    const sbx_grid_state& g = sc.grid;
+    const sbx_rigid_body& fb = sc.fil.body;
+    const int nSeg = a.nSeg;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = i < a.cap ? g.bodyCell[i] : -1;
+    float span = 0.f;
+    if (c >= 0 && SBX_IDX_OK(c, a.C, CK_CELL)) {
+        const int o0 = g.gridCellOffsets[c], n = g.gridCellOffsets[c + 1] - o0;
+        const bool seg = i < nSeg;
+        float c3[3], e1[3], e2[3];
+        int q0 = 0;
+        bool fil = false;
+        if (seg) {
+            q0 = a.segCellOff[c];
+            fil = g.ownerStore[i] == STORE_FILAMENT;
+            for (int k = 0; k < 3; k++) {
+                c3[k] = g.center[k * a.cap + i];
+                e1[k] = fb.end1[k * nSeg + i];
+                e2[k] = fb.end2[k * nSeg + i];
+            }
+        }
+        const int rank = row_rank<WIDE_CELL_SLOTS>(a, n, a.cellSlot, a.cellUse, a.cellHead, a.cellNext, c, i, a.cap);
+        if (SBX_IDX_OK(o0 + rank, a.cap, CK_CSR_POS)) {
+            g.gridCellContents[o0 + rank] = i;
+            if (seg && SBX_IDX_OK(q0 + rank, nSeg, CK_CSR_POS)) {
+                if (fil) {
+                    span = segment_span(c3, e1, e2);
+                    a.segE1[q0 + rank] = make_float4(e1[0], e1[1], e1[2], __int_as_float(i));
+                    a.segE2[q0 + rank] = make_float4(e2[0], e2[1], e2[2], 0.f);
+                } else {
+                    a.segE1[q0 + rank] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+                    a.segE2[q0 + rank] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+        }
+    }
+    __syncwarp();
+    span_max(a.reachMax, span);
+}
+
+// ---------------------------------------------------------------- bind
+// Release, reach walk with the nearest choice, nucleotide cycle and the bound head's entry in
+// its rod's motor row (as the fused kernel's binding phase): a warp takes BIND_HEADS consecutive
+// heads, 32 / BIND_LANES of them side by side, BIND_LANES lanes a head.
+constexpr int BIND_LANES = 8, BIND_HEADS = 8;
+template <bool B>
+__global__ void __launch_bounds__(128) k_wide_bind(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_dense_scene& sc = a.sc;
+    const sbx_motor_store& mot = sc.mot;
+    const float* kp = mot.kinParams;
+    const int lane = threadIdx.x & 31, nM = a.nM;
+    const int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * BIND_HEADS;
+    if (base >= nM) return;
+    const int t = mot.counts[1];
+    const int myM = base + lane;
+    const bool mine = lane < BIND_HEADS && myM < nM;
+    int bs = 0, cd = 0, sb = 0, sr = 0, cs = 0, seed = sc.seed;
+    int2 key = make_int2(0, 0);
+    if (mine) {
+        key = key_of<B>(w.bt.motKey, myM);
+        if (B) seed = w.bt.seeds[3 * key.x];
+        bs = mot.boundSeg[myM]; cd = mot.cooldown[myM]; sb = mot.stats[2 * myM]; sr = mot.stats[2 * myM + 1];
+        cs = mot.capStats[myM];
+        release_one(key.y, bs, cd, sb, sr, cs, mot.forceDotFil[myM], mot.forceMag[myM], kp, t, seed);
+    }
+    for (int j = 0; j < BIND_HEADS; j += 32 / BIND_LANES) {
+        const int m = base + j + lane / BIND_LANES;
+        const bool valid = m < nM;
+        const int mm = valid ? m : base;
+        const GridView gv = grid_view<B>(w, key_of<B>(w.bt.motKey, mm).x);
+        int best;
+        float arc;
+        const int rc = group_reach_bind<BIND_LANES>(
+            a, gv, lane, valid, mot.head[mm], mot.head[nM + mm], mot.head[2 * nM + mm], mot.uVec[mm],
+            mot.uVec[nM + mm], mot.uVec[2 * nM + mm], mot.rodUVec[mm], mot.rodUVec[nM + mm], mot.rodUVec[2 * nM + mm],
+            sc.grid.reachSeg + (int64_t)mm * MAX_CAND, kp[7], kp[8], &best, &arc);
+        if ((lane & (BIND_LANES - 1)) == 0 && valid) {
+            sc.grid.reachCount[m] = rc;
+            if (rc > MAX_CAND) {
+                atomicOr(a.err, ERR_REACH_OVERFLOW);
+                stat_add(a, ST_REACH_OVER, 1);
+            }
+        }
+        const bool owner = lane >= j && lane < j + 32 / BIND_LANES;
+        const int src = owner ? (lane - j) * BIND_LANES : 0;
+        const int bb = __shfl_sync(0xffffffffu, best, src);
+        const float ab = __shfl_sync(0xffffffffu, arc, src);
+        if (owner && bs == FREE_BINDABLE && bb >= 0) {
+            bs = bb;
+            if (mine) mot.bindArc[myM] = ab;
+        }
+    }
+    int row = -1, over = 0;
+    if (mine) {
+        mot.boundSeg[myM] = bs; mot.cooldown[myM] = cd; mot.stats[2 * myM] = sb; mot.stats[2 * myM + 1] = sr;
+        mot.capStats[myM] = cs;
+        mot.nucleotideState[myM] = cycle_one(key.y, mot.nucleotideState[myM], bs >= 0, mot.forceDotHist + 10 * myM,
+                                             mot.nucParams, t, seed);
+        if (bs >= 0 && SBX_IDX_OK(bs, a.nSeg, CK_BOUND_SEG) && bs < a.nSeg) {
+            row = bs;
+            over = row_insert(a.cntM, a.slotM, FUSED_MOTOR_SLOTS, a.mRowUse, a.headM, a.nextM, bs, myM);
+        } else if (bs >= 0 && w.errDev) {
+            *(volatile int*)w.errDev = 1;
+        }
+    }
+    __syncwarp();
+    tile_add(w.sumM, row >= 0 ? row / WIDE_TILE : -1);
+    stat_add(a, ST_MOTOR_LIST, over);
+}
+
+// ---------------------------------------------------------------- terms and mini
+// The position-only myosin terms, one a thread, beside the grid kernels: FP64 chains of some
+// thousand cycles that would otherwise sit between binding and integration.
+__global__ void __launch_bounds__(128) k_wide_terms(const __grid_constant__ WideArgs w) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < 2 * w.a.nM + 4 * w.a.nD) myosin_term(w.a, k);
+}
+
+// One block a minifilament: a warp for its heads (with their bonds), its rods, its levers, then
+// the integration of its sub-bodies in body order. The backbones, one a thread, take the
+// blocks after them.
+constexpr int MINI_THREADS = 96;
+template <bool B>
+__global__ void __launch_bounds__(MINI_THREADS) k_wide_mini(const __grid_constant__ WideArgs w) {
+    __shared__ MiniSmem sm;
+    const FusedArgs& a = w.a;
+    const sbx_minifilament_store& mini = a.sc.mini;
+    if ((int)blockIdx.x < a.nBb) {
+        mini_bodies(a, sm, blockIdx.x, GlobalTerms{a});
+        return;
+    }
+    const int u = (blockIdx.x - a.nBb) * MINI_THREADS + threadIdx.x;
+    if (u >= a.nBb) return;
+    mini_backbone(a, u, mini.bbCounts[1], GlobalTerms{a}, B ? w.bt.boxParams + 8 * w.bt.bbKey[2 * u] : a.sc.boxParams,
+                  B ? mini.bbBodyParams[0] : a.sc.boxParams[7]);
+}
+
+// ---------------------------------------------------------------- links
+// Crosslinker forces and torsion (CrosslinkerSystem.java:61-123, :777-806), one thread a link,
+// and the link at its rank in both CSRs: the lists, and its two payload rows in list order
+// (zeros for a FREE link)
+__global__ void __launch_bounds__(128) k_wide_links(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_crosslinker_store& xl = a.sc.xl;
+    const sbx_rigid_body& fb = a.sc.fil.body;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= a.nL) return;
+    int la = xl.linkFilA[k], lb = xl.linkFilB[k];
+    if (!end_ok(w, la)) la = -1;
+    if (!end_ok(w, lb)) lb = -1;
+    int pA = -1, pB = -1;
+    if (la >= 0) {
+        const int o0 = xl.segOffsetsA[la], n = xl.segOffsetsA[la + 1] - o0;
+        pA = o0 + row_rank<FUSED_ROW_SLOTS>(a, n, a.slotA, a.rowUse, a.headA, a.nextA, la, k, a.nL);
+    }
+    if (lb >= 0) {
+        const int o0 = xl.segOffsetsB[lb], n = xl.segOffsetsB[lb + 1] - o0;
+        pB = o0 + row_rank<FUSED_ROW_SLOTS>(a, n, a.slotB, a.rowUse, a.headB, a.nextB, lb, k, a.nL);
+    }
+    const int state = xl.linkState[k];
+    float out[XL_STRIDE];
+    link_forces_one(k, a.nSeg, fb.coord, fb.uVec, fb.end1, fb.bTransGam, la, lb, xl.loc1[k], xl.loc2[k], a.cntAct,
+                    xl.xlParams, out);
+    if (xl.torsionParams[1] >= 0.5f)
+        link_torsion_row(k, a.nSeg, fb.uVec, la, lb, state, xl.linkOrientSame[k], xl.torqueMagHist, xl.torqueMagPlace,
+                         out, xl.torsionParams[0]);
+    // (a row is 48 bytes: 16-byte stores where the array is aligned)
+    float* row = xl.xlinkData + (int64_t)k * XL_STRIDE;
+    if (((uintptr_t)xl.xlinkData & 15u) == 0)
+        for (int j = 0; j < 3; j++)
+            reinterpret_cast<float4*>(row)[j] = make_float4(out[4 * j], out[4 * j + 1], out[4 * j + 2], out[4 * j + 3]);
+    else
+        for (int j = 0; j < XL_STRIDE; j++) row[j] = out[j];
+    if (pA >= 0) xl.segIdxA[pA] = k;
+    if (pB >= 0) xl.segIdxB[pB] = k;
+    const bool on = state >= 0;
+    float2* oA = reinterpret_cast<float2*>(w.payA + 6 * (int64_t)(pA < 0 ? 0 : pA));
+    float2* oB = reinterpret_cast<float2*>(w.payB + 6 * (int64_t)(pB < 0 ? 0 : pB));
+    for (int j = 0; j < 3; j++) {
+        if (pA >= 0) oA[j] = on ? make_float2(out[2 * j], out[2 * j + 1]) : make_float2(0.f, 0.f);
+        if (pB >= 0) oB[j] = on ? make_float2(out[6 + 2 * j], out[7 + 2 * j]) : make_float2(0.f, 0.f);
+    }
+}
+
+// ---------------------------------------------------------------- motor CSR
+// The reference's motor CSR arrays (CrossBridgeSystem.java:190-217), outputs of the step that
+// the rods kernel does not wait for (it reads the row slots; the row lengths stay in cntM)
+__global__ void __launch_bounds__(256) k_wide_motor_scan(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    scan_one_tile(blockIdx.x, w.tilesS, a.cntM, a.nSeg, w.sumM, a.sc.segMotorOffsets, a.sc.segMotorCount, a.nM, nullptr,
+                  true);
+}
+
+// the motors at their ranks; the overflow lists' heads of the cells (last read by the place
+// kernel) and every scan's tile sums are emptied for the next step, which begins after this
+__global__ void __launch_bounds__(256) k_wide_motor_place(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_dense_scene& sc = a.sc;
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m < a.C) a.cellHead[m] = -1;
+    if (m < w.tilesC) { w.sumCell[m * WIDE_SUM_STRIDE] = 0; w.sumSeg[m * WIDE_SUM_STRIDE] = 0; }
+    if (m < w.tilesS) w.sumM[m * WIDE_SUM_STRIDE] = 0;
+    if (m >= a.nM) return;
+    const int bs = sc.mot.boundSeg[m];
+    if (bs < 0 || bs >= a.nSeg) return;
+    const int pos = sc.segMotorOffsets[bs] + row_rank<FUSED_MOTOR_SLOTS>(a, a.cntM, a.slotM, a.mRowUse, a.headM,
+                                                                         a.nextM, bs, m, a.nM);
+    if (pos < a.nM) sc.segMotorMyo[pos] = m;
+}
+
+// ---------------------------------------------------------------- rods
+// Adds row [k0, k1) of a link payload in list order, FP64, into the float sums (segGatherA/B,
+// CrosslinkerSystem.java:129-173)
+__device__ __forceinline__ void add_row(const float* pay, int k0, int k1, float F[3], float T[3]) {
+    double f[3] = {0.0, 0.0, 0.0}, t[3] = {0.0, 0.0, 0.0};
+    for (int k = k0; k < k1; k++) {
+        const float2* q = reinterpret_cast<const float2*>(pay + 6 * (int64_t)k);
+        const float2 x = q[0], y = q[1], z = q[2];
+        f[0] += x.x; f[1] += x.y; f[2] += y.x;
+        t[0] += y.y; t[1] += z.x; t[2] += z.y;
+    }
+    for (int k = 0; k < 3; k++) { F[k] = (float)(F[k] + f[k]); T[k] = (float)(T[k] + t[k]); }
+}
+
+// a neighbour rod as the step found it
+__device__ __forceinline__ RodGeom start_rod(const FusedArgs& a, int j) {
+    const sbx_rigid_body& fb = a.sc.fil.body;
+    const float* c = a.sc.grid.center;
+    const int n = a.nSeg, cap = a.cap;
+    RodGeom r;
+    r.cx = c[j]; r.cy = c[cap + j]; r.cz = c[2 * cap + j];
+    r.ux = a.uSnap[j]; r.uy = a.uSnap[n + j]; r.uz = a.uSnap[2 * n + j];
+    r.len = fb.segLength[j];
+    r.bTGx = fb.bTransGam[j]; r.bTGy = fb.bTransGam[n + j]; r.bRGy = fb.bRotGam[n + j];
+    return r;
+}
+
+// Chain forces from the joints made ahead, the crosslinker and motor gathers, the walls and the
+// Langevin update of one rod a thread, in the reference's order; the rod's histograms are reset
+// for the next step. A joint whose neighbour does not point back is computed from this side.
+template <bool B>
+__global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ WideArgs w) {
+    const FusedArgs& a = w.a;
+    const sbx_dense_scene& sc = a.sc;
+    const sbx_filament_store& fs = sc.fil;
+    const sbx_rigid_body& fb = fs.body;
+    const sbx_crosslinker_store& xl = sc.xl;
+    const int n = a.nSeg, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    // what does not wait for anything first, all in flight together
+    const int t = fs.counts[1];
+    const int nm = a.cntM[i];
+    int slots[2] = {fs.end2NbrSlot[i], fs.end1NbrSlot[i]};
+    const int sides[2] = {fs.end2NbrSide[i], fs.end1NbrSide[i]};
+    int a0 = 0, a1 = 0, b0 = 0, b1 = 0, act = 0;
+    if (a.xlOn) {
+        a0 = xl.segOffsetsA[i]; a1 = xl.segOffsetsA[i + 1];
+        b0 = xl.segOffsetsB[i]; b1 = xl.segOffsetsB[i + 1];
+        act = a.cntAct[i];
+    }
+    const BodyIn in = body_load(fb, i);
+    if (i == 0) {
+        *a.d_step = t + 1;               // (every reader of this step's index has run)
+        *a.reachMax = 0;
+    }
+    if (a.xlOn) {
+        xl.activeLinkCount[i] = act;
+        a.cntAct[i] = 0; a.headA[i] = -1; a.headB[i] = -1;
+        if (i < w.tilesS) { w.sumA[i * WIDE_SUM_STRIDE] = 0; w.sumB[i * WIDE_SUM_STRIDE] = 0; }
+    }
+    const ChainParams cp = chain_params(fs.chainParams);
+    double fd[3] = {0.0, 0.0, 0.0}, td[3] = {0.0, 0.0, 0.0};
+    RodGeom me;
+    me.cx = in.p.c[0]; me.cy = in.p.c[1]; me.cz = in.p.c[2];
+    me.ux = in.p.u[0]; me.uy = in.p.u[1]; me.uz = in.p.u[2];
+    me.len = in.len; me.bTGx = in.gT[0]; me.bTGy = in.gT[1]; me.bRGy = in.gR[1];
+    const ChainJoint* Jg = reinterpret_cast<const ChainJoint*>(a.joints);
+    for (int side = 0; side < 2; side++) {
+        int slot = slots[side];
+        const int nside = sides[side];
+        if (!SBX_IDX_OK_OR_NONE(slot, n, CK_NEIGHBOUR)) slot = -1;
+        if (slot < 0) continue;
+        const RodGeom nb = start_rod(a, slot);
+        ChainJoint J;
+        bool have = slot > i;
+        if (have) {
+            J = Jg[2 * (int64_t)i + side];
+        } else if (nside == 0 || nside == 1) {
+            const int ps = 1 - nside;                    // the partner's side facing rod i
+            const int back = ps == 0 ? fs.end2NbrSlot[slot] : fs.end1NbrSlot[slot];
+            const int backSide = ps == 0 ? fs.end2NbrSide[slot] : fs.end1NbrSide[slot];
+            have = slot < i && back == i && backSide == 1 - side;
+            if (have) J = Jg[2 * (int64_t)slot + ps];
+        }
+        if (!have) J = chain_joint(cp, i, side, slot, nside, me, nb);
+        chain_apply(cp, i, side, slot, nside, me, nb, J, fd, td);
+    }
+    float F[3], T[3];
+    for (int k = 0; k < 3; k++) { F[k] = (float)(0.0f + fd[k]); T[k] = (float)(0.0f + td[k]); }
+    if (a.xlOn) {
+        add_row(w.payA, a0, a1, F, T);
+        add_row(w.payB, b0, b1, F, T);
+    }
+    // CrossBridgeSystem.segGather (CrossBridgeSystem.java:302-320): the bound motors' reactions
+    // in ascending slot, taken from the row's slots (and list) by repeated minimum
+    double gf[3] = {0.0, 0.0, 0.0}, gt[3] = {0.0, 0.0, 0.0};
+    for (int q = 0, last = -1; q < nm; q++) {
+        int next = 0x7fffffff;
+        for (int j = 0; j < FUSED_MOTOR_SLOTS && j < nm && j < a.mRowUse; j++) {
+            const int m = a.slotM[(size_t)i * FUSED_MOTOR_SLOTS + j];
+            if (m > last && m < next) next = m;
+        }
+        if (nm > a.mRowUse) {
+            int it = 0;
+            for (int m = a.headM[i]; m >= 0 && it <= a.nM; m = a.nextM[m], it++) {
+                if (!SBX_IDX_OK(m, a.nM, CK_MOTOR_SLOT)) break;
+                if (m > last && m < next) next = m;
+            }
+        }
+        if (next == 0x7fffffff || !SBX_IDX_OK(next, a.nM, CK_MOTOR_SLOT)) {
+            atomicOr(a.err, ERR_LIST);
+            break;
+        }
+        const float* p = sc.bondData + (int64_t)next * XB_STRIDE + 6;
+        gf[0] += p[0]; gf[1] += p[1]; gf[2] += p[2];
+        gt[0] += p[3]; gt[1] += p[4]; gt[2] += p[5];
+        last = next;
+    }
+    for (int k = 0; k < 3; k++) { F[k] = (float)(F[k] + gf[k]); T[k] = (float)(T[k] + gt[k]); }
+    const float* box = B ? w.bt.boxParams + 8 * w.bt.segKey[2 * i] : sc.boxParams;
+    const BoxParams bx = box_params(box, t);
+    if (bx.active) confine_one(bx, in.p.c, in.p.u, in.len, in.gT[0], F, T);
+    body_step(fb, i, in, F, T, B ? fs.params[0] : sc.boxParams[7]);
+}
+
+}  // namespace
+
+bool wide_streams_create(WideStreams& ws) {
+    for (cudaStream_t* s : {&ws.ahead, &ws.link, &ws.csr})
+        if (cudaStreamCreateWithFlags(s, cudaStreamNonBlocking) != cudaSuccess) return false;
+    for (cudaEvent_t* e : {&ws.start, &ws.drawn, &ws.bound, &ws.joined, &ws.linkDone, &ws.csrDone})
+        if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return false;
+    return true;
+}
+
+void wide_streams_destroy(WideStreams& ws) {
+    for (cudaStream_t s : {ws.ahead, ws.link, ws.csr})
+        if (s) cudaStreamDestroy(s);
+    for (cudaEvent_t e : {ws.start, ws.drawn, ws.bound, ws.joined, ws.linkDone, ws.csrDone})
+        if (e) cudaEventDestroy(e);
+    ws = WideStreams{};
+}
+
+namespace {
+
+template <bool B>
+sbx_status wide_step_impl(sbx_ctx* ctx, const WideArgs& w, const WideStreams& ws) {
+    const FusedArgs& a = w.a;
+    cudaStream_t s = ctx->stream;
+    cudaError_t e = cudaSuccess;
+    auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
+    auto fork = [&](cudaEvent_t ev, cudaStream_t to) { ok(cudaEventRecord(ev, s)); ok(cudaStreamWaitEvent(to, ev, 0)); };
+    auto join = [&](cudaEvent_t ev, cudaStream_t from) { ok(cudaEventRecord(ev, from)); ok(cudaStreamWaitEvent(s, ev, 0)); };
+#define WIDE_LAUNCH(stream, kernel, items, block)                                  \
+    do {                                                                           \
+        kernel<<<blocks(items, block), block, 0, stream>>>(w);                     \
+        ctx->launches++;                                                           \
+    } while (0)
+    fork(ws.start, ws.ahead);
+    if (a.xlOn) ok(cudaStreamWaitEvent(ws.link, ws.start, 0));
+    WIDE_LAUNCH(ws.ahead, k_wide_draws<B>, (int64_t)a.nB + a.nBb + a.nSeg, 256);
+    WIDE_LAUNCH(ws.ahead, k_wide_terms, 2 * (int64_t)a.nM + 4 * (int64_t)a.nD, 128);
+    ok(cudaEventRecord(ws.drawn, ws.ahead));
+    WIDE_LAUNCH(ws.ahead, k_wide_joints, a.nSeg, 128);
+    if (a.xlOn) {
+        WIDE_LAUNCH(ws.link, k_wide_link_rows<B>, a.nL, 128);
+        WIDE_LAUNCH(ws.link, k_wide_link_scan, (int64_t)2 * w.tilesS * 256, 256);
+        WIDE_LAUNCH(ws.link, k_wide_links, a.nL, 128);
+    }
+    WIDE_LAUNCH(s, k_wide_publish<B>, a.cap, 256);
+    WIDE_LAUNCH(s, k_wide_cell_scan, (int64_t)2 * w.tilesC * 256, 256);
+    WIDE_LAUNCH(s, k_wide_place, a.cap, 256);
+    WIDE_LAUNCH(s, k_wide_bind<B>, ((int64_t)a.nM + BIND_HEADS - 1) / BIND_HEADS * 32, 128);
+    fork(ws.bound, ws.csr);
+    WIDE_LAUNCH(ws.csr, k_wide_motor_scan, (int64_t)w.tilesS * 256, 256);
+    WIDE_LAUNCH(ws.csr, k_wide_motor_place, std::max(std::max(a.nM, a.C), w.tilesS), 256);
+    ok(cudaStreamWaitEvent(s, ws.drawn, 0));
+    k_wide_mini<B><<<a.nBb + (a.nBb + MINI_THREADS - 1) / MINI_THREADS, MINI_THREADS, 0, s>>>(w);
+    ctx->launches++;
+    join(ws.joined, ws.ahead);
+    if (a.xlOn) join(ws.linkDone, ws.link);
+    WIDE_LAUNCH(s, k_wide_rods<B>, a.nSeg, 128);
+    join(ws.csrDone, ws.csr);
+#undef WIDE_LAUNCH
+    if (e != cudaSuccess) return fail(ctx, SBX_ECUDA, std::string("dense step: streams: ") + cudaGetErrorString(e));
+    return check_launch(ctx, "dense step");
+}
+
+}  // namespace
+
+sbx_status wide_step(sbx_ctx* ctx, const WideArgs& w, bool batched, const WideStreams& ws) {
+    SBX_TRACE("sbx.dense.step");
+    return batched ? wide_step_impl<true>(ctx, w, ws) : wide_step_impl<false>(ctx, w, ws);
+}
+
+SBX_CHECK_EXPORT(wide)

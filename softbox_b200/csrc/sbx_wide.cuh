@@ -1,0 +1,34 @@
+// sbx_wide.cuh — the dense step as a few wide kernels (sbx_wide.cu).
+#pragma once
+#include "sbx_fused.cuh"
+
+constexpr int WIDE_CELL_SLOTS = 8;    // fixed slots per grid cell (one 32-byte sector)
+constexpr int WIDE_TILE = 4096;       // rows of a scan tile
+constexpr int WIDE_SUM_STRIDE = 8;    // ints between two tiles' sums: each in a sector of its own
+
+// `a` holds the scene, the noise and this path's own scratch (not the fused kernel's)
+struct WideArgs {
+    FusedArgs a;
+    int tilesC, tilesS;      // scan tiles of the cells and of the rods
+    // per tile: bodies and segments of the cells, A ends, B ends, bound motors of the rods
+    int *sumCell, *sumSeg, *sumA, *sumB, *sumM;
+    sbx_batch bt;            // packed networks' tables (packed plans)
+    int* noiseErr;           // set when a step outside the supplied noise's range runs, or null
+    int* errDev;             // the context's input-range error word
+    float *payA, *payB;      // the links' A-side and B-side payloads in CSR order, 6 floats each
+};
+
+// the streams and events of one step: `ahead` runs what needs only the step's start view, `link`
+// the crosslinkers, `csr` the motor CSR
+struct WideStreams {
+    cudaStream_t ahead = nullptr, link = nullptr, csr = nullptr;
+    cudaEvent_t start = nullptr, drawn = nullptr, bound = nullptr, joined = nullptr, linkDone = nullptr,
+                csrDone = nullptr;
+};
+
+bool wide_streams_create(WideStreams& ws);
+void wide_streams_destroy(WideStreams& ws);
+
+// queues one step on the context's stream (for capture); the step index is *d_step, advanced at
+// the end
+sbx_status wide_step(sbx_ctx* ctx, const WideArgs& w, bool batched, const WideStreams& ws);

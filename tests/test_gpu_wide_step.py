@@ -1,0 +1,84 @@
+"""The graph path's wide kernels (sbx_wide.cu) where they can go wrong: rows past their fixed
+slots, chain neighbours that do not point back, and scenes of another layout, which keep the
+per-system sequence. The reference of each is the per-system path of the same scene
+(bit-identical to the oracle: tests/test_gpu_parity.py)."""
+import copy
+
+import numpy as np
+import pytest
+
+from helpers import assert_same, compare_scenes, oracle_dense_run, small_dense
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from softbox_b200 import device as D  # noqa: E402
+
+
+@pytest.fixture(scope="module")
+def warm(orc_dm):
+    sc = small_dense(0.05)
+    oracle_dense_run(orc_dm, sc, 0, 300)
+    return sc
+
+
+def _run(sc, mode, steps=40, caps=None):
+    from softbox_b200.engine import DenseNetwork
+    net = DenseNetwork(copy.deepcopy(sc))
+    if caps is not None:
+        net.test_caps(**caps)
+    net.run(300, steps, mode=mode)
+    net.status()
+    stats, n = net.fused_stats(), net.kernels_per_step
+    out = D.to_host(net.dev)
+    net.close()
+    return out, stats, n
+
+
+@pytest.mark.parametrize("caps", [dict(cell_slots=0), dict(row_slots=0), dict(cell_slots=1, row_slots=1)],
+                         ids=["cells", "rows", "both"])
+def test_rows_past_their_slots(warm, caps):
+    ref, _, _ = _run(warm, "unfused")
+    got, stats, _ = _run(warm, "graph", caps=caps)
+    assert stats["cell_list"] > 0 if "cell_slots" in caps else stats["link_list"] > 0 and stats["motor_list"] > 0
+    assert len(compare_scenes(ref, got)) > 80
+
+
+def test_neighbours_that_do_not_point_back(warm):
+    sc = copy.deepcopy(warm)
+    f = sc["fil"]
+    for k in (3, 4, 57, 200):                      # rod k + 1 forgets rod k, which keeps its joint
+        assert f["end2NbrSlot"][k] == k + 1
+        f["end1NbrSlot"][k + 1] = -1
+    for k in (21, 121):                            # and the other way round
+        assert f["end2NbrSlot"][k] == k + 1
+        f["end2NbrSlot"][k] = -1
+    ref, _, _ = _run(sc, "unfused")
+    got, _, _ = _run(sc, "graph")
+    assert len(compare_scenes(ref, got)) > 80
+
+
+def test_other_layouts_keep_the_per_system_sequence(warm):
+    sc = copy.deepcopy(warm)
+    a, b = sc["dim"]["motorA"].copy(), sc["dim"]["motorB"].copy()
+    sc["dim"]["motorA"][0], sc["dim"]["motorB"][0] = b[0], a[0]
+    ref, _, n_wide = _run(warm, "graph", steps=1)
+    ref, _, _ = _run(sc, "unfused")
+    got, _, n = _run(sc, "graph")
+    assert n > 40 > n_wide
+    assert len(compare_scenes(ref, got)) > 80
+
+
+def test_graph_and_fused_steps_alternate(warm):
+    from softbox_b200.engine import DenseNetwork
+    ref, _, _ = _run(warm, "unfused", steps=12)
+    net = DenseNetwork(copy.deepcopy(warm))
+    t = 300
+    for mode, k in (("graph", 1), ("fused", 3), ("graph", 2), ("unfused", 1), ("graph", 1), ("fused", 1), ("graph", 3)):
+        net.run(t, k, mode=mode)
+        t += k
+    assert t == 312 and net.status() == 0
+    assert len(compare_scenes(ref, D.to_host(net.dev))) > 80
+    assert_same(np.asarray(ref["mot"]["boundSeg"]), net.pull("mot", "boundSeg"), "boundSeg")
+    net.close()
