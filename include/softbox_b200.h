@@ -747,13 +747,14 @@ sbx_status sbx_dense_plan_create(sbx_ctx* ctx, const sbx_dense_scene* scene, sbx
 /* Advances steps t0, t0+1, ..., t0+nsteps-1 (the step index feeds every RNG key and
  * the containment cadence). mode 0: the call sequence of the per-system entry points
  * (zero + draws and confine + integrate + derive as the MechanicsFusion passes, which give
- * the same values); 1: one CUDA-graph replay per step of that sequence; 2: the fused persistent kernel (all nsteps in one
- * cooperative launch; available when the scene has the harness layout, see
- * sbx_dense_plan_fused_available). All three give the same bits. mode 3 (auto): the fused
- * kernel up to SBX_DENSE_AUTO_MAX_FUSED_RODS rods when available, the graph path above it,
- * where the per-system kernels' occupancy beats the persistent kernel's (measured, fused vs
- * graph ms per step: 0.070 / 0.157 at 2e4 rods, 0.092 / 0.177 at 4e4, 0.298 / 0.181 at 5e4,
- * 0.202 / 0.198 at 1e5, 1.01 / 0.44 at 5e5). */
+ * the same values); 1: one CUDA-graph replay per step (wide kernels for a scene of the harness
+ * layout, else that sequence); 2: the fused persistent kernel (all nsteps in one cooperative
+ * launch; available when the scene has the harness layout, see
+ * sbx_dense_plan_fused_available). All three give the same bits. mode 3 (auto): the graph of
+ * wide kernels, which leads at every size (us per step, graph / fused: 48 / 57 at 1,000 rods one
+ * step a call; 55 / 64 at 2e4 and 67 / 172 at 4e4, 20 steps a call); without it, or on a stream
+ * under capture, the fused kernel up to SBX_DENSE_AUTO_MAX_FUSED_RODS rods when available, the
+ * graph path above it. */
 #define SBX_DENSE_AUTO_MAX_FUSED_RODS 40960
 sbx_status sbx_dense_plan_run(sbx_dense_plan* plan, int32_t t0, int32_t nsteps, int32_t mode);
 /* Runs one step as the unfused per-system call sequence (reference granularity). */
@@ -768,10 +769,11 @@ int32_t sbx_dense_plan_kernels_per_step(sbx_dense_plan* plan);
 sbx_status sbx_dense_plan_status(sbx_dense_plan* plan, int32_t* flags);
 /* 1 when the fused persistent path is available for this scene (else mode 2 returns SBX_ESTATE) */
 int32_t sbx_dense_plan_fused_available(sbx_dense_plan* plan);
-/* Re-reads the chain topology for the fused path after the scene's filament topology changed
- * (a turnover cadence: growth splits, deaths, births into FREE slots): rod groups, whether
- * neighbours cross groups, joint sharing. Synchronises the plan's stream. The graph and
- * per-system paths need no refresh. */
+/* Tells the plan that the scene's filament topology changed (a turnover cadence: growth splits,
+ * deaths, births into FREE slots). The fused path depends on it (rod groups, whether
+ * neighbours cross groups, joint sharing): it is read again, which synchronises the plan's
+ * stream, when the fused kernel next runs, or here when the plan has no wide kernels. The
+ * graph and per-system paths need no refresh. */
 sbx_status sbx_dense_plan_refresh(sbx_dense_plan* plan);
 /* cooperative grid size (CTAs) of the fused path */
 int32_t sbx_dense_plan_fused_grid(sbx_dense_plan* plan);

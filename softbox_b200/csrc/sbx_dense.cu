@@ -396,6 +396,7 @@ struct sbx_dense_plan {
     // fused persistent path
     bool fused_ok = false;
     bool fused_prepared = false;  // its scratch exists (the topology may still be refused)
+    bool fused_stale = false;    // the chain topology has changed since its groups were made
     bool fused_dirty = true;     // scratch must be (re)initialised before the next fused run
     std::string fused_why;
     FusedArgs fa{};
@@ -403,6 +404,7 @@ struct sbx_dense_plan {
     std::vector<void*> allocs;
     // the graph path's wide kernels (harness layouts); other scenes capture the per-system sequence
     bool wide_ok = false;
+    bool reportReach = false;      // an "auto" run of fused size ran: its reach overflows are reported
     WideArgs wide{};
     WideStreams wideStreams{};
     // packed networks (graph and per-system paths only)
@@ -843,8 +845,21 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
     if (nsteps == 0) return SBX_OK;
     if (p->noiseOn && ((int64_t)t0 < p->noise.t0 || (int64_t)t0 + nsteps > (int64_t)p->noise.t0 + p->noise.nsteps))
         return fail(ctx, SBX_EINVAL, "sbx_dense_plan_run: steps outside the supplied-noise range");
-    if (mode == 3) mode = (p->fused_ok && p->scene.fil.body.n <= SBX_DENSE_AUTO_MAX_FUSED_RODS) ? 2 : 1;
+    if (mode == 3) {
+        // the wide kernels lead at every size: 48 / 57 us a step at 1,000 rods (one step a call),
+        // 55 / 64 at 20,000 and 67 / 172 at 40,000 (20 steps a call) against the fused kernel
+        const bool fused = p->fused_ok && p->scene.fil.body.n <= SBX_DENSE_AUTO_MAX_FUSED_RODS;
+        // (a stream under capture takes the fused kernel as one node; a graph cannot be launched there)
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (fused && p->wide_ok && cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) cudaGetLastError();
+        mode = fused && (!p->wide_ok || (capture != cudaStreamCaptureStatusNone && !p->fused_stale)) ? 2 : 1;
+        if (fused) p->reportReach = true;
+    }
     if (mode == 2) {
+        if (p->fused_stale) {
+            p->fused_stale = false;
+            p->fused_ok = fused_topology(p);
+        }
         if (!p->fused_ok) return fail(ctx, SBX_ESTATE, "fused path unavailable: " + p->fused_why);
         // the kernel leaves its histograms zeroed and its barrier words consistent at the
         // end of every completed run; they are reset here only after a failed run
@@ -893,11 +908,16 @@ extern "C" sbx_status sbx_dense_plan_status(sbx_dense_plan* p, int32_t* flags) {
         int we = 0;
         cudaMemcpyAsync(&we, p->wide.a.err, sizeof(int), cudaMemcpyDeviceToHost, p->ctx->stream);
         CHK(sbx_ctx_sync(p->ctx));
+        const bool reach = (we & 2) && p->reportReach;
         if (we) cudaMemsetAsync(p->wide.a.err, 0, 16, p->ctx->stream);
         if (we & 8) {
             wide_reset(p);
             *flags = 8;
             return fail(p->ctx, SBX_ESTATE, "graph step: a linked-list walk ran past its bound");
+        }
+        if (reach) {
+            *flags = 2;
+            return fail(p->ctx, SBX_EOVERFLOW, "dense step: a reach list exceeded SBX_MAX_CAND");
         }
     }
     if (!p->fused_ok) return SBX_OK;
@@ -913,12 +933,22 @@ extern "C" sbx_status sbx_dense_plan_status(sbx_dense_plan* p, int32_t* flags) {
     return SBX_OK;
 }
 
-extern "C" int32_t sbx_dense_plan_fused_available(sbx_dense_plan* p) { return p && p->fused_ok ? 1 : 0; }
+extern "C" int32_t sbx_dense_plan_fused_available(sbx_dense_plan* p) {
+    if (!p) return 0;
+    if (p->fused_stale) {
+        p->fused_stale = false;
+        p->fused_ok = fused_topology(p);
+    }
+    return p->fused_ok ? 1 : 0;
+}
 
 extern "C" sbx_status sbx_dense_plan_refresh(sbx_dense_plan* p) {
     if (!p) return SBX_EINVAL;
     if (p->batched || !p->fused_prepared) return SBX_OK;
-    p->fused_ok = fused_topology(p);
+    // the wide kernels take the chains as they are on the device; the fused kernel's groups are
+    // made again when it next runs
+    if (p->wide_ok) p->fused_stale = true;
+    else p->fused_ok = fused_topology(p);
     return SBX_OK;
 }
 

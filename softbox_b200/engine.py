@@ -1,7 +1,7 @@
 """Device-resident networks: the public Python API over the fused step plans.
 
     net = DenseNetwork(scenes.dense_contractile(scenes.C1))
-    net.run(t0=0, nsteps=100)          # "auto": one fused launch up to 40,960 rods, CUDA graphs above
+    net.run(t0=0, nsteps=100)          # "auto": one CUDA-graph replay a step
     pose = net.pull("fil", "coord", sub="body")    # UNDER_DEMAND host copy
 
     rods = FreeRods(scenes.free_rods_box())
@@ -48,11 +48,10 @@ class DenseNetwork:
         return LIB.sbx_dense_plan_fused_grid(self.plan)
 
     def run(self, t0, nsteps, mode=None):
-        """Advance steps t0..t0+nsteps-1. mode: "auto" (default: the fused kernel for
-        networks up to SBX_DENSE_AUTO_MAX_FUSED_RODS rods when available, else the graph
-        path), "fused" (one persistent cooperative launch for all steps), "graph" (one
-        CUDA-graph replay per step) or "unfused" (the per-system call sequence). All give
-        the same bits."""
+        """Advance steps t0..t0+nsteps-1. mode: "auto" (default: the graph path; the fused
+        kernel for a network of its size on a stream under capture), "fused" (one persistent
+        cooperative launch for all steps), "graph" (one CUDA-graph replay per step) or
+        "unfused" (the per-system call sequence). All give the same bits."""
         if mode is None:
             mode = "auto"
         st = LIB.sbx_dense_plan_run(self.plan, int(t0), int(nsteps), self.MODES[mode])
@@ -139,10 +138,10 @@ class TurnoverNetwork(DenseNetwork):
     """A dense network with actin turnover (scenes.dense_turnover): at every biochem cadence
     the turnover block (growth, depolymerisation, death, severing, splits), the release of
     links and heads on dead slots, and constant-actin births run before that step's
-    mechanics, all on the library's stream. The mechanics run on any path; on the fused
-    path (mode "fused", or "auto" below the fused size limit) the plan re-reads the chain
-    topology after each cadence (sbx_dense_plan_refresh: one stream synchronisation per
-    cadence), since splits and births into FREE slots change the rod groups."""
+    mechanics, all on the library's stream. The mechanics run on any path. The fused
+    kernel's rod groups depend on the chain topology, which splits and births into FREE slots
+    change: sbx_dense_plan_refresh notes that after each cadence, and a "fused" run then
+    re-reads it (one stream synchronisation); the graph path reads it on the device."""
 
     def __init__(self, host_scene, ctx=None, fp64_coords=False, device="cuda"):
         from .turnover import Turnover

@@ -82,3 +82,20 @@ def test_graph_and_fused_steps_alternate(warm):
     assert len(compare_scenes(ref, D.to_host(net.dev))) > 80
     assert_same(np.asarray(ref["mot"]["boundSeg"]), net.pull("mot", "boundSeg"), "boundSeg")
     net.close()
+
+
+def test_auto_takes_the_graph_and_fused_runs_after_a_refresh(warm):
+    from softbox_b200.engine import DenseNetwork
+    from softbox_b200.runtime import LIB
+    ref, _, _ = _run(warm, "unfused", steps=6)
+    net = DenseNetwork(copy.deepcopy(warm))
+    k = net.kernels_per_step
+    n0 = net.ctx.launches()
+    net.run(300, 2)
+    assert net.ctx.launches() - n0 >= 2 * k                # (one launch for both steps on the fused path)
+    assert LIB.sbx_dense_plan_refresh(net.plan) == 0
+    net.run(302, 2, mode="fused")
+    net.run(304, 2)
+    assert net.fused_available and net.status() == 0
+    assert len(compare_scenes(ref, D.to_host(net.dev))) > 80
+    net.close()
