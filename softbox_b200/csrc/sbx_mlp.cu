@@ -308,9 +308,9 @@ __device__ __forceinline__ bool wait_mma(unsigned long long* mbar, unsigned pari
     return __syncthreads_and(done_ok ? 1 : 0) != 0;
 }
 
-// 16 accumulator columns of this warp's 32 rows (TMEM lanes 32 * quarter ..)
-__device__ __forceinline__ void load_acc16(unsigned tmem, int quarter, int c0, float v[16]) {
-    unsigned r[16];
+// 16 accumulator columns of this warp's 32 rows (TMEM lanes 32 * quarter ..): the load is
+// issued here, its registers are valid after acc_wait
+__device__ __forceinline__ void acc_load16(unsigned tmem, int quarter, int c0, unsigned r[16]) {
     unsigned taddr = tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)c0;
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
@@ -318,9 +318,29 @@ __device__ __forceinline__ void load_acc16(unsigned tmem, int quarter, int c0, f
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;");
+}
+// waits for the warp's loads; the registers pass through, so that no use moves before it
+__device__ __forceinline__ void acc_wait(unsigned r[16], float v[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
+                   "+r"(r[15])::"memory");
 #pragma unroll
     for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
+}
+__device__ __forceinline__ float4 load_acc4(unsigned tmem, int quarter, int c0) {
+    unsigned r[4];
+    unsigned taddr = tmem + ((unsigned)(quarter * 32) << 16) + (unsigned)c0;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3])::"memory");
+    return make_float4(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]), __uint_as_float(r[3]));
+}
+__device__ __forceinline__ void load_acc16(unsigned tmem, int quarter, int c0, float v[16]) {
+    unsigned r[16];
+    acc_load16(tmem, quarter, c0, r);
+    acc_wait(r, v);
 }
 
 __device__ __forceinline__ void pack16(const float a[16], uint4& lo, uint4& hi) {
@@ -339,20 +359,29 @@ __device__ __forceinline__ int core_at(int r, int c, int Kp) {
     return ((r >> 3) * (Kp >> 3) + (c >> 3)) * 128 + (r & 7) * 16 + (c & 7) * 2;
 }
 
-// rows [0, rows) x [0, Kp) of a row-major BF16 matrix (16-byte aligned rows) into the
-// core-matrix layout by 16-byte async copies; rows past rowsValid are zero
+// rows [0, rows) x [0, Kp) of a row-major BF16 matrix (16-byte aligned rows, rows a multiple of
+// 8) into the core-matrix layout by 16-byte async copies; rows past rowsValid are zero. Item u
+// is row u & 7 of core matrix u >> 3, so the shared addresses run with u and a warp's copies
+// meet no bank twice (with the row's columns along the lanes they all met one: staging 160
+// rows of 256 took 3.2 us of a 10 us pass).
 __device__ __forceinline__ void stage_rows(char* dst, const __nv_bfloat16* src, int ld, int rows, int rowsValid,
                                            int Kp) {
-    const int kg = Kp >> 3;
-    for (int u = threadIdx.x; u < rows * kg; u += blockDim.x) {
-        const int r = u / kg, c = u - r * kg;
-        char* d = dst + ((r >> 3) * kg + c) * 128 + (r & 7) * 16;
+    const int kg = Kp >> 3, r8 = threadIdx.x & 7, step = blockDim.x >> 3, cores = (rows >> 3) * kg;
+    // a thread keeps its 8 columns where the block holds whole rows of core matrices
+    const bool even = step % kg == 0;
+    int v = threadIdx.x >> 3, rg = v / kg, c = v - rg * kg;
+    const int dr = step / kg;
+    for (; v < cores; v += step) {
+        if (!even) { rg = v / kg; c = v - rg * kg; }
+        const int r = rg * 8 + r8;
+        char* d = dst + v * 128 + r8 * 16;
         if (r < rowsValid) {
             const __nv_bfloat16* p = src + (long long)r * ld + c * 8;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(d)), "l"(p));
         } else {
             *reinterpret_cast<uint4*>(d) = make_uint4(0, 0, 0, 0);
         }
+        rg += dr;
     }
 }
 
@@ -436,9 +465,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_predict(const __grid_consta
             if (!last) weights(l + 1, phase);
             else if (tile + (int)gridDim.x < tiles) weights(0, phase);
             const int r = quarter * 32 + lane, row = m0 + r;
+            unsigned acc[16];
+            if (cgroup * 16 < Np) acc_load16(tmem, quarter, cgroup * 16, acc);
             for (int c0 = cgroup * 16; c0 < Np; c0 += COL_GROUPS * 16) {
                 float v[16];
-                load_acc16(tmem, quarter, c0, v);
+                acc_wait(acc, v);
+                // the next columns are on their way while these are worked on
+                if (c0 + COL_GROUPS * 16 < Np) acc_load16(tmem, quarter, c0 + COL_GROUPS * 16, acc);
 #pragma unroll
                 for (int j = 0; j < 16; j++) v[j] += bias[c0 + j];
                 if (!last) {
@@ -484,7 +517,7 @@ __global__ void k_predict_stats(int nz, long long n, double* out) {
 
 // ---------------------------------------------------------------- training
 // Whole Adam steps of the ensemble in one cooperative launch. A network's blocks (gridDim.x of
-// them, at most one an SM) work on its passes together and meet at a barrier of their own
+// them, all resident) work on its passes together and meet at a barrier of their own
 // after each: L forward products, then for each layer from the last the input gradient
 // together with the weight gradient and Adam update of the layer above it (whose weights
 // nothing reads any more). Every product is split into 128 x 32 tiles; the epilogues take in
@@ -552,7 +585,7 @@ __device__ __forceinline__ float adam_one(const TrainArgs& g, int s, float gg, f
     return w - g.lr * (m / g.c1[s]) / (sqrtf(v / g.c2[s]) + g.eps);
 }
 
-__global__ void __launch_bounds__(TRAIN_THREADS, 1) k_train(const __grid_constant__ TrainArgs g) {
+__global__ void __launch_bounds__(TRAIN_THREADS, 2) k_train(const __grid_constant__ TrainArgs g) {
     extern __shared__ __align__(1024) char smem[];
     char* sA = smem;                               // 128 x 256
     char* sB = smem + MT * KMAX * 2;               // 32 x 256
@@ -620,16 +653,14 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) k_train(const __grid_constan
         stage_rows(sB, prevT + ((long long)z * K + k0) * B, B, kc, kc, B);
         const int n = n0 + quarter * 32 + lane, c0 = 16 * half;
         const bool mine = n < N && c0 < kc;
-        float w[16], m[16], v[16];
         const long long o = wz + (long long)n * K + k0 + c0;
-        if (mine) {
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                *reinterpret_cast<float4*>(w + 4 * j) = reinterpret_cast<const float4*>(g.W[l] + o)[j];
-                *reinterpret_cast<float4*>(m + 4 * j) = reinterpret_cast<const float4*>(g.mW[l] + o)[j];
-                *reinterpret_cast<float4*>(v + 4 * j) = reinterpret_cast<const float4*>(g.vW[l] + o)[j];
-            }
-        }
+        float4 w = {}, m = {}, v = {};
+        auto fetch = [&](int j) {
+            w = reinterpret_cast<const float4*>(g.W[l] + o)[j];
+            m = reinterpret_cast<const float4*>(g.mW[l] + o)[j];
+            v = reinterpret_cast<const float4*>(g.vW[l] + o)[j];
+        };
+        if (mine) fetch(0);
         if (!product(kc, B)) return false;
         if (kt == 0 && threadIdx.x < MT && n0 + (int)threadIdx.x < N) {
             // the bias gradient: the row's B values in row order, from the staged operand
@@ -651,25 +682,33 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) k_train(const __grid_constan
             g.mb[l][bo] = mm;
             g.vb[l][bo] = vv;
         }
-        float d[16];
-        if (c0 < kc) load_acc16(tmem, quarter, c0, d);
-        if (mine) {
-#pragma unroll
-            for (int j = 0; j < 16; j++) w[j] = adam_one(g, s, d[j], m[j], v[j], w[j]);
-#pragma unroll
+        // four columns at a time, the next four's state on its way
+        if (c0 < kc) {
+#pragma unroll 1
             for (int j = 0; j < 4; j++) {
-                reinterpret_cast<float4*>(g.dW[l] + o)[j] = *reinterpret_cast<float4*>(d + 4 * j);
-                reinterpret_cast<float4*>(g.W[l] + o)[j] = *reinterpret_cast<float4*>(w + 4 * j);
-                reinterpret_cast<float4*>(g.mW[l] + o)[j] = *reinterpret_cast<float4*>(m + 4 * j);
-                reinterpret_cast<float4*>(g.vW[l] + o)[j] = *reinterpret_cast<float4*>(v + 4 * j);
+                __syncwarp();                          // the load below is the whole warp's
+                const float4 d = load_acc4(tmem, quarter, c0 + 4 * j);
+                if (mine) {
+                    float4 w1 = w, m1 = m, v1 = v;
+                    if (j < 3) fetch(j + 1);
+                    w1.x = adam_one(g, s, d.x, m1.x, v1.x, w1.x);
+                    w1.y = adam_one(g, s, d.y, m1.y, v1.y, w1.y);
+                    w1.z = adam_one(g, s, d.z, m1.z, v1.z, w1.z);
+                    w1.w = adam_one(g, s, d.w, m1.w, v1.w, w1.w);
+                    reinterpret_cast<float4*>(g.dW[l] + o)[j] = d;
+                    reinterpret_cast<float4*>(g.W[l] + o)[j] = w1;
+                    reinterpret_cast<float4*>(g.mW[l] + o)[j] = m1;
+                    reinterpret_cast<float4*>(g.vW[l] + o)[j] = v1;
+                    __nv_bfloat162 h[2] = {__floats2bfloat162_rn(w1.x, w1.y), __floats2bfloat162_rn(w1.z, w1.w)};
+                    *reinterpret_cast<uint2*>(g.Wb[l] + o + 4 * j) = *reinterpret_cast<uint2*>(h);
+                    __nv_bfloat16* t = g.WbT[l] + wz + (long long)(k0 + c0 + 4 * j) * N + n;
+                    t[0] = h[0].x;
+                    t[N] = h[0].y;
+                    t[2 * N] = h[1].x;
+                    t[3 * N] = h[1].y;
+                }
             }
-            uint4 lo, hi;
-            pack16(w, lo, hi);
-            uint4* wb = reinterpret_cast<uint4*>(g.Wb[l] + o);
-            wb[0] = lo;
-            wb[1] = hi;
-#pragma unroll
-            for (int j = 0; j < 16; j++) g.WbT[l][wz + (long long)(k0 + c0 + j) * N + n] = __float2bfloat16_rn(w[j]);
+            __syncwarp();
         }
         release();
         return true;
@@ -784,7 +823,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) k_train(const __grid_constan
         // ---- the updates that are left: layer 0, and layer 1 of a network with more than one
         const int w1 = L > 1 ? weight_tiles(1) : 0, w0 = weight_tiles(0);
         for (int tile = blockIdx.x; tile < w1 + w0 && ok; tile += gridDim.x)
-            ok = tile < w1 ? weight_tile(1, tile, s) : weight_tile(0, tile - w1, s);
+            ok = weight_tile(tile < w1 ? 1 : 0, tile < w1 ? tile : tile - w1, s);
         ok = ok && net_sync(g.bar + z, target, g.err);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -1014,9 +1053,9 @@ extern "C" sbx_status sbx_mlp_train(sbx_ctx* ctx, const sbx_mlp_net* net, const 
     int per = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_train, TRAIN_THREADS, smem) != cudaSuccess || per < 1)
         return fail(ctx, SBX_ECUDA, "sbx_mlp_train: occupancy");
-    // a network's blocks: one an SM, no more than a backward pass has tiles (two products of 16)
-    int gx = sm_count(ctx) / net->nz;
-    if (gx < 1) return fail(ctx, SBX_EINVAL, "sbx_mlp_train: more networks than SMs");
+    // a network's blocks: all resident, no more than a backward pass has tiles (two products of 16)
+    int gx = per * sm_count(ctx) / net->nz;
+    if (gx < 1) return fail(ctx, SBX_EINVAL, "sbx_mlp_train: more networks than resident blocks");
     if (gx > 32) gx = 32;
     TrainArgs g{};
     g.net = net_of(net);
