@@ -615,8 +615,8 @@ void step_carve(Arena& m, FusedArgs& a, int cellSlots) {
     m.take(a.cellHead, 4 * C); m.take(a.cellNext, 4 * (size_t)a.cap);
     m.take(a.nextA, 4 * nLk); m.take(a.nextB, 4 * nLk); m.take(a.nextM, 4 * (size_t)a.nM);
     m.take(a.segE1, 16 * nS); m.take(a.segE2, 16 * nS);
-    m.take(a.joints, 2 * nS * FUSED_JOINT_BYTES);
-    m.take(a.terms, (2 * (size_t)a.nM + 4 * (size_t)a.nD) * FUSED_TERM_BYTES);
+    m.take(a.joints, 8 * nS * FUSED_JOINT_PLANES);
+    m.take(a.terms, 8 * (FUSED_MOTOR_PLANES * (size_t)a.nM + FUSED_DIMER_PLANES * (size_t)a.nD));
     m.take(a.uSnap, 12 * nS);
     m.take(a.reachMax, 4);
     m.take(a.err, 16);

@@ -386,9 +386,8 @@ __device__ void phase_motors_links(const FusedArgs& a, FusedSmem& sm, int t) {
     for (int w = blockIdx.x; w < units; w += gridDim.x) {
         if (w < a.nBb) {
             // the sub-bodies on three warps, the backbone on the fourth
-            if (threadIdx.x < 96) mini_bodies(a, sm.mini, w, GlobalTerms{a});
-            else if (threadIdx.x == 96)
-                mini_backbone(a, w, t, GlobalTerms{a}, a.sc.boxParams, a.sc.mini.bbBodyParams[0]);
+            if (threadIdx.x < 96) mini_bodies(a, sm.mini, w);
+            else if (threadIdx.x == 96) mini_backbone(a, w, t, a.sc.boxParams, a.sc.mini.bbBodyParams[0]);
             __syncthreads();
         } else {
             int k = (w - a.nBb) * blockDim.x + threadIdx.x;
@@ -405,7 +404,6 @@ __device__ void phase_motors_links(const FusedArgs& a, FusedSmem& sm, int t) {
     int helpers = (int)gridDim.x - units, h0 = units;
     if (helpers <= 0) { helpers = gridDim.x; h0 = 0; }
     if ((int)blockIdx.x >= h0) {
-        ChainJoint* J = reinterpret_cast<ChainJoint*>(a.joints);
         const int n = a.nSeg;
         const int nJ = a.jointShare ? n : 0, total = nJ + 3 * n;
         const int g = ((int)blockIdx.x - h0) * blockDim.x + threadIdx.x, H = helpers * blockDim.x;
@@ -426,13 +424,14 @@ __device__ void phase_motors_links(const FusedArgs& a, FusedSmem& sm, int t) {
                     ChainParams cp = chain_params(fs.chainParams);
                     const RodGeom me = load_rod(n, i, fb.coord, fb.uVec, fb.segLength, fb.bTransGam, fb.bRotGam);
                     const int side = s2 > i ? 0 : 1, nb = side == 0 ? s2 : s1;
-                    J[2 * i + side] = chain_joint(cp, i, side, nb, side == 0 ? d2 : d1, me,
-                                                  load_rod(n, nb, fb.coord, fb.uVec, fb.segLength, fb.bTransGam,
-                                                           fb.bRotGam));
+                    joint_store(a, i, side,
+                                chain_joint(cp, i, side, nb, side == 0 ? d2 : d1, me,
+                                            load_rod(n, nb, fb.coord, fb.uVec, fb.segLength, fb.bTransGam, fb.bRotGam)));
                     if (side == 0 && s1 > i)
-                        J[2 * i + 1] = chain_joint(cp, i, 1, s1, d1, me,
-                                                   load_rod(n, s1, fb.coord, fb.uVec, fb.segLength, fb.bTransGam,
-                                                            fb.bRotGam));
+                        joint_store(a, i, 1,
+                                    chain_joint(cp, i, 1, s1, d1, me,
+                                                load_rod(n, s1, fb.coord, fb.uVec, fb.segLength, fb.bTransGam,
+                                                         fb.bRotGam)));
                 }
             } else {
                 const int r = q - nJ, c = r / n, i = r - c * n;
@@ -595,11 +594,10 @@ __device__ bool rod_unit(const FusedArgs& a, RodSmem& rs, int u, int t, uint64_t
         return r;
     };
     // this rod's two joints (computed in the minifilament phase), loaded ahead of use
-    const ChainJoint* Jg = reinterpret_cast<const ChainJoint*>(a.joints);
     ChainJoint j2, j1;
     if (a.jointShare && tid < cnt) {
-        if (s2 >= 0) j2 = Jg[s2 > i ? 2 * i : 2 * s2 + (1 - n2)];
-        if (s1 >= 0) j1 = Jg[s1 > i ? 2 * i + 1 : 2 * s1 + (1 - n1)];
+        if (s2 >= 0) j2 = s2 > i ? joint_load(a, i, 0) : joint_load(a, s2, 1 - n2);
+        if (s1 >= 0) j1 = s1 > i ? joint_load(a, i, 1) : joint_load(a, s1, 1 - n1);
     }
     // the link CSR payloads of the group's rows (link A, link B), one entry per thread
     const int eA = a.xlOn ? rs.off[0][cnt] - rs.off[0][0] : 0;

@@ -11,8 +11,11 @@ constexpr int FUSED_ENT_CAP = 256;    // CSR payload entries a rod CTA stages in
 constexpr int FUSED_MCAP = 16;        // motor reactions per segment a rod CTA stages in shared memory
 constexpr int FUSED_MIDS = 16;        // motor slots per segment a rod CTA sorts (more: repeated-minimum walk)
 constexpr int FUSED_CELL_SLOTS = 4;   // fixed slots per grid cell
-constexpr int FUSED_JOINT_BYTES = 64; // one chain joint (ChainJoint, padded)
-constexpr int FUSED_TERM_BYTES = 80;  // one position-only myosin term (MotorJoint, CoupleTerm, LeverTerm, TetherTerm)
+// planes of a rod's chain joints (two sides: six doubles and a flag each) and of the position-only
+// myosin terms: a motor's two joints (nine doubles each), a dimer's two end variants (nine and a
+// flag), lever torsion (three and a flag) and tether (six, a flag and six floats)
+constexpr int FUSED_JOINT_PLANES = 13;
+constexpr int FUSED_MOTOR_PLANES = 18, FUSED_DIMER_PLANES = 34;
 constexpr int FUSED_ROW_SLOTS = 4;    // fixed slots per segment row of link A ends, of link B ends
 constexpr int FUSED_MOTOR_SLOTS = 16; // fixed slots per segment row of bound motors
 constexpr int FUSED_MIN_HELPERS = 16; // CTAs kept free of rod units in the rod phase
@@ -32,11 +35,10 @@ struct FusedArgs {
     // private scratch (plan-owned)
     int *cntCell, *cntSeg, *cntAct, *cntA, *cntB, *cntM;   // cntSeg: segments per cell
     int* segCellOff;         // segment-only exclusive prefix over cells (C + 1)
-    void* joints;            // chain joints at (owner rod, owner side): 2 * nSeg slots of FUSED_JOINT_BYTES
-    // the position-only myosin terms of the step, 2 nM + 4 nD slots of FUSED_TERM_BYTES:
-    // motor joints [which][motor], coupling end variants [dimer][variant], lever torsion
-    // [dimer], tethers [dimer]
-    void* terms;
+    double* joints;          // chain joints by owner rod: FUSED_JOINT_PLANES planes of nSeg
+    // the position-only myosin terms of the step: FUSED_MOTOR_PLANES planes of nM doubles, then
+    // FUSED_DIMER_PLANES planes of nD
+    double* terms;
     int* tileSum;            // tile sums of the step's scans (cells, segments, link A, link B)
     int* mTileSum;           // tile sums of the motor CSR scan
     // rows of the step's inverse maps (cells -> bodies, segments -> link A/B ends,

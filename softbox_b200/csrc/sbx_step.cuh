@@ -18,10 +18,6 @@ constexpr int ERR_REACH_OVERFLOW = 2, ERR_LIST = 8;
 struct MiniSmem {
     float sF[3 * FUSED_MAX_SUB], sT[3 * FUSED_MAX_SUB];
 };
-static_assert(sizeof(ChainJoint) <= FUSED_JOINT_BYTES, "joint slot size");
-static_assert(sizeof(MotorJoint) <= FUSED_TERM_BYTES && sizeof(CoupleTerm) <= FUSED_TERM_BYTES &&
-                  sizeof(LeverTerm) <= FUSED_TERM_BYTES && sizeof(TetherTerm) <= FUSED_TERM_BYTES,
-              "myosin term slot size");
 
 // BrownianForceSystem.brownianForce (BrownianForceSystem.java:44-106), component j (0..2) of
 // one slot: the slot's j-th Box-Muller pair gives its random force and torque components j
@@ -190,27 +186,98 @@ __device__ void tile_scan(const ScanArr* arrs, int narr, const int* tileSum, int
 }
 
 // ---------------------------------------------------------------- binding and minifilaments
-// slots of the step's myosin terms (FusedArgs::terms)
-__device__ __forceinline__ MotorJoint& term_joint(const FusedArgs& a, int m, int which) {
-    return *reinterpret_cast<MotorJoint*>((char*)a.terms + ((size_t)which * a.nM + m) * FUSED_TERM_BYTES);
+// The step's joints and myosin terms as planes: the lanes of a warp write and read consecutive
+// items of a plane (as one struct after another a warp's 16-byte accesses touched 20 lines
+// each: at 500,000 rods the terms kernel went from 42 to 27 us, the step from 377 to 370, at
+// 100,000 from 102 to 96.5).
+__device__ __forceinline__ void joint_store(const FusedArgs& a, int i, int side, const ChainJoint& J) {
+    const size_t n = a.nSeg;
+    double* p = a.joints + 6 * n * side + i;
+    p[0] = J.forceMag; p[n] = J.luX; p[2 * n] = J.luY; p[3 * n] = J.luZ; p[4 * n] = J.invMag; p[5 * n] = J.torsionMag;
+    reinterpret_cast<int*>(a.joints + 12 * n)[n * side + i] = J.tvOK;
 }
-__device__ __forceinline__ CoupleTerm& term_couple(const FusedArgs& a, int d, int variant) {
-    return *reinterpret_cast<CoupleTerm*>((char*)a.terms + (2 * (size_t)a.nM + 2 * d + variant) * FUSED_TERM_BYTES);
-}
-__device__ __forceinline__ LeverTerm& term_lever(const FusedArgs& a, int d) {
-    return *reinterpret_cast<LeverTerm*>((char*)a.terms + (2 * (size_t)a.nM + 2 * (size_t)a.nD + d) * FUSED_TERM_BYTES);
-}
-__device__ __forceinline__ TetherTerm& term_tether(const FusedArgs& a, int d) {
-    return *reinterpret_cast<TetherTerm*>((char*)a.terms + (2 * (size_t)a.nM + 3 * (size_t)a.nD + d) * FUSED_TERM_BYTES);
+__device__ __forceinline__ ChainJoint joint_load(const FusedArgs& a, int i, int side) {
+    const size_t n = a.nSeg;
+    const double* p = a.joints + 6 * n * side + i;
+    ChainJoint J;
+    J.forceMag = p[0]; J.luX = p[n]; J.luY = p[2 * n]; J.luZ = p[3 * n]; J.invMag = p[4 * n]; J.torsionMag = p[5 * n];
+    J.tvOK = reinterpret_cast<const int*>(a.joints + 12 * n)[n * side + i];
+    return J;
 }
 
-// the step's terms in global memory
 struct GlobalTerms {
     const FusedArgs& a;
-    __device__ __forceinline__ const MotorJoint& joint(int m, int which) const { return term_joint(a, m, which); }
-    __device__ __forceinline__ const CoupleTerm& couple(int d, int v) const { return term_couple(a, d, v); }
-    __device__ __forceinline__ const LeverTerm& lever(int d) const { return term_lever(a, d); }
-    __device__ __forceinline__ const TetherTerm& tether(int d) const { return term_tether(a, d); }
+    __device__ __forceinline__ double* motor(int which, int m) const { return a.terms + (size_t)9 * a.nM * which + m; }
+    __device__ __forceinline__ double* dimer(int plane, int d) const {
+        return a.terms + (size_t)FUSED_MOTOR_PLANES * a.nM + (size_t)plane * a.nD + d;
+    }
+    __device__ __forceinline__ MotorJoint joint(int m, int which) const {
+        const double* p = motor(which, m);
+        const size_t n = a.nM;
+        MotorJoint J;
+        J.forceMag = p[0]; J.lx = p[n]; J.ly = p[2 * n]; J.lz = p[3 * n];
+        J.tvx = p[4 * n]; J.tvy = p[5 * n]; J.tvz = p[6 * n]; J.tm[0] = p[7 * n]; J.tm[1] = p[8 * n];
+        return J;
+    }
+    __device__ __forceinline__ void put(int m, int which, const MotorJoint& J) const {
+        double* p = motor(which, m);
+        const size_t n = a.nM;
+        p[0] = J.forceMag; p[n] = J.lx; p[2 * n] = J.ly; p[3 * n] = J.lz;
+        p[4 * n] = J.tvx; p[5 * n] = J.tvy; p[6 * n] = J.tvz; p[7 * n] = J.tm[0]; p[8 * n] = J.tm[1];
+    }
+    __device__ __forceinline__ CoupleTerm couple(int d, int v) const {
+        const double* p = dimer(10 * v, d);
+        const size_t n = a.nD;
+        CoupleTerm C;
+        C.FAx = p[0]; C.FAy = p[n]; C.FAz = p[2 * n]; C.TAx = p[3 * n]; C.TAy = p[4 * n]; C.TAz = p[5 * n];
+        C.TBx = p[6 * n]; C.TBy = p[7 * n]; C.TBz = p[8 * n];
+        C.ok = *reinterpret_cast<const int*>(p + 9 * n);
+        return C;
+    }
+    __device__ __forceinline__ void put(int d, int v, const CoupleTerm& C) const {
+        double* p = dimer(10 * v, d);
+        const size_t n = a.nD;
+        *reinterpret_cast<int*>(p + 9 * n) = C.ok;
+        if (!C.ok) return;
+        p[0] = C.FAx; p[n] = C.FAy; p[2 * n] = C.FAz; p[3 * n] = C.TAx; p[4 * n] = C.TAy; p[5 * n] = C.TAz;
+        p[6 * n] = C.TBx; p[7 * n] = C.TBy; p[8 * n] = C.TBz;
+    }
+    __device__ __forceinline__ LeverTerm lever(int d) const {
+        const double* p = dimer(20, d);
+        const size_t n = a.nD;
+        LeverTerm L;
+        L.px = p[0]; L.py = p[n]; L.pz = p[2 * n];
+        L.ok = *reinterpret_cast<const int*>(p + 3 * n);
+        return L;
+    }
+    __device__ __forceinline__ void put(int d, const LeverTerm& L) const {
+        double* p = dimer(20, d);
+        const size_t n = a.nD;
+        *reinterpret_cast<int*>(p + 3 * n) = L.ok;
+        if (!L.ok) return;
+        p[0] = L.px; p[n] = L.py; p[2 * n] = L.pz;
+    }
+    // (the rows' floats take three planes of doubles, as six planes of floats)
+    __device__ __forceinline__ float* row(int d) const { return reinterpret_cast<float*>(dimer(31, 0)) + d; }
+    __device__ __forceinline__ TetherTerm tether(int d) const {
+        const double* p = dimer(24, d);
+        const size_t n = a.nD;
+        TetherTerm T;
+        T.Fx = p[0]; T.Fy = p[n]; T.Fz = p[2 * n]; T.Tx = p[3 * n]; T.Ty = p[4 * n]; T.Tz = p[5 * n];
+        const int ok = *reinterpret_cast<const int*>(p + 6 * n);
+        T.fOK = ok & 1;
+        T.tOK = ok >> 1;
+        return T;
+    }
+    __device__ __forceinline__ void put(int d, const TetherTerm& T) const {
+        double* p = dimer(24, d);
+        const size_t n = a.nD;
+        if (T.fOK) { p[0] = T.Fx; p[n] = T.Fy; p[2 * n] = T.Fz; }
+        if (T.tOK) { p[3 * n] = T.Tx; p[4 * n] = T.Ty; p[5 * n] = T.Tz; }
+        *reinterpret_cast<int*>(p + 6 * n) = (T.fOK ? 1 : 0) | (T.tOK ? 2 : 0);
+        float* q = row(d);
+        for (int j = 0; j < 6; j++) q[j * n] = T.row[j];
+    }
 };
 
 // The reach of a segment's points from its centre, the largest coordinate difference of its ends
@@ -381,9 +448,8 @@ __device__ __forceinline__ void bond_store(const FusedArgs& a, int m, float out[
 // MiniFilamentSystem.backboneGather over backbone u's CSR row (its dimers, ascending;
 // MiniFilamentSystem.java:140-147), then walls, integration and derived geometry; the
 // reference's CSR arrays (rows = backbones, items = dimers in index order)
-template <class Terms>
-__device__ __forceinline__ void mini_backbone(const FusedArgs& a, int u, int t, const Terms& terms,
-                                              const float* boxParams, float dt) {
+__device__ __forceinline__ void mini_backbone(const FusedArgs& a, int u, int t, const float* boxParams, float dt) {
+    const GlobalTerms terms{a};
     const sbx_minifilament_store& mini = a.sc.mini;
     const sbx_rigid_body& bb = mini.backbone;
     const int dpm = a.dpm, nBb = a.nBb, d0 = u * dpm;
@@ -392,9 +458,10 @@ __device__ __forceinline__ void mini_backbone(const FusedArgs& a, int u, int t, 
     if (u == nBb - 1) mini.bbDimerOffsets[nBb] = d0 + dpm;
     double f[3] = {0, 0, 0}, tq[3] = {0, 0, 0};
     for (int d = d0; d < d0 + dpm; d++) {
-        const float* p = terms.tether(d).row;        // the dimer's miniData row
-        f[0] += p[0]; f[1] += p[1]; f[2] += p[2];
-        tq[0] += p[3]; tq[1] += p[4]; tq[2] += p[5];
+        const float* p = terms.row(d);                // the dimer's miniData row
+        const size_t n = a.nD;
+        f[0] += p[0]; f[1] += p[n]; f[2] += p[2 * n];
+        tq[0] += p[3 * n]; tq[1] += p[4 * n]; tq[2] += p[5 * n];
     }
     float F[3], T[3];
     for (int k = 0; k < 3; k++) { F[k] = (float)(0.0f + f[k]); T[k] = (float)(0.0f + tq[k]); }
@@ -409,8 +476,8 @@ __device__ __forceinline__ void mini_backbone(const FusedArgs& a, int u, int t, 
 // the position-only terms ran before). Each sub-body accumulates its terms in the order of the
 // reference's System sequence (joints, coupling, tether; the head's bond after its joint): a
 // warp for the heads, the rods, the levers; then they integrate in body order.
-template <class Terms>
-__device__ __forceinline__ void mini_bodies(const FusedArgs& a, MiniSmem& ms, int u, const Terms& terms) {
+__device__ __forceinline__ void mini_bodies(const FusedArgs& a, MiniSmem& ms, int u) {
+    const GlobalTerms terms{a};
     const sbx_dense_scene& sc = a.sc;
     const sbx_motor_store& mot = sc.mot;
     const sbx_rigid_body& mb = mot.body;
@@ -494,23 +561,23 @@ __device__ __forceinline__ void myosin_term(const FusedArgs& a, int k) {
     const sbx_minifilament_store& mini = sc.mini;
     const sbx_rigid_body& bb = mini.backbone;
     const int nM = a.nM, nD = a.nD, nB = a.nB;
+    const GlobalTerms terms{a};
     if (k < 2 * nM) {
         const int which = k >= nM, m = k - which * nM;
-        term_joint(a, m, which) = motor_joint(m, which, nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam,
-                                              mb.bRotGam, mot.jointParams);
+        terms.put(m, which, motor_joint(m, which, nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam, mb.bRotGam,
+                                        mot.jointParams));
     } else if (k < 2 * nM + 2 * nD) {
-        const int q = k - 2 * nM, d = q >> 1;
-        term_couple(a, d, q & 1) = couple_variant(nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam, mb.bRotGam,
-                                                  2 * d, 2 * d + 1, sc.dim.parallel[d] != 0, sc.dim.dimerParams,
-                                                  q & 1);
+        const int v = k >= 2 * nM + nD, d = k - 2 * nM - v * nD;
+        terms.put(d, v, couple_variant(nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam, mb.bRotGam, 2 * d, 2 * d + 1,
+                                       sc.dim.parallel[d] != 0, sc.dim.dimerParams, v));
     } else if (k < 2 * nM + 3 * nD) {
         const int d = k - 2 * nM - 2 * nD;
-        term_lever(a, d) = couple_lever(nB, mb.uVec, mb.bRotGam, 2 * d, 2 * d + 1, sc.dim.dimerParams);
+        terms.put(d, couple_lever(nB, mb.uVec, mb.bRotGam, 2 * d, 2 * d + 1, sc.dim.dimerParams));
     } else {
         const int d = k - 2 * nM - 3 * nD, u = d / a.dpm;
         TetherTerm T = tether_terms(nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam, mb.bRotGam, a.nBb, bb.coord,
                                     bb.uVec, mini.bbInvDragY, u, 2 * d, mini.attachAxial[d], mini.miniParams);
-        term_tether(a, d) = T;
+        terms.put(d, T);
         float* o = mini.miniData + (int64_t)MINI_STRIDE * d;
         for (int j = 0; j < 6; j++) o[j] = T.row[j];
         // backbone CSR of the reference (rows = backbones, items = dimers in index order)

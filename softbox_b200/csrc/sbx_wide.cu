@@ -16,8 +16,8 @@
 // what a later kernel reads again is written once.
 // Every slot is computed by the same device functions as the per-system kernels, in the
 // reference's accumulation order: the same bits.
-// A step takes 105 us at 100,000 rods and 375 us at 500,000 (200 and 434 as the per-system
-// sequence), a packed step of 12 networks (0.17e6 rods, 0.18e6 heads) 280 us (366).
+// A step takes 97 us at 100,000 rods and 370 us at 500,000 (200 and 434 as the per-system
+// sequence), a packed step of 12 networks (0.17e6 rods, 0.18e6 heads) 269 us (366).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -130,15 +130,14 @@ __global__ void __launch_bounds__(128, 5) k_wide_joints(const __grid_constant__ 
     int s2 = fs.end2NbrSlot[i], s1 = fs.end1NbrSlot[i];
     if (!SBX_IDX_OK_OR_NONE(s2, n, CK_NEIGHBOUR)) s2 = -1;
     if (!SBX_IDX_OK_OR_NONE(s1, n, CK_NEIGHBOUR)) s1 = -1;
-    ChainJoint* J = reinterpret_cast<ChainJoint*>(a.joints);
     const ChainParams cp = chain_params(fs.chainParams);
     for (int side = 0; side < 2; side++) {
         const int nb = side == 0 ? s2 : s1;
         if (nb <= i) continue;
-        J[2 * (int64_t)i + side] =
-            chain_joint(cp, i, side, nb, side == 0 ? fs.end2NbrSide[i] : fs.end1NbrSide[i],
-                        load_rod(n, i, fb.coord, fb.uVec, fb.segLength, fb.bTransGam, fb.bRotGam),
-                        load_rod(n, nb, fb.coord, fb.uVec, fb.segLength, fb.bTransGam, fb.bRotGam));
+        joint_store(a, i, side,
+                    chain_joint(cp, i, side, nb, side == 0 ? fs.end2NbrSide[i] : fs.end1NbrSide[i],
+                                load_rod(n, i, fb.coord, fb.uVec, fb.segLength, fb.bTransGam, fb.bRotGam),
+                                load_rod(n, nb, fb.coord, fb.uVec, fb.segLength, fb.bTransGam, fb.bRotGam)));
     }
 }
 
@@ -476,12 +475,12 @@ __global__ void __launch_bounds__(MINI_THREADS) k_wide_mini(const __grid_constan
     const FusedArgs& a = w.a;
     const sbx_minifilament_store& mini = a.sc.mini;
     if ((int)blockIdx.x < a.nBb) {
-        mini_bodies(a, sm, blockIdx.x, GlobalTerms{a});
+        mini_bodies(a, sm, blockIdx.x);
         return;
     }
     const int u = (blockIdx.x - a.nBb) * MINI_THREADS + threadIdx.x;
     if (u >= a.nBb) return;
-    mini_backbone(a, u, mini.bbCounts[1], GlobalTerms{a}, B ? w.bt.boxParams + 8 * w.bt.bbKey[2 * u] : a.sc.boxParams,
+    mini_backbone(a, u, mini.bbCounts[1], B ? w.bt.boxParams + 8 * w.bt.bbKey[2 * u] : a.sc.boxParams,
                   B ? mini.bbBodyParams[0] : a.sc.boxParams[7]);
 }
 
@@ -624,7 +623,6 @@ __global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ Wi
     me.cx = in.p.c[0]; me.cy = in.p.c[1]; me.cz = in.p.c[2];
     me.ux = in.p.u[0]; me.uy = in.p.u[1]; me.uz = in.p.u[2];
     me.len = in.len; me.bTGx = in.gT[0]; me.bTGy = in.gT[1]; me.bRGy = in.gR[1];
-    const ChainJoint* Jg = reinterpret_cast<const ChainJoint*>(a.joints);
     for (int side = 0; side < 2; side++) {
         int slot = slots[side];
         const int nside = sides[side];
@@ -634,13 +632,13 @@ __global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ Wi
         ChainJoint J;
         bool have = slot > i;
         if (have) {
-            J = Jg[2 * (int64_t)i + side];
+            J = joint_load(a, i, side);
         } else if (nside == 0 || nside == 1) {
             const int ps = 1 - nside;                    // the partner's side facing rod i
             const int back = ps == 0 ? fs.end2NbrSlot[slot] : fs.end1NbrSlot[slot];
             const int backSide = ps == 0 ? fs.end2NbrSide[slot] : fs.end1NbrSide[slot];
             have = slot < i && back == i && backSide == 1 - side;
-            if (have) J = Jg[2 * (int64_t)slot + ps];
+            if (have) J = joint_load(a, slot, ps);
         }
         if (!have) J = chain_joint(cp, i, side, slot, nside, me, nb);
         chain_apply(cp, i, side, slot, nside, me, nb, J, fd, td);
