@@ -330,10 +330,14 @@ struct GridView {
     int nX, nY, nZ;
     const int* off;              // segment-only cell offsets of the grid's first cell
 };
-template <int W>
+struct NoWait {
+    __device__ void operator()() const {}
+};
+// (ready() comes before the first read of the endpoints)
+template <int W, class Ready = NoWait>
 __device__ int group_reach_bind(const FusedArgs& a, const GridView& gv, int lane, bool valid, float mx, float my, float mz, float mux,
                                 float muy, float muz, float rux, float ruy, float ruz, int* out, float tol,
-                                float align, int* bestSeg, float* bestArc) {
+                                float align, int* bestSeg, float* bestArc, Ready ready = Ready()) {
     static_assert(W == 8 || W == 16, "a group of 8 or 16 lanes walks one head");
     const float* gp = gv.gp;
     const int* off = gv.off;
@@ -386,6 +390,7 @@ __device__ int group_reach_bind(const FusedArgs& a, const GridView& gv, int lane
     const unsigned lower = (1u << hl) - 1u;
     int cnt = 0, best = -1;
     float bestD = 1.0e30f, arc = 0.f;
+    ready();
     for (int k0 = 0; k0 < totalMax; k0 += W) {
         const int k = k0 + hl;
         bool pass = false;

@@ -1,14 +1,20 @@
 // sbx_wide.cu — the dense contractile step (DenseContractileHarness.cpuStep,
 // DenseContractileHarness.java:350-429) as fourteen wide kernels, single or packed networks.
 //
-//   main stream                                    ahead         link               csr
-//   publish: body view, cells, row slots           draws         rows, unbinding
-//   scan: cell offsets                             myosin terms  scan
-//   place: contents, endpoints in cell order       joints        forces, lists
-//   bind: release, reach, nearest, cycle
-//   mini: one block a minifilament  <- draws, terms                                 scan
-//   rods: gathers, walls, integrate <- joints, link                                 lists
+//   main stream                                      ahead          link               csr
+//   publish: body view, release, cells, row slots    draws          rows, unbinding
+//   scan: cell offsets                               myosin terms   scan
+//   place: contents, endpoints in cell order         joints         forces, lists
+//   bind: reach, nearest, cycle
+//   mini: one block a minifilament <- all ahead, links                                 scan
+//   rods: gathers, walls, integration                                                  lists
 //
+// At the small sizes a step is a chain of latencies, so a kernel with one predecessor starts
+// before that one is done (programmatic dependent launch): it reads and computes what it does not
+// take from it, then waits (after_previous). A kernel lets the next start after its own wait
+// (let_next_start), so that whatever comes before the predecessor is complete by then. mini has
+// several predecessors and waits for all of them at its launch; rods then has one, and does the
+// chain and the links while the minifilaments are computed.
 // The per-system sequence (sbx_dense.cu: dense_sequence) takes 53 launches: five counting sorts
 // of five kernels and many kernels of 3-5 us each, in a row. Here the inverse maps are made as
 // the fused kernel makes them (fixed slots per row filled by atomics, placed by rank), what
@@ -16,8 +22,9 @@
 // what a later kernel reads again is written once.
 // Every slot is computed by the same device functions as the per-system kernels, in the
 // reference's accumulation order: the same bits.
-// A step takes 97 us at 100,000 rods and 370 us at 500,000 (200 and 434 as the per-system
-// sequence), a packed step of 12 networks (0.17e6 rods, 0.18e6 heads) 269 us (366).
+// A step takes 35 us at 1,000 rods, 47 at 20,000, 90 at 100,000 and 356 at 500,000 (46, 57, 97 and
+// 370 with full waits; 200 and 434 at the last two as the per-system sequence), a packed
+// step of 12 networks (0.17e6 rods, 0.18e6 heads) 250 us (269; 366).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -45,6 +52,15 @@ __device__ __forceinline__ GridView grid_view(const WideArgs& w, int net) {
     }
     return GridView{g.gridParams, g.gridDims[0], g.gridDims[1], g.gridDims[2], w.a.segCellOff};
 }
+
+// the kernel before this one in its stream is complete, and what it wrote can be read
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// the next kernel of the stream may start its blocks once every block is here or done
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+struct AfterPrevious {
+    __device__ __forceinline__ void operator()() const { after_previous(); }
+};
 
 // a link end names a rod; one at or past the rod count is left out and reported
 __device__ __forceinline__ bool end_ok(const WideArgs& w, int s) {
@@ -142,11 +158,13 @@ __global__ void __launch_bounds__(128, 5) k_wide_joints(const __grid_constant__ 
 }
 
 // ---------------------------------------------------------------- publish
-// The body view, the cells with their row slots and tile sums, the start view's orientations
+// The body view, the release of the heads, the cells with their row slots and tile sums, the
+// largest reach of a segment from its centre, the start view's orientations
 // (the rods kernel reads a neighbour from the start view: its own block may have stepped it
 // already) and the step's counts.
 template <bool B>
 __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ WideArgs w) {
+    let_next_start();
     const FusedArgs& a = w.a;
     const sbx_dense_scene& sc = a.sc;
     const sbx_grid_state& g = sc.grid;
@@ -160,6 +178,7 @@ __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ Wi
         if (a.xlOn) { sc.xl.counts[1] = t; sc.xl.counts[2] = sc.seed; }
     }
     int cell = -1;
+    float span = 0.f;
     if (i < nSeg + nM) {
         float c[3];
         int net;
@@ -167,11 +186,17 @@ __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ Wi
             const sbx_rigid_body& fb = sc.fil.body;
             const int* state = sc.fil.filState;              // FREE (< 0) slots of turnover, or none
             // (all loads before the first store: nothing tells the compiler that they differ)
-            float u[3];
-            for (int k = 0; k < 3; k++) { c[k] = fb.coord[k * nSeg + i]; u[k] = fb.uVec[k * nSeg + i]; }
+            float u[3], e1[3], e2[3];
+            for (int k = 0; k < 3; k++) {
+                c[k] = fb.coord[k * nSeg + i];
+                u[k] = fb.uVec[k * nSeg + i];
+                e1[k] = fb.end1[k * nSeg + i];
+                e2[k] = fb.end2[k * nSeg + i];
+            }
             const float r = 0.5f * fb.segLength[i] + g.viewParams[0];
             const int owner = (state && state[i] < 0) ? STORE_NONE : STORE_FILAMENT;
             net = key_of<B>(w.bt.segKey, i).x;
+            if (owner == STORE_FILAMENT) span = segment_span(c, e1, e2);
             for (int k = 0; k < 3; k++) a.uSnap[k * nSeg + i] = u[k];
             g.boundingRadius[i] = r;
             g.ownerStore[i] = owner;
@@ -189,7 +214,14 @@ __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ Wi
                 ru[k] = mb.uVec[k * nB + r];
                 c[k] = mb.coord[k * nB + h] + 0.5f * hl * u[k];
             }
-            net = key_of<B>(w.bt.motKey, m).x;
+            // the catch-slip release and cooldown (NucleotideCycleSystem.java:77-134): previous step's
+            // forces only
+            const sbx_motor_store& mot = sc.mot;
+            const int2 key = key_of<B>(w.bt.motKey, m);
+            int bs = mot.boundSeg[m], cd = mot.cooldown[m], sb = mot.stats[2 * m], sr = mot.stats[2 * m + 1],
+                cs = mot.capStats[m];
+            const float dot = mot.forceDotFil[m], mag = mot.forceMag[m];
+            net = key.x;
             for (int k = 0; k < 3; k++) {
                 sc.mot.head[k * nM + m] = c[k];
                 sc.mot.uVec[k * nM + m] = u[k];
@@ -198,6 +230,9 @@ __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ Wi
             g.boundingRadius[i] = reach;
             g.ownerStore[i] = STORE_MOTOR;
             g.ownerSlot[i] = m;
+            release_one(key.y, bs, cd, sb, sr, cs, dot, mag, mot.kinParams, *a.d_step, B ? w.bt.seeds[3 * key.x] : sc.seed);
+            mot.boundSeg[m] = bs; mot.cooldown[m] = cd; mot.stats[2 * m] = sb; mot.stats[2 * m + 1] = sr;
+            mot.capStats[m] = cs;
         }
         for (int k = 0; k < 3; k++) g.center[k * cap + i] = c[k];
         if (i < g.gridCounts[1]) {
@@ -216,6 +251,7 @@ __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ Wi
     const int tile = cell >= 0 ? cell / WIDE_TILE : -1;
     tile_add(w.sumCell, tile);
     tile_add(w.sumSeg, i < nSeg ? tile : -1);
+    span_max(a.reachMax, span);
     stat_add(a, ST_CELL_LIST, over);
 }
 
@@ -224,6 +260,7 @@ __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ Wi
 // (CrosslinkerSystem.java:727-756) and the active counts (:694-708)
 template <bool B>
 __global__ void __launch_bounds__(128) k_wide_link_rows(const __grid_constant__ WideArgs w) {
+    let_next_start();
     const FusedArgs& a = w.a;
     const sbx_dense_scene& sc = a.sc;
     const sbx_crosslinker_store& xl = sc.xl;
@@ -319,78 +356,69 @@ __device__ void scan_one_tile(int tile, int tiles, int* cnt, int n, const int* s
 }
 
 __global__ void __launch_bounds__(256) k_wide_cell_scan(const __grid_constant__ WideArgs w) {
+    after_previous();
+    let_next_start();
     const FusedArgs& a = w.a;
     const sbx_grid_state& g = a.sc.grid;
     const int b = blockIdx.x;
     if (b < w.tilesC)
-        scan_one_tile(b, w.tilesC, a.cntCell, a.C, w.sumCell, g.gridCellOffsets, g.cellCount, a.cap, g.chunkSum, false);
+        scan_one_tile(b, w.tilesC, a.cntCell, a.C, w.sumCell, g.gridCellOffsets, g.cellCount, a.cap, g.chunkSum, true);
     else
         scan_one_tile(b - w.tilesC, w.tilesC, a.cntSeg, a.C, w.sumSeg, a.segCellOff, nullptr, a.nSeg, nullptr, false);
 }
 
 __global__ void __launch_bounds__(256) k_wide_link_scan(const __grid_constant__ WideArgs w) {
+    after_previous();
+    let_next_start();
     const FusedArgs& a = w.a;
     const sbx_crosslinker_store& xl = a.sc.xl;
     const int b = blockIdx.x;
     if (b < w.tilesS)
-        scan_one_tile(b, w.tilesS, a.cntA, a.nSeg, w.sumA, xl.segOffsetsA, xl.segCountA, a.nL, nullptr, false);
+        scan_one_tile(b, w.tilesS, a.cntA, a.nSeg, w.sumA, xl.segOffsetsA, xl.segCountA, a.nL, nullptr, true);
     else
-        scan_one_tile(b - w.tilesS, w.tilesS, a.cntB, a.nSeg, w.sumB, xl.segOffsetsB, xl.segCountB, a.nL, nullptr, false);
+        scan_one_tile(b - w.tilesS, w.tilesS, a.cntB, a.nSeg, w.sumB, xl.segOffsetsB, xl.segCountB, a.nL, nullptr, true);
 }
 
 // ---------------------------------------------------------------- place
 // Each body at its rank in its cell: the serial scatter's position. The segments' endpoints go
 // into cell order for the reach walk (segments precede heads within a cell, so a segment's
-// rank in its cell is its rank among the cell's segments), and the largest reach of a segment
-// from its centre is kept for it.
+// rank in its cell is its rank among the cell's segments). Only the offsets come from the scan:
+// the rest is read before it is done.
 __global__ void __launch_bounds__(256) k_wide_place(const __grid_constant__ WideArgs w) {
     const FusedArgs& a = w.a;
-    const sbx_dense_scene& sc = a.sc;
-    const sbx_grid_state& g = sc.grid;
-    const sbx_rigid_body& fb = sc.fil.body;
+    const sbx_grid_state& g = a.sc.grid;
+    const sbx_rigid_body& fb = a.sc.fil.body;
     const int nSeg = a.nSeg;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int c = i < a.cap ? g.bodyCell[i] : -1;
-    float span = 0.f;
-    if (c >= 0 && SBX_IDX_OK(c, a.C, CK_CELL)) {
-        const int o0 = g.gridCellOffsets[c], n = g.gridCellOffsets[c + 1] - o0;
-        const bool seg = i < nSeg;
-        float c3[3], e1[3], e2[3];
-        int q0 = 0;
-        bool fil = false;
-        if (seg) {
-            q0 = a.segCellOff[c];
-            fil = g.ownerStore[i] == STORE_FILAMENT;
-            for (int k = 0; k < 3; k++) {
-                c3[k] = g.center[k * a.cap + i];
-                e1[k] = fb.end1[k * nSeg + i];
-                e2[k] = fb.end2[k * nSeg + i];
-            }
+    int c = i < a.cap ? g.bodyCell[i] : -1;
+    if (!SBX_IDX_OK_OR_NONE(c, a.C, CK_CELL)) c = -1;
+    const bool seg = i < nSeg;
+    int rank = 0;
+    float4 e1 = make_float4(0.f, 0.f, 0.f, __int_as_float(-1)), e2 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c >= 0) {
+        if (seg && g.ownerStore[i] == STORE_FILAMENT) {
+            e1 = make_float4(fb.end1[i], fb.end1[nSeg + i], fb.end1[2 * nSeg + i], __int_as_float(i));
+            e2 = make_float4(fb.end2[i], fb.end2[nSeg + i], fb.end2[2 * nSeg + i], 0.f);
         }
-        const int rank = row_rank<WIDE_CELL_SLOTS>(a, n, a.cellSlot, a.cellUse, a.cellHead, a.cellNext, c, i, a.cap);
-        if (SBX_IDX_OK(o0 + rank, a.cap, CK_CSR_POS)) {
-            g.gridCellContents[o0 + rank] = i;
-            if (seg && SBX_IDX_OK(q0 + rank, nSeg, CK_CSR_POS)) {
-                if (fil) {
-                    span = segment_span(c3, e1, e2);
-                    a.segE1[q0 + rank] = make_float4(e1[0], e1[1], e1[2], __int_as_float(i));
-                    a.segE2[q0 + rank] = make_float4(e2[0], e2[1], e2[2], 0.f);
-                } else {
-                    a.segE1[q0 + rank] = make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
-                    a.segE2[q0 + rank] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
-        }
+        rank = row_rank<WIDE_CELL_SLOTS>(a, a.cntCell, a.cellSlot, a.cellUse, a.cellHead, a.cellNext, c, i, a.cap);
     }
-    __syncwarp();
-    span_max(a.reachMax, span);
+    after_previous();
+    let_next_start();
+    if (c < 0) return;
+    const int pos = g.gridCellOffsets[c] + rank, q = seg ? a.segCellOff[c] + rank : 0;
+    if (!SBX_IDX_OK(pos, a.cap, CK_CSR_POS)) return;
+    g.gridCellContents[pos] = i;
+    if (seg && SBX_IDX_OK(q, nSeg, CK_CSR_POS)) {
+        a.segE1[q] = e1;
+        a.segE2[q] = e2;
+    }
 }
 
 // ---------------------------------------------------------------- bind
-// Release, reach walk with the nearest choice, nucleotide cycle and the bound head's entry in
-// its rod's motor row (as the fused kernel's binding phase): a warp takes BIND_HEADS consecutive
-// heads, 32 / BIND_LANES of them side by side, BIND_LANES lanes a head.
-constexpr int BIND_LANES = 8, BIND_HEADS = 8;
+constexpr int BIND_LANES = 8;        // lanes a head
+// The reach walk with the nearest choice, the nucleotide cycle and the bound head's entry in its
+// rod's motor row: a warp takes 32 / BIND_LANES consecutive heads.
+constexpr int BIND_HEADS = 32 / BIND_LANES;
 template <bool B>
 __global__ void __launch_bounds__(128) k_wide_bind(const __grid_constant__ WideArgs w) {
     const FusedArgs& a = w.a;
@@ -399,55 +427,37 @@ __global__ void __launch_bounds__(128) k_wide_bind(const __grid_constant__ WideA
     const float* kp = mot.kinParams;
     const int lane = threadIdx.x & 31, nM = a.nM;
     const int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * BIND_HEADS;
-    if (base >= nM) return;
-    const int t = mot.counts[1];
-    const int myM = base + lane;
-    const bool mine = lane < BIND_HEADS && myM < nM;
-    int bs = 0, cd = 0, sb = 0, sr = 0, cs = 0, seed = sc.seed;
-    int2 key = make_int2(0, 0);
-    if (mine) {
-        key = key_of<B>(w.bt.motKey, myM);
-        if (B) seed = w.bt.seeds[3 * key.x];
-        bs = mot.boundSeg[myM]; cd = mot.cooldown[myM]; sb = mot.stats[2 * myM]; sr = mot.stats[2 * myM + 1];
-        cs = mot.capStats[myM];
-        release_one(key.y, bs, cd, sb, sr, cs, mot.forceDotFil[myM], mot.forceMag[myM], kp, t, seed);
-    }
-    for (int j = 0; j < BIND_HEADS; j += 32 / BIND_LANES) {
-        const int m = base + j + lane / BIND_LANES;
-        const bool valid = m < nM;
-        const int mm = valid ? m : base;
-        const GridView gv = grid_view<B>(w, key_of<B>(w.bt.motKey, mm).x);
-        int best;
-        float arc;
-        const int rc = group_reach_bind<BIND_LANES>(
-            a, gv, lane, valid, mot.head[mm], mot.head[nM + mm], mot.head[2 * nM + mm], mot.uVec[mm],
-            mot.uVec[nM + mm], mot.uVec[2 * nM + mm], mot.rodUVec[mm], mot.rodUVec[nM + mm], mot.rodUVec[2 * nM + mm],
-            sc.grid.reachSeg + (int64_t)mm * MAX_CAND, kp[7], kp[8], &best, &arc);
-        if ((lane & (BIND_LANES - 1)) == 0 && valid) {
-            sc.grid.reachCount[m] = rc;
-            if (rc > MAX_CAND) {
-                atomicOr(a.err, ERR_REACH_OVERFLOW);
-                stat_add(a, ST_REACH_OVER, 1);
-            }
-        }
-        const bool owner = lane >= j && lane < j + 32 / BIND_LANES;
-        const int src = owner ? (lane - j) * BIND_LANES : 0;
-        const int bb = __shfl_sync(0xffffffffu, best, src);
-        const float ab = __shfl_sync(0xffffffffu, arc, src);
-        if (owner && bs == FREE_BINDABLE && bb >= 0) {
-            bs = bb;
-            if (mine) mot.bindArc[myM] = ab;
-        }
-    }
+    if (base >= nM) { after_previous(); return; }
+    const int m = base + lane / BIND_LANES;
+    const bool valid = m < nM, mine = valid && (lane & (BIND_LANES - 1)) == 0;
+    const int mm = valid ? m : base;
+    const int2 key = key_of<B>(w.bt.motKey, mm);
+    const float mx = mot.head[mm], my = mot.head[nM + mm], mz = mot.head[2 * nM + mm];
+    const float ux = mot.uVec[mm], uy = mot.uVec[nM + mm], uz = mot.uVec[2 * nM + mm];
+    const float rx = mot.rodUVec[mm], ry = mot.rodUVec[nM + mm], rz = mot.rodUVec[2 * nM + mm];
+    int bs = mot.boundSeg[mm], state = mot.nucleotideState[mm];
+    int best;
+    float arc;
+    const int rc = group_reach_bind<BIND_LANES>(
+        a, grid_view<B>(w, key.x), lane, valid, mx, my, mz, ux, uy, uz, rx, ry, rz,
+        sc.grid.reachSeg + (int64_t)mm * MAX_CAND, kp[7], kp[8], &best, &arc, AfterPrevious());
     int row = -1, over = 0;
     if (mine) {
-        mot.boundSeg[myM] = bs; mot.cooldown[myM] = cd; mot.stats[2 * myM] = sb; mot.stats[2 * myM + 1] = sr;
-        mot.capStats[myM] = cs;
-        mot.nucleotideState[myM] = cycle_one(key.y, mot.nucleotideState[myM], bs >= 0, mot.forceDotHist + 10 * myM,
-                                             mot.nucParams, t, seed);
+        sc.grid.reachCount[m] = rc;
+        if (rc > MAX_CAND) {
+            atomicOr(a.err, ERR_REACH_OVERFLOW);
+            stat_add(a, ST_REACH_OVER, 1);
+        }
+        if (bs == FREE_BINDABLE && best >= 0) {
+            bs = best;
+            mot.boundSeg[m] = bs;
+            mot.bindArc[m] = arc;
+        }
+        mot.nucleotideState[m] = cycle_one(key.y, state, bs >= 0, mot.forceDotHist + 10 * m, mot.nucParams,
+                                           mot.counts[1], B ? w.bt.seeds[3 * key.x] : sc.seed);
         if (bs >= 0 && SBX_IDX_OK(bs, a.nSeg, CK_BOUND_SEG) && bs < a.nSeg) {
             row = bs;
-            over = row_insert(a.cntM, a.slotM, FUSED_MOTOR_SLOTS, a.mRowUse, a.headM, a.nextM, bs, myM);
+            over = row_insert(a.cntM, a.slotM, FUSED_MOTOR_SLOTS, a.mRowUse, a.headM, a.nextM, bs, m);
         } else if (bs >= 0 && w.errDev) {
             *(volatile int*)w.errDev = 1;
         }
@@ -471,6 +481,7 @@ __global__ void __launch_bounds__(128) k_wide_terms(const __grid_constant__ Wide
 constexpr int MINI_THREADS = 96;
 template <bool B>
 __global__ void __launch_bounds__(MINI_THREADS) k_wide_mini(const __grid_constant__ WideArgs w) {
+    let_next_start();
     __shared__ MiniSmem sm;
     const FusedArgs& a = w.a;
     const sbx_minifilament_store& mini = a.sc.mini;
@@ -493,19 +504,10 @@ __global__ void __launch_bounds__(128) k_wide_links(const __grid_constant__ Wide
     const sbx_crosslinker_store& xl = a.sc.xl;
     const sbx_rigid_body& fb = a.sc.fil.body;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.nL) return;
+    if (k >= a.nL) { after_previous(); return; }
     int la = xl.linkFilA[k], lb = xl.linkFilB[k];
     if (!end_ok(w, la)) la = -1;
     if (!end_ok(w, lb)) lb = -1;
-    int pA = -1, pB = -1;
-    if (la >= 0) {
-        const int o0 = xl.segOffsetsA[la], n = xl.segOffsetsA[la + 1] - o0;
-        pA = o0 + row_rank<FUSED_ROW_SLOTS>(a, n, a.slotA, a.rowUse, a.headA, a.nextA, la, k, a.nL);
-    }
-    if (lb >= 0) {
-        const int o0 = xl.segOffsetsB[lb], n = xl.segOffsetsB[lb + 1] - o0;
-        pB = o0 + row_rank<FUSED_ROW_SLOTS>(a, n, a.slotB, a.rowUse, a.headB, a.nextB, lb, k, a.nL);
-    }
     const int state = xl.linkState[k];
     float out[XL_STRIDE];
     link_forces_one(k, a.nSeg, fb.coord, fb.uVec, fb.end1, fb.bTransGam, la, lb, xl.loc1[k], xl.loc2[k], a.cntAct,
@@ -513,6 +515,12 @@ __global__ void __launch_bounds__(128) k_wide_links(const __grid_constant__ Wide
     if (xl.torsionParams[1] >= 0.5f)
         link_torsion_row(k, a.nSeg, fb.uVec, la, lb, state, xl.linkOrientSame[k], xl.torqueMagHist, xl.torqueMagPlace,
                          out, xl.torsionParams[0]);
+    int pA = 0, pB = 0;
+    if (la >= 0) pA = row_rank<FUSED_ROW_SLOTS>(a, a.cntA, a.slotA, a.rowUse, a.headA, a.nextA, la, k, a.nL);
+    if (lb >= 0) pB = row_rank<FUSED_ROW_SLOTS>(a, a.cntB, a.slotB, a.rowUse, a.headB, a.nextB, lb, k, a.nL);
+    after_previous();                    // the offsets
+    pA = la >= 0 ? pA + xl.segOffsetsA[la] : -1;
+    pB = lb >= 0 ? pB + xl.segOffsetsB[lb] : -1;
     // (a row is 48 bytes: 16-byte stores where the array is aligned)
     float* row = xl.xlinkData + (int64_t)k * XL_STRIDE;
     if (((uintptr_t)xl.xlinkData & 15u) == 0)
@@ -546,7 +554,7 @@ __global__ void __launch_bounds__(256) k_wide_motor_place(const __grid_constant_
     const FusedArgs& a = w.a;
     const sbx_dense_scene& sc = a.sc;
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m < a.C) a.cellHead[m] = -1;
+    if (m < a.C) { a.cntCell[m] = 0; a.cellHead[m] = -1; }
     if (m < w.tilesC) { w.sumCell[m * WIDE_SUM_STRIDE] = 0; w.sumSeg[m * WIDE_SUM_STRIDE] = 0; }
     if (m < w.tilesS) w.sumM[m * WIDE_SUM_STRIDE] = 0;
     if (m >= a.nM) return;
@@ -595,7 +603,7 @@ __global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ Wi
     const sbx_rigid_body& fb = fs.body;
     const sbx_crosslinker_store& xl = sc.xl;
     const int n = a.nSeg, i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n) { after_previous(); return; }
     // what does not wait for anything first, all in flight together
     const int t = fs.counts[1];
     const int nm = a.cntM[i];
@@ -608,15 +616,6 @@ __global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ Wi
         act = a.cntAct[i];
     }
     const BodyIn in = body_load(fb, i);
-    if (i == 0) {
-        *a.d_step = t + 1;               // (every reader of this step's index has run)
-        *a.reachMax = 0;
-    }
-    if (a.xlOn) {
-        xl.activeLinkCount[i] = act;
-        a.cntAct[i] = 0; a.headA[i] = -1; a.headB[i] = -1;
-        if (i < w.tilesS) { w.sumA[i * WIDE_SUM_STRIDE] = 0; w.sumB[i * WIDE_SUM_STRIDE] = 0; }
-    }
     const ChainParams cp = chain_params(fs.chainParams);
     double fd[3] = {0.0, 0.0, 0.0}, td[3] = {0.0, 0.0, 0.0};
     RodGeom me;
@@ -648,6 +647,16 @@ __global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ Wi
     if (a.xlOn) {
         add_row(w.payA, a0, a1, F, T);
         add_row(w.payB, b0, b1, F, T);
+    }
+    after_previous();                    // the bonds; nothing is written before them
+    if (i == 0) {
+        *a.d_step = t + 1;               // (every reader of this step's index has run)
+        *a.reachMax = 0;
+    }
+    if (a.xlOn) {
+        xl.activeLinkCount[i] = act;
+        a.cntAct[i] = 0; a.cntA[i] = 0; a.cntB[i] = 0; a.headA[i] = -1; a.headB[i] = -1;
+        if (i < w.tilesS) { w.sumA[i * WIDE_SUM_STRIDE] = 0; w.sumB[i * WIDE_SUM_STRIDE] = 0; }
     }
     // CrossBridgeSystem.segGather (CrossBridgeSystem.java:302-320): the bound motors' reactions
     // in ascending slot, taken from the row's slots (and list) by repeated minimum
@@ -686,7 +695,7 @@ __global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ Wi
 bool wide_streams_create(WideStreams& ws) {
     for (cudaStream_t* s : {&ws.ahead, &ws.link, &ws.csr})
         if (cudaStreamCreateWithFlags(s, cudaStreamNonBlocking) != cudaSuccess) return false;
-    for (cudaEvent_t* e : {&ws.start, &ws.drawn, &ws.bound, &ws.joined, &ws.linkDone, &ws.csrDone})
+    for (cudaEvent_t* e : {&ws.start, &ws.bound, &ws.joined, &ws.linkDone, &ws.csrDone})
         if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return false;
     return true;
 }
@@ -694,7 +703,7 @@ bool wide_streams_create(WideStreams& ws) {
 void wide_streams_destroy(WideStreams& ws) {
     for (cudaStream_t s : {ws.ahead, ws.link, ws.csr})
         if (s) cudaStreamDestroy(s);
-    for (cudaEvent_t e : {ws.start, ws.drawn, ws.bound, ws.joined, ws.linkDone, ws.csrDone})
+    for (cudaEvent_t e : {ws.start, ws.bound, ws.joined, ws.linkDone, ws.csrDone})
         if (e) cudaEventDestroy(e);
     ws = WideStreams{};
 }
@@ -709,37 +718,43 @@ sbx_status wide_step_impl(sbx_ctx* ctx, const WideArgs& w, const WideStreams& ws
     auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     auto fork = [&](cudaEvent_t ev, cudaStream_t to) { ok(cudaEventRecord(ev, s)); ok(cudaStreamWaitEvent(to, ev, 0)); };
     auto join = [&](cudaEvent_t ev, cudaStream_t from) { ok(cudaEventRecord(ev, from)); ok(cudaStreamWaitEvent(s, ev, 0)); };
-#define WIDE_LAUNCH(stream, kernel, items, block)                                  \
-    do {                                                                           \
-        kernel<<<blocks(items, block), block, 0, stream>>>(w);                     \
-        ctx->launches++;                                                           \
-    } while (0)
+    // early: the kernel waits for its predecessor itself
+    auto launch = [&](cudaStream_t to, bool early, auto kernel, int64_t items, int block) {
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(blocks(items, block));
+        cfg.blockDim = dim3(block);
+        cfg.stream = to;
+        cfg.attrs = &attr;
+        cfg.numAttrs = early ? 1 : 0;
+        ok(cudaLaunchKernelEx(&cfg, kernel, w));
+        ctx->launches++;
+    };
     fork(ws.start, ws.ahead);
     if (a.xlOn) ok(cudaStreamWaitEvent(ws.link, ws.start, 0));
-    WIDE_LAUNCH(ws.ahead, k_wide_draws<B>, (int64_t)a.nB + a.nBb + a.nSeg, 256);
-    WIDE_LAUNCH(ws.ahead, k_wide_terms, 2 * (int64_t)a.nM + 4 * (int64_t)a.nD, 128);
-    ok(cudaEventRecord(ws.drawn, ws.ahead));
-    WIDE_LAUNCH(ws.ahead, k_wide_joints, a.nSeg, 128);
+    launch(ws.ahead, false, k_wide_draws<B>, (int64_t)a.nB + a.nBb + a.nSeg, 256);
+    launch(ws.ahead, false, k_wide_terms, 2 * (int64_t)a.nM + 4 * (int64_t)a.nD, 128);
+    launch(ws.ahead, false, k_wide_joints, a.nSeg, 128);
     if (a.xlOn) {
-        WIDE_LAUNCH(ws.link, k_wide_link_rows<B>, a.nL, 128);
-        WIDE_LAUNCH(ws.link, k_wide_link_scan, (int64_t)2 * w.tilesS * 256, 256);
-        WIDE_LAUNCH(ws.link, k_wide_links, a.nL, 128);
+        launch(ws.link, false, k_wide_link_rows<B>, a.nL, 128);
+        launch(ws.link, true, k_wide_link_scan, (int64_t)2 * w.tilesS * 256, 256);
+        launch(ws.link, true, k_wide_links, a.nL, 128);
     }
-    WIDE_LAUNCH(s, k_wide_publish<B>, a.cap, 256);
-    WIDE_LAUNCH(s, k_wide_cell_scan, (int64_t)2 * w.tilesC * 256, 256);
-    WIDE_LAUNCH(s, k_wide_place, a.cap, 256);
-    WIDE_LAUNCH(s, k_wide_bind<B>, ((int64_t)a.nM + BIND_HEADS - 1) / BIND_HEADS * 32, 128);
+    launch(s, false, k_wide_publish<B>, a.cap, 256);
+    launch(s, true, k_wide_cell_scan, (int64_t)2 * w.tilesC * 256, 256);
+    launch(s, true, k_wide_place, a.cap, 256);
+    launch(s, true, k_wide_bind<B>, ((int64_t)a.nM + BIND_HEADS - 1) / BIND_HEADS * 32, 128);
     fork(ws.bound, ws.csr);
-    WIDE_LAUNCH(ws.csr, k_wide_motor_scan, (int64_t)w.tilesS * 256, 256);
-    WIDE_LAUNCH(ws.csr, k_wide_motor_place, std::max(std::max(a.nM, a.C), w.tilesS), 256);
-    ok(cudaStreamWaitEvent(s, ws.drawn, 0));
-    k_wide_mini<B><<<a.nBb + (a.nBb + MINI_THREADS - 1) / MINI_THREADS, MINI_THREADS, 0, s>>>(w);
-    ctx->launches++;
+    launch(ws.csr, false, k_wide_motor_scan, (int64_t)w.tilesS * 256, 256);
+    launch(ws.csr, false, k_wide_motor_place, std::max(std::max(a.nM, a.C), w.tilesS), 256);
     join(ws.joined, ws.ahead);
     if (a.xlOn) join(ws.linkDone, ws.link);
-    WIDE_LAUNCH(s, k_wide_rods<B>, a.nSeg, 128);
+    launch(s, false, k_wide_mini<B>, ((int64_t)a.nBb + (a.nBb + MINI_THREADS - 1) / MINI_THREADS) * MINI_THREADS,
+           MINI_THREADS);
+    launch(s, true, k_wide_rods<B>, a.nSeg, 128);
     join(ws.csrDone, ws.csr);
-#undef WIDE_LAUNCH
     if (e != cudaSuccess) return fail(ctx, SBX_ECUDA, std::string("dense step: streams: ") + cudaGetErrorString(e));
     return check_launch(ctx, "dense step");
 }

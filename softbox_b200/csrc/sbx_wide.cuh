@@ -22,7 +22,7 @@ struct WideArgs {
 // the crosslinkers, `csr` the motor CSR
 struct WideStreams {
     cudaStream_t ahead = nullptr, link = nullptr, csr = nullptr;
-    cudaEvent_t start = nullptr, drawn = nullptr, bound = nullptr, joined = nullptr, linkDone = nullptr,
+    cudaEvent_t start = nullptr, bound = nullptr, joined = nullptr, linkDone = nullptr,
                 csrDone = nullptr;
 };
 
