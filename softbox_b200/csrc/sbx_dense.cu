@@ -604,13 +604,13 @@ struct Arena {
 };
 
 // the row slots, lists, snapshots and terms both shapes of the step use (each its own set)
-void step_carve(Arena& m, FusedArgs& a, int cellSlots) {
+void step_carve(Arena& m, FusedArgs& a, int cellSlots, int rowSlots) {
     const size_t nS = a.nSeg, nLk = (size_t)std::max(a.nL, 1), C = a.C;
     m.take(a.cntCell, 4 * C); m.take(a.cntSeg, 4 * C);
     m.take(a.segCellOff, 4 * (C + 1));
     for (int** q : {&a.cntAct, &a.cntA, &a.cntB, &a.cntM, &a.headA, &a.headB, &a.headM}) m.take(*q, 4 * nS);
     m.take(a.cellSlot, 4 * C * cellSlots);
-    m.take(a.slotA, 4 * nS * FUSED_ROW_SLOTS); m.take(a.slotB, 4 * nS * FUSED_ROW_SLOTS);
+    m.take(a.slotA, 4 * nS * rowSlots); m.take(a.slotB, 4 * nS * rowSlots);
     m.take(a.slotM, 4 * nS * FUSED_MOTOR_SLOTS);
     m.take(a.cellHead, 4 * C); m.take(a.cellNext, 4 * (size_t)a.cap);
     m.take(a.nextA, 4 * nLk); m.take(a.nextB, 4 * nLk); m.take(a.nextM, 4 * (size_t)a.nM);
@@ -651,7 +651,7 @@ bool fused_prepare(sbx_dense_plan* p) {
     a.filSeed = fc[2];
     Arena m;
     if (!m.build(p, [&] {
-            step_carve(m, a, FUSED_CELL_SLOTS);
+            step_carve(m, a, FUSED_CELL_SLOTS, FUSED_ROW_SLOTS);
             m.take(a.tileSum, 4 * (size_t)(2 * a.tilesC + 2 * a.tilesS + 1));
             m.take(a.mTileSum, 4 * (size_t)(a.tilesS + 1));
             m.take(a.bar, 32);
@@ -679,13 +679,14 @@ bool wide_prepare(sbx_dense_plan* p) {
     if (p->batched) w.bt = p->batch;
     w.errDev = p->ctx->err_dev;
     a.cellUse = WIDE_CELL_SLOTS;
+    a.rowUse = WIDE_ROW_SLOTS;
     w.tilesC = (a.C + WIDE_TILE - 1) / WIDE_TILE;
     w.tilesS = (a.nSeg + WIDE_TILE - 1) / WIDE_TILE;
     const size_t nLk = (size_t)std::max(a.nL, 1), words = WIDE_SUM_STRIDE * (2 * (size_t)w.tilesC + 3 * (size_t)w.tilesS);
     int* sums = nullptr;
     Arena m;
     if (!m.build(p, [&] {
-            step_carve(m, a, WIDE_CELL_SLOTS);
+            step_carve(m, a, WIDE_CELL_SLOTS, WIDE_ROW_SLOTS);
             m.take(w.payA, 24 * nLk);
             m.take(w.payB, 24 * nLk);
             m.take(sums, 4 * words);
@@ -1027,7 +1028,7 @@ extern "C" sbx_status sbx_dense_plan_test_caps(sbx_dense_plan* p, int32_t entCap
         a->entCap = clampCap(entCap, FUSED_ENT_CAP);
         a->mCap = clampCap(motorCap, FUSED_MCAP);
         a->mIds = clampCap(motorIds, FUSED_MIDS);
-        a->rowUse = clampCap(rowSlots, FUSED_ROW_SLOTS);
+        a->rowUse = clampCap(rowSlots, a == &p->fa ? FUSED_ROW_SLOTS : WIDE_ROW_SLOTS);
         a->mRowUse = clampCap(rowSlots, FUSED_MOTOR_SLOTS);
         a->cellUse = clampCap(cellSlots, a == &p->fa ? FUSED_CELL_SLOTS : WIDE_CELL_SLOTS);
     }

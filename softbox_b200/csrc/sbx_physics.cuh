@@ -837,48 +837,78 @@ SBX_DEV void csr_gather_row(int s, const int* offsets, const int* list, const fl
 }
 
 // CrosslinkerSystem.linkForces per link (CrosslinkerSystem.java:61-123) -> 12 floats
-SBX_DEV void link_forces_one(int k, int nSeg, const float* fC, const float* fU, const float* fE1, const float* fBTG,
-                             int a, int b, float loc1k, float loc2k, const int* ct, const float* xp,
-                             float out[XL_STRIDE]) {
-    for (int j = 0; j < XL_STRIDE; j++) out[j] = 0.f;
-    if (a < 0 || b < 0) return;
+// what a link's force takes of the rod at one of its ends
+struct LinkEnd {
+    float c[3], u[3], e1[3], bTG;
+    int links;                   // active links on the rod
+};
+SBX_DEV LinkEnd link_end(int a, int nSeg, const float* fC, const float* fU, const float* fE1, const float* fBTG,
+                         const int* ct) {
+    LinkEnd e;
+    for (int k = 0; k < 3; k++) { e.c[k] = fC[k * nSeg + a]; e.u[k] = fU[k * nSeg + a]; e.e1[k] = fE1[k * nSeg + a]; }
+    e.bTG = fBTG[a];
+    e.links = ct[a];
+    return e;
+}
+SBX_DEV void link_forces(const LinkEnd& a, const LinkEnd& b, float loc1k, float loc2k, const float* xp,
+                         float out[XL_STRIDE]) {
     double restLength = xp[0], fracMoveBase = xp[1], dt = xp[2];
     double l1 = loc1k;
-    double uax = fU[a], uay = fU[nSeg + a], uaz = fU[2 * nSeg + a];
-    double p1x = fE1[a] + l1 * uax;
-    double p1y = fE1[nSeg + a] + l1 * uay;
-    double p1z = fE1[2 * nSeg + a] + l1 * uaz;
+    double uax = a.u[0], uay = a.u[1], uaz = a.u[2];
+    double p1x = a.e1[0] + l1 * uax;
+    double p1y = a.e1[1] + l1 * uay;
+    double p1z = a.e1[2] + l1 * uaz;
     double l2 = loc2k;
-    double ubx = fU[b], uby = fU[nSeg + b], ubz = fU[2 * nSeg + b];
-    double p2x = fE1[b] + l2 * ubx;
-    double p2y = fE1[nSeg + b] + l2 * uby;
-    double p2z = fE1[2 * nSeg + b] + l2 * ubz;
+    double ubx = b.u[0], uby = b.u[1], ubz = b.u[2];
+    double p2x = b.e1[0] + l2 * ubx;
+    double p2y = b.e1[1] + l2 * uby;
+    double p2z = b.e1[2] + l2 * ubz;
     double lvx = p2x - p1x, lvy = p2y - p1y, lvz = p2z - p1z;
     double linkLength = sqrt(lvx * lvx + lvy * lvy + lvz * lvz);
     double stretch = linkLength - restLength;
     if (stretch < 0.0) stretch = 0.0;
-    int ctA = ct[a], ctB = ct[b];
+    int ctA = a.links, ctB = b.links;
     int maxLinks = ctA > ctB ? ctA : ctB;
     if (maxLinks < 1) maxLinks = 1;
     double fracMove = fracMoveBase / maxLinks;
-    double g1 = fBTG[a], g2 = fBTG[b];
+    double g1 = a.bTG, g2 = b.bTG;
     double curForceMag = (fracMove * 1.0e-6 * stretch / dt) / (1.0 / g1 + 1.0 / g2);
     double Fx = curForceMag * lvx, Fy = curForceMag * lvy, Fz = curForceMag * lvz;
-    double rax = (p1x - fC[a]) * 1e-6, ray = (p1y - fC[nSeg + a]) * 1e-6, raz = (p1z - fC[2 * nSeg + a]) * 1e-6;
+    double rax = (p1x - a.c[0]) * 1e-6, ray = (p1y - a.c[1]) * 1e-6, raz = (p1z - a.c[2]) * 1e-6;
     double TAx = ray * Fz - raz * Fy, TAy = raz * Fx - rax * Fz, TAz = rax * Fy - ray * Fx;
     double nFx = -Fx, nFy = -Fy, nFz = -Fz;
-    double rbx = (p2x - fC[b]) * 1e-6, rby = (p2y - fC[nSeg + b]) * 1e-6, rbz = (p2z - fC[2 * nSeg + b]) * 1e-6;
+    double rbx = (p2x - b.c[0]) * 1e-6, rby = (p2y - b.c[1]) * 1e-6, rbz = (p2z - b.c[2]) * 1e-6;
     double TBx = rby * nFz - rbz * nFy, TBy = rbz * nFx - rbx * nFz, TBz = rbx * nFy - rby * nFx;
     out[0] = (float)Fx; out[1] = (float)Fy; out[2] = (float)Fz;
     out[3] = (float)TAx; out[4] = (float)TAy; out[5] = (float)TAz;
     out[6] = (float)nFx; out[7] = (float)nFy; out[8] = (float)nFz;
     out[9] = (float)TBx; out[10] = (float)TBy; out[11] = (float)TBz;
 }
+SBX_DEV void link_forces_one(int k, int nSeg, const float* fC, const float* fU, const float* fE1, const float* fBTG,
+                             int a, int b, float loc1k, float loc2k, const int* ct, const float* xp,
+                             float out[XL_STRIDE]) {
+    for (int j = 0; j < XL_STRIDE; j++) out[j] = 0.f;
+    if (a < 0 || b < 0) return;
+    link_forces(link_end(a, nSeg, fC, fU, fE1, fBTG, ct), link_end(b, nSeg, fC, fU, fE1, fBTG, ct), loc1k, loc2k, xp,
+                out);
+}
+
+// a link's window of torque magnitudes, as the step found it
+struct TorsionWindow {
+    int p;
+    float w[TORQUE_WIN];
+};
+SBX_DEV TorsionWindow torsion_window(int k, const float* hist, const int* place) {
+    TorsionWindow t;
+    t.p = place[k];
+    for (int j = 0; j < TORQUE_WIN; j++) t.w[j] = hist[k * TORQUE_WIN + j];
+    return t;
+}
 
 // CrosslinkerSystem.linkTorsion per link (CrosslinkerSystem.java:777-806); adds into the link's
 // payload row r
-SBX_DEV void link_torsion_row(int k, int nSeg, const float* fU, int a, int b, int state, int orient, float* hist,
-                              int* place, float* r, double spring) {
+SBX_DEV void link_torsion_row(int k, int nSeg, const float* fU, int a, int b, int state, int orient,
+                              const TorsionWindow& win, float* hist, int* place, float* r, double spring) {
     if (state < 0) return;
     if (a < 0 || b < 0) return;
     double uax = fU[a], uay = fU[nSeg + a], uaz = fU[2 * nSeg + a];
@@ -895,12 +925,12 @@ SBX_DEV void link_torsion_row(int k, int nSeg, const float* fU, int a, int b, in
     if (dot < -1.0) dot = -1.0;
     double angT = same ? fast_acos(dot) : fabs(fast_acos(dot) - PI_D);
     double curMag = spring * angT;
-    int base = k * TORQUE_WIN;
-    int p = place[k];
-    hist[base + p] = (float)curMag;
+    // the window with this step's entry replaced, summed in slot order
+    const int p = win.p;
+    hist[k * TORQUE_WIN + p] = (float)curMag;
     place[k] = (p + 1) % TORQUE_WIN;
     double avg = 0.0;
-    for (int j = 0; j < TORQUE_WIN; j++) avg += hist[base + j];
+    for (int j = 0; j < TORQUE_WIN; j++) avg += (j == p) ? (float)curMag : win.w[j];
     avg /= TORQUE_WIN;
     double Tx = avg * tx, Ty = avg * ty, Tz = avg * tz;
     r[3] = (float)(r[3] + Tx);
@@ -913,7 +943,9 @@ SBX_DEV void link_torsion_row(int k, int nSeg, const float* fU, int a, int b, in
 
 SBX_DEV void link_torsion_one(int k, int nSeg, const float* fU, int a, int b, int state, int orient, float* hist,
                               int* place, float* xd, double spring) {
-    link_torsion_row(k, nSeg, fU, a, b, state, orient, hist, place, xd + (int64_t)k * XL_STRIDE, spring);
+    if (state < 0 || a < 0 || b < 0) return;
+    link_torsion_row(k, nSeg, fU, a, b, state, orient, torsion_window(k, hist, place), hist, place,
+                     xd + (int64_t)k * XL_STRIDE, spring);
 }
 
 // CrosslinkerSystem.unbind per ACTIVE link (CrosslinkerSystem.java:245-280); true = break

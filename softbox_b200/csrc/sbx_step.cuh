@@ -60,18 +60,20 @@ __device__ __forceinline__ int list_rank(const FusedArgs& a, int head, const int
     return r;
 }
 
-// Appends `item` to row r: the histogram's old count is its arrival index; the first `use`
+// Appends `item` to row r: the histogram's old count is its arrival index j; the first `use`
 // (<= S, the slot stride) arrivals take the row's fixed slots, later ones join the row's
 // overflow list (returns 1).
-__device__ __forceinline__ int row_insert(int* cnt, int* slot, int S, int use, int* head, int* next, int r,
-                                          int item) {
-    int j = atomicAdd(&cnt[r], 1);
+__device__ __forceinline__ int row_put(int* slot, int S, int use, int* head, int* next, int r, int item, int j) {
     if (j < use) {
         slot[(size_t)r * S + j] = item;
         return 0;
     }
     next[item] = atomicExch(&head[r], item);
     return 1;
+}
+__device__ __forceinline__ int row_insert(int* cnt, int* slot, int S, int use, int* head, int* next, int r,
+                                          int item) {
+    return row_put(slot, S, use, head, next, r, item, atomicAdd(&cnt[r], 1));
 }
 
 // adds a thread's count of a capacity fallback to the plan's counters, one addition per warp (of

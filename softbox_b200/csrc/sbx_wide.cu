@@ -22,9 +22,9 @@
 // what a later kernel reads again is written once.
 // Every slot is computed by the same device functions as the per-system kernels, in the
 // reference's accumulation order: the same bits.
-// A step takes 35 us at 1,000 rods, 47 at 20,000, 90 at 100,000 and 356 at 500,000 (46, 57, 97 and
-// 370 with full waits; 200 and 434 at the last two as the per-system sequence), a packed
-// step of 12 networks (0.17e6 rods, 0.18e6 heads) 250 us (269; 366).
+// A step takes 29 us at 1,000 rods, 37 at 20,000, 85 at 100,000 and 353 at 500,000 (46, 57, 97 and
+// 370 with full waits and serial gathers; 200 and 434 at the last two as the per-system
+// sequence), a packed step of 12 networks (0.17e6 rods, 0.18e6 heads) 250 us (269; 366).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -83,6 +83,7 @@ __device__ __forceinline__ void tile_add(int* sums, int tile) {
 // independent chains of FP64 operations.
 template <bool B>
 __global__ void __launch_bounds__(256) k_wide_draws(const __grid_constant__ WideArgs w) {
+    let_next_start();
     const FusedArgs& a = w.a;
     const sbx_dense_scene& sc = a.sc;
     const int nB = a.nB, nBb = a.nBb;
@@ -155,6 +156,7 @@ __global__ void __launch_bounds__(128, 5) k_wide_joints(const __grid_constant__ 
                                 load_rod(n, i, fb.coord, fb.uVec, fb.segLength, fb.bTransGam, fb.bRotGam),
                                 load_rod(n, nb, fb.coord, fb.uVec, fb.segLength, fb.bTransGam, fb.bRotGam)));
     }
+    after_previous();                    // (done when the kernels before it are)
 }
 
 // ---------------------------------------------------------------- publish
@@ -267,31 +269,38 @@ __global__ void __launch_bounds__(128) k_wide_link_rows(const __grid_constant__ 
     const sbx_rigid_body& fb = sc.fil.body;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     int la = -1, lb = -1, over = 0;
+    bool act = false;
     if (k < a.nL) {
         la = xl.linkFilA[k];
         lb = xl.linkFilB[k];
+        const bool on = xl.linkState[k] >= 0;
         if (!end_ok(w, la)) la = -1;
         if (!end_ok(w, lb)) lb = -1;
-        if (la >= 0) over += row_insert(a.cntA, a.slotA, FUSED_ROW_SLOTS, a.rowUse, a.headA, a.nextA, la, k);
-        if (lb >= 0) over += row_insert(a.cntB, a.slotB, FUSED_ROW_SLOTS, a.rowUse, a.headB, a.nextB, lb, k);
+        // (the two counters and the unbinding's inputs are in flight together)
+        int jA = 0, jB = 0;
+        if (la >= 0) jA = atomicAdd(&a.cntA[la], 1);
+        if (lb >= 0) jB = atomicAdd(&a.cntB[lb], 1);
+        act = la >= 0 && lb >= 0 && on;
+        if (act && a.xlUnbind) {
+            const int2 key = key_of<B>(w.bt.linkKey, k);
+            // the draw is keyed by the local index, which also indexes the strain ring: shift the
+            // ring pointers so that it addresses this link's own ring
+            const int off = k - key.y;
+            if (unbind_one(key.y, a.nSeg, fb.uVec, fb.end1, la, lb, xl.loc1[k], xl.loc2[k],
+                           xl.strainHist + (int64_t)off * STRAIN_WIN, xl.strainPlace + off, xl.offParams, *a.d_step,
+                           B ? w.bt.seeds[3 * key.x] : sc.seed)) {
+                xl.linkState[k] = LINK_FREE;
+                act = false;
+            }
+        }
+        if (la >= 0) over += row_put(a.slotA, WIDE_ROW_SLOTS, a.rowUse, a.headA, a.nextA, la, k, jA);
+        if (lb >= 0) over += row_put(a.slotB, WIDE_ROW_SLOTS, a.rowUse, a.headB, a.nextB, lb, k, jB);
     }
     __syncwarp();
     tile_add(w.sumA, la >= 0 ? la / WIDE_TILE : -1);
     tile_add(w.sumB, lb >= 0 ? lb / WIDE_TILE : -1);
     stat_add(a, ST_LINK_LIST, over);
-    if (la < 0 || lb < 0 || xl.linkState[k] < 0) return;
-    if (a.xlUnbind) {
-        const int2 key = key_of<B>(w.bt.linkKey, k);
-        // the draw is keyed by the local index, which also indexes the strain ring: shift the
-        // ring pointers so that it addresses this link's own ring
-        const int off = k - key.y;
-        if (unbind_one(key.y, a.nSeg, fb.uVec, fb.end1, la, lb, xl.loc1[k], xl.loc2[k],
-                       xl.strainHist + (int64_t)off * STRAIN_WIN, xl.strainPlace + off, xl.offParams, *a.d_step,
-                       B ? w.bt.seeds[3 * key.x] : sc.seed)) {
-            xl.linkState[k] = LINK_FREE;
-            return;
-        }
-    }
+    if (!act) return;
     atomicAdd(&a.cntAct[la], 1);
     atomicAdd(&a.cntAct[lb], 1);
 }
@@ -471,8 +480,10 @@ __global__ void __launch_bounds__(128) k_wide_bind(const __grid_constant__ WideA
 // The position-only myosin terms, one a thread, beside the grid kernels: FP64 chains of some
 // thousand cycles that would otherwise sit between binding and integration.
 __global__ void __launch_bounds__(128) k_wide_terms(const __grid_constant__ WideArgs w) {
+    let_next_start();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < 2 * w.a.nM + 4 * w.a.nD) myosin_term(w.a, k);
+    after_previous();                    // (done when the kernels before it are)
 }
 
 // One block a minifilament: a warp for its heads (with their bonds), its rods, its levers, then
@@ -496,28 +507,55 @@ __global__ void __launch_bounds__(MINI_THREADS) k_wide_mini(const __grid_constan
 }
 
 // ---------------------------------------------------------------- links
+// how many of the slots v, the first of them slot q of n, hold items below k
+__device__ __forceinline__ int below(int4 v, int q, int n, int k) {
+    return (q < n && v.x < k) + (q + 1 < n && v.y < k) + (q + 2 < n && v.z < k) + (q + 3 < n && v.w < k);
+}
+
 // Crosslinker forces and torsion (CrosslinkerSystem.java:61-123, :777-806), one thread a link,
 // and the link at its rank in both CSRs: the lists, and its two payload rows in list order
-// (zeros for a FREE link)
+// (zeros for a FREE link). The minifilaments wait for it, and it is a chain of latencies: with
+// the loads of each round together, and the rank from a row's slots (a row of nine links was a
+// list walked entry by entry), it takes 10 us at 20,000 rods (13 before) and ends 5 us earlier.
 __global__ void __launch_bounds__(128) k_wide_links(const __grid_constant__ WideArgs w) {
     const FusedArgs& a = w.a;
     const sbx_crosslinker_store& xl = a.sc.xl;
     const sbx_rigid_body& fb = a.sc.fil.body;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.nL) { after_previous(); return; }
+    // two rounds of loads, each in flight together: what the link's index names, then what its
+    // ends name (row 0 stands in for an end that is left out)
     int la = xl.linkFilA[k], lb = xl.linkFilB[k];
+    const int state = xl.linkState[k], orient = xl.linkOrientSame[k];
+    const float loc1 = xl.loc1[k], loc2 = xl.loc2[k];
+    const bool torsion = xl.torsionParams[1] >= 0.5f;
+    TorsionWindow win;
+    if (torsion) win = torsion_window(k, xl.torqueMagHist, xl.torqueMagPlace);
     if (!end_ok(w, la)) la = -1;
     if (!end_ok(w, lb)) lb = -1;
-    const int state = xl.linkState[k];
+    const int ia = la < 0 ? 0 : la, ib = lb < 0 ? 0 : lb;
+    const LinkEnd ea = link_end(ia, a.nSeg, fb.coord, fb.uVec, fb.end1, fb.bTransGam, a.cntAct);
+    const LinkEnd eb = link_end(ib, a.nSeg, fb.coord, fb.uVec, fb.end1, fb.bTransGam, a.cntAct);
+    const int nA = a.cntA[ia], nB = a.cntB[ib];
+    const int4* sA = reinterpret_cast<const int4*>(a.slotA + (size_t)ia * WIDE_ROW_SLOTS);
+    const int4* sB = reinterpret_cast<const int4*>(a.slotB + (size_t)ib * WIDE_ROW_SLOTS);
+    const int4 vA = sA[0], vB = sB[0];
+    int pA = below(vA, 0, min(nA, a.rowUse), k), pB = below(vB, 0, min(nB, a.rowUse), k);
     float out[XL_STRIDE];
-    link_forces_one(k, a.nSeg, fb.coord, fb.uVec, fb.end1, fb.bTransGam, la, lb, xl.loc1[k], xl.loc2[k], a.cntAct,
-                    xl.xlParams, out);
-    if (xl.torsionParams[1] >= 0.5f)
-        link_torsion_row(k, a.nSeg, fb.uVec, la, lb, state, xl.linkOrientSame[k], xl.torqueMagHist, xl.torqueMagPlace,
-                         out, xl.torsionParams[0]);
-    int pA = 0, pB = 0;
-    if (la >= 0) pA = row_rank<FUSED_ROW_SLOTS>(a, a.cntA, a.slotA, a.rowUse, a.headA, a.nextA, la, k, a.nL);
-    if (lb >= 0) pB = row_rank<FUSED_ROW_SLOTS>(a, a.cntB, a.slotB, a.rowUse, a.headB, a.nextB, lb, k, a.nL);
+#pragma unroll
+    for (int j = 0; j < XL_STRIDE; j++) out[j] = 0.f;
+    if (la >= 0 && lb >= 0) {
+        link_forces(ea, eb, loc1, loc2, xl.xlParams, out);
+        if (torsion)
+            link_torsion_row(k, a.nSeg, fb.uVec, la, lb, state, orient, win, xl.torqueMagHist, xl.torqueMagPlace, out,
+                             xl.torsionParams[0]);
+    }
+    for (int q = 1; q < WIDE_ROW_SLOTS / 4; q++) {
+        if (nA > 4 * q) pA += below(sA[q], 4 * q, min(nA, a.rowUse), k);
+        if (nB > 4 * q) pB += below(sB[q], 4 * q, min(nB, a.rowUse), k);
+    }
+    if (la >= 0 && nA > a.rowUse) pA += list_rank(a, a.headA[la], a.nextA, k, a.nL);
+    if (lb >= 0 && nB > a.rowUse) pB += list_rank(a, a.headB[lb], a.nextB, k, a.nL);
     after_previous();                    // the offsets
     pA = la >= 0 ? pA + xl.segOffsetsA[la] : -1;
     pB = lb >= 0 ? pB + xl.segOffsetsB[lb] : -1;
@@ -577,6 +615,22 @@ __device__ __forceinline__ void add_row(const float* pay, int k0, int k1, float 
         t[0] += y.y; t[1] += z.x; t[2] += z.y;
     }
     for (int k = 0; k < 3; k++) { F[k] = (float)(F[k] + f[k]); T[k] = (float)(T[k] + t[k]); }
+}
+
+constexpr int ROD_MOTORS = 16;        // bound motors of a rod that are held in registers
+static_assert(ROD_MOTORS % 4 == 0 && ROD_MOTORS <= FUSED_MOTOR_SLOTS && FUSED_MOTOR_SLOTS % 4 == 0, "16-byte loads");
+
+// sorts the first N of a row's slots, ascending (odd-even transposition)
+template <int N>
+__device__ __forceinline__ void sort_slots(int (&v)[ROD_MOTORS]) {
+#pragma unroll
+    for (int r = 0; r < N; r++)
+#pragma unroll
+        for (int j = r & 1; j + 1 < N; j += 2) {
+            const int lo = min(v[j], v[j + 1]), hi = max(v[j], v[j + 1]);
+            v[j] = lo;
+            v[j + 1] = hi;
+        }
 }
 
 // a neighbour rod as the step found it
@@ -648,6 +702,20 @@ __global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ Wi
         add_row(w.payA, a0, a1, F, T);
         add_row(w.payB, b0, b1, F, T);
     }
+    // the bound motors in ascending slot: a short row is sorted here
+    int ids[ROD_MOTORS];
+    const bool fits = nm <= a.mRowUse && nm <= ROD_MOTORS;
+#pragma unroll
+    for (int q = 0; q < ROD_MOTORS; q += 4) {
+        const int4 v = fits && nm > q ? *reinterpret_cast<const int4*>(a.slotM + (size_t)i * FUSED_MOTOR_SLOTS + q)
+                                      : make_int4(0, 0, 0, 0);
+        ids[q] = v.x; ids[q + 1] = v.y; ids[q + 2] = v.z; ids[q + 3] = v.w;
+    }
+#pragma unroll
+    for (int j = 0; j < ROD_MOTORS; j++)
+        if (j >= nm) ids[j] = 0x7fffffff;
+    if (fits && nm > 4) sort_slots<ROD_MOTORS>(ids);
+    else if (fits && nm > 1) sort_slots<4>(ids);
     after_previous();                    // the bonds; nothing is written before them
     if (i == 0) {
         *a.d_step = t + 1;               // (every reader of this step's index has run)
@@ -659,9 +727,32 @@ __global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ Wi
         if (i < w.tilesS) { w.sumA[i * WIDE_SUM_STRIDE] = 0; w.sumB[i * WIDE_SUM_STRIDE] = 0; }
     }
     // CrossBridgeSystem.segGather (CrossBridgeSystem.java:302-320): the bound motors' reactions
-    // in ascending slot, taken from the row's slots (and list) by repeated minimum
+    // in ascending slot, GATHER of them in flight (one after another a rod with 15 motors held
+    // its warp, and the step, for 9 us at 20,000 rods; now 3); a longer row by repeated minimum over its slots
+    // and list
     double gf[3] = {0.0, 0.0, 0.0}, gt[3] = {0.0, 0.0, 0.0};
-    for (int q = 0, last = -1; q < nm; q++) {
+    constexpr int GATHER = 4;
+#pragma unroll
+    for (int q = 0; q < ROD_MOTORS; q += GATHER) {
+        if (!fits || q >= nm) break;
+        float p[GATHER][6];
+#pragma unroll
+        for (int j = 0; j < GATHER; j++) {
+            const int m = ids[q + j];
+            const bool on = m != 0x7fffffff && SBX_IDX_OK(m, a.nM, CK_MOTOR_SLOT);
+            const float* r = sc.bondData + (int64_t)(on ? m : 0) * XB_STRIDE + 6;
+#pragma unroll
+            for (int k = 0; k < 6; k++) p[j][k] = on ? r[k] : 0.f;
+            if (!on && q + j < nm) atomicOr(a.err, ERR_LIST);
+        }
+#pragma unroll
+        for (int j = 0; j < GATHER; j++) {
+            if (q + j >= nm) break;
+            gf[0] += p[j][0]; gf[1] += p[j][1]; gf[2] += p[j][2];
+            gt[0] += p[j][3]; gt[1] += p[j][4]; gt[2] += p[j][5];
+        }
+    }
+    for (int q = 0, last = -1; !fits && q < nm; q++) {
         int next = 0x7fffffff;
         for (int j = 0; j < FUSED_MOTOR_SLOTS && j < nm && j < a.mRowUse; j++) {
             const int m = a.slotM[(size_t)i * FUSED_MOTOR_SLOTS + j];
@@ -734,9 +825,14 @@ sbx_status wide_step_impl(sbx_ctx* ctx, const WideArgs& w, const WideStreams& ws
     };
     fork(ws.start, ws.ahead);
     if (a.xlOn) ok(cudaStreamWaitEvent(ws.link, ws.start, 0));
+    // The three kernels ahead need nothing of each other: they start together while their threads
+    // fit on the chip at once (148 SMs of 2048), else one after another, as their blocks would go
+    // before the main stream's. Together and in turn: 28.8 and 30.0 us a step at 1,000 rods, 85.0
+    // and 86.4 at 100,000; 360 and 356 at 500,000 with all three let through.
+    const bool side = (int64_t)a.nB + a.nBb + a.nSeg <= 148 * 2048;
     launch(ws.ahead, false, k_wide_draws<B>, (int64_t)a.nB + a.nBb + a.nSeg, 256);
-    launch(ws.ahead, false, k_wide_terms, 2 * (int64_t)a.nM + 4 * (int64_t)a.nD, 128);
-    launch(ws.ahead, false, k_wide_joints, a.nSeg, 128);
+    launch(ws.ahead, side, k_wide_terms, 2 * (int64_t)a.nM + 4 * (int64_t)a.nD, 128);
+    launch(ws.ahead, side, k_wide_joints, a.nSeg, 128);
     if (a.xlOn) {
         launch(ws.link, false, k_wide_link_rows<B>, a.nL, 128);
         launch(ws.link, true, k_wide_link_scan, (int64_t)2 * w.tilesS * 256, 256);

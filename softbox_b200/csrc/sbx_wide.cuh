@@ -3,6 +3,9 @@
 #include "sbx_fused.cuh"
 
 constexpr int WIDE_CELL_SLOTS = 8;    // fixed slots per grid cell (one 32-byte sector)
+// fixed slots per segment row of link A ends, of link B ends: four are read with the row's
+// count, the rest only by longer rows
+constexpr int WIDE_ROW_SLOTS = 16;
 constexpr int WIDE_TILE = 4096;       // rows of a scan tile
 constexpr int WIDE_SUM_STRIDE = 8;    // ints between two tiles' sums: each in a sector of its own
 

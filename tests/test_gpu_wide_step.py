@@ -45,6 +45,24 @@ def test_rows_past_their_slots(warm, caps):
     assert len(compare_scenes(ref, got)) > 80
 
 
+@pytest.mark.parametrize("heads,links", [(2, 4), (4, 5), (5, 8), (15, 9), (16, 16), (17, 17), (40, 33)])
+def test_long_rows(warm, heads, links):
+    # one rod with many bound heads and both ends of many links, around the sizes of a row's parts
+    sc = copy.deepcopy(warm)
+    rng = np.random.default_rng(heads)
+    m = rng.permutation(len(sc["mot"]["boundSeg"]))[:heads]
+    sc["mot"]["boundSeg"][m] = 7
+    sc["mot"]["bindArc"][m] = 0.0
+    k = rng.permutation(len(sc["xl"]["linkFilA"]))
+    sc["xl"]["linkFilA"][k[:links]] = 7
+    sc["xl"]["linkFilB"][k[links:2 * links]] = 7
+    ref, _, _ = _run(sc, "unfused", steps=2)
+    got, stats, _ = _run(sc, "graph", steps=2)
+    assert np.asarray(ref["xl"]["segCountA"])[7] >= links and np.asarray(ref["xl"]["segCountB"])[7] >= links
+    assert (stats["link_list"] > 0) == (links > 16) and (stats["motor_list"] > 0) == (heads > 16)
+    assert len(compare_scenes(ref, got)) > 80
+
+
 def test_neighbours_that_do_not_point_back(warm):
     sc = copy.deepcopy(warm)
     f = sc["fil"]
