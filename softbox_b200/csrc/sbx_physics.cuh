@@ -1046,7 +1046,7 @@ SBX_DEV void motor_joint_apply(const MotorJoint& J, int which, bool second, int 
                                const float* uVec, const float* segLength, const float* jp, double f[3],
                                double t[3]) {
     double fracR = which == 0 ? (double)jp[6] : (double)jp[2];
-    double tm = J.tm[(which == 1 && nucState == NUC_ADPPI) ? 1 : 0];
+    double tm = which == 1 && nucState == NUC_ADPPI ? J.tm[1] : J.tm[0];      // (an index would put J in memory)
     double ux = uVec[s], uy = uVec[nB + s], uz = uVec[2 * nB + s];
     double len = segLength[s];
     if (!second) {

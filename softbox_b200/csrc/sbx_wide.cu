@@ -22,9 +22,9 @@
 // what a later kernel reads again is written once.
 // Every slot is computed by the same device functions as the per-system kernels, in the
 // reference's accumulation order: the same bits.
-// A step takes 29 us at 1,000 rods, 37 at 20,000, 85 at 100,000 and 353 at 500,000 (46, 57, 97 and
-// 370 with full waits and serial gathers; 200 and 434 at the last two as the per-system
-// sequence), a packed step of 12 networks (0.17e6 rods, 0.18e6 heads) 250 us (269; 366).
+// A step takes 29 us at 1,000 rods, 37 at 20,000, 79 at 100,000 and 330 at 500,000 (46, 57, 97 and
+// 370 with full waits, serial gathers and fewer warps; 200 and 434 at the last two as the
+// per-system sequence), a packed step of 12 networks (0.17e6 rods, 0.18e6 heads) 222 us (269; 366).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -137,8 +137,9 @@ __global__ void __launch_bounds__(256) k_wide_draws(const __grid_constant__ Wide
     for (int k = 0; k < 3; k++) { b->randForce[k * n + i] = rf[k]; b->randTorque[k * n + i] = rt[k]; }
 }
 
-// the chain joints, each by its lower-slot rod (as k_chain)
-__global__ void __launch_bounds__(128, 5) k_wide_joints(const __grid_constant__ WideArgs w) {
+// the chain joints, each by its lower-slot rod (as k_chain); the latency of the FP64 chains is
+// hidden by warps: 64 registers, eight blocks an SM
+__global__ void __launch_bounds__(128, 8) k_wide_joints(const __grid_constant__ WideArgs w) {
     const FusedArgs& a = w.a;
     const sbx_filament_store& fs = a.sc.fil;
     const sbx_rigid_body& fb = fs.body;
@@ -426,10 +427,11 @@ __global__ void __launch_bounds__(256) k_wide_place(const __grid_constant__ Wide
 // ---------------------------------------------------------------- bind
 constexpr int BIND_LANES = 8;        // lanes a head
 // The reach walk with the nearest choice, the nucleotide cycle and the bound head's entry in its
-// rod's motor row: a warp takes 32 / BIND_LANES consecutive heads.
+// rod's motor row: a warp takes 32 / BIND_LANES consecutive heads. (64 registers here and in the
+// terms: 222 us a packed step of 12 networks, 228 with 68 and 76.)
 constexpr int BIND_HEADS = 32 / BIND_LANES;
 template <bool B>
-__global__ void __launch_bounds__(128) k_wide_bind(const __grid_constant__ WideArgs w) {
+__global__ void __launch_bounds__(128, 8) k_wide_bind(const __grid_constant__ WideArgs w) {
     const FusedArgs& a = w.a;
     const sbx_dense_scene& sc = a.sc;
     const sbx_motor_store& mot = sc.mot;
@@ -479,7 +481,7 @@ __global__ void __launch_bounds__(128) k_wide_bind(const __grid_constant__ WideA
 // ---------------------------------------------------------------- terms and mini
 // The position-only myosin terms, one a thread, beside the grid kernels: FP64 chains of some
 // thousand cycles that would otherwise sit between binding and integration.
-__global__ void __launch_bounds__(128) k_wide_terms(const __grid_constant__ WideArgs w) {
+__global__ void __launch_bounds__(128, 8) k_wide_terms(const __grid_constant__ WideArgs w) {
     let_next_start();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < 2 * w.a.nM + 4 * w.a.nD) myosin_term(w.a, k);
@@ -488,10 +490,13 @@ __global__ void __launch_bounds__(128) k_wide_terms(const __grid_constant__ Wide
 
 // One block a minifilament: a warp for its heads (with their bonds), its rods, its levers, then
 // the integration of its sub-bodies in body order. The backbones, one a thread, take the
-// blocks after them.
+// blocks after them. A block waits for memory twice (terms, then bodies), so blocks in flight
+// count for more than registers: at ten an SM (64 registers, 150 bytes spilled) a step of
+// 500,000 rods takes 337 us, at seven (88 registers) 355; a packed step of 12 networks 228 and
+// 250. (Twelve an SM gave the same as ten; prefetching the bodies to L1 was slower.)
 constexpr int MINI_THREADS = 96;
 template <bool B>
-__global__ void __launch_bounds__(MINI_THREADS) k_wide_mini(const __grid_constant__ WideArgs w) {
+__global__ void __launch_bounds__(MINI_THREADS, 10) k_wide_mini(const __grid_constant__ WideArgs w) {
     let_next_start();
     __shared__ MiniSmem sm;
     const FusedArgs& a = w.a;
