@@ -747,12 +747,12 @@ sbx_status sbx_dense_plan_create(sbx_ctx* ctx, const sbx_dense_scene* scene, sbx
 /* Advances steps t0, t0+1, ..., t0+nsteps-1 (the step index feeds every RNG key and
  * the containment cadence). mode 0: the call sequence of the per-system entry points
  * (zero + draws and confine + integrate + derive as the MechanicsFusion passes, which give
- * the same values); 1: one CUDA-graph replay per step (wide kernels for a scene of the harness
+ * the same values); 1: CUDA-graph replays of one step, or of a few (wide kernels for a scene of the harness
  * layout, else that sequence); 2: the fused persistent kernel (all nsteps in one cooperative
  * launch; available when the scene has the harness layout, see
  * sbx_dense_plan_fused_available). All three give the same bits. mode 3 (auto): the graph of
- * wide kernels, which leads at every size (us per step, graph / fused: 48 / 57 at 1,000 rods one
- * step a call; 55 / 64 at 2e4 and 67 / 172 at 4e4, 20 steps a call); without it, or on a stream
+ * wide kernels, which leads at every size (us per step, graph / fused: 30 / 57 at 1,000 rods one
+ * step a call; 35 / 64 at 2e4 and 54 / 172 at 4e4, 20 steps a call); without it, or on a stream
  * under capture, the fused kernel up to SBX_DENSE_AUTO_MAX_FUSED_RODS rods when available, the
  * graph path above it. */
 #define SBX_DENSE_AUTO_MAX_FUSED_RODS 40960

@@ -390,8 +390,10 @@ struct sbx_dense_plan {
     sbx_ctx* ctx = nullptr;
     sbx_dense_scene scene;
     int* d_step = nullptr;
-    cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    cudaGraphExec_t execMany = nullptr;      // GRAPH_STEPS steps, or none
+    int64_t stepNow = INT64_MIN;             // *d_step once the queued work is done, if known
+    bool stepShared = false;                 // a fused run, which a captured graph may replay, sets *d_step too
     int kernels_per_step = 0;
     // fused persistent path
     bool fused_ok = false;
@@ -709,17 +711,52 @@ extern "C" sbx_status sbx_dense_step_unfused(sbx_ctx* ctx, const sbx_dense_scene
     return dense_sequence(ctx, sc, nullptr, t);
 }
 
+// Runs of at least GRAPH_STEPS steps take graphs of that many. Between two graphs of one step
+// each there are about 5 us, between two steps of one graph 2 to 3: a step of 20 takes 25.7 us
+// (28.8) at 1,000 rods, 34.8 (37.1) at 20,000, 77.4 (79) at 100,000; eight steps a graph gave 26.1,
+// 35.5 and 77. Above GRAPH_STEPS_RODS the gap is lost in the step and its branches start in a
+// worse order: 106 and 109.5 us at 150,000 rods, 203 and 207 at 300,000, one step a graph first.
+// The first plan of a process takes 15 ms more to make, a later one 0.6.
+constexpr int GRAPH_STEPS = 4, GRAPH_STEPS_RODS = 1 << 17;
+
+// Captures `steps` steps into a graph, ready to launch
+static sbx_status capture_steps(sbx_dense_plan* p, int steps, cudaGraphExec_t* exec, int* launches) {
+    sbx_ctx* ctx = p->ctx;
+    const int64_t l0 = ctx->launches;
+    if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
+        return fail(ctx, SBX_ECUDA, "dense plan: begin capture");
+    sbx_status st = SBX_OK;
+    for (int k = 0; k < steps && st == SBX_OK; k++) {
+        if (p->wide_ok) {
+            st = wide_step(ctx, p->wide, p->batched, p->wideStreams);
+        } else {
+            StepNoise sn{p->noise, p->noiseErr};
+            PlanScratch use(p);
+            st = dense_sequence(ctx, &p->scene, p->d_step, 0, p->batched ? &p->batch : nullptr, &p->side,
+                                p->noiseOn ? &sn : nullptr);
+            if (st == SBX_OK) SBX_LAUNCH(ctx, k_step_advance, 1, 1, p->d_step);
+        }
+    }
+    *launches = (int)(ctx->launches - l0);
+    ctx->launches = l0;
+    cudaGraph_t g = nullptr;
+    cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
+    if (st == SBX_OK && ce == cudaSuccess) ce = cudaGraphInstantiate(exec, g, 0);
+    if (st == SBX_OK && ce == cudaSuccess) ce = cudaGraphUpload(*exec, ctx->stream);    // not in the first launch
+    if (g) cudaGraphDestroy(g);                  // (the executable graph holds its own copy)
+    if (st != SBX_OK || ce != cudaSuccess) {
+        cudaGetLastError();
+        return st != SBX_OK ? st : fail(ctx, SBX_ECUDA, std::string("dense plan: graph: ") + cudaGetErrorString(ce));
+    }
+    return SBX_OK;
+}
+
 // Captures one step (the sequence, then the step-counter advance) into the plan's graph,
 // replacing a previous capture; the supplied noise, when on, is part of the capture.
 static sbx_status capture_step(sbx_dense_plan* p) {
     SBX_TRACE("sbx.dense.capture");
     sbx_ctx* ctx = p->ctx;
     cudaStreamSynchronize(ctx->stream);
-    int64_t l0 = ctx->launches;
-    if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-        return fail(ctx, SBX_ECUDA, "dense plan: begin capture");
-    sbx_status st;
-    StepNoise sn{p->noise, p->noiseErr};
     if (p->wide_ok) {
         FusedArgs& a = p->wide.a;
         a.nzFil = p->noiseOn ? p->noise.fil : nullptr;
@@ -728,34 +765,21 @@ static sbx_status capture_step(sbx_dense_plan* p) {
         a.nzT0 = p->noise.t0;
         a.nzN = p->noise.nsteps;
         p->wide.noiseErr = p->noiseErr;
-        st = wide_step(ctx, p->wide, p->batched, p->wideStreams);
-    } else {
-        PlanScratch use(p);
-        st = dense_sequence(ctx, &p->scene, p->d_step, 0, p->batched ? &p->batch : nullptr, &p->side,
-                            p->noiseOn ? &sn : nullptr);
     }
-    if (st == SBX_OK && !p->wide_ok) SBX_LAUNCH(ctx, k_step_advance, 1, 1, p->d_step);
-    cudaGraph_t g = nullptr;
-    cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
-    if (st != SBX_OK || ce != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        ctx->launches = l0;
-        cudaGetLastError();
-        return st != SBX_OK ? st : fail(ctx, SBX_ECUDA, std::string("end capture: ") + cudaGetErrorString(ce));
+    cudaGraphExec_t one = nullptr, many = nullptr;
+    int launches = 0;
+    sbx_status st = capture_steps(p, 1, &one, &launches);
+    if (st == SBX_OK && p->wide_ok && p->scene.fil.body.n <= GRAPH_STEPS_RODS) {
+        int all = 0;
+        st = capture_steps(p, GRAPH_STEPS, &many, &all);
+        if (st != SBX_OK) cudaGraphExecDestroy(one);
     }
-    cudaGraphExec_t ex = nullptr;
-    if (cudaGraphInstantiate(&ex, g, 0) != cudaSuccess) {
-        cudaGraphDestroy(g);
-        ctx->launches = l0;
-        cudaGetLastError();
-        return fail(ctx, SBX_ECUDA, "dense plan: graph instantiate");
-    }
+    if (st != SBX_OK) return st;
     if (p->exec) cudaGraphExecDestroy(p->exec);
-    if (p->graph) cudaGraphDestroy(p->graph);
-    p->graph = g;
-    p->exec = ex;
-    p->kernels_per_step = (int)(ctx->launches - l0);
-    ctx->launches = l0;
+    if (p->execMany) cudaGraphExecDestroy(p->execMany);
+    p->exec = one;
+    p->execMany = many;
+    p->kernels_per_step = launches;
     return SBX_OK;
 }
 
@@ -847,8 +871,8 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
     if (p->noiseOn && ((int64_t)t0 < p->noise.t0 || (int64_t)t0 + nsteps > (int64_t)p->noise.t0 + p->noise.nsteps))
         return fail(ctx, SBX_EINVAL, "sbx_dense_plan_run: steps outside the supplied-noise range");
     if (mode == 3) {
-        // the wide kernels lead at every size: 48 / 57 us a step at 1,000 rods (one step a call),
-        // 55 / 64 at 20,000 and 67 / 172 at 40,000 (20 steps a call) against the fused kernel
+        // the wide kernels lead at every size: 30 / 57 us a step at 1,000 rods (one step a call),
+        // 35 / 64 at 20,000 and 54 / 172 at 40,000 (20 steps a call) against the fused kernel
         const bool fused = p->fused_ok && p->scene.fil.body.n <= SBX_DENSE_AUTO_MAX_FUSED_RODS;
         // (a stream under capture takes the fused kernel as one node; a graph cannot be launched there)
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -869,18 +893,26 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
             cudaMemsetAsync(p->fa.bar, 0, 32, ctx->stream);
             p->fused_dirty = false;
         }
+        p->stepShared = true;
         SBX_TRACE("sbx.dense.fused_launch");
         return fused_launch(ctx, p->fa, p->fused_grid, t0, nsteps);
     }
     if (mode == 1) {
         SBX_TRACE("sbx.dense.graph_replay");
-        SBX_LAUNCH(ctx, k_step_set, 1, 1, p->d_step, t0);
-        for (int k = 0; k < nsteps; k++) {
-            if (cudaGraphLaunch(p->exec, ctx->stream) != cudaSuccess)
+        // a run that goes on where the last one ended finds its step index in place
+        if (p->stepShared || p->stepNow != t0) SBX_LAUNCH(ctx, k_step_set, 1, 1, p->d_step, t0);
+        p->stepNow = INT64_MIN;
+        for (int k = 0; k < nsteps;) {
+            const bool many = p->execMany && nsteps - k >= GRAPH_STEPS;
+            const int n = many ? GRAPH_STEPS : 1;
+            if (cudaGraphLaunch(many ? p->execMany : p->exec, ctx->stream) != cudaSuccess)
                 return fail(ctx, SBX_ECUDA, "sbx_dense_plan_run: graph launch");
-            ctx->launches += p->kernels_per_step;
+            ctx->launches += (int64_t)n * p->kernels_per_step;
+            k += n;
         }
-        return check_launch(ctx, "sbx_dense_plan_run");
+        CHK(check_launch(ctx, "sbx_dense_plan_run"));
+        p->stepNow = (int64_t)t0 + nsteps;
+        return SBX_OK;
     }
     SBX_TRACE("sbx.dense.unfused");
     PlanScratch use(p);
@@ -1041,7 +1073,7 @@ extern "C" sbx_status sbx_dense_plan_destroy(sbx_dense_plan* p) {
     // exit), so it touches no context state here: a device-wide wait before the frees
     cudaDeviceSynchronize();
     if (p->exec) cudaGraphExecDestroy(p->exec);
-    if (p->graph) cudaGraphDestroy(p->graph);
+    if (p->execMany) cudaGraphExecDestroy(p->execMany);
     if (p->d_step) cudaFree(p->d_step);
     if (p->scratch) cudaFree(p->scratch);
     if (p->noiseErr) cudaFree(p->noiseErr);

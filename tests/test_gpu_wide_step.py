@@ -102,6 +102,27 @@ def test_graph_and_fused_steps_alternate(warm):
     net.close()
 
 
+@pytest.mark.parametrize("runs", [((300, 3), (303, 4), (307, 5), (312, 1)), ((300, 9), (400, 2), (402, 8), (0, 1))],
+                         ids=["on", "jumps"])
+def test_runs_of_any_length(warm, runs):
+    # runs around the steps of a graph, each going on from the last one or from another step index
+    from softbox_b200.engine import DenseNetwork
+    out = []
+    for mode in ("unfused", "graph"):
+        net = DenseNetwork(copy.deepcopy(warm))
+        for t, n in runs:
+            net.run(t, n, mode=mode)
+        if mode == "graph":                            # the fused kernel moves the step index as well
+            net.run(20, 2, mode="fused")
+            net.run(22, 5, mode="graph")
+        else:
+            net.run(20, 7, mode=mode)
+        assert net.status() == 0
+        out.append(D.to_host(net.dev))
+        net.close()
+    assert len(compare_scenes(*out)) > 80
+
+
 def test_auto_takes_the_graph_and_fused_runs_after_a_refresh(warm):
     from softbox_b200.engine import DenseNetwork
     from softbox_b200.runtime import LIB
