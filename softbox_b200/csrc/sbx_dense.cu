@@ -605,23 +605,34 @@ struct Arena {
     }
 };
 
-// the row slots, lists, snapshots and terms both shapes of the step use (each its own set)
-void step_carve(Arena& m, FusedArgs& a, int cellSlots, int rowSlots) {
+// The row slots, lists, snapshots and terms both shapes of the step use. What a completed step
+// leaves empty for the next one (histograms, list heads) is each shape's own; what lives within
+// a step is taken from the other shape's set when that is given, whose strides are the larger.
+void step_carve(Arena& m, FusedArgs& a, int cellSlots, int rowSlots, const FusedArgs* other) {
     const size_t nS = a.nSeg, nLk = (size_t)std::max(a.nL, 1), C = a.C;
     m.take(a.cntCell, 4 * C); m.take(a.cntSeg, 4 * C);
-    m.take(a.segCellOff, 4 * (C + 1));
     for (int** q : {&a.cntAct, &a.cntA, &a.cntB, &a.cntM, &a.headA, &a.headB, &a.headM}) m.take(*q, 4 * nS);
+    m.take(a.cellHead, 4 * C);
+    m.take(a.reachMax, 4);
+    m.take(a.err, 16);
+    if (other) {
+        a.segCellOff = other->segCellOff;
+        a.cellSlot = other->cellSlot; a.slotA = other->slotA; a.slotB = other->slotB; a.slotM = other->slotM;
+        a.cellNext = other->cellNext; a.nextA = other->nextA; a.nextB = other->nextB; a.nextM = other->nextM;
+        a.segE1 = other->segE1; a.segE2 = other->segE2;
+        a.joints = other->joints; a.terms = other->terms; a.uSnap = other->uSnap;
+        return;
+    }
+    m.take(a.segCellOff, 4 * (C + 1));
     m.take(a.cellSlot, 4 * C * cellSlots);
     m.take(a.slotA, 4 * nS * rowSlots); m.take(a.slotB, 4 * nS * rowSlots);
     m.take(a.slotM, 4 * nS * FUSED_MOTOR_SLOTS);
-    m.take(a.cellHead, 4 * C); m.take(a.cellNext, 4 * (size_t)a.cap);
+    m.take(a.cellNext, 4 * (size_t)a.cap);
     m.take(a.nextA, 4 * nLk); m.take(a.nextB, 4 * nLk); m.take(a.nextM, 4 * (size_t)a.nM);
     m.take(a.segE1, 16 * nS); m.take(a.segE2, 16 * nS);
     m.take(a.joints, 8 * nS * FUSED_JOINT_PLANES);
     m.take(a.terms, 8 * (FUSED_MOTOR_PLANES * (size_t)a.nM + FUSED_DIMER_PLANES * (size_t)a.nD));
     m.take(a.uSnap, 12 * nS);
-    m.take(a.reachMax, 4);
-    m.take(a.err, 16);
 }
 
 // empty histograms and lists, as every completed step leaves them
@@ -635,6 +646,7 @@ void step_reset(sbx_ctx* ctx, FusedArgs& a) {
     cudaMemsetAsync(a.err, 0, 16, ctx->stream);
 }
 
+static_assert(FUSED_CELL_SLOTS <= WIDE_CELL_SLOTS && FUSED_ROW_SLOTS <= WIDE_ROW_SLOTS, "the shared sets' strides");
 bool fused_prepare(sbx_dense_plan* p) {
     const sbx_dense_scene& sc = p->scene;
     cudaStream_t st = p->ctx->stream;
@@ -653,7 +665,7 @@ bool fused_prepare(sbx_dense_plan* p) {
     a.filSeed = fc[2];
     Arena m;
     if (!m.build(p, [&] {
-            step_carve(m, a, FUSED_CELL_SLOTS, FUSED_ROW_SLOTS);
+            step_carve(m, a, FUSED_CELL_SLOTS, FUSED_ROW_SLOTS, p->wide_ok ? &p->wide.a : nullptr);
             m.take(a.tileSum, 4 * (size_t)(2 * a.tilesC + 2 * a.tilesS + 1));
             m.take(a.mTileSum, 4 * (size_t)(a.tilesS + 1));
             m.take(a.bar, 32);
@@ -688,7 +700,7 @@ bool wide_prepare(sbx_dense_plan* p) {
     int* sums = nullptr;
     Arena m;
     if (!m.build(p, [&] {
-            step_carve(m, a, WIDE_CELL_SLOTS, WIDE_ROW_SLOTS);
+            step_carve(m, a, WIDE_CELL_SLOTS, WIDE_ROW_SLOTS, nullptr);
             m.take(w.payA, 24 * nLk);
             m.take(w.payB, 24 * nLk);
             m.take(sums, 4 * words);
