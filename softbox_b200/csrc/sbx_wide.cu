@@ -22,9 +22,9 @@
 // what a later kernel reads again is written once.
 // Every slot is computed by the same device functions as the per-system kernels, in the
 // reference's accumulation order: the same bits.
-// A step takes 29 us at 1,000 rods, 37 at 20,000, 79 at 100,000 and 330 at 500,000 (46, 57, 97 and
+// A step takes 26 us at 1,000 rods, 35 at 20,000, 75 at 100,000 and 325 at 500,000 (46, 57, 97 and
 // 370 with full waits, serial gathers and fewer warps; 200 and 434 at the last two as the
-// per-system sequence), a packed step of 12 networks (0.17e6 rods, 0.18e6 heads) 222 us (269; 366).
+// per-system sequence), a packed step of 12 networks (0.17e6 rods, 0.18e6 heads) 219 us (269; 366).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -57,6 +57,8 @@ __device__ __forceinline__ GridView grid_view(const WideArgs& w, int net) {
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // the next kernel of the stream may start its blocks once every block is here or done
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 struct AfterPrevious {
     __device__ __forceinline__ void operator()() const { after_previous(); }
@@ -654,8 +656,13 @@ __device__ __forceinline__ RodGeom start_rod(const FusedArgs& a, int j) {
 // Chain forces from the joints made ahead, the crosslinker and motor gathers, the walls and the
 // Langevin update of one rod a thread, in the reference's order; the rod's histograms are reset
 // for the next step. A joint whose neighbour does not point back is computed from this side.
-template <bool B>
-__global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ WideArgs w) {
+// MANY: for more rods than are on the chip at once at four blocks an SM, six (80 registers): what
+// only the integration takes goes towards L1 first and is read after the bonds. 78.5 and 74.5 us
+// a step at 100,000 rods, 329 and 325 at 500,000, 221 and 218.6 a packed step of 12 networks; but
+// 25.9 and 26.6 at 1,000, 35.3 and 36.7 at 20,000, where the last read is on the step's path.
+constexpr int RODS_AT_ONCE = 148 * 4 * 128;
+template <bool B, bool MANY>
+__global__ void __launch_bounds__(128, MANY ? 6 : 4) k_wide_rods(const __grid_constant__ WideArgs w) {
     const FusedArgs& a = w.a;
     const sbx_dense_scene& sc = a.sc;
     const sbx_filament_store& fs = sc.fil;
@@ -674,7 +681,17 @@ __global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ Wi
         b0 = xl.segOffsetsB[i]; b1 = xl.segOffsetsB[i + 1];
         act = a.cntAct[i];
     }
-    const BodyIn in = body_load(fb, i);
+    BodyIn in;
+    if (MANY) {
+        for (int k = 0; k < 3; k++) { in.p.c[k] = fb.coord[k * n + i]; in.p.u[k] = fb.uVec[k * n + i]; }
+        in.len = fb.segLength[i]; in.gT[0] = fb.bTransGam[i]; in.gT[1] = fb.bTransGam[n + i]; in.gR[1] = fb.bRotGam[n + i];
+        for (int k = 0; k < 3; k++) {
+            prefetch_l1(fb.yVec + k * n + i); prefetch_l1(fb.randForce + k * n + i); prefetch_l1(fb.randTorque + k * n + i);
+            if (fb.coord64) prefetch_l1(fb.coord64 + k * n + i);
+        }
+    } else {
+        in = body_load(fb, i);
+    }
     const ChainParams cp = chain_params(fs.chainParams);
     double fd[3] = {0.0, 0.0, 0.0}, td[3] = {0.0, 0.0, 0.0};
     RodGeom me;
@@ -780,6 +797,7 @@ __global__ void __launch_bounds__(128, 4) k_wide_rods(const __grid_constant__ Wi
         last = next;
     }
     for (int k = 0; k < 3; k++) { F[k] = (float)(F[k] + gf[k]); T[k] = (float)(T[k] + gt[k]); }
+    if (MANY) in = body_load(fb, i);
     const float* box = B ? w.bt.boxParams + 8 * w.bt.segKey[2 * i] : sc.boxParams;
     const BoxParams bx = box_params(box, t);
     if (bx.active) confine_one(bx, in.p.c, in.p.u, in.len, in.gT[0], F, T);
@@ -854,7 +872,8 @@ sbx_status wide_step_impl(sbx_ctx* ctx, const WideArgs& w, const WideStreams& ws
     if (a.xlOn) join(ws.linkDone, ws.link);
     launch(s, false, k_wide_mini<B>, ((int64_t)a.nBb + (a.nBb + MINI_THREADS - 1) / MINI_THREADS) * MINI_THREADS,
            MINI_THREADS);
-    launch(s, true, k_wide_rods<B>, a.nSeg, 128);
+    if (a.nSeg > RODS_AT_ONCE) launch(s, true, k_wide_rods<B, true>, a.nSeg, 128);
+    else launch(s, true, k_wide_rods<B, false>, a.nSeg, 128);
     join(ws.csrDone, ws.csr);
     if (e != cudaSuccess) return fail(ctx, SBX_ECUDA, std::string("dense step: streams: ") + cudaGetErrorString(e));
     return check_launch(ctx, "dense step");

@@ -88,6 +88,23 @@ def test_other_layouts_keep_the_per_system_sequence(warm):
     assert len(compare_scenes(ref, got)) > 80
 
 
+@pytest.mark.parametrize("rods", [75_770, 75_780])
+def test_rods_kernel_on_both_sides_of_its_rule(rods):
+    # above 148 x 4 x 128 rods the kernel with more blocks an SM
+    from softbox_b200 import scenes
+    from softbox_b200.engine import DenseNetwork
+    sc = scenes.dense_contractile(scenes.dense_scaled(rods))
+    n = len(sc["fil"]["end1NbrSlot"])
+    out = []
+    for mode in ("unfused", "graph"):
+        net = DenseNetwork(copy.deepcopy(sc), fp64_coords=True)
+        net.run(0, 6, mode=mode)
+        assert net.status() == 0
+        out.append(D.to_host(net.dev))
+        net.close()
+    assert len(compare_scenes(*out)) > 80 and n == rods
+
+
 def test_graph_and_fused_steps_alternate(warm):
     from softbox_b200.engine import DenseNetwork
     ref, _, _ = _run(warm, "unfused", steps=12)
