@@ -12,8 +12,8 @@ scene builder with these counts); no dataset.
 Both arms first advance the network WARM_STEPS steps untimed, to the state where binding
 has built up (about 700 bound heads; a fresh scene has about 120 in its first 25 steps),
 then take W untimed warm-up steps and time K steps.
-Our arm: each step is one launch of the fused persistent kernel; timed with CUDA events
-on the library's stream, one step at a time, with L2 flushed (a 256 MiB write) between
+Our arm: each step is one call of the library's step in its default mode (a CUDA graph of
+wide kernels); timed with CUDA events on the library's stream, one step at a time, with L2 flushed (a 256 MiB write) between
 timed steps. The reference arm times the reference's CPU path: the C++ restatement of
 the Java System classes (oracle/), on all host threads, on the same workload, for at
 least REF_MIN_STEPS timed steps.
@@ -44,12 +44,11 @@ from softbox_b200.roofline import peaks, step_bytes  # noqa: E402
 
 WARM_STEPS = 3000      # untimed steps before the warm-up: bound heads have built up
 REF_MIN_STEPS = 200    # the reference arm times at least this many steps
-# DRAM bytes (read + write) of one launch of the fused kernel advancing one step of this
-# workload (FP64 centres, warmed state, L2 flushed before the launch), from one ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum, mean of three launches of
-# `python bench.py --steps 3 --warmup 3 --no-cpu --sweep-points 0` under
-# `ncu --clock-control none -k regex:k_dense_fused -s 1 -c 3`)
-FUSED_STEP_DRAM_BYTES = 12_302_000
+# DRAM bytes (read + write) of the 14 kernels of one step of this workload (FP64 centres, warmed
+# state), the caches flushed before each kernel, from one ncu capture (dram__bytes_read.sum +
+# dram__bytes_write.sum, mean of three steps of `python bench.py --steps 3 --warmup 3 --no-cpu
+# --sweep-points 0` under `ncu --clock-control none -k regex:k_wide -s 42042 -c 42`)
+STEP_DRAM_BYTES = 20_777_000
 
 
 def workload_config(sc_host, warmup):
@@ -204,16 +203,15 @@ def run_ours(args):
     ctx = Context(local)
     sc_host = scenes.dense_contractile(scenes.C1)
     net = DenseNetwork(sc_host, ctx=ctx, fp64_coords=True)
-    assert net.fused_available, "the benchmark network must qualify for the fused path"
     stream = torch.cuda.ExternalStream(LIB.sbx_ctx_stream(ctx.h))
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=f"cuda:{local}")
     nrods = sc_host["fil"]["body"]["n"]
 
     def one_step(t):
-        net.run(t, 1, mode="fused")
+        net.run(t, 1)
 
-    # advance to the warmed state (one persistent launch), untimed
-    net.run(0, WARM_STEPS, mode="fused")
+    # advance to the warmed state, untimed
+    net.run(0, WARM_STEPS)
     net.status()
     t = WARM_STEPS
     with torch.cuda.stream(stream):
@@ -250,7 +248,7 @@ def run_ours(args):
 
     # e2e through the C ABI: per step, H2D of the step's counts blocks (the reference's
     # EVERY_EXECUTION upload: motor, backbone and filament counts, 3 x 16 B, contiguous on
-    # the device, so one copy) from pinned memory, one fused step, D2H of the step's binding
+    # the device, so one copy) from pinned memory, one step, D2H of the step's binding
     # state (boundSeg) into pinned memory.
     # Pipelined as a streaming host would run it: step k is queued (upload, launch, result
     # copy, marker) before the host waits for step k - 1's result; two pinned buffers each.
@@ -276,7 +274,7 @@ def run_ours(args):
         ctx("sbx_upload", C.c_void_p(net.counts_block.data_ptr()), C.c_void_p(counts_host[b].data_ptr()), h2d)
         if k > 0:
             ctx("sbx_ctx_stream_wait_mark", 1 - b)       # the step rewrites boundSeg: after k - 1's copy
-        st = LIB.sbx_dense_plan_run(net.plan, t, 1, 2)
+        st = LIB.sbx_dense_plan_run(net.plan, t, 1, 3)
         assert st == 0, ctx.last_error()
         ctx("sbx_download_async_side", C.c_void_p(bound_host[b].data_ptr()),
             C.c_void_p(d["mot"]["boundSeg"].data_ptr()), d2h)
@@ -294,11 +292,12 @@ def run_ours(args):
         e2e_s = float(tt.item())
     e2e = ws * nrods * e2e_steps / e2e_s
 
-    # roofline of the dominant (only) kernel: the fused step
+    # roofline of the step
     hbm, how = peaks()
     bytes_step = step_bytes(sc_host, fp64=True)
     achieved = bytes_step / (float(np.mean(step_ms)) / 1e3) / 1e9
-    traffic = FUSED_STEP_DRAM_BYTES
+    traffic = STEP_DRAM_BYTES
+    launches = net.kernels_per_step
 
     cpu = None
     if rank == 0 and ws == 1 and not args.no_cpu:
@@ -322,16 +321,16 @@ def run_ours(args):
                 "warmup": max(3, args.warmup), "ms_per_step": total_ms / args.steps, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "f32 forces, f64 centres", "data": "synthetic",
                 "config": workload_config(sc_host, max(3, args.warmup)),
-                "arm": {"path": "fused persistent cooperative kernel, 1 launch per step",
-                        "parallelism": f"replicas x{ws}", "grid_ctas": net.fused_grid, "state_at_timing": state},
+                "arm": {"path": f"CUDA graph of wide kernels, {launches} kernels per step",
+                        "parallelism": f"replicas x{ws}", "state_at_timing": state},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                              "frac": achieved / hbm, "traffic": traffic, "peak_source": how,
-                             "kernel": "k_dense_fused", "algorithmic_bytes_per_launch": bytes_step},
+                             "kernel": "k_wide_* (one step)", "algorithmic_bytes_per_launch": bytes_step},
                 "cpu_baseline": cpu,
                 "e2e": {"value": e2e, "unit": "rod-steps/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                         "host_loop": "C ABI from Python; each step's upload, launch and result copy (on the copy stream) queued "
                                      "before the host waits for the previous step's result (L2 not flushed)"},
-                "gpu_launches": args.steps,
+                "gpu_launches": args.steps * launches,
                 "clocks": clocks,
                 "step_ms_median": float(np.median(step_ms)), "step_ms_p90": float(np.percentile(step_ms, 90)),
                 "sweep": sweep}
