@@ -362,8 +362,8 @@ __device__ __forceinline__ int core_at(int r, int c, int Kp) {
 // rows [0, rows) x [0, Kp) of a row-major BF16 matrix (16-byte aligned rows, rows a multiple of
 // 8) into the core-matrix layout by 16-byte async copies; rows past rowsValid are zero. Item u
 // is row u & 7 of core matrix u >> 3, so the shared addresses run with u and a warp's copies
-// meet no bank twice (with the row's columns along the lanes they all met one: staging 160
-// rows of 256 took 3.2 us of a 10 us pass).
+// meet no bank twice (the copies' latency bounds it: with the columns along the lanes, and all
+// copies on one bank, a pass took the same time).
 __device__ __forceinline__ void stage_rows(char* dst, const __nv_bfloat16* src, int ld, int rows, int rowsValid,
                                            int Kp) {
     const int kg = Kp >> 3, r8 = threadIdx.x & 7, step = blockDim.x >> 3, cores = (rows >> 3) * kg;
@@ -526,7 +526,7 @@ __global__ void k_predict_stats(int nz, long long n, double* out) {
 // in row order. The arithmetic, element by element, is that of the separate kernels.
 // What bounds it is latency: per pass an operand fetch from L2, a short MMA chain, an
 // epilogue and a barrier. As 42 launches a step the host's calls bounded it: 551 us a step of 5 networks at a batch of 256,
-// 127 us now.
+// 110 us now.
 constexpr int TRAIN_THREADS = 256;
 constexpr int TRAIN_N = 32;                        // columns of a tile
 constexpr int TRAIN_STEPS = 64;                    // steps a launch takes (the bias corrections are arguments)
