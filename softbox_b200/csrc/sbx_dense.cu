@@ -393,7 +393,7 @@ struct sbx_dense_plan {
     cudaGraphExec_t exec = nullptr;
     cudaGraphExec_t execMany = nullptr;      // GRAPH_STEPS steps, or none
     int64_t stepNow = INT64_MIN;             // *d_step once the queued work is done, if known
-    bool stepShared = false;                 // a fused run, which a captured graph may replay, sets *d_step too
+    bool stepShared = false;                 // others set *d_step: the fused kernel, a graph that captured a run
     int kernels_per_step = 0;
     // fused persistent path
     bool fused_ok = false;
@@ -911,14 +911,20 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
     }
     if (mode == 1) {
         SBX_TRACE("sbx.dense.graph_replay");
-        // a run that goes on where the last one ended finds its step index in place
+        // A run that goes on where the last one ended finds its step index in place; not where a
+        // graph that captured a run may be replayed in between.
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) cudaGetLastError();
+        if (capture != cudaStreamCaptureStatusNone) p->stepShared = true;
         if (p->stepShared || p->stepNow != t0) SBX_LAUNCH(ctx, k_step_set, 1, 1, p->d_step, t0);
         p->stepNow = INT64_MIN;
         for (int k = 0; k < nsteps;) {
             const bool many = p->execMany && nsteps - k >= GRAPH_STEPS;
             const int n = many ? GRAPH_STEPS : 1;
-            if (cudaGraphLaunch(many ? p->execMany : p->exec, ctx->stream) != cudaSuccess)
+            if (cudaGraphLaunch(many ? p->execMany : p->exec, ctx->stream) != cudaSuccess) {
+                cudaGetLastError();
                 return fail(ctx, SBX_ECUDA, "sbx_dense_plan_run: graph launch");
+            }
             ctx->launches += (int64_t)n * p->kernels_per_step;
             k += n;
         }

@@ -140,6 +140,32 @@ def test_runs_of_any_length(warm, runs):
     assert len(compare_scenes(*out)) > 80
 
 
+def test_step_index_beside_a_captured_run(warm):
+    # a captured run (the fused kernel) moves the step index at its replay, not at its capture
+    from softbox_b200.engine import DenseNetwork
+    from softbox_b200.runtime import LIB
+    ref = DenseNetwork(copy.deepcopy(warm))
+    for t, n in ((300, 3), (303, 5), (303, 2), (308, 4), (312, 1)):
+        ref.run(t, n, mode="unfused")
+    net = DenseNetwork(copy.deepcopy(warm))
+    net.run(300, 3, mode="graph")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(LIB.sbx_ctx_stream(net.ctx.h))):
+        net.run(303, 2)
+    net.run(303, 5, mode="graph")
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    net.run(308, 4, mode="graph")
+    net.run(312, 1, mode="graph")
+    assert net.status() == 0 and ref.status() == 0
+    assert len(compare_scenes(D.to_host(ref.dev), D.to_host(net.dev))) > 80
+    del g
+    ref.close()
+    net.close()
+
+
 def test_auto_takes_the_graph_and_fused_runs_after_a_refresh(warm):
     from softbox_b200.engine import DenseNetwork
     from softbox_b200.runtime import LIB
