@@ -753,8 +753,8 @@ sbx_status sbx_dense_plan_create(sbx_ctx* ctx, const sbx_dense_scene* scene, sbx
  * sbx_dense_plan_fused_available). All three give the same bits. mode 3 (auto): the graph of
  * wide kernels, which leads at every size (us per step, graph / fused: 30 / 57 at 1,000 rods one
  * step a call; 35 / 64 at 2e4 and 54 / 172 at 4e4, 20 steps a call); without it, or on a stream
- * under capture, the fused kernel up to SBX_DENSE_AUTO_MAX_FUSED_RODS rods when available, the
- * graph path above it. */
+ * under capture, the fused kernel up to SBX_DENSE_AUTO_MAX_FUSED_RODS rods when available (mode 0
+ * under capture after a refresh), the graph path above it. */
 #define SBX_DENSE_AUTO_MAX_FUSED_RODS 40960
 sbx_status sbx_dense_plan_run(sbx_dense_plan* plan, int32_t t0, int32_t nsteps, int32_t mode);
 /* Runs one step as the unfused per-system call sequence (reference granularity). */

@@ -886,10 +886,13 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
         // the wide kernels lead at every size: 30 / 57 us a step at 1,000 rods (one step a call),
         // 35 / 64 at 20,000 and 54 / 172 at 40,000 (20 steps a call) against the fused kernel
         const bool fused = p->fused_ok && p->scene.fil.body.n <= SBX_DENSE_AUTO_MAX_FUSED_RODS;
-        // (a stream under capture takes the fused kernel as one node; a graph cannot be launched there)
+        // (a graph cannot be launched on a stream under capture: that takes the fused kernel as one
+        // node, or the per-system kernels while the fused topology, which the host reads, is stale)
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (fused && p->wide_ok && cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) cudaGetLastError();
-        mode = fused && (!p->wide_ok || (capture != cudaStreamCaptureStatusNone && !p->fused_stale)) ? 2 : 1;
+        if (fused && cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) cudaGetLastError();
+        if (!fused) mode = 1;
+        else if (capture != cudaStreamCaptureStatusNone) mode = p->fused_stale ? 0 : 2;
+        else mode = p->wide_ok ? 1 : 2;
         if (fused) p->reportReach = true;
     }
     if (mode == 2) {

@@ -140,8 +140,10 @@ def test_runs_of_any_length(warm, runs):
     assert len(compare_scenes(*out)) > 80
 
 
-def test_step_index_beside_a_captured_run(warm):
-    # a captured run (the fused kernel) moves the step index at its replay, not at its capture
+@pytest.mark.parametrize("refresh", [False, True])
+def test_step_index_beside_a_captured_run(warm, refresh):
+    # a captured run (the fused kernel) moves the step index at its replay, not at its capture;
+    # after a refresh the per-system kernels are captured, as the topology cannot be read there
     from softbox_b200.engine import DenseNetwork
     from softbox_b200.runtime import LIB
     ref = DenseNetwork(copy.deepcopy(warm))
@@ -149,6 +151,8 @@ def test_step_index_beside_a_captured_run(warm):
         ref.run(t, n, mode="unfused")
     net = DenseNetwork(copy.deepcopy(warm))
     net.run(300, 3, mode="graph")
+    if refresh:
+        assert LIB.sbx_dense_plan_refresh(net.plan) == 0
     torch.cuda.synchronize()
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(LIB.sbx_ctx_stream(net.ctx.h))):
