@@ -690,6 +690,7 @@ bool wide_prepare(sbx_dense_plan* p) {
     WideArgs& w = p->wide;
     FusedArgs& a = w.a;
     if (step_layout(p, a)) return false;
+    if (a.S > a.nSeg + a.nM) return false;       // bodies of the caller's beyond the published ones
     if (p->batched) w.bt = p->batch;
     w.errDev = p->ctx->err_dev;
     a.cellUse = WIDE_CELL_SLOTS;

@@ -15,8 +15,9 @@ struct sbx_ctx {
     void* scratch = nullptr;          // grow-only device scratch for scans / unordered scatters
     size_t scratch_bytes = 0;
     int* host_flag = nullptr;         // pinned word for device -> host status flags
-    // mapped pinned word that kernels set when an input breaks a documented range (a CSR key
-    // >= its row count); sbx_ctx_sync reports and clears it. err_dev is its device address.
+    // mapped pinned word that kernels set when an input breaks a documented range (1: a CSR key
+    // >= its row count, 2: a wait that ran out, ERR_DEV_VIEW); sbx_ctx_sync reports and clears
+    // it. err_dev is its device address.
     int* err_host = nullptr;
     int* err_dev = nullptr;
     // stream markers of sbx_ctx_mark / sbx_ctx_wait_mark (created on first use)
@@ -27,6 +28,9 @@ struct sbx_ctx {
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t copy_after = nullptr;
 };
+
+// err_dev: a captured step met a body view that is not its plan's
+constexpr int ERR_DEV_VIEW = 3;
 
 sbx_status fail(sbx_ctx* ctx, sbx_status code, const std::string& msg);
 sbx_status check_launch(sbx_ctx* ctx, const char* what);

@@ -53,6 +53,14 @@ __device__ __forceinline__ GridView grid_view(const WideArgs& w, int net) {
     return GridView{g.gridParams, g.gridDims[0], g.gridDims[1], g.gridDims[2], w.a.segCellOff};
 }
 
+// the cell of a centre in its network's grid
+template <bool B>
+__device__ __forceinline__ int body_cell(const WideArgs& w, int net, const float c[3]) {
+    const GridView v = grid_view<B>(w, net);
+    return (int)(v.off - w.a.segCellOff) + cell_coord(c[0], v.gp[0], v.gp[4], v.nX) +
+           cell_coord(c[1], v.gp[1], v.gp[4], v.nY) * v.nX + cell_coord(c[2], v.gp[2], v.gp[4], v.nZ) * (v.nX * v.nY);
+}
+
 // the kernel before this one in its stream is complete, and what it wrote can be read
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // the next kernel of the stream may start its blocks once every block is here or done
@@ -181,6 +189,7 @@ __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ Wi
         int* bc = sc.mini.bbCounts; bc[0] = a.nBb; bc[1] = t; bc[2] = sc.seedBb; bc[3] = a.nBb;
         sc.fil.counts[1] = t;
         if (a.xlOn) { sc.xl.counts[1] = t; sc.xl.counts[2] = sc.seed; }
+        if (sc.mot.publishParams[0] != nSeg && w.errDev) *(volatile int*)w.errDev = ERR_DEV_VIEW;
     }
     int cell = -1;
     float span = 0.f;
@@ -240,11 +249,12 @@ __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ Wi
             mot.capStats[m] = cs;
         }
         for (int k = 0; k < 3; k++) g.center[k * cap + i] = c[k];
-        if (i < g.gridCounts[1]) {
-            const GridView v = grid_view<B>(w, net);
-            cell = (int)(v.off - a.segCellOff) + cell_coord(c[0], v.gp[0], v.gp[4], v.nX) +
-                   cell_coord(c[1], v.gp[1], v.gp[4], v.nY) * v.nX + cell_coord(c[2], v.gp[2], v.gp[4], v.nZ) * (v.nX * v.nY);
-        }
+        if (i < g.gridCounts[1]) cell = body_cell<B>(w, net, c);
+    } else if (!B && i < cap && i < g.gridCounts[1]) {
+        // a body of the caller's beyond the published ones (counted in after the plan was made)
+        const float c[3] = {g.center[i], g.center[cap + i], g.center[2 * cap + i]};
+        cell = body_cell<B>(w, 0, c);
+        if (g.ownerStore[i] == STORE_FILAMENT && w.errDev) *(volatile int*)w.errDev = ERR_DEV_VIEW;
     }
     if (i < cap) g.bodyCell[i] = cell;
     int over = 0;

@@ -185,3 +185,49 @@ def test_auto_takes_the_graph_and_fused_runs_after_a_refresh(warm):
     assert net.fused_available and net.status() == 0
     assert len(compare_scenes(ref, D.to_host(net.dev))) > 80
     net.close()
+
+
+def _with_bodies(sc, extra, counted):
+    # `extra` bodies of the caller's after the heads in the body view, owned by no store
+    sc = copy.deepcopy(sc)
+    g = sc["grid"]
+    cap, rng = g["cap"], np.random.default_rng(extra)
+    head = np.asarray(sc["mot"]["body"]["coord"]).reshape(3, -1)[:, :extra]
+    center = np.zeros((3, cap + extra), np.float32)
+    center[:, cap:] = head + rng.normal(scale=0.02, size=head.shape).astype(np.float32)
+    g["center"] = center.reshape(-1)
+    for k, v in (("boundingRadius", 0.05), ("ownerStore", -1), ("ownerSlot", -1), ("bodyCell", -1),
+                 ("gridCellContents", -1)):
+        g[k] = np.concatenate([g[k], np.full(extra, v, g[k].dtype)])
+    g["cap"] = cap + extra
+    g["gridCounts"][1] = cap + (extra if counted else 0)
+    return sc
+
+
+@pytest.mark.parametrize("counted", [True, False], ids=["before", "after"])
+def test_bodies_past_the_published_ones(warm, counted):
+    # counted into the view before the plan is made, or on the device afterwards
+    from softbox_b200.engine import DenseNetwork
+    sc, out = _with_bodies(warm, 40, counted), []
+    for mode in ("unfused", "graph"):
+        net = DenseNetwork(copy.deepcopy(sc))
+        if not counted:
+            net.dev["grid"]["gridCounts"][1] = sc["grid"]["cap"]
+        net.run(300, 9, mode=mode)
+        assert net.status() == 0
+        net.ctx.sync()
+        out.append(D.to_host(net.dev))
+        net.close()
+    assert (np.asarray(out[0]["grid"]["bodyCell"])[-40:] >= 0).all()
+    assert len(compare_scenes(*out)) > 80
+
+
+def test_a_moved_body_view_is_reported(warm):
+    from softbox_b200.engine import DenseNetwork
+    from softbox_b200.runtime import SbxError
+    net = DenseNetwork(copy.deepcopy(warm))
+    net.dev["mot"]["publishParams"][0] = 0
+    net.run(300, 1, mode="graph")
+    with pytest.raises(SbxError, match="publishParams"):
+        net.ctx.sync()
+    net.close()
