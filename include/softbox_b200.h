@@ -773,7 +773,10 @@ int32_t sbx_dense_plan_fused_available(sbx_dense_plan* plan);
  * deaths, births into FREE slots). The fused path depends on it (rod groups, whether
  * neighbours cross groups, joint sharing): it is read again, which synchronises the plan's
  * stream, when the fused kernel next runs, or here when the plan has no wide kernels. The
- * graph and per-system paths need no refresh. */
+ * graph and per-system paths need no refresh: they take the chains, the dimer and
+ * minifilament tables and the count of the body view as the device has them at each step.
+ * (publishParams stays what it was when the plan was made, and bodies past the heads are no
+ * filament's: a graph step that finds otherwise makes sbx_ctx_sync return SBX_EINVAL.) */
 sbx_status sbx_dense_plan_refresh(sbx_dense_plan* plan);
 /* cooperative grid size (CTAs) of the fused path */
 int32_t sbx_dense_plan_fused_grid(sbx_dense_plan* plan);

@@ -539,7 +539,8 @@ bool fused_topology(sbx_dense_plan* p) {
 
 // Sizes and the harness layout that the fused kernel and the wide kernels rely on: motors 2d and
 // 2d + 1 of dimer d, the same number of dimers on every backbone in backbone order, the body
-// view = segments then heads. Returns why a scene has another layout, or null.
+// view = segments then heads. Returns why a scene has another layout, or null. (The wide kernels
+// keep to the dimer tables when these change later: myosin_term, odd_sums.)
 const char* step_layout(sbx_dense_plan* p, FusedArgs& a) {
     const sbx_dense_scene& sc = p->scene;
     cudaStream_t st = p->ctx->stream;
@@ -681,6 +682,7 @@ bool fused_prepare(sbx_dense_plan* p) {
 void wide_reset(sbx_dense_plan* p) {
     const WideArgs& w = p->wide;
     step_reset(p->ctx, p->wide.a);
+    cudaMemsetAsync(w.a.odd, 0, 4, p->ctx->stream);
     cudaMemsetAsync(w.sumCell, 0, 4 * (size_t)WIDE_SUM_STRIDE * (2 * (size_t)w.tilesC + 3 * (size_t)w.tilesS),
                     p->ctx->stream);
 }
@@ -704,6 +706,7 @@ bool wide_prepare(sbx_dense_plan* p) {
             step_carve(m, a, WIDE_CELL_SLOTS, WIDE_ROW_SLOTS, nullptr);
             m.take(w.payA, 24 * nLk);
             m.take(w.payB, 24 * nLk);
+            m.take(a.odd, 4);
             m.take(sums, 4 * words);
         }) || !wide_streams_create(p->wideStreams))
         return false;

@@ -241,7 +241,7 @@ __device__ void myosin_terms(const FusedArgs& a, int firstWarp) {
     if (firstWarp >= nw) firstWarp = 0;
     if (w < firstWarp) return;
     const int total = 2 * a.nM + 4 * a.nD;
-    for (int k = (w - firstWarp) * 32 + (threadIdx.x & 31); k < total; k += (nw - firstWarp) * 32) myosin_term(a, k);
+    for (int k = (w - firstWarp) * 32 + (threadIdx.x & 31); k < total; k += (nw - firstWarp) * 32) myosin_term<false>(a, k);
 }
 
 // ---------------------------------------------------------------- E: stable placement
@@ -386,8 +386,8 @@ __device__ void phase_motors_links(const FusedArgs& a, FusedSmem& sm, int t) {
     for (int w = blockIdx.x; w < units; w += gridDim.x) {
         if (w < a.nBb) {
             // the sub-bodies on three warps, the backbone on the fourth
-            if (threadIdx.x < 96) mini_bodies(a, sm.mini, w);
-            else if (threadIdx.x == 96) mini_backbone(a, w, t, a.sc.boxParams, a.sc.mini.bbBodyParams[0]);
+            if (threadIdx.x < 96) mini_bodies<false>(a, sm.mini, w);
+            else if (threadIdx.x == 96) mini_backbone<false>(a, w, t, a.sc.boxParams, a.sc.mini.bbBodyParams[0]);
             __syncthreads();
         } else {
             int k = (w - a.nBb) * blockDim.x + threadIdx.x;

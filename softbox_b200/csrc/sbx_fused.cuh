@@ -46,6 +46,9 @@ struct FusedArgs {
     // rest in a singly linked overflow list (head per row, next per item; -1 ends)
     int *cellSlot, *slotA, *slotB, *slotM;
     int *cellHead, *cellNext, *headA, *nextA, *headB, *nextB, *headM, *nextM;
+    // set while the dimer tables on the device are not the harness layout's (the wide kernels
+    // read them at every step; null for the fused kernel)
+    int* odd;
     int* reachMax;           // float bits: the largest reach of a segment from its centre, this step
     float4 *segE1, *segE2;   // segment endpoints in cell order: {end1, slot}, {end2, 0}
     unsigned long long* bar; // arrival counters (monotonic): [0] grid barrier, [1] rod-phase helpers

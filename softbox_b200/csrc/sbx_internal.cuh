@@ -29,7 +29,7 @@ struct sbx_ctx {
     cudaEvent_t copy_after = nullptr;
 };
 
-// err_dev: a captured step met a body view that is not its plan's
+// err_dev: a captured step met a body view or dimer tables that its plan cannot follow
 constexpr int ERR_DEV_VIEW = 3;
 
 sbx_status fail(sbx_ctx* ctx, sbx_status code, const std::string& msg);

@@ -14,9 +14,11 @@ __device__ __forceinline__ int vload(const int* p) { return *(const volatile int
 // error word: a reach list past MAX_CAND, a linked-list walk past its bound
 constexpr int ERR_REACH_OVERFLOW = 2, ERR_LIST = 8;
 
-// force and torque sums of one minifilament's sub-bodies
+// force and torque sums of one minifilament's sub-bodies; with odd dimer tables each of its
+// motors' place in a dimer (2 d, 2 d + 1 as motor B, or -1) and the dimer that tethers its rod
 struct MiniSmem {
     float sF[3 * FUSED_MAX_SUB], sT[3 * FUSED_MAX_SUB];
+    int dimer[32], tether[32];
 };
 
 // BrownianForceSystem.brownianForce (BrownianForceSystem.java:44-106), component j (0..2) of
@@ -261,22 +263,24 @@ struct GlobalTerms {
     }
     // (the rows' floats take three planes of doubles, as six planes of floats)
     __device__ __forceinline__ float* row(int d) const { return reinterpret_cast<float*>(dimer(31, 0)) + d; }
-    __device__ __forceinline__ TetherTerm tether(int d) const {
+    __device__ __forceinline__ TetherTerm tether(int d, int& odd) const {
         const double* p = dimer(24, d);
         const size_t n = a.nD;
         TetherTerm T;
         T.Fx = p[0]; T.Fy = p[n]; T.Fz = p[2 * n]; T.Tx = p[3 * n]; T.Ty = p[4 * n]; T.Tz = p[5 * n];
         const int ok = *reinterpret_cast<const int*>(p + 6 * n);
         T.fOK = ok & 1;
-        T.tOK = ok >> 1;
+        T.tOK = (ok >> 1) & 1;
+        odd = ok >> 2;
         return T;
     }
-    __device__ __forceinline__ void put(int d, const TetherTerm& T) const {
+    // (odd: the device's tables have another dimer there than the harness layout)
+    __device__ __forceinline__ void put(int d, const TetherTerm& T, bool odd) const {
         double* p = dimer(24, d);
         const size_t n = a.nD;
         if (T.fOK) { p[0] = T.Fx; p[n] = T.Fy; p[2 * n] = T.Fz; }
         if (T.tOK) { p[3 * n] = T.Tx; p[4 * n] = T.Ty; p[5 * n] = T.Tz; }
-        *reinterpret_cast<int*>(p + 6 * n) = (T.fOK ? 1 : 0) | (T.tOK ? 2 : 0);
+        *reinterpret_cast<int*>(p + 6 * n) = (T.fOK ? 1 : 0) | (T.tOK ? 2 : 0) | (odd ? 4 : 0);
         float* q = row(d);
         for (int j = 0; j < 6; j++) q[j * n] = T.row[j];
     }
@@ -455,21 +459,39 @@ __device__ __forceinline__ void bond_store(const FusedArgs& a, int m, float out[
 // MiniFilamentSystem.backboneGather over backbone u's CSR row (its dimers, ascending;
 // MiniFilamentSystem.java:140-147), then walls, integration and derived geometry; the
 // reference's CSR arrays (rows = backbones, items = dimers in index order)
+template <bool LIVE>
 __device__ __forceinline__ void mini_backbone(const FusedArgs& a, int u, int t, const float* boxParams, float dt) {
     const GlobalTerms terms{a};
     const sbx_minifilament_store& mini = a.sc.mini;
     const sbx_rigid_body& bb = mini.backbone;
-    const int dpm = a.dpm, nBb = a.nBb, d0 = u * dpm;
+    const int nBb = a.nBb, nD = a.nD;
+    int dpm = a.dpm, d0 = u * dpm;
+    double f[3] = {0, 0, 0}, tq[3] = {0, 0, 0};
+    auto add = [&](int d) {
+        const float* p = terms.row(d);                // the dimer's miniData row
+        const size_t n = nD;
+        f[0] += p[0]; f[1] += p[n]; f[2] += p[2 * n];
+        tq[0] += p[3 * n]; tq[1] += p[4 * n]; tq[2] += p[5 * n];
+    };
+    if (LIVE && vload(a.odd)) {
+        // (any table: the row's place from all dimers, its members where they are)
+        dpm = d0 = 0;
+        for (int d = 0; d < nD; d++) {
+            const int h = mini.headBackboneSlot[d];
+            dpm += h == u;
+            d0 += h >= 0 && h < u;
+        }
+        for (int d = 0, q = d0; d < nD; d++)
+            if (mini.headBackboneSlot[d] == u) {
+                mini.bbDimerList[q++] = d;
+                add(d);
+            }
+    } else {
+        for (int d = d0; d < d0 + dpm; d++) add(d);
+    }
     mini.bbDimerCount[u] = dpm;
     mini.bbDimerOffsets[u] = d0;
     if (u == nBb - 1) mini.bbDimerOffsets[nBb] = d0 + dpm;
-    double f[3] = {0, 0, 0}, tq[3] = {0, 0, 0};
-    for (int d = d0; d < d0 + dpm; d++) {
-        const float* p = terms.row(d);                // the dimer's miniData row
-        const size_t n = a.nD;
-        f[0] += p[0]; f[1] += p[n]; f[2] += p[2 * n];
-        tq[0] += p[3 * n]; tq[1] += p[4 * n]; tq[2] += p[5 * n];
-    }
     float F[3], T[3];
     for (int k = 0; k < 3; k++) { F[k] = (float)(0.0f + f[k]); T[k] = (float)(0.0f + tq[k]); }
     BoxParams bx = box_params(boxParams, t);
@@ -479,10 +501,71 @@ __device__ __forceinline__ void mini_backbone(const FusedArgs& a, int u, int t, 
     integrate_derive_store(bb, u, F, T, dt);
 }
 
+// the sums of motor ml's rod (role 0) or lever (1) of minifilament u begin with its joints; returns
+// the sub-body
+__device__ __forceinline__ int joint_sums(const FusedArgs& a, MiniSmem& ms, int u, int role, int ml) {
+    const GlobalTerms terms{a};
+    const sbx_motor_store& mot = a.sc.mot;
+    const sbx_rigid_body& mb = mot.body;
+    const int nB = a.nB, spm = 6 * a.dpm;
+    const int m = 2 * u * a.dpm + ml, sl = 3 * ml + role, s = u * spm + sl;
+    int nuc = mot.nucleotideState[m];
+    double f[3] = {0.0, 0.0, 0.0}, tq[3] = {0.0, 0.0, 0.0};
+    if (role == 0) {
+        motor_joint_apply(terms.joint(m, 0), 0, false, nuc, s, nB, mb.uVec, mb.segLength, mot.jointParams, f, tq);
+    } else {
+        motor_joint_apply(terms.joint(m, 0), 0, true, nuc, s, nB, mb.uVec, mb.segLength, mot.jointParams, f, tq);
+        motor_joint_apply(terms.joint(m, 1), 1, false, nuc, s, nB, mb.uVec, mb.segLength, mot.jointParams, f, tq);
+    }
+    for (int k = 0; k < 3; k++) {
+        ms.sF[k * spm + sl] = (float)(0.0 + f[k]);
+        ms.sT[k * spm + sl] = (float)(0.0 + tq[k]);
+    }
+    return s;
+}
+
+// The rods' and levers' sums of minifilament u again, with the dimers as odd tables have them (96
+// threads): each motor's dimer by a scan of all, its terms computed here. Such a scene keeps
+// its bits, not its speed; the others pay for a vote. (A motor belongs to one dimer, so where
+// a minifilament's own dimers are the layout's, so are its motors'.)
+__device__ __noinline__ void odd_sums(const FusedArgs& a, MiniSmem& ms, int u) {
+    const sbx_dense_scene& sc = a.sc;
+    const sbx_rigid_body& mb = sc.mot.body;
+    const int mpm = 2 * a.dpm, spm = 6 * a.dpm, m0 = u * mpm, tid = threadIdx.x, ml = tid & 31;
+    if (tid < 32) ms.dimer[tid] = ms.tether[tid] = -1;
+    asm volatile("bar.sync 1, 96;" ::: "memory");
+    for (int d = tid; d < a.nD; d += 96) {
+        const int mA = sc.dim.motorA[d] - m0, mB = sc.dim.motorB[d] - m0, rA = sc.mini.motorA[d] - m0;
+        if (mA >= 0 && mA < mpm) ms.dimer[mA] = 2 * d;
+        if (mB >= 0 && mB < mpm) ms.dimer[mB] = 2 * d + 1;
+        if (rA >= 0 && rA < mpm) ms.tether[rA] = d;
+    }
+    asm volatile("bar.sync 1, 96;" ::: "memory");
+    if (tid < 32 || ml >= mpm) return;
+    LocalAcc acc{ms.sF, ms.sT, u * spm, spm};
+    const int role = (tid - 32) >> 5, s = joint_sums(a, ms, u, role, ml);
+    const int at = ms.dimer[ml], d = at >> 1;
+    const bool isA = (at & 1) == 0;
+    const int mA = at < 0 ? -1 : sc.dim.motorA[d], mB = at < 0 ? -1 : sc.dim.motorB[d];
+    const bool paired = mA >= 0 && mA < a.nM && mB >= 0 && mB < a.nM;
+    const bool par = paired && sc.dim.parallel[d] != 0;
+    if (role == 0) {
+        for (int v = 0; v < 2 && paired; v++)
+            couple_apply_rod(acc, s, isA, couple_variant(a.nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam, mb.bRotGam,
+                                                         mA, mB, par, sc.dim.dimerParams, v));
+        int odd;
+        if (ms.tether[ml] >= 0) tether_apply(acc, s, GlobalTerms{a}.tether(ms.tether[ml], odd));
+    } else if (par && !(sc.mot.boundSeg[mA] >= 0 && sc.mot.boundSeg[mB] >= 0)) {
+        couple_apply_lever(acc, s, isA, couple_lever(a.nB, mb.uVec, mb.bRotGam, mA, mB, sc.dim.dimerParams));
+    }
+}
+
 // The sub-bodies of minifilament u on the first three warps of a block (its heads' binding and
 // the position-only terms ran before). Each sub-body accumulates its terms in the order of the
 // reference's System sequence (joints, coupling, tether; the head's bond after its joint): a
-// warp for the heads, the rods, the levers; then they integrate in body order.
+// warp for the heads, the rods, the levers; then they integrate in body order. LIVE: the dimers
+// as the device's tables have them now, else as the harness layout has them.
+template <bool LIVE>
 __device__ __forceinline__ void mini_bodies(const FusedArgs& a, MiniSmem& ms, int u) {
     const GlobalTerms terms{a};
     const sbx_dense_scene& sc = a.sc;
@@ -495,6 +578,7 @@ __device__ __forceinline__ void mini_bodies(const FusedArgs& a, MiniSmem& ms, in
     float* sF = ms.sF;
     float* sT = ms.sT;
     LocalAcc acc{sF, sT, s0, spm};
+    int odd = 0;
     if (tid < 32) {
         if (tid < mpm) {
             // CrossBridgeSystem.bondForces, then the head's sums: joint 1, then the bond
@@ -514,35 +598,27 @@ __device__ __forceinline__ void mini_bodies(const FusedArgs& a, MiniSmem& ms, in
     } else {
         const int role = (tid - 32) >> 5, ml = tid & 31;      // 0 rods, 1 levers
         if (ml < mpm) {
-            int m = m0 + ml, sl = 3 * ml + role, s = s0 + sl;
-            int nuc = mot.nucleotideState[m];
-            double f[3] = {0.0, 0.0, 0.0}, tq[3] = {0.0, 0.0, 0.0};
-            if (role == 0) {
-                motor_joint_apply(terms.joint(m, 0), 0, false, nuc, s, nB, mb.uVec, mb.segLength, mot.jointParams, f,
-                                  tq);
-            } else {
-                motor_joint_apply(terms.joint(m, 0), 0, true, nuc, s, nB, mb.uVec, mb.segLength, mot.jointParams, f,
-                                  tq);
-                motor_joint_apply(terms.joint(m, 1), 1, false, nuc, s, nB, mb.uVec, mb.segLength, mot.jointParams, f,
-                                  tq);
-            }
-            for (int k = 0; k < 3; k++) {
-                sF[k * spm + sl] = (float)(0.0 + f[k]);
-                sT[k * spm + sl] = (float)(0.0 + tq[k]);
-            }
+            const int s = joint_sums(a, ms, u, role, ml);
             int dl = ml >> 1, d = d0 + dl;
             bool isA = (ml & 1) == 0;            // motorA = 2d, motorB = 2d + 1
             if (role == 0) {
                 couple_apply_rod(acc, s, isA, terms.couple(d, 0));
                 couple_apply_rod(acc, s, isA, terms.couple(d, 1));
-                if (isA) tether_apply(acc, s, terms.tether(d));
+                if (isA) tether_apply(acc, s, terms.tether(d, odd));
             } else {
                 bool bothBound = mot.boundSeg[2 * d] >= 0 && mot.boundSeg[2 * d + 1] >= 0;
                 if (sc.dim.parallel[d] != 0 && !bothBound) couple_apply_lever(acc, s, isA, terms.lever(d));
             }
         }
     }
-    asm volatile("bar.sync 1, 96;" ::: "memory");             // the three warps, without a fourth
+    if (LIVE) {
+        if (__syncthreads_or(odd)) {
+            odd_sums(a, ms, u);
+            __syncthreads();
+        }
+    } else {
+        asm volatile("bar.sync 1, 96;" ::: "memory");         // the three warps, without a fourth
+    }
     // integrate + derive the sub-bodies; force-dot registry
     if (tid < spm) {
         int s = s0 + tid;
@@ -557,16 +633,33 @@ __device__ __forceinline__ void mini_bodies(const FusedArgs& a, MiniSmem& ms, in
     }
 }
 
+// dimer d's tether to backbone u by motor mA's rod, with its row
+__device__ __forceinline__ void tether_term(const FusedArgs& a, int d, int u, int mA, bool odd) {
+    const sbx_minifilament_store& mini = a.sc.mini;
+    const sbx_rigid_body &mb = a.sc.mot.body, &bb = mini.backbone;
+    TetherTerm T = tether_terms(a.nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam, mb.bRotGam, a.nBb, bb.coord,
+                                bb.uVec, mini.bbInvDragY, u, mA, mini.attachAxial[d], mini.miniParams);
+    GlobalTerms{a}.put(d, T, odd);
+    float* o = mini.miniData + (int64_t)MINI_STRIDE * d;
+    for (int j = 0; j < 6; j++) o[j] = T.row[j];
+}
+// (out of line: the layout's own term is made while the tables are read)
+__device__ __noinline__ void odd_tether_term(const FusedArgs& a, int d, int u, int mA) {
+    tether_term(a, d, u, mA, true);
+}
+
 // The position-only terms of the myosin mechanics, none of which depends on a step's binding or
 // forces (MotorJointSystem.java:72-123 joint geometry, DimerCouplingSystem.java:99-182 end
 // variants and lever torsion, MiniFilamentSystem tethers with their backbone reaction rows):
-// item k of 2 nM + 4 nD
-__device__ __forceinline__ void myosin_term(const FusedArgs& a, int k) {
+// item k of 2 nM + 4 nD, of the harness layout's dimers. LIVE: a dimer's tether item looks at the
+// dimer tables as the device has them now, sets *a.odd where they are not the layout's and
+// makes that tether from them (the rest: odd_sums); false where they name no motor or backbone.
+template <bool LIVE>
+__device__ __forceinline__ bool myosin_term(const FusedArgs& a, int k) {
     const sbx_dense_scene& sc = a.sc;
     const sbx_motor_store& mot = sc.mot;
     const sbx_rigid_body& mb = mot.body;
     const sbx_minifilament_store& mini = sc.mini;
-    const sbx_rigid_body& bb = mini.backbone;
     const int nM = a.nM, nD = a.nD, nB = a.nB;
     const GlobalTerms terms{a};
     if (k < 2 * nM) {
@@ -582,14 +675,19 @@ __device__ __forceinline__ void myosin_term(const FusedArgs& a, int k) {
         terms.put(d, couple_lever(nB, mb.uVec, mb.bRotGam, 2 * d, 2 * d + 1, sc.dim.dimerParams));
     } else {
         const int d = k - 2 * nM - 3 * nD, u = d / a.dpm;
-        TetherTerm T = tether_terms(nB, mb.coord, mb.uVec, mb.segLength, mb.bTransGam, mb.bRotGam, a.nBb, bb.coord,
-                                    bb.uVec, mini.bbInvDragY, u, 2 * d, mini.attachAxial[d], mini.miniParams);
-        terms.put(d, T);
-        float* o = mini.miniData + (int64_t)MINI_STRIDE * d;
-        for (int j = 0; j < 6; j++) o[j] = T.row[j];
+        int h = u, r = 2 * d, mA = 2 * d, mB = 2 * d + 1;
+        if (LIVE) { h = mini.headBackboneSlot[d]; r = mini.motorA[d]; mA = sc.dim.motorA[d]; mB = sc.dim.motorB[d]; }
+        tether_term(a, d, u, 2 * d, false);
         // backbone CSR of the reference (rows = backbones, items = dimers in index order)
         mini.bbDimerList[d] = d;
+        if (LIVE && (h != u || r != 2 * d || mA != 2 * d || mB != 2 * d + 1)) {
+            *(volatile int*)a.odd = 1;
+            const bool ok = h >= 0 && h < a.nBb && r >= 0 && r < nM && mA >= 0 && mA < nM && mB >= 0 && mB < nM;
+            odd_tether_term(a, d, ok ? h : u, ok ? r : 2 * d);
+            return ok;
+        }
     }
+    return true;
 }
 
 }  // namespace

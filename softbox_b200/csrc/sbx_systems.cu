@@ -95,8 +95,8 @@ extern "C" sbx_status sbx_ctx_sync(sbx_ctx* ctx) {
         *(volatile int*)ctx->err_host = 0;
         if (w == 2) return fail(ctx, SBX_ETIMEOUT, "a staged reach walk's bulk copies did not complete in time");
         if (w == ERR_DEV_VIEW)
-            return fail(ctx, SBX_EINVAL, "dense step: publishParams or a filament's body past the heads is not as the "
-                                         "plan was made for");
+            return fail(ctx, SBX_EINVAL, "dense step: publishParams, a filament's body past the heads or a dimer's "
+                                         "motor or backbone is outside what the plan was made for");
         return fail(ctx, SBX_EINVAL, "a CSR key was >= its row count (the item was skipped)");
     }
     return SBX_OK;
@@ -245,8 +245,8 @@ extern "C" sbx_status sbx_ctx_wait_mark(sbx_ctx* ctx, int32_t slot) {
         *(volatile int*)ctx->err_host = 0;
         if (w == 2) return fail(ctx, SBX_ETIMEOUT, "a staged reach walk's bulk copies did not complete in time");
         if (w == ERR_DEV_VIEW)
-            return fail(ctx, SBX_EINVAL, "dense step: publishParams or a filament's body past the heads is not as the "
-                                         "plan was made for");
+            return fail(ctx, SBX_EINVAL, "dense step: publishParams, a filament's body past the heads or a dimer's "
+                                         "motor or backbone is outside what the plan was made for");
         return fail(ctx, SBX_EINVAL, "a CSR key was >= its row count (the item was skipped)");
     }
     return SBX_OK;

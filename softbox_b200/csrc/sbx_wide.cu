@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(256) k_wide_draws(const __grid_constant__ Wide
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nB + nBb + a.nSeg) return;
     const int t = *a.d_step;
+    if (j == 0 && sc.mot.publishParams[0] != a.nSeg && w.errDev) *(volatile int*)w.errDev = ERR_DEV_VIEW;
     if (j == 0 && a.nzFil && w.noiseErr && (t < a.nzT0 || t >= a.nzT0 + a.nzN)) atomicOr(w.noiseErr, 1);
     const sbx_rigid_body* b;
     const float* noise;
@@ -175,7 +176,8 @@ __global__ void __launch_bounds__(128, 8) k_wide_joints(const __grid_constant__ 
 // largest reach of a segment from its centre, the start view's orientations
 // (the rods kernel reads a neighbour from the start view: its own block may have stepped it
 // already) and the step's counts.
-template <bool B>
+// (MORE: the view has room for bodies of the caller's)
+template <bool B, bool MORE>
 __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ WideArgs w) {
     let_next_start();
     const FusedArgs& a = w.a;
@@ -189,7 +191,6 @@ __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ Wi
         int* bc = sc.mini.bbCounts; bc[0] = a.nBb; bc[1] = t; bc[2] = sc.seedBb; bc[3] = a.nBb;
         sc.fil.counts[1] = t;
         if (a.xlOn) { sc.xl.counts[1] = t; sc.xl.counts[2] = sc.seed; }
-        if (sc.mot.publishParams[0] != nSeg && w.errDev) *(volatile int*)w.errDev = ERR_DEV_VIEW;
     }
     int cell = -1;
     float span = 0.f;
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(256) k_wide_publish(const __grid_constant__ Wi
         }
         for (int k = 0; k < 3; k++) g.center[k * cap + i] = c[k];
         if (i < g.gridCounts[1]) cell = body_cell<B>(w, net, c);
-    } else if (!B && i < cap && i < g.gridCounts[1]) {
+    } else if (MORE && !B && i < cap && i < g.gridCounts[1]) {
         // a body of the caller's beyond the published ones (counted in after the plan was made)
         const float c[3] = {g.center[i], g.center[cap + i], g.center[2 * cap + i]};
         cell = body_cell<B>(w, 0, c);
@@ -496,7 +497,7 @@ __global__ void __launch_bounds__(128, 8) k_wide_bind(const __grid_constant__ Wi
 __global__ void __launch_bounds__(128, 8) k_wide_terms(const __grid_constant__ WideArgs w) {
     let_next_start();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < 2 * w.a.nM + 4 * w.a.nD) myosin_term(w.a, k);
+    if (k < 2 * w.a.nM + 4 * w.a.nD && !myosin_term<true>(w.a, k) && w.errDev) *(volatile int*)w.errDev = ERR_DEV_VIEW;
     after_previous();                    // (done when the kernels before it are)
 }
 
@@ -514,12 +515,12 @@ __global__ void __launch_bounds__(MINI_THREADS, 10) k_wide_mini(const __grid_con
     const FusedArgs& a = w.a;
     const sbx_minifilament_store& mini = a.sc.mini;
     if ((int)blockIdx.x < a.nBb) {
-        mini_bodies(a, sm, blockIdx.x);
+        mini_bodies<true>(a, sm, blockIdx.x);
         return;
     }
     const int u = (blockIdx.x - a.nBb) * MINI_THREADS + threadIdx.x;
     if (u >= a.nBb) return;
-    mini_backbone(a, u, mini.bbCounts[1], B ? w.bt.boxParams + 8 * w.bt.bbKey[2 * u] : a.sc.boxParams,
+    mini_backbone<true>(a, u, mini.bbCounts[1], B ? w.bt.boxParams + 8 * w.bt.bbKey[2 * u] : a.sc.boxParams,
                   B ? mini.bbBodyParams[0] : a.sc.boxParams[7]);
 }
 
@@ -752,6 +753,7 @@ __global__ void __launch_bounds__(128, MANY ? 6 : 4) k_wide_rods(const __grid_co
     if (i == 0) {
         *a.d_step = t + 1;               // (every reader of this step's index has run)
         *a.reachMax = 0;
+        *a.odd = 0;
     }
     if (a.xlOn) {
         xl.activeLinkCount[i] = act;
@@ -871,7 +873,8 @@ sbx_status wide_step_impl(sbx_ctx* ctx, const WideArgs& w, const WideStreams& ws
         launch(ws.link, true, k_wide_link_scan, (int64_t)2 * w.tilesS * 256, 256);
         launch(ws.link, true, k_wide_links, a.nL, 128);
     }
-    launch(s, false, k_wide_publish<B>, a.cap, 256);
+    if (a.cap > a.nSeg + a.nM) launch(s, false, k_wide_publish<B, true>, a.cap, 256);
+    else launch(s, false, k_wide_publish<B, false>, a.cap, 256);
     launch(s, true, k_wide_cell_scan, (int64_t)2 * w.tilesC * 256, 256);
     launch(s, true, k_wide_place, a.cap, 256);
     launch(s, true, k_wide_bind<B>, ((int64_t)a.nM + BIND_HEADS - 1) / BIND_HEADS * 32, 128);

@@ -231,3 +231,36 @@ def test_a_moved_body_view_is_reported(warm):
     with pytest.raises(SbxError, match="publishParams"):
         net.ctx.sync()
     net.close()
+
+
+@pytest.mark.parametrize("change", ["sides", "partners", "backbones", "tethers"])
+def test_dimer_tables_changed_on_the_device(warm, change):
+    # the graph path takes the dimer tables as they are at each step: changed after the plan was
+    # made, and changed back
+    from softbox_b200.engine import DenseNetwork
+    out = []
+    for mode in ("unfused", "graph"):
+        net = DenseNetwork(copy.deepcopy(warm))
+        dim, mini = net.dev["dim"], net.dev["mini"]
+        keep = [x.clone() for x in (dim["motorA"], dim["motorB"], mini["headBackboneSlot"], mini["motorA"])]
+        n, far = dim["motorA"].numel(), dim["motorA"].numel() - 1
+        net.run(300, 5, mode=mode)
+        if change == "sides":
+            dim["motorA"][3], dim["motorB"][3] = keep[1][3], keep[0][3]
+        elif change == "partners":
+            dim["motorB"][1], dim["motorB"][far] = keep[1][far], keep[1][1]
+        elif change == "backbones":
+            rows = torch.randint(0, n, (n,), generator=torch.Generator().manual_seed(4)).cuda()
+            mini["headBackboneSlot"].copy_(keep[2][rows])           # of unequal lengths, some empty
+        else:
+            mini["motorA"][0], mini["motorA"][far] = keep[3][far], keep[3][0]
+        net.run(305, 6, mode=mode)
+        mid = D.to_host(net.dev)
+        for x, k in zip((dim["motorA"], dim["motorB"], mini["headBackboneSlot"], mini["motorA"]), keep):
+            x.copy_(k)
+        net.run(311, 5, mode=mode)
+        assert net.status() == 0
+        out.append((mid, D.to_host(net.dev)))
+        net.close()
+    for ref, got in zip(*out):
+        assert len(compare_scenes(ref, got)) > 80
