@@ -754,7 +754,7 @@ sbx_status sbx_dense_plan_create(sbx_ctx* ctx, const sbx_dense_scene* scene, sbx
  * wide kernels, which leads at every size (us per step, graph / fused: 30 / 57 at 1,000 rods one
  * step a call; 35 / 64 at 2e4 and 54 / 172 at 4e4, 20 steps a call); without it, or on a stream
  * under capture, the fused kernel up to SBX_DENSE_AUTO_MAX_FUSED_RODS rods when available (mode 0
- * under capture after a refresh), the graph path above it. */
+ * after a refresh in the same capture), the graph path above it. */
 #define SBX_DENSE_AUTO_MAX_FUSED_RODS 40960
 sbx_status sbx_dense_plan_run(sbx_dense_plan* plan, int32_t t0, int32_t nsteps, int32_t mode);
 /* Runs one step as the unfused per-system call sequence (reference granularity). */
@@ -771,8 +771,10 @@ sbx_status sbx_dense_plan_status(sbx_dense_plan* plan, int32_t* flags);
 int32_t sbx_dense_plan_fused_available(sbx_dense_plan* plan);
 /* Tells the plan that the scene's filament topology changed (a turnover cadence: growth splits,
  * deaths, births into FREE slots). The fused path depends on it (rod groups, whether
- * neighbours cross groups, joint sharing): it is read again, which synchronises the plan's
- * stream, when the fused kernel next runs, or here when the plan has no wide kernels. The
+ * neighbours cross groups, joint sharing): it is read again, which waits for the work queued
+ * before this call, when the fused kernel next runs (on a stream under capture too), or here
+ * when the plan has no wide kernels. After a refresh that is itself under capture the fused
+ * kernel returns SBX_ESTATE in that capture. The
  * graph and per-system paths need no refresh: they take the chains, the dimer and
  * minifilament tables and the count of the body view as the device has them at each step.
  * (publishParams stays what it was when the plan was made, and bodies past the heads are no

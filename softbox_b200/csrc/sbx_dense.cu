@@ -399,6 +399,8 @@ struct sbx_dense_plan {
     bool fused_ok = false;
     bool fused_prepared = false;  // its scratch exists (the topology may still be refused)
     bool fused_stale = false;    // the chain topology has changed since its groups were made
+    cudaEvent_t changed = nullptr;   // on the stream, after that change (recorded: changedAt)
+    bool changedAt = false;
     bool fused_dirty = true;     // scratch must be (re)initialised before the next fused run
     std::string fused_why;
     FusedArgs fa{};
@@ -471,21 +473,37 @@ std::vector<T> d2h(const T* d, size_t n, cudaStream_t s) {
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
+// the chain topology, read through a stream, which is synchronised; false if that fails
+struct Chains {
+    std::vector<int> e1, e2, d1, d2;
+    bool read(const sbx_filament_store& fil, cudaStream_t s) {
+        const size_t n = fil.body.n;
+        cudaError_t e = cudaSuccess;
+        auto take = [&](std::vector<int>& h, const int* d) {
+            h.resize(n);
+            if (n && e == cudaSuccess) e = cudaMemcpyAsync(h.data(), d, n * sizeof(int), cudaMemcpyDeviceToHost, s);
+        };
+        take(e1, fil.end1NbrSlot); take(e2, fil.end2NbrSlot);
+        take(d1, fil.end1NbrSide); take(d2, fil.end2NbrSide);
+        const cudaError_t w = cudaStreamSynchronize(s);
+        if (e == cudaSuccess && w == cudaSuccess) return true;
+        cudaGetLastError();
+        return false;
+    }
+};
+
 // Checks that the scene has the harness's structure the fused kernel relies on and fills
 // the kernel arguments; on failure records why (the graph path remains available).
-// The fused kernel's view of the chain topology, read from the device (the plan's stream
-// is synchronised): rod groups (FUSED_MAX_ROD slots at most, a multiple of 4), whether every
+// The fused kernel's view of the chain topology: rod groups (FUSED_MAX_ROD slots at most, a multiple of 4), whether every
 // chain neighbour lies in its own group (else the rod phase reads cross-group neighbours from
 // the step's start view), whether each joint can be computed once. FREE filament slots of
-// turnover are allowed: the body view leaves them out of the grid's segments. Called at plan
-// creation and by sbx_dense_plan_refresh after a topology change.
-bool fused_topology(sbx_dense_plan* p) {
+// turnover are allowed: the body view leaves them out of the grid's segments. Made at plan
+// creation and again after a topology change.
+bool fused_topology(sbx_dense_plan* p, const Chains& chains) {
     const sbx_dense_scene& sc = p->scene;
-    cudaStream_t st = p->ctx->stream;
     FusedArgs& a = p->fa;
     auto why = [&](const char* w) { p->fused_why = w; return false; };
-    auto e1 = d2h(sc.fil.end1NbrSlot, a.nSeg, st), e2 = d2h(sc.fil.end2NbrSlot, a.nSeg, st);
-    auto d1 = d2h(sc.fil.end1NbrSide, a.nSeg, st), d2 = d2h(sc.fil.end2NbrSide, a.nSeg, st);
+    const std::vector<int>&e1 = chains.e1, &e2 = chains.e2, &d1 = chains.d1, &d2 = chains.d2;
     std::vector<int> lo(a.nSeg), hi(a.nSeg);
     for (int i = 0; i < a.nSeg; i++) {
         lo[i] = i; hi[i] = i;
@@ -661,7 +679,9 @@ bool fused_prepare(sbx_dense_plan* p) {
     int per = fused_max_blocks_per_sm();
     if (!coop || per <= 0) return why("cooperative launch unavailable");
     p->fused_grid = sms * per;
-    if (!fused_topology(p)) return false;
+    Chains chains;
+    if (!chains.read(sc.fil, st)) return why("the chain topology could not be read");
+    if (!fused_topology(p, chains)) return false;
     auto fc = d2h(sc.fil.counts, 4, st);
     a.filSeed = fc[2];
     Arena m;
@@ -845,10 +865,12 @@ static sbx_status plan_create(sbx_ctx* ctx, const sbx_dense_scene* sc, const sbx
         return fail(ctx, SBX_ENOMEM, "sbx_dense_plan_create: counters");
     }
     p->wide_ok = wide_prepare(p);
+    if (cudaEventCreateWithFlags(&p->changed, cudaEventDisableTiming) != cudaSuccess) cudaGetLastError();
     // capture one step into a graph
     sbx_status st = capture_step(p);
     if (st != SBX_OK) {
         wide_streams_destroy(p->wideStreams);
+        if (p->changed) cudaEventDestroy(p->changed);
         for (void* q : p->allocs) cudaFree(q);
         cudaFree(p->stats);
         cudaFree(p->d_step);
@@ -880,6 +902,45 @@ extern "C" sbx_status sbx_dense_plan_create_batched(sbx_ctx* ctx, const sbx_dens
     return plan_create(ctx, sc, batch, out);
 }
 
+static bool capturing(sbx_ctx* ctx) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &c) != cudaSuccess) cudaGetLastError();
+    return c != cudaStreamCaptureStatusNone;
+}
+
+// Makes the fused kernel's groups anew if the topology has changed. The read goes through a
+// stream of the plan's own, behind the change, so that it may come while the context's stream
+// is under capture (the thread's capture mode is relaxed for it); a change that is itself part
+// of the capture has not happened yet and cannot be read.
+static sbx_status fused_current(sbx_dense_plan* p) {
+    if (!p->fused_stale) return SBX_OK;
+    sbx_ctx* ctx = p->ctx;
+    if (!p->changedAt) {
+        if (capturing(ctx))
+            return fail(ctx, SBX_ESTATE, "dense plan: the chain topology changed in this capture: the fused kernel "
+                                         "cannot be prepared for it");
+        if (cudaEventRecord(p->changed, ctx->stream) != cudaSuccess) {
+            cudaGetLastError();
+            return fail(ctx, SBX_ECUDA, "dense plan: topology event");
+        }
+        p->changedAt = true;
+    }
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaStream_t s = p->wideStreams.ahead;       // (idle but for the plan's own captures)
+    Chains chains;
+    bool ok = cudaStreamWaitEvent(s, p->changed, 0) == cudaSuccess;
+    ok = chains.read(p->scene.fil, s) && ok;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!ok) {
+        cudaGetLastError();
+        return fail(ctx, SBX_ECUDA, "dense plan: the chain topology could not be read");
+    }
+    p->fused_stale = false;
+    p->fused_ok = fused_topology(p, chains);
+    return SBX_OK;
+}
+
 extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t nsteps, int32_t mode) {
     if (!p || nsteps < 0 || mode < 0 || mode > 3) return SBX_EINVAL;
     sbx_ctx* ctx = p->ctx;
@@ -891,19 +952,14 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
         // 35 / 64 at 20,000 and 54 / 172 at 40,000 (20 steps a call) against the fused kernel
         const bool fused = p->fused_ok && p->scene.fil.body.n <= SBX_DENSE_AUTO_MAX_FUSED_RODS;
         // (a graph cannot be launched on a stream under capture: that takes the fused kernel as one
-        // node, or the per-system kernels while the fused topology, which the host reads, is stale)
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (fused && cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) cudaGetLastError();
+        // node, or the per-system kernels where its topology is not to be had)
         if (!fused) mode = 1;
-        else if (capture != cudaStreamCaptureStatusNone) mode = p->fused_stale ? 0 : 2;
+        else if (capturing(ctx)) mode = fused_current(p) == SBX_OK && p->fused_ok ? 2 : 0;
         else mode = p->wide_ok ? 1 : 2;
         if (fused) p->reportReach = true;
     }
     if (mode == 2) {
-        if (p->fused_stale) {
-            p->fused_stale = false;
-            p->fused_ok = fused_topology(p);
-        }
+        CHK(fused_current(p));
         if (!p->fused_ok) return fail(ctx, SBX_ESTATE, "fused path unavailable: " + p->fused_why);
         // the kernel leaves its histograms zeroed and its barrier words consistent at the
         // end of every completed run; they are reset here only after a failed run
@@ -920,9 +976,7 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
         SBX_TRACE("sbx.dense.graph_replay");
         // A run that goes on where the last one ended finds its step index in place; not where a
         // graph that captured a run may be replayed in between.
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) cudaGetLastError();
-        if (capture != cudaStreamCaptureStatusNone) p->stepShared = true;
+        if (capturing(ctx)) p->stepShared = true;
         if (p->stepShared || p->stepNow != t0) SBX_LAUNCH(ctx, k_step_set, 1, 1, p->d_step, t0);
         p->stepNow = INT64_MIN;
         for (int k = 0; k < nsteps;) {
@@ -992,12 +1046,9 @@ extern "C" sbx_status sbx_dense_plan_status(sbx_dense_plan* p, int32_t* flags) {
 }
 
 extern "C" int32_t sbx_dense_plan_fused_available(sbx_dense_plan* p) {
-    if (!p) return 0;
-    if (p->fused_stale) {
-        p->fused_stale = false;
-        p->fused_ok = fused_topology(p);
-    }
-    return p->fused_ok ? 1 : 0;
+    // (a topology that cannot be read now: the answer of the last one)
+    if (p && p->fused_stale && (p->changedAt || !capturing(p->ctx))) fused_current(p);
+    return p && p->fused_ok ? 1 : 0;
 }
 
 extern "C" sbx_status sbx_dense_plan_refresh(sbx_dense_plan* p) {
@@ -1005,9 +1056,15 @@ extern "C" sbx_status sbx_dense_plan_refresh(sbx_dense_plan* p) {
     if (p->batched || !p->fused_prepared) return SBX_OK;
     // the wide kernels take the chains as they are on the device; the fused kernel's groups are
     // made again when it next runs
-    if (p->wide_ok) p->fused_stale = true;
-    else p->fused_ok = fused_topology(p);
-    return SBX_OK;
+    p->fused_stale = true;
+    p->changedAt = false;
+    if (capturing(p->ctx)) return SBX_OK;
+    if (cudaEventRecord(p->changed, p->ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(p->ctx, SBX_ECUDA, "sbx_dense_plan_refresh: event");
+    }
+    p->changedAt = true;
+    return p->wide_ok ? SBX_OK : fused_current(p);
 }
 
 extern "C" int32_t sbx_dense_plan_fused_grid(sbx_dense_plan* p) { return p ? p->fused_grid : 0; }
@@ -1105,6 +1162,7 @@ extern "C" sbx_status sbx_dense_plan_destroy(sbx_dense_plan* p) {
     if (p->stats) cudaFree(p->stats);
     release_side(p);
     wide_streams_destroy(p->wideStreams);
+    if (p->changed) cudaEventDestroy(p->changed);
     for (void* q : p->allocs) cudaFree(q);
     delete p;
     return SBX_OK;

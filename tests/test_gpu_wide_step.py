@@ -264,3 +264,52 @@ def test_dimer_tables_changed_on_the_device(warm, change):
         net.close()
     for ref, got in zip(*out):
         assert len(compare_scenes(ref, got)) > 80
+
+
+@pytest.mark.parametrize("mode", ["fused", "auto"])
+def test_captured_fused_run_after_a_refresh(warm, mode):
+    # the topology of a refresh is read behind the change while the context's stream is captured
+    from softbox_b200.engine import DenseNetwork
+    from softbox_b200.runtime import LIB
+    sc = copy.deepcopy(warm)
+    ref, _, _ = _run(sc, "unfused", steps=6)
+    net = DenseNetwork(sc)
+    net.run(300, 2)
+    assert LIB.sbx_dense_plan_refresh(net.plan) == 0
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    n0 = net.ctx.launches()
+    with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(LIB.sbx_ctx_stream(net.ctx.h))):
+        assert net.fused_available
+        net.run(302, 2, mode=mode)
+    assert net.ctx.launches() - n0 == 1                # one launch for both steps
+    g.replay()
+    torch.cuda.synchronize()
+    net.run(304, 2)
+    assert net.status() == 0
+    assert len(compare_scenes(ref, D.to_host(net.dev))) > 80
+    del g
+    net.close()
+
+
+def test_a_refresh_inside_a_capture_keeps_the_capture(warm):
+    from softbox_b200.engine import DenseNetwork
+    from softbox_b200.runtime import LIB, SbxError
+    ref, _, _ = _run(warm, "unfused", steps=5)
+    net = DenseNetwork(copy.deepcopy(warm))
+    net.run(300, 2)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(LIB.sbx_ctx_stream(net.ctx.h))):
+        assert LIB.sbx_dense_plan_refresh(net.plan) == 0
+        assert net.fused_available
+        with pytest.raises(SbxError, match="capture"):
+            net.run(302, 2, mode="fused")
+        net.run(302, 2)
+    g.replay()
+    torch.cuda.synchronize()
+    net.run(304, 1, mode="fused")
+    assert net.status() == 0
+    assert len(compare_scenes(ref, D.to_host(net.dev))) > 80
+    del g
+    net.close()
