@@ -401,7 +401,7 @@ struct sbx_dense_plan {
     bool fused_stale = false;    // the chain topology has changed since its groups were made
     cudaEvent_t changed = nullptr;   // on the stream, after that change (recorded: changedAt)
     bool changedAt = false;
-    bool fused_dirty = true;     // scratch must be (re)initialised before the next fused run
+    bool fused_dirty = false;    // scratch must be initialised again before the next fused run
     std::string fused_why;
     FusedArgs fa{};
     int fused_grid = 0;
@@ -666,6 +666,11 @@ void step_reset(sbx_ctx* ctx, FusedArgs& a) {
 }
 
 static_assert(FUSED_CELL_SLOTS <= WIDE_CELL_SLOTS && FUSED_ROW_SLOTS <= WIDE_ROW_SLOTS, "the shared sets' strides");
+void fused_reset(sbx_dense_plan* p) {
+    step_reset(p->ctx, p->fa);
+    cudaMemsetAsync(p->fa.bar, 0, 32, p->ctx->stream);
+}
+
 bool fused_prepare(sbx_dense_plan* p) {
     const sbx_dense_scene& sc = p->scene;
     cudaStream_t st = p->ctx->stream;
@@ -692,9 +697,7 @@ bool fused_prepare(sbx_dense_plan* p) {
             m.take(a.bar, 32);
         }))
         return why("scratch allocation failed");
-    // the error word and barrier counters are read by the plan status before any fused run
-    cudaMemsetAsync(a.err, 0, 16, st);
-    cudaMemsetAsync(a.bar, 0, 32, st);
+    fused_reset(p);      // (here, as the first fused run may be a captured one)
     p->fused_prepared = true;
     return true;
 }
@@ -964,9 +967,8 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
         // the kernel leaves its histograms zeroed and its barrier words consistent at the
         // end of every completed run; they are reset here only after a failed run
         if (p->fused_dirty) {
-            step_reset(ctx, p->fa);
-            cudaMemsetAsync(p->fa.bar, 0, 32, ctx->stream);
-            p->fused_dirty = false;
+            fused_reset(p);
+            p->fused_dirty = capturing(ctx);     // (a captured reset comes with the replay)
         }
         p->stepShared = true;
         SBX_TRACE("sbx.dense.fused_launch");

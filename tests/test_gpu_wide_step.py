@@ -313,3 +313,22 @@ def test_a_refresh_inside_a_capture_keeps_the_capture(warm):
     assert len(compare_scenes(ref, D.to_host(net.dev))) > 80
     del g
     net.close()
+
+
+def test_fused_run_between_a_first_capture_and_its_replay(warm):
+    # the plan's first fused run is a captured one: another may come before the replay
+    from softbox_b200.engine import DenseNetwork
+    from softbox_b200.runtime import LIB
+    ref, _, _ = _run(warm, "unfused", steps=5)
+    net = DenseNetwork(copy.deepcopy(warm))
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(LIB.sbx_ctx_stream(net.ctx.h))):
+        net.run(302, 2)
+    net.run(300, 2, mode="fused")
+    g.replay()
+    torch.cuda.synchronize()
+    net.run(304, 1, mode="fused")
+    assert net.status() == 0
+    assert len(compare_scenes(ref, D.to_host(net.dev))) > 80
+    del g
+    net.close()
