@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(256) k_wide_draws(const __grid_constant__ Wide
     if (j >= nB + nBb + a.nSeg) return;
     const int t = *a.d_step;
     if (j == 0 && sc.mot.publishParams[0] != a.nSeg && w.errDev) *(volatile int*)w.errDev = ERR_DEV_VIEW;
-    if (j == 0 && a.nzFil && w.noiseErr && (t < a.nzT0 || t >= a.nzT0 + a.nzN)) atomicOr(w.noiseErr, 1);
+    const WideNoise nz = *w.noise;
+    if (j == 0 && nz.fil && nz.err && (t < nz.t0 || t >= nz.t0 + nz.n)) atomicOr(nz.err, 1);
     const sbx_rigid_body* b;
     const float* noise;
     int i, key, seed;
@@ -114,7 +115,7 @@ __global__ void __launch_bounds__(256) k_wide_draws(const __grid_constant__ Wide
         key = 3 * k.y + (j - 3 * m);
         seed = B ? w.bt.seeds[3 * k.x] : sc.seed;
         mag = sc.mot.bodyParams[1];
-        noise = a.nzMot;
+        noise = nz.mot;
     } else if (j < nB + nBb) {
         b = &sc.mini.backbone;
         i = j - nB;
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(256) k_wide_draws(const __grid_constant__ Wide
         key = k.y;
         seed = B ? w.bt.seeds[3 * k.x + 1] : sc.seedBb;
         mag = sc.mini.bbBodyParams[1];
-        noise = a.nzBb;
+        noise = nz.bb;
     } else {
         b = &sc.fil.body;
         i = j - nB - nBb;
@@ -130,13 +131,13 @@ __global__ void __launch_bounds__(256) k_wide_draws(const __grid_constant__ Wide
         key = k.y;
         seed = B ? w.bt.seeds[3 * k.x + 2] : sc.fil.counts[2];
         mag = sc.fil.params[1];
-        noise = a.nzFil;
+        noise = nz.fil;
     }
     const int n = b->n;
     float g[6];
     if (noise) {
-        const int s = t - a.nzT0;
-        const bool in = s >= 0 && s < a.nzN;
+        const int s = t - nz.t0;
+        const bool in = s >= 0 && s < nz.n;
         const float* q = noise + (int64_t)(in ? s : 0) * 6 * n + i;
         for (int k = 0; k < 6; k++) g[k] = in ? q[(int64_t)k * n] : 0.f;
     } else {
@@ -816,7 +817,14 @@ __global__ void __launch_bounds__(128, MANY ? 6 : 4) k_wide_rods(const __grid_co
     body_step(fb, i, in, F, T, B ? fs.params[0] : sc.boxParams[7]);
 }
 
+__global__ void k_wide_noise(WideNoise* dst, const WideNoise noise) { *dst = noise; }
+
 }  // namespace
+
+sbx_status wide_set_noise(sbx_ctx* ctx, const WideArgs& w, const WideNoise& noise) {
+    SBX_LAUNCH(ctx, k_wide_noise, 1, 1, w.noise, noise);
+    return check_launch(ctx, "dense step: noise");
+}
 
 bool wide_streams_create(WideStreams& ws) {
     for (cudaStream_t* s : {&ws.ahead, &ws.link, &ws.csr})

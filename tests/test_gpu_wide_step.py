@@ -332,3 +332,25 @@ def test_fused_run_between_a_first_capture_and_its_replay(warm):
     assert len(compare_scenes(ref, D.to_host(net.dev))) > 80
     del g
     net.close()
+
+
+def test_noise_in_chunks(warm):
+    # noise set anew between runs, on and off, without new graphs
+    from softbox_b200.engine import DenseNetwork
+    out = []
+    for mode in ("unfused", "graph"):
+        net = DenseNetwork(copy.deepcopy(warm))
+        d, t = net.dev, 300
+        sizes = (d["fil"]["body"]["n"], d["mot"]["body"]["n"], d["mini"]["backbone"]["n"])
+        rng = torch.Generator("cuda").manual_seed(9)
+        for steps in (1, 6, 0, 5, 4):
+            if steps:
+                net.set_noise(*(torch.randn(steps, 6, n, device="cuda", generator=rng) for n in sizes), t)
+            else:
+                net.set_noise(None, None, None, 0)
+            net.run(t, steps or 3, mode=mode)
+            t += steps or 3
+        assert net.status() == 0
+        out.append(D.to_host(net.dev))
+        net.close()
+    assert len(compare_scenes(*out)) > 80
