@@ -761,9 +761,12 @@ sbx_status sbx_dense_plan_run(sbx_dense_plan* plan, int32_t t0, int32_t nsteps, 
 sbx_status sbx_dense_step_unfused(sbx_ctx* ctx, const sbx_dense_scene* scene, int32_t t);
 /* Number of kernels one fused step launches. */
 int32_t sbx_dense_plan_kernels_per_step(sbx_dense_plan* plan);
-/* Synchronises and reports the fused path's flags for the last run: bit0 a grid-barrier
+/* Synchronises and reports the flags of the last fused run and of the graph's runs since the
+ * last call: bit0 a grid-barrier
  * wait ran out (SBX_ETIMEOUT; the state of that run is partial), bit1 a reach list
- * exceeded SBX_MAX_CAND (SBX_EOVERFLOW; counts continue past the cap, as the reference),
+ * exceeded SBX_MAX_CAND (SBX_EOVERFLOW; counts continue past the cap, as the reference) in a
+ * run of mode 2, or of mode 3 up to SBX_DENSE_AUTO_MAX_FUSED_RODS rods where the fused path is
+ * available (runs of the other kinds truncate the list without a report, as mode 0),
  * bit2 a bulk-copy wait ran out (SBX_ETIMEOUT), bit3 a linked-list walk ran past its bound
  * (SBX_ESTATE). */
 sbx_status sbx_dense_plan_status(sbx_dense_plan* plan, int32_t* flags);

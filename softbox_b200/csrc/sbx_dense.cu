@@ -36,6 +36,14 @@ __global__ void k_dense_set_counts(const int* d_step, int t_host, int* motCounts
 
 __global__ void k_step_set(int* d_step, int t) { *d_step = t; }
 
+// the wide kernels' error word: a reach list past its capacity, a list walk past its bound, and
+// a reach overflow of a run that reports it
+constexpr int WIDE_REACH = 2, WIDE_LIST = 8, WIDE_REACH_REPORT = 16;
+// takes a reach overflow out of the word, or keeps it as `as`
+__global__ void k_reach_settle(int* err, int as) {
+    if (*err & WIDE_REACH) *err = (*err & ~WIDE_REACH) | as;
+}
+
 // MechanicsFusion.forceBuild (zero + BrownianForceSystem.brownianForce) in supplied-noise
 // mode: the step's six Gaussians of slot i are noise[counts[1] - t0][k][i]. A step outside
 // the supplied range (the host rejects such runs before launching) draws zeros and sets *err.
@@ -408,7 +416,9 @@ struct sbx_dense_plan {
     std::vector<void*> allocs;
     // the graph path's wide kernels (harness layouts); other scenes capture the per-system sequence
     bool wide_ok = false;
-    bool reportReach = false;      // an "auto" run of fused size ran: its reach overflows are reported
+    // the last run of the wide kernels (wideRan: there was one) was an "auto" one of fused size,
+    // whose reach overflows the status reports
+    bool wideRan = false, reportReach = false;
     WideArgs wide{};
     WideStreams wideStreams{};
     // packed networks (graph and per-system paths only)
@@ -944,6 +954,7 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
     if (nsteps == 0) return SBX_OK;
     if (p->noiseOn && ((int64_t)t0 < p->noise.t0 || (int64_t)t0 + nsteps > (int64_t)p->noise.t0 + p->noise.nsteps))
         return fail(ctx, SBX_EINVAL, "sbx_dense_plan_run: steps outside the supplied-noise range");
+    bool report = false;
     if (mode == 3) {
         // the wide kernels lead at every size: 30 / 57 us a step at 1,000 rods (one step a call),
         // 35 / 64 at 20,000 and 54 / 172 at 40,000 (20 steps a call) against the fused kernel
@@ -953,7 +964,7 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
         if (!fused) mode = 1;
         else if (capturing(ctx)) mode = fused_current(p) == SBX_OK && p->fused_ok ? 2 : 0;
         else mode = p->wide_ok ? 1 : 2;
-        if (fused) p->reportReach = true;
+        report = fused;
     }
     if (mode == 2) {
         CHK(fused_current(p));
@@ -972,7 +983,15 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
         SBX_TRACE("sbx.dense.graph_replay");
         // A run that goes on where the last one ended finds its step index in place; not where a
         // graph that captured a run may be replayed in between.
-        if (capturing(ctx)) p->stepShared = true;
+        const bool captured = capturing(ctx);
+        if (captured) p->stepShared = true;
+        if (p->wide_ok && !captured) {
+            // an overflow belongs to the run it came from: settled where the two kinds follow each other
+            if (p->wideRan && p->reportReach != report)
+                SBX_LAUNCH(ctx, k_reach_settle, 1, 1, p->wide.a.err, p->reportReach ? WIDE_REACH_REPORT : 0);
+            p->wideRan = true;
+            p->reportReach = report;
+        }
         if (p->stepShared || p->stepNow != t0) SBX_LAUNCH(ctx, k_step_set, 1, 1, p->d_step, t0);
         p->stepNow = INT64_MIN;
         for (int k = 0; k < nsteps;) {
@@ -1016,9 +1035,9 @@ extern "C" sbx_status sbx_dense_plan_status(sbx_dense_plan* p, int32_t* flags) {
         int we = 0;
         cudaMemcpyAsync(&we, p->wide.a.err, sizeof(int), cudaMemcpyDeviceToHost, p->ctx->stream);
         CHK(sbx_ctx_sync(p->ctx));
-        const bool reach = (we & 2) && p->reportReach;
+        const bool reach = (we & WIDE_REACH_REPORT) || ((we & WIDE_REACH) && p->reportReach);
         if (we) cudaMemsetAsync(p->wide.a.err, 0, 16, p->ctx->stream);
-        if (we & 8) {
+        if (we & WIDE_LIST) {
             wide_reset(p);
             *flags = 8;
             return fail(p->ctx, SBX_ESTATE, "graph step: a linked-list walk ran past its bound");

@@ -354,3 +354,31 @@ def test_noise_in_chunks(warm):
         out.append(D.to_host(net.dev))
         net.close()
     assert len(compare_scenes(*out)) > 80
+
+
+@pytest.mark.parametrize("runs,reported", [(("graph",), False), (("auto",), True), (("graph", "auto"), True),
+                                           (("auto", "graph"), True), (("graph", "unfused"), False)])
+def test_a_reach_overflow_is_its_runs(runs, reported):
+    # reported for the runs of fused size, whatever ran before or after them; not for the graph's
+    import physics_gates as G
+    from softbox_b200.engine import DenseNetwork
+    from softbox_b200.runtime import SbxError
+    net = DenseNetwork(G.crowded_dense())
+    assert net.fused_available
+    t = 0
+    for first in (("auto",), ()):                      # once after an auto run whose report was taken
+        for mode in first:
+            net.run(t, 1, mode=mode)
+            t += 1
+            with pytest.raises(SbxError):
+                net.status()
+            assert net.status() == 0
+        for mode in runs:
+            net.run(t, 1, mode=mode)
+            t += 1
+        if reported:
+            with pytest.raises(SbxError) as e:
+                net.status()
+            assert e.value.code == -3
+        assert net.status() == 0
+    net.close()
