@@ -967,7 +967,10 @@ typedef struct sbx_mlp_train_state {
     int32_t* err;
 } sbx_mlp_train_state;
 /* 1 if the whole-network kernels take this ensemble: at most 16 inputs and outputs, hidden
- * widths multiples of 32 up to 256, at most SBX_MLP_MAX_LAYERS layers (training: at least 2) */
+ * widths multiples of 32 up to 256, at most SBX_MLP_MAX_LAYERS layers. For training (at least 2
+ * layers) it also asks the current device whether a block of every network is resident at once,
+ * which sbx_mlp_train requires, and whether so few blocks a network still lead the separate
+ * kernels. */
 int32_t sbx_mlp_net_fits(const sbx_mlp_net* net, int32_t train);
 /* Predictions for P points X [P][nin] (FP64, not normalised): out [2 + nz][P][nout] FP64 holds
  * the ensemble mean, its population standard deviation and each network's outputs.

@@ -1018,7 +1018,39 @@ static int sm_count(sbx_ctx* ctx) {
     return sms;
 }
 
-extern "C" int32_t sbx_mlp_net_fits(const sbx_mlp_net* net, int32_t train) { return net_fits(net, train != 0) ? 1 : 0; }
+constexpr size_t TRAIN_SMEM = (size_t)(MT + TRAIN_N) * KMAX * 2;
+
+// blocks of the training kernel that the current device holds at once; 0 if it cannot tell
+static int train_blocks() {
+    int dev = 0, sms = 0, per = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+        cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRAIN_SMEM) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_train, TRAIN_THREADS, TRAIN_SMEM) == cudaSuccess)
+        return per * sms;
+    cudaGetLastError();
+    return 0;
+}
+
+// Where the one launch leads the separate kernels. A network's blocks must all be resident: more
+// networks than that cannot run whole. With two blocks a network or more it leads at every width
+// and batch that was measured (32 to 256 wide, 2 to 8 layers, batches of 16 to 256): 1.06 to 8
+// times. With one block it depends on how many tiles of a layer's weights that block walks
+// through: up to ONE_BLOCK_TILES it leads or is even (75 to 148 networks: 96 wide 3 tiles, 1.5 to
+// 2.4 times; 256-64-256 8 tiles, 1.04 to 1.36; 160 wide 10 tiles, 0.97 to 1.23), beyond them
+// mostly not (192 wide 12 tiles, 0.86 to 1.14; 256 wide 16 tiles, 0.67 to 1.03).
+constexpr int ONE_BLOCK_TILES = 10;
+static bool train_leads(const sbx_mlp_net* n) {
+    const int per = train_blocks() / n->nz;
+    if (per != 1) return per > 1;
+    for (int l = 0; l < n->nLayers; l++)
+        if (((n->Np[l] + MT - 1) / MT) * ((n->Kp[l] + TRAIN_N - 1) / TRAIN_N) > ONE_BLOCK_TILES) return false;
+    return true;
+}
+
+extern "C" int32_t sbx_mlp_net_fits(const sbx_mlp_net* net, int32_t train) {
+    return net_fits(net, train != 0) && (!train || train_leads(net)) ? 1 : 0;
+}
 
 extern "C" sbx_status sbx_mlp_predict(sbx_ctx* ctx, const sbx_mlp_net* net, const double* X, int32_t P,
                                       const double* xMean, const double* xStd, const double* yMean,
@@ -1047,14 +1079,9 @@ extern "C" sbx_status sbx_mlp_train(sbx_ctx* ctx, const sbx_mlp_net* net, const 
         SBX_REQUIRE(st->W[l] && st->mW[l] && st->vW[l] && st->mb[l] && st->vb[l] && st->dW[l] && st->db[l] &&
                     st->WbT[l] && st->Z[l] && st->G[l] && st->GT[l] &&
                     (l == net->nLayers - 1 || (st->A[l] && st->AT[l])));
-    const size_t smem = (size_t)(MT + TRAIN_N) * KMAX * 2;
-    if (cudaFuncSetAttribute(k_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return fail(ctx, SBX_ECUDA, "sbx_mlp_train: shared memory attribute");
-    int per = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_train, TRAIN_THREADS, smem) != cudaSuccess || per < 1)
-        return fail(ctx, SBX_ECUDA, "sbx_mlp_train: occupancy");
+    const size_t smem = TRAIN_SMEM;
     // a network's blocks: all resident, no more than a backward pass has tiles (two products of 16)
-    int gx = per * sm_count(ctx) / net->nz;
+    int gx = train_blocks() / net->nz;
     if (gx < 1) return fail(ctx, SBX_EINVAL, "sbx_mlp_train: more networks than resident blocks");
     if (gx > 32) gx = 32;
     TrainArgs g{};

@@ -72,3 +72,19 @@ def test_one_step_on_given_batches_equals_fit():
     torch.cuda.synchronize()
     for l in range(a.L):
         assert torch.equal(a.W[l], b.W[l]) and torch.equal(a.b[l], b.b[l])
+
+
+@pytest.mark.parametrize("dims,nz,whole", [((6, 32, 3), 64, True), ((6, 32, 3), 148, True), ((6, 32, 3), 300, False),
+                                           ((6, 256, 256, 3), 64, True), ((6, 256, 256, 3), 148, False)])
+def test_many_networks_train(dims, nz, whole, monkeypatch):
+    # past the resident blocks, or with too much work for a network's one block, the separate kernels
+    a, x, y = _ensemble(dims, nz, 16)
+    b, _, _ = _ensemble(dims, nz, 16)
+    assert (a._trains_whole() is not None) == whole
+    ha = a.fit(x[:32], y[:32], epochs=1, seed=5)
+    monkeypatch.setattr(type(b), "_net", lambda self, train: None)
+    hb = b.fit(x[:32], y[:32], epochs=1, seed=5)
+    assert abs(ha[0] - hb[0]) <= 1e-5 * abs(hb[0])
+    for l in range(a.L):
+        p, q = a.W[l].double(), b.W[l].double()
+        assert (p - q).norm() <= 2e-5 * q.norm(), l
