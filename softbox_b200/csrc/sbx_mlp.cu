@@ -544,7 +544,7 @@ struct TrainArgs {
     float* Z[NET_MAX_LAYERS];
     float* loss;
     float lr, b1, b2, eps, c1[TRAIN_STEPS], c2[TRAIN_STEPS];
-    unsigned long long* bar;                       // [nz] arrival counters, zero at launch
+    unsigned long long* bar;                       // [nz] arrival counters (and NET_FAILED), zero at launch
     int* err;                                      // bit 0: an MMA or barrier wait ran out
 };
 
@@ -554,25 +554,36 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
     return v;
 }
 
-// barrier of a network's blocks; false (for the whole block) once a wait has run out anywhere
-__device__ bool net_sync(unsigned long long* ctr, unsigned long long& target, int* err) {
+// A network's counter also carries the word that its launch is given up: with NET_FAILED set its
+// blocks leave their barrier, whatever they have counted; the next launch begins from zero.
+constexpr unsigned long long NET_FAILED = 1ULL << 63;
+
+// this launch of the network is given up (a wait ran out), its loss not a number
+__device__ void net_fail(const TrainArgs& g, int z) {
+    asm volatile("red.release.gpu.global.or.b64 [%0], %1;" ::"l"(g.bar + z), "l"(NET_FAILED) : "memory");
+    *(volatile float*)(g.loss + z) = __int_as_float(0x7fc00000);
+    atomicOr(g.err, 1);
+}
+
+// barrier of a network's blocks; false (for the whole block) once a wait of theirs has run out
+__device__ bool net_sync(const TrainArgs& g, int z, unsigned long long& target) {
     __shared__ int s_ok;
+    unsigned long long* ctr = g.bar + z;
     __syncthreads();
     if (threadIdx.x == 0) {
         target += gridDim.x;
         asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(ctr), "l"(1ULL) : "memory");
-        bool ok = true;
+        unsigned long long at;
         long long t0 = 0;
         unsigned it = 0;
-        while (ld_acquire_u64(ctr) < target) {
+        while ((at = ld_acquire_u64(ctr)) < target) {      // (a failed network's counter is past any target)
             if ((++it & 63u) == 0) {
-                if (*(volatile int*)err & 1) { ok = false; break; }
                 long long now = gtimer();
                 if (t0 == 0) t0 = now;
-                else if (now - t0 > WAIT_NS) { atomicOr(err, 1); ok = false; break; }
+                else if (now - t0 > WAIT_NS) { net_fail(g, z); at = NET_FAILED; break; }
             }
         }
-        s_ok = ok;
+        s_ok = (at & NET_FAILED) == 0;
     }
     __syncthreads();
     return s_ok != 0;
@@ -619,7 +630,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 2) k_train(const __grid_constan
         if (threadIdx.x == 0) issue_mma(tmem, smem_u32(sA), smem_u32(sB), N, Kp, &mbar);
         const bool done = wait_mma(&mbar, phase);
         phase ^= 1u;
-        if (!done && threadIdx.x == 0) atomicOr(g.err, 1);
+        if (!done && threadIdx.x == 0) net_fail(g, z);
         asm volatile("tcgen05.fence::after_thread_sync;");
         return done;
     };
@@ -784,7 +795,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 2) k_train(const __grid_constan
                 }
                 if (ok) release();
             }
-            ok = ok && net_sync(g.bar + z, target, g.err);
+            ok = ok && net_sync(g, z, target);
         }
         // ---- backward: the gradient of layer l's input, with the update of layer l + 1
         for (int l = L - 1; l >= 1 && ok; l--) {
@@ -818,13 +829,13 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 2) k_train(const __grid_constan
                 }
                 if (ok) release();
             }
-            ok = ok && net_sync(g.bar + z, target, g.err);
+            ok = ok && net_sync(g, z, target);
         }
         // ---- the updates that are left: layer 0, and layer 1 of a network with more than one
         const int w1 = L > 1 ? weight_tiles(1) : 0, w0 = weight_tiles(0);
         for (int tile = blockIdx.x; tile < w1 + w0 && ok; tile += gridDim.x)
             ok = weight_tile(tile < w1 ? 1 : 0, tile < w1 ? tile : tile - w1, s);
-        ok = ok && net_sync(g.bar + z, target, g.err);
+        ok = ok && net_sync(g, z, target);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();

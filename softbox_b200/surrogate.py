@@ -64,7 +64,9 @@ class MLPEnsemble:
         self._refresh_bf16()
         self._alloc(batch)
         self.x_mean = self.x_std = self.y_mean = self.y_std = None
-        self.err = torch.zeros(1, dtype=torch.int32, device=device)
+        # what a training epoch reports in one read: the mean loss, and the kernels' error word
+        self._report = torch.zeros(2, **f32)
+        self.err = self._report.view(torch.int32)[1:]
         self.graph = None
 
     # ---------------------------------------------------------------- buffers
@@ -98,6 +100,14 @@ class MLPEnsemble:
             wb = self.W[l].to(t.bfloat16)
             self.Wb[l].copy_(wb.view(t.int16))
             self.WbT[l].copy_(wb.transpose(1, 2).contiguous().view(t.int16))
+
+    def _raise_on(self, err):
+        """Raises if the error word says that a wait in a kernel ran out, and clears it: the weights
+        of a training step, or a prediction, are then not to be used."""
+        if err:
+            from .runtime import SbxError
+            self.err.zero_()
+            raise SbxError(-4, "surrogate: a tensor-core or barrier wait ran out; this call's results are partial")
 
     # ---------------------------------------------------------------- whole networks
     def _net(self, train):
@@ -197,7 +207,8 @@ class MLPEnsemble:
 
     def train_step(self, xb, tb):
         """One Adam step per member on its own batch: xb [nz, B, nin], tb [nz, B, nout]
-        (normalised, device). Returns nothing; the losses stay in self.loss."""
+        (normalised, device). Returns nothing; the losses stay in self.loss (not a number where a
+        whole-network step was given up; fit and predict raise then)."""
         t = self.torch
         shapes = ((xb, (self.nz, self.B, self.nin)), (tb, (self.nz, self.B, self.nout)))
         net = self._trains_whole()
@@ -236,7 +247,10 @@ class MLPEnsemble:
                 if idx.shape[1] < self.B:
                     break
                 self.train_step(Xn[idx], Yn[idx])
-            hist.append(float(self.loss.mean().item()))
+            t.mean(self.loss, dim=0, keepdim=True, out=self._report[:1])
+            report = self._report.cpu()
+            self._raise_on(int(report.view(t.int32)[1]))
+            hist.append(float(report[0]))
             if log:
                 log(ep, hist[-1])
         return hist
@@ -290,6 +304,7 @@ class MLPEnsemble:
             self._inf_X0[:, :m].copy_(xp.view(t.int16).unsqueeze(0).expand(self.nz, m, KPAD_IN))
             outs.append(self._forward_infer(m)[:, :m, :self.nout].clone())
         y = t.cat(outs, dim=1).cpu().numpy().astype(np.float64) * self.y_std + self.y_mean
+        self._raise_on(self.err.item())
         return y.mean(axis=0), y.std(axis=0), y
 
     def _predict_whole(self, net, X):
@@ -309,6 +324,7 @@ class MLPEnsemble:
         host = np.empty(out.shape)
         host.reshape(-1)[::512] = 0.0
         t.from_numpy(host).copy_(out)
+        self._raise_on(self.err.item())
         return host[0], host[1], host[2:]
 
 

@@ -88,3 +88,27 @@ def test_many_networks_train(dims, nz, whole, monkeypatch):
     for l in range(a.L):
         p, q = a.W[l].double(), b.W[l].double()
         assert (p - q).norm() <= 2e-5 * q.norm(), l
+
+
+@pytest.mark.parametrize("whole", [True, False])
+def test_a_failed_wait_is_raised_once(whole, monkeypatch):
+    # a kernel's error word (set from the host here) ends the call that finds it with an error,
+    # and neither stops that call's kernels nor the next call
+    from softbox_b200.runtime import SbxError
+    a, x, y = _ensemble((6, 64, 64, 3), 2, 64)
+    b, _, _ = _ensemble((6, 64, 64, 3), 2, 64)
+    if not whole:
+        monkeypatch.setattr(type(a), "_net", lambda self, train: None)
+    a.err.fill_(1)
+    with pytest.raises(SbxError, match="wait ran out"):
+        a.fit(x[:1024], y[:1024], epochs=1, seed=5)
+    b.fit(x[:1024], y[:1024], epochs=1, seed=5)
+    ha, hb = (e.fit(x[:1024], y[:1024], epochs=2, seed=6) for e in (a, b))
+    assert np.allclose(ha, hb, rtol=1e-5)               # (the loss is summed in no order)
+    for l in range(a.L):
+        assert torch.equal(a.W[l], b.W[l]) and torch.equal(a.b[l], b.b[l])
+    a.err.fill_(1)
+    with pytest.raises(SbxError, match="wait ran out"):
+        a.predict(x[:300])
+    for p, q in zip(a.predict(x[:300]), b.predict(x[:300])):
+        assert np.array_equal(p, q)
