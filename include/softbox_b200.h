@@ -954,7 +954,8 @@ typedef struct sbx_mlp_net {
  * transposed BF16 weights [nz][Kp][Np], and buffers of a pass of B rows: activations A and
  * their transposes AT (not for the last layer), pre-activations Z, gradients G and GT, the
  * transposed inputs X0T [nz][16][B]. loss: nz floats (the last step's). bar: nz uint64 words
- * of scratch. err gets bit 0 when a wait ran out (it is not read or cleared here); that
+ * of scratch. All but the biases' arrays (mb, vb, db), loss, bar and err begin on 16-byte
+ * boundaries, and so does Wb. err gets bit 0 when a wait ran out (it is not read or cleared here); that
  * network's launch is then given up with its weights partly updated, its loss not a number. */
 typedef struct sbx_mlp_train_state {
     float *W[SBX_MLP_MAX_LAYERS], *mW[SBX_MLP_MAX_LAYERS], *vW[SBX_MLP_MAX_LAYERS], *mb[SBX_MLP_MAX_LAYERS],

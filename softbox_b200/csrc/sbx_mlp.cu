@@ -1086,10 +1086,12 @@ extern "C" sbx_status sbx_mlp_train(sbx_ctx* ctx, const sbx_mlp_net* net, const 
                                     int32_t nsteps, int32_t stepNumber, float lr, float beta1, float beta2, float eps) {
     SBX_REQUIRE(ctx && net_fits(net, true) && st && B >= 16 && B <= KMAX && B % 16 == 0 && X && Y && nsteps >= 0 &&
                 stepNumber >= 1 && st->X0T && st->loss && st->bar && st->err);
+    auto aligned = [](const void* p) { return p && ((uintptr_t)p & 15) == 0; };
+    SBX_REQUIRE(aligned(st->X0T) && ((uintptr_t)st->bar & 7) == 0);
     for (int l = 0; l < net->nLayers; l++)
-        SBX_REQUIRE(st->W[l] && st->mW[l] && st->vW[l] && st->mb[l] && st->vb[l] && st->dW[l] && st->db[l] &&
-                    st->WbT[l] && st->Z[l] && st->G[l] && st->GT[l] &&
-                    (l == net->nLayers - 1 || (st->A[l] && st->AT[l])));
+        SBX_REQUIRE(aligned(st->W[l]) && aligned(st->mW[l]) && aligned(st->vW[l]) && aligned(st->dW[l]) && st->mb[l] &&
+                    st->vb[l] && st->db[l] && aligned(st->WbT[l]) && aligned(st->Z[l]) && aligned(st->G[l]) &&
+                    aligned(st->GT[l]) && (l == net->nLayers - 1 || (aligned(st->A[l]) && aligned(st->AT[l]))));
     const size_t smem = TRAIN_SMEM;
     // a network's blocks: all resident, no more than a backward pass has tiles (two products of 16)
     int gx = train_blocks() / net->nz;

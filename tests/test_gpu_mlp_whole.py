@@ -112,3 +112,22 @@ def test_a_failed_wait_is_raised_once(whole, monkeypatch):
         a.predict(x[:300])
     for p, q in zip(a.predict(x[:300]), b.predict(x[:300])):
         assert np.array_equal(p, q)
+
+
+@pytest.mark.parametrize("name", ["W", "mW", "vW", "dW", "WbT", "A", "AT", "G", "GT", "Z", "X0T", "bar", "Wb"])
+def test_unaligned_training_arrays_are_refused(name):
+    from softbox_b200 import abi_types as T
+    a, x, y = _ensemble((6, 32, 32, 3), 2, 16)
+    net, s = a._net(True), T.MlpTrainState()
+    for l in range(a.L):
+        for k in ("W", "mW", "vW", "mb", "vb", "dW", "db", "WbT", "A", "AT", "G", "GT", "Z"):
+            getattr(s, k)[l] = getattr(a, k)[l].data_ptr()
+    s.X0T, s.loss, s.bar, s.err = (v.data_ptr() for v in (a.X0T, a.loss, a.bar, a.err))
+    if name in ("X0T", "bar"):
+        setattr(s, name, getattr(s, name) + 4)
+    else:
+        at = net.Wb if name == "Wb" else getattr(s, name)
+        at[1] += 4
+    X, Y = (torch.zeros(64, n, device="cuda") for n in (6, 3))
+    st = a._ctx().raw("sbx_mlp_train", net, s, 16, X, Y, None, 0, 1, 1, 1e-3, 0.9, 0.999, 1e-8)
+    assert st == -1                                    # SBX_EINVAL, before anything is launched
