@@ -559,16 +559,15 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 constexpr unsigned long long NET_FAILED = 1ULL << 63;
 
 // this launch of the network is given up (a wait ran out), its loss not a number
-__device__ void net_fail(const TrainArgs& g, int z) {
-    asm volatile("red.release.gpu.global.or.b64 [%0], %1;" ::"l"(g.bar + z), "l"(NET_FAILED) : "memory");
-    *(volatile float*)(g.loss + z) = __int_as_float(0x7fc00000);
-    atomicOr(g.err, 1);
+__device__ __forceinline__ void net_fail(unsigned long long* ctr, float* loss, int* err) {
+    asm volatile("red.release.gpu.global.or.b64 [%0], %1;" ::"l"(ctr), "l"(NET_FAILED) : "memory");
+    *(volatile float*)loss = __int_as_float(0x7fc00000);
+    atomicOr(err, 1);
 }
 
 // barrier of a network's blocks; false (for the whole block) once a wait of theirs has run out
-__device__ bool net_sync(const TrainArgs& g, int z, unsigned long long& target) {
+__device__ bool net_sync(unsigned long long* ctr, unsigned long long& target, float* loss, int* err) {
     __shared__ int s_ok;
-    unsigned long long* ctr = g.bar + z;
     __syncthreads();
     if (threadIdx.x == 0) {
         target += gridDim.x;
@@ -580,7 +579,7 @@ __device__ bool net_sync(const TrainArgs& g, int z, unsigned long long& target) 
             if ((++it & 63u) == 0) {
                 long long now = gtimer();
                 if (t0 == 0) t0 = now;
-                else if (now - t0 > WAIT_NS) { net_fail(g, z); at = NET_FAILED; break; }
+                else if (now - t0 > WAIT_NS) { net_fail(ctr, loss, err); at = NET_FAILED; break; }
             }
         }
         s_ok = (at & NET_FAILED) == 0;
@@ -630,7 +629,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 2) k_train(const __grid_constan
         if (threadIdx.x == 0) issue_mma(tmem, smem_u32(sA), smem_u32(sB), N, Kp, &mbar);
         const bool done = wait_mma(&mbar, phase);
         phase ^= 1u;
-        if (!done && threadIdx.x == 0) net_fail(g, z);
+        if (!done && threadIdx.x == 0) net_fail(g.bar + z, g.loss + z, g.err);
         asm volatile("tcgen05.fence::after_thread_sync;");
         return done;
     };
@@ -795,7 +794,7 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 2) k_train(const __grid_constan
                 }
                 if (ok) release();
             }
-            ok = ok && net_sync(g, z, target);
+            ok = ok && net_sync(g.bar + z, target, g.loss + z, g.err);
         }
         // ---- backward: the gradient of layer l's input, with the update of layer l + 1
         for (int l = L - 1; l >= 1 && ok; l--) {
@@ -829,13 +828,13 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 2) k_train(const __grid_constan
                 }
                 if (ok) release();
             }
-            ok = ok && net_sync(g, z, target);
+            ok = ok && net_sync(g.bar + z, target, g.loss + z, g.err);
         }
         // ---- the updates that are left: layer 0, and layer 1 of a network with more than one
         const int w1 = L > 1 ? weight_tiles(1) : 0, w0 = weight_tiles(0);
         for (int tile = blockIdx.x; tile < w1 + w0 && ok; tile += gridDim.x)
             ok = weight_tile(tile < w1 ? 1 : 0, tile < w1 ? tile : tile - w1, s);
-        ok = ok && net_sync(g, z, target);
+        ok = ok && net_sync(g.bar + z, target, g.loss + z, g.err);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();

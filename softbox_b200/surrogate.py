@@ -64,9 +64,8 @@ class MLPEnsemble:
         self._refresh_bf16()
         self._alloc(batch)
         self.x_mean = self.x_std = self.y_mean = self.y_std = None
-        # what a training epoch reports in one read: the mean loss, and the kernels' error word
-        self._report = torch.zeros(2, **f32)
-        self.err = self._report.view(torch.int32)[1:]
+        # the kernels' error word, in mapped host memory: read after a call's results, without a copy
+        self.err = torch.zeros(1, dtype=torch.int32, pin_memory=True)
         self.graph = None
 
     # ---------------------------------------------------------------- buffers
@@ -101,10 +100,10 @@ class MLPEnsemble:
             self.Wb[l].copy_(wb.view(t.int16))
             self.WbT[l].copy_(wb.transpose(1, 2).contiguous().view(t.int16))
 
-    def _raise_on(self, err):
+    def _raise_on_error(self):
         """Raises if the error word says that a wait in a kernel ran out, and clears it: the weights
         of a training step, or a prediction, are then not to be used."""
-        if err:
+        if self.err.item():
             from .runtime import SbxError
             self.err.zero_()
             raise SbxError(-4, "surrogate: a tensor-core or barrier wait ran out; this call's results are partial")
@@ -247,10 +246,8 @@ class MLPEnsemble:
                 if idx.shape[1] < self.B:
                     break
                 self.train_step(Xn[idx], Yn[idx])
-            t.mean(self.loss, dim=0, keepdim=True, out=self._report[:1])
-            report = self._report.cpu()
-            self._raise_on(int(report.view(t.int32)[1]))
-            hist.append(float(report[0]))
+            hist.append(float(self.loss.mean().item()))
+            self._raise_on_error()
             if log:
                 log(ep, hist[-1])
         return hist
@@ -304,7 +301,7 @@ class MLPEnsemble:
             self._inf_X0[:, :m].copy_(xp.view(t.int16).unsqueeze(0).expand(self.nz, m, KPAD_IN))
             outs.append(self._forward_infer(m)[:, :m, :self.nout].clone())
         y = t.cat(outs, dim=1).cpu().numpy().astype(np.float64) * self.y_std + self.y_mean
-        self._raise_on(self.err.item())
+        self._raise_on_error()
         return y.mean(axis=0), y.std(axis=0), y
 
     def _predict_whole(self, net, X):
@@ -324,7 +321,7 @@ class MLPEnsemble:
         host = np.empty(out.shape)
         host.reshape(-1)[::512] = 0.0
         t.from_numpy(host).copy_(out)
-        self._raise_on(self.err.item())
+        self._raise_on_error()
         return host[0], host[1], host[2:]
 
 
