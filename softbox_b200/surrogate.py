@@ -316,13 +316,17 @@ class MLPEnsemble:
         Xd = t.from_numpy(np.ascontiguousarray(X, dtype=np.float64)).to(self.dev)
         out = t.empty((2 + self.nz, P, self.nout), dtype=t.float64, device=self.dev)
         self._ctx()("sbx_mlp_predict", net, Xd, P, xm, xs, ym, ys, out, self.err)
-        # the result's pages are touched while the kernel runs: fresh memory costs as much as the
-        # copy into it
-        host = np.empty(out.shape)
-        host.reshape(-1)[::512] = 0.0
-        t.from_numpy(host).copy_(out)
+        # Of a large result each part is an array of its own, so that a mean that is kept does not keep
+        # every network's outputs; a small one comes in one read. The pages are touched while the
+        # kernel runs: fresh memory costs as much as the copy into it.
+        parts = (out[0], out[1], out[2:]) if out.numel() > 1 << 17 else (out,)
+        host = [np.empty(v.shape) for v in parts]
+        for h in host:
+            h.reshape(-1)[::512] = 0.0
+        for h, v in zip(host, parts):
+            t.from_numpy(h).copy_(v)
         self._raise_on_error()
-        return host[0], host[1], host[2:]
+        return tuple(host) if len(host) == 3 else (host[0][0], host[0][1], host[0][2:])
 
 
 def fallback_mask(mean, std, threshold=0.10, outputs=None, scale=None):

@@ -131,3 +131,12 @@ def test_unaligned_training_arrays_are_refused(name):
     X, Y = (torch.zeros(64, n, device="cuda") for n in (6, 3))
     st = a._ctx().raw("sbx_mlp_train", net, s, 16, X, Y, None, 0, 1, 1, 1e-3, 0.9, 0.999, 1e-8)
     assert st == -1                                    # SBX_EINVAL, before anything is launched
+
+
+def test_large_predictions_are_arrays_of_their_own():
+    # a mean that is kept does not keep every network's outputs
+    a, x, _ = _ensemble((6, 32, 16), 3, 16)
+    mean, std, y = a.predict(x)
+    assert mean.shape == std.shape == (2048, 16) and y.shape == (3, 2048, 16)
+    for v in (mean, std, y):
+        assert v.flags.owndata and v.flags.writeable and v.base is None
