@@ -61,3 +61,25 @@ def test_extent_and_clusters(sizes, links):
         p = xyz[:, s][:, m]
         want = np.sqrt(((p - p.mean(axis=1, keepdims=True)) ** 2).sum(axis=0).mean()) if m.any() else 0.0
         assert ex[k, 1] == m.sum() and abs(ex[k, 0] - want) <= 1e-12 * max(want, 1.0)
+
+
+@pytest.mark.parametrize("n,links", [(300_000, 0), (300_000, 1), (1 << 21, 0)])
+def test_one_long_chain(n, links):
+    # a walk along the chain takes fewer steps than a walk's limit (2^20), and every label is right
+    from softbox_b200.runtime import default_context
+    dev = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")  # noqa: E731
+    ctx = default_context()
+    e2 = torch.arange(1, n + 1, dtype=torch.int32, device="cuda")
+    e2[-1] = -1
+    label, size = (torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(2))
+    flags, out, ends = dev([0, 0, 0]), dev([0, 0]), dev([0, n - 1, 0])
+    for _ in range(3):                                 # (the third call is timed)
+        torch.cuda.synchronize()
+        s, e = torch.cuda.Event(True), torch.cuda.Event(True)
+        s.record()
+        ctx("sbx_obs_clusters", 1, dev([0, n]), n, None, e2, links, ends[:1], ends[1:2], ends[2:], 0, None, None, 0, 2,
+            label, size, flags, out)
+        e.record()
+        torch.cuda.synchronize()
+    assert out.tolist() == [n, n] and flags[1].item() == 0 and label.max().item() == 0
+    assert s.elapsed_time(e) < 20                      # ms: hooking and compressing in rounds takes 3 at 2^21
