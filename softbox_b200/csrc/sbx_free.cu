@@ -188,26 +188,41 @@ __global__ void __launch_bounds__(PipeShape<RODS>::THREADS) k_free_pipe(const Fr
     if (steps) rod_store(a, first + lane, r);                // (the last step's forces: stored by its draw)
 }
 
-// The pipeline while the rods leave the GPU idle: as few rods a block as give at most two
-// blocks an SM, 32 up to four blocks an SM. More rods fill the GPU one thread a rod, where the
-// pipeline's stepping warps are in the way. Measured before the velocities moved to the drawing
-// warps, us a step, pipeline / one thread a rod: 4,096 rods 0.67 (16 a block; 1.25 with 8)
-// / 1.71, 8,192 0.72 (32) / 1.71, 16,384 1.44 (32) / 1.73, 32,768 2.84 (32) / 2.02. A few
-// steps are not worth filling the pipeline.
-constexpr int PIPE_MIN_STEPS = 4;
+// Rods a block of the pipeline, 0 for one thread a rod. As few rods a block as give at most two
+// blocks an SM, else 32. Its registers let two blocks on an SM (three with supplied noise), so up
+// to there it leads from a few steps on; more blocks follow one another, and then the steps
+// must be worth the filling of the pipeline twice, up to where the draws fill the GPU anyway.
+// us a call, pipeline / one thread a rod (rods without, and with, external forces; the former
+// also leave the velocities to the drawing warps), on 148 SMs:
+//   4,736 rods, Philox        8 steps 18 / 25, 20 / 25     32 steps 31 / 66, 38 / 66
+//   9,472 (two blocks an SM)  8 steps 18 / 25, 20 / 25     32 steps 32 / 66, 38 / 66
+//   14,208 (three)            8 steps 22 / 24, 26 / 24     16 steps 30 / 37, 36.5 / 37
+//   18,944 (four)             8 steps 23 / 24, 26 / 24     24 steps 42 / 50, 51.5 / 50.5
+//   14,208, supplied noise   16 steps 41 / 44, 41 / 41    100 steps 90 / 116, 112 / 116
+//   18,944, supplied noise   16 steps 46 / 41, 54 / 40     64 steps 102 / 88, 131 / 88
+constexpr int pipe_rods(int n, int nsteps, int sms, bool supplied) {
+    const int64_t wave = (int64_t)32 * sms;            // rods at one block of 32 an SM
+    if (n > 4 * wave || (supplied && n > 3 * wave) || nsteps > 0x7fffffff - 64) return 0;
+    if (nsteps < (n <= 2 * wave ? 4 : n <= 3 * wave ? 16 : 24)) return 0;
+    return n <= 16 * (int64_t)sms ? 8 : n <= 32 * (int64_t)sms ? 16 : 32;
+}
+static_assert(pipe_rods(2368, 4, 148, false) == 8 && pipe_rods(2369, 4, 148, true) == 16 &&
+              pipe_rods(4737, 4, 148, false) == 32 && pipe_rods(2368, 3, 148, false) == 0, "few rods");
+static_assert(pipe_rods(9473, 15, 148, false) == 0 && pipe_rods(9473, 16, 148, true) == 32 &&
+              pipe_rods(14209, 23, 148, false) == 0 && pipe_rods(14209, 24, 148, false) == 32 &&
+              pipe_rods(14209, 1000, 148, true) == 0 && pipe_rods(18945, 1000, 148, false) == 0, "more than two blocks an SM");
+static_assert(pipe_rods(1, 0x7fffffff, 148, false) == 0, "a step index past the chunks");
+
 template <int MODE>
 void free_launch(sbx_ctx* ctx, const FreeArgs& a) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess) sms = 0;
-    const int64_t two = 2 * (int64_t)sms;
-    if (a.nsteps < PIPE_MIN_STEPS || a.n > 2 * 32 * two)
-        SBX_LAUNCH(ctx, k_free_rods<MODE>, blocks(a.n, 128), 128, a);
-    else if (a.n <= 8 * two)
-        SBX_LAUNCH(ctx, (k_free_pipe<MODE, 8>), blocks(a.n, 8), PipeShape<8>::THREADS, a);
-    else if (a.n <= 16 * two)
-        SBX_LAUNCH(ctx, (k_free_pipe<MODE, 16>), blocks(a.n, 16), PipeShape<16>::THREADS, a);
-    else
-        SBX_LAUNCH(ctx, (k_free_pipe<MODE, 32>), blocks(a.n, 32), PipeShape<32>::THREADS, a);
+    switch (pipe_rods(a.n, a.nsteps, sms, MODE == 2)) {
+    case 8: SBX_LAUNCH(ctx, (k_free_pipe<MODE, 8>), blocks(a.n, 8), PipeShape<8>::THREADS, a); break;
+    case 16: SBX_LAUNCH(ctx, (k_free_pipe<MODE, 16>), blocks(a.n, 16), PipeShape<16>::THREADS, a); break;
+    case 32: SBX_LAUNCH(ctx, (k_free_pipe<MODE, 32>), blocks(a.n, 32), PipeShape<32>::THREADS, a); break;
+    default: SBX_LAUNCH(ctx, k_free_rods<MODE>, blocks(a.n, 128), 128, a);
+    }
 }
 
 }  // namespace
