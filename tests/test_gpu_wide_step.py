@@ -382,3 +382,18 @@ def test_a_reach_overflow_is_its_runs(runs, reported):
             assert e.value.code == -3
         assert net.status() == 0
     net.close()
+
+
+def test_more_rods_than_graphs_of_several_steps_take():
+    # above 2^17 rods a graph holds one step: the largest size's rule, on more than one scan tile a row
+    from softbox_b200 import scenes
+    from softbox_b200.engine import DenseNetwork
+    sc, out = scenes.dense_contractile(scenes.dense_scaled(131_080)), []
+    for mode in ("unfused", "graph"):
+        net = DenseNetwork(copy.deepcopy(sc), fp64_coords=True)
+        net.run(0, 5, mode=mode)
+        net.run(5, 1, mode=mode)
+        assert net.status() == 0
+        out.append(D.to_host(net.dev))
+        net.close()
+    assert len(sc["fil"]["end1NbrSlot"]) > 1 << 17 and len(compare_scenes(*out)) > 80
