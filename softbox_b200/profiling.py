@@ -1,7 +1,7 @@
-"""Timing helpers for the fused dense step.
+"""Timing helpers for the dense step.
 
-    python -m softbox_b200.profiling phases [--steps 200] [--warm 3000] [--fp64]   # per-phase times
-    python -m softbox_b200.profiling onestep                 # two one-step fused launches (for ncu -s 1 -c 1)
+    python -m softbox_b200.profiling phases [--steps 200] [--warm 3000] [--fp64]   # the fused kernel's phases
+    python -m softbox_b200.profiling onestep [--mode fused]  # two one-step runs in the default mode (for ncu)
 
 `phases` switches on the plan's %globaltimer stamps (sbx_dense_plan_phase_times): the
 fused kernel writes the device time after every grid barrier of every step, so the
@@ -49,11 +49,11 @@ def phase_times(steps=200, fp64_coords=False, cfg=None, warm=20):
     return out
 
 
-def one_step_launches():
+def one_step_launches(mode="auto"):
     import torch
     net = DenseNetwork(scenes.dense_contractile(scenes.C1))
-    net.run(0, 1, mode="fused")
-    net.run(1, 1, mode="fused")
+    net.run(0, 1, mode=mode)
+    net.run(1, 1, mode=mode)
     torch.cuda.synchronize()
     return net.status()
 
@@ -64,12 +64,13 @@ def main():
     ap.add_argument("--steps", type=int, default=200)
     ap.add_argument("--fp64", action="store_true")
     ap.add_argument("--warm", type=int, default=3000)
+    ap.add_argument("--mode", default="auto")
     a = ap.parse_args()
     if a.what == "phases":
         for k, v in phase_times(a.steps, a.fp64, warm=a.warm).items():
             print(f"{k:48s} {v:9.2f} {'ms' if k.startswith('ms') else 'us'}")
     else:
-        print("status", one_step_launches())
+        print("status", one_step_launches(a.mode))
 
 
 if __name__ == "__main__":

@@ -1,7 +1,6 @@
 """Scale sweep of the dense step: the benchmark network's composition at fixed density.
 
-    python -m softbox_b200.scale [--rods 20000 100000 500000 2000000] [--steps 20] [--modes fused graph]
-                                 [--turnover]
+    python -m softbox_b200.scale [--rods 20000 100000 500000 2000000] [--steps 20] [--modes auto] [--turnover]
 
 For every size: build the network (slab side scaled by sqrt(n / 20,000), crosslinkers by
 the KD-tree builder), then time `steps` consecutive steps per path with CUDA events on the
@@ -13,7 +12,7 @@ and path; FP64 rod centres throughout.
 
 --turnover runs the same networks with actin turnover on (scenes.dense_turnover: growth
 10 subunits/s at barbed ends, severing 0.01/s per rod, constant-actin births into dead
-slots) on the graph path, timing whole 100-step biochem cadences (the turnover block, the
+slots), timing whole 100-step biochem cadences (the turnover block, the
 release of dead attachments, births, and 100 mechanics steps with the grid rebuilt every
 step).
 """
@@ -25,7 +24,7 @@ from . import scenes
 from .roofline import peaks, step_bytes
 
 
-def measure(n_rods, steps=20, modes=("fused", "graph")):
+def measure(n_rods, steps=20, modes=("auto",)):
     import torch
     from .engine import DenseNetwork
     from .runtime import LIB
@@ -62,7 +61,7 @@ def measure(n_rods, steps=20, modes=("fused", "graph")):
     return out
 
 
-def measure_turnover(n_rods, steps=1000, mode="graph"):
+def measure_turnover(n_rods, steps=1000, mode="auto"):
     import torch
     from .engine import TurnoverNetwork
     from .runtime import LIB
@@ -106,7 +105,7 @@ def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--rods", type=int, nargs="+", default=[20000, 100000, 500000, 2000000])
     ap.add_argument("--steps", type=int, default=20)
-    ap.add_argument("--modes", nargs="+", default=["fused", "graph"])
+    ap.add_argument("--modes", nargs="+", default=["auto"])
     ap.add_argument("--turnover", action="store_true")
     a = ap.parse_args()
     if a.turnover:
