@@ -668,11 +668,12 @@ __device__ __forceinline__ RodGeom start_rod(const FusedArgs& a, int j) {
 // Chain forces from the joints made ahead, the crosslinker and motor gathers, the walls and the
 // Langevin update of one rod a thread, in the reference's order; the rod's histograms are reset
 // for the next step. A joint whose neighbour does not point back is computed from this side.
-// MANY: for more rods than are on the chip at once at four blocks an SM, six (80 registers): what
-// only the integration takes goes towards L1 first and is read after the bonds. 78.5 and 74.5 us
-// a step at 100,000 rods, 329 and 325 at 500,000, 221 and 218.6 a packed step of 12 networks; but
-// 25.9 and 26.6 at 1,000, 35.3 and 36.7 at 20,000, where the last read is on the step's path.
-constexpr int RODS_AT_ONCE = 148 * 4 * 128;
+// MANY: for more rods than are on the chip at once at four blocks an SM (75,776 on 148 SMs), six
+// (80 registers): what only the integration takes goes towards L1 first and is read after the
+// bonds. 78.5 and 74.5 us a step at 100,000 rods, 329 and 325 at 500,000, 221 and 218.6 a packed
+// step of 12 networks; but 25.9 and 26.6 at 1,000, 35.3 and 36.7 at 20,000, where the last read
+// is on the step's path.
+constexpr int RODS_AN_SM = 4 * 128;
 template <bool B, bool MANY>
 __global__ void __launch_bounds__(128, MANY ? 6 : 4) k_wide_rods(const __grid_constant__ WideArgs w) {
     const FusedArgs& a = w.a;
@@ -850,6 +851,8 @@ sbx_status wide_step_impl(sbx_ctx* ctx, const WideArgs& w, const WideStreams& ws
     cudaStream_t s = ctx->stream;
     cudaError_t e = cudaSuccess;
     auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
+    int sms = 0;
+    ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     auto fork = [&](cudaEvent_t ev, cudaStream_t to) { ok(cudaEventRecord(ev, s)); ok(cudaStreamWaitEvent(to, ev, 0)); };
     auto join = [&](cudaEvent_t ev, cudaStream_t from) { ok(cudaEventRecord(ev, from)); ok(cudaStreamWaitEvent(s, ev, 0)); };
     // early: the kernel waits for its predecessor itself
@@ -869,10 +872,10 @@ sbx_status wide_step_impl(sbx_ctx* ctx, const WideArgs& w, const WideStreams& ws
     fork(ws.start, ws.ahead);
     if (a.xlOn) ok(cudaStreamWaitEvent(ws.link, ws.start, 0));
     // The three kernels ahead need nothing of each other: they start together while their threads
-    // fit on the chip at once (148 SMs of 2048), else one after another, as their blocks would go
+    // fit on the chip at once (2048 an SM), else one after another, as their blocks would go
     // before the main stream's. Together and in turn: 28.8 and 30.0 us a step at 1,000 rods, 85.0
     // and 86.4 at 100,000; 360 and 356 at 500,000 with all three let through.
-    const bool side = (int64_t)a.nB + a.nBb + a.nSeg <= 148 * 2048;
+    const bool side = (int64_t)a.nB + a.nBb + a.nSeg <= (int64_t)sms * 2048;
     launch(ws.ahead, false, k_wide_draws<B>, (int64_t)a.nB + a.nBb + a.nSeg, 256);
     launch(ws.ahead, side, k_wide_terms, 2 * (int64_t)a.nM + 4 * (int64_t)a.nD, 128);
     launch(ws.ahead, side, k_wide_joints, a.nSeg, 128);
@@ -893,7 +896,7 @@ sbx_status wide_step_impl(sbx_ctx* ctx, const WideArgs& w, const WideStreams& ws
     if (a.xlOn) join(ws.linkDone, ws.link);
     launch(s, false, k_wide_mini<B>, ((int64_t)a.nBb + (a.nBb + MINI_THREADS - 1) / MINI_THREADS) * MINI_THREADS,
            MINI_THREADS);
-    if (a.nSeg > RODS_AT_ONCE) launch(s, true, k_wide_rods<B, true>, a.nSeg, 128);
+    if (a.nSeg > (int64_t)sms * RODS_AN_SM) launch(s, true, k_wide_rods<B, true>, a.nSeg, 128);
     else launch(s, true, k_wide_rods<B, false>, a.nSeg, 128);
     join(ws.csrDone, ws.csr);
     if (e != cudaSuccess) return fail(ctx, SBX_ECUDA, std::string("dense step: streams: ") + cudaGetErrorString(e));
