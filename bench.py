@@ -44,11 +44,12 @@ from softbox_b200.roofline import peaks, step_bytes  # noqa: E402
 
 WARM_STEPS = 3000      # untimed steps before the warm-up: bound heads have built up
 REF_MIN_STEPS = 200    # the reference arm times at least this many steps
-# DRAM bytes (read + write) of the 14 kernels of one step of this workload (FP64 centres, warmed
-# state), the caches flushed before each kernel, from one ncu capture (dram__bytes_read.sum +
-# dram__bytes_write.sum, mean of three steps of `python bench.py --steps 3 --warmup 3 --no-cpu
-# --sweep-points 0` under `ncu --clock-control none -k regex:k_wide -s 42042 -c 42`)
-STEP_DRAM_BYTES = 20_777_000
+# DRAM bytes that the 14 kernels of one step of this workload read (FP64 centres, warmed state), with
+# the flush before the step and none between its kernels: one ncu capture (dram__bytes_read.sum, mean
+# of three steps of `python bench.py --steps 3 --warmup 3 --no-cpu --sweep-points 0` under
+# `ncu --cache-control none --clock-control none -k regex:k_wide -s 42042 -c 42`). What is written
+# meanwhile (17 MB) is mostly the flush's own dirty lines, so no traffic of the step is given.
+STEP_DRAM_READ_BYTES = 8_708_000
 
 
 def workload_config(sc_host, warmup):
@@ -296,7 +297,6 @@ def run_ours(args):
     hbm, how = peaks()
     bytes_step = step_bytes(sc_host, fp64=True)
     achieved = bytes_step / (float(np.mean(step_ms)) / 1e3) / 1e9
-    traffic = STEP_DRAM_BYTES
     launches = net.kernels_per_step
 
     cpu = None
@@ -324,7 +324,8 @@ def run_ours(args):
                 "arm": {"path": f"CUDA graph of wide kernels, {launches} kernels per step",
                         "parallelism": f"replicas x{ws}", "state_at_timing": state},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
-                             "frac": achieved / hbm, "traffic": traffic, "peak_source": how,
+                             "frac": achieved / hbm, "traffic": None, "dram_read_bytes": STEP_DRAM_READ_BYTES,
+                             "peak_source": how,
                              "kernel": "k_wide_* (one step)", "algorithmic_bytes_per_launch": bytes_step},
                 "cpu_baseline": cpu,
                 "e2e": {"value": e2e, "unit": "rod-steps/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,

@@ -751,8 +751,8 @@ sbx_status sbx_dense_plan_create(sbx_ctx* ctx, const sbx_dense_scene* scene, sbx
  * layout, else that sequence); 2: the fused persistent kernel (all nsteps in one cooperative
  * launch; available when the scene has the harness layout, see
  * sbx_dense_plan_fused_available). All three give the same bits. mode 3 (auto): the graph of
- * wide kernels, which leads at every size (us per step, graph / fused: 30 / 57 at 1,000 rods one
- * step a call; 35 / 64 at 2e4 and 54 / 172 at 4e4, 20 steps a call); without it, or on a stream
+ * wide kernels, which leads at every size (us per step, graph / fused: 31 / 63 at 1,000 rods one
+ * step a call; 35 / 64 at 2e4 and 40 / 101 at 4e4, 20 steps a call); without it, or on a stream
  * under capture, the fused kernel up to SBX_DENSE_AUTO_MAX_FUSED_RODS rods when available (mode 0
  * after a refresh in the same capture), the graph path above it. */
 #define SBX_DENSE_AUTO_MAX_FUSED_RODS 40960
@@ -818,7 +818,8 @@ sbx_status sbx_dense_plan_set_noise(sbx_dense_plan* plan, const sbx_dense_noise*
  * the rod CTA's staging capacity, out[4] motor reactions read from global memory past the
  * staged ones, out[5] motor rows longer than the sorted-slot capacity (repeated-minimum
  * walk), out[6] reach lists longer than SBX_MAX_CAND, out[7] reserved; `out` holds
- * SBX_FUSED_STATS values. */
+ * SBX_FUSED_STATS values. The graph's wide kernels add to out[0..2], by their own row slots, and
+ * to out[6]. */
 #define SBX_FUSED_STATS 8
 sbx_status sbx_dense_plan_fused_stats(sbx_dense_plan* plan, int64_t* out, int32_t reset);
 /* Test hook: lowers the fused kernel's capacities (link payload entries a rod CTA stages,
@@ -882,8 +883,8 @@ sbx_status sbx_confine_batched(sbx_ctx* ctx, int32_t n, const float* coord, cons
                                const int32_t* counts, const int32_t* key);
 /* ---------------------------------------------------------------- observables
  * Per network k of a single or packed scene (segBase/linkBase/motBase: nNet+1 device
- * offsets of the network's index ranges). Deterministic FP64 reductions: one block per
- * network, thread t sums items t, t+256, ... in index order, then a fixed tree.
+ * offsets of the network's index ranges). Deterministic FP64 reductions: 256 partial sums a
+ * network, sum t of items t, t+256, ... in index order, then a fixed tree.
  * RMS extent of the ACTIVE filament rods about their mean (FullSystemDemoHarness.filRms,
  * FullSystemDemoHarness.java:1047-1055): out[2k] = R_rms (um), out[2k+1] = rods counted.
  * coord64 (FP64 centres) is used when given; filState may be NULL (all ACTIVE). */
@@ -901,7 +902,7 @@ sbx_status sbx_obs_stress(sbx_ctx* ctx, int32_t nNet, int32_t nSeg, const float*
                           const float* bondData, double headLen, const float* volume, double* out);
 /* Largest cluster: components over ACTIVE segments and backbones joined by chain links,
  * ACTIVE crosslinks and bound heads (segment -- its head's backbone, motorBackbone[m]).
- * One pass joins the edges' components completely; `rounds` is the length of flags less one
+ * The edges' components are joined completely, chain links first; `rounds` is the length of flags less one
  * (rounds + 1 words), and flags[rounds-1] != 0 afterwards means not converged. label
  * receives each node's component id (its smallest node id; -1 for FREE segments), size the
  * component sizes in segments; out[2k] = largest component (segments), out[2k+1] = ACTIVE

@@ -956,8 +956,8 @@ extern "C" sbx_status sbx_dense_plan_run(sbx_dense_plan* p, int32_t t0, int32_t 
         return fail(ctx, SBX_EINVAL, "sbx_dense_plan_run: steps outside the supplied-noise range");
     bool report = false;
     if (mode == 3) {
-        // the wide kernels lead at every size: 30 / 57 us a step at 1,000 rods (one step a call),
-        // 35 / 64 at 20,000 and 54 / 172 at 40,000 (20 steps a call) against the fused kernel
+        // the wide kernels lead at every size: 31 / 63 us a step at 1,000 rods (one step a call),
+        // 35 / 64 at 20,000 and 40 / 101 at 40,000 (20 steps a call) against the fused kernel
         const bool fused = p->fused_ok && p->scene.fil.body.n <= SBX_DENSE_AUTO_MAX_FUSED_RODS;
         // (a graph cannot be launched on a stream under capture: that takes the fused kernel as one
         // node, or the per-system kernels where its topology is not to be had)

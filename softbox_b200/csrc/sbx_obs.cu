@@ -15,14 +15,14 @@
 // per network took 159 us and 103 us.
 //
 // Clusters: nodes are the segments and the backbones; edges are chain links, ACTIVE
-// crosslinks and bound heads (segment -- the head's backbone). One pass over the edges joins
-// their components completely: the larger root is hooked onto the smaller one with a
-// compare-and-swap and the edge tries again from the roots it finds when another edge was
-// first. A root only ever gets a smaller parent, so the final root of a component is its
-// smallest node id and the labelling does not depend on the order in which edges are
-// processed. Rounds of hooking and compressing, launched up to the caller's limit whether or
-// not anything was left to do, took 128 launches and 425 us on the 12 networks; the one pass
-// takes 90 us with its labelling.
+// crosslinks and bound heads (segment -- the head's backbone). Each edge joins its components
+// completely: the larger root is hooked onto the smaller one with a compare-and-swap and the
+// edge tries again from the roots it finds when another edge was first. A root only ever gets
+// a smaller parent, so the final root of a component is its smallest node id and the
+// labelling does not depend on the order in which edges are processed. The chain links go
+// first, then paths are flattened, then the other edges join and every node is labelled.
+// Rounds of hooking and compressing, launched up to the caller's limit whether or not anything
+// was left to do, took 128 launches and 425 us on the 12 networks; the six launches take 44.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

@@ -50,8 +50,8 @@ class DenseNetwork:
     def run(self, t0, nsteps, mode=None):
         """Advance steps t0..t0+nsteps-1. mode: "auto" (default: the graph path; the fused
         kernel for a network of its size on a stream under capture), "fused" (one persistent
-        cooperative launch for all steps), "graph" (one CUDA-graph replay per step) or
-        "unfused" (the per-system call sequence). All give the same bits."""
+        cooperative launch for all steps), "graph" (CUDA-graph replays of one step, or of four
+        up to 2^17 rods) or "unfused" (the per-system call sequence). All give the same bits."""
         if mode is None:
             mode = "auto"
         st = LIB.sbx_dense_plan_run(self.plan, int(t0), int(nsteps), self.MODES[mode])
@@ -141,7 +141,7 @@ class TurnoverNetwork(DenseNetwork):
     mechanics, all on the library's stream. The mechanics run on any path. The fused
     kernel's rod groups depend on the chain topology, which splits and births into FREE slots
     change: sbx_dense_plan_refresh notes that after each cadence, and a "fused" run then
-    re-reads it (one stream synchronisation); the graph path reads it on the device."""
+    reads it again (waiting for the cadence); the graph path reads it on the device."""
 
     def __init__(self, host_scene, ctx=None, fp64_coords=False, device="cuda"):
         from .turnover import Turnover
