@@ -65,7 +65,7 @@ class MLPEnsemble:
         self._alloc(batch)
         self.x_mean = self.x_std = self.y_mean = self.y_std = None
         # the kernels' error word, in mapped host memory: read after a call's results, without a copy
-        self.err = torch.zeros(1, dtype=torch.int32, pin_memory=True)
+        self.err = torch.zeros(1, dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
         self.graph = None
 
     # ---------------------------------------------------------------- buffers
@@ -276,9 +276,10 @@ class MLPEnsemble:
         return self._inf_Z
 
     def predict(self, X, chunk=65536):
-        """Ensemble mean and standard deviation of the de-normalised outputs for X [P, nin].
-        An ensemble that does not run whole uses inference buffers for `chunk` points
-        (allocated on first use of a chunk size, then reused)."""
+        """Ensemble mean and standard deviation of the de-normalised outputs for X [P, nin], and each
+        member's outputs. `chunk` is how many points a pass of the separate kernels takes (buffers
+        for that many are allocated on first use, then reused); an ensemble that runs whole takes
+        all points at once."""
         t = self.torch
         X = np.asarray(X)
         net = self._net(False)

@@ -44,3 +44,11 @@ def test_backward_matches_finite_differences(monkeypatch):
         bm[l][1] -= h
         fd = (loss_of(W, bp) - loss_of(W, bm)) / (2 * h)
         assert abs(fd - db[l][1]) <= 1e-6 * max(1.0, abs(fd))
+
+
+def test_an_ensemble_can_be_made_without_a_gpu():
+    import pytest
+    torch = pytest.importorskip("torch")
+    from softbox_b200.surrogate import MLPEnsemble
+    ens = MLPEnsemble(n_nets=2, dims=(6, 32, 3), batch=16, device="cpu")
+    assert ens.W[0].shape == (2, 32, 16) and ens.err.item() == 0 and not torch.any(ens.mW[0])
